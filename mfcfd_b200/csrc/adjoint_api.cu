@@ -261,7 +261,8 @@ int record(mfcfd_t *h, AdjointState *a, const R4 *from) {
         b.res_part = h->d_res_part;
         b.flux_dbg = reinterpret_cast<double *>(a->tfr[rk - 1]);
         b.kstape = ks_at(a, rk);
-        launch_flux(h->geom, h->consts, h->sched, b, rk, rk == rks, h->flux_grid, h->stream);
+        launch_flux(h->geom, h->consts, h->sched, b, rk, rk == rks, h->flux_grid,
+                    h->inst_h.ntiles, h->stream);
     }
     h->launches += 1 + (long long)rks * (2 + m);
     a->forward_iters += 1;

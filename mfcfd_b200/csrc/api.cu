@@ -68,7 +68,7 @@ void free_all(mfcfd_t *h) {
         for (auto &g : row)
             if (g) cudaGraphExecDestroy(g);
     void *bufs[] = {h->d_xy, h->d_nrm, h->d_eps2, h->d_obc, h->d_conn, h->d_nbhs, h->d_mx,
-                    h->d_my, h->d_hoff, h->d_hrow, h->d_hloc, h->d_prim[0], h->d_prim[1], h->d_q[0], h->d_q[1], h->d_dq[0],
+                    h->d_my, h->d_hoff, h->d_hrow, h->d_hloc, h->d_fco, h->d_wsl, h->d_prim[0], h->d_prim[1], h->d_q[0], h->d_q[1], h->d_dq[0],
                     h->d_dq[1], h->d_dq[2], h->d_qm, h->d_delta, h->d_spd, h->d_res_part, h->d_flux_dbg,
                     h->d_hist, h->d_forces, h->d_ctl, h->d_sh_idx, h->d_sh_shape, h->d_sh_geo,
                     h->d_sh_my, h->f_prim[0], h->f_prim[1], h->f_q[0], h->f_q[1],
@@ -143,7 +143,7 @@ void launch_stage(mfcfd_t *h, cudaStream_t s, int rk, int A, int B, F after) {
         b.spd = h->d_spd;
         b.res_part = h->d_res_part;
         b.flux_dbg = h->keep_diag ? h->d_flux_dbg : nullptr;
-        launch_flux(h->geom, h->consts, h->sched, b, rk, last, h->flux_grid, s);
+        launch_flux(h->geom, h->consts, h->sched, b, rk, last, h->flux_grid, h->inst_h.ntiles, s);
         after();
     } else {
         const float4 *q_in = h->f_q[h->qcur];
@@ -814,6 +814,8 @@ static int create_handle(const mfcfd_grid *grid, const mfcfd_params *params, int
         }
         for (int b = 0; b < 3; ++b) ALLOC(h->d_dq[b], (size_t)8 * n);
         ALLOC(h->d_qm, (size_t)8 * n);
+        ALLOC(h->d_fco, (size_t)8 * n);
+        if (P.power != 0.0) ALLOC(h->d_wsl, (size_t)kp * n);
     } else {
         ALLOC(h->d_prim[0], n);  // FP64 copy of the state for forces/diagnostics
         for (int b = 0; b < 2; ++b) {
@@ -880,6 +882,12 @@ static int create_handle(const mfcfd_grid *grid, const mfcfd_params *params, int
         h->geom.hkp = halo.hkp;
         h->geom.hc = halo.hc;
     }
+    if (!h->fp32) {
+        // on the stream of the uploads above, and before the copies below
+        launch_flux_coef(h->geom, 0, nl, nw, no, P.power, h->d_fco, h->d_wsl, nullptr);
+        h->geom.fco = h->d_fco;
+        h->geom.wsl = h->d_wsl;
+    }
     h->consts.cfl = P.cfl;
     h->consts.power = P.power;
     h->consts.euler = P.euler;
@@ -898,7 +906,7 @@ static int create_handle(const mfcfd_grid *grid, const mfcfd_params *params, int
                              wave_blocks(h->dev, 0, h->point_block, 0, h->fp32));
     h->inner_grid = std::min((nl + h->point_block - 1) / h->point_block,
                              wave_blocks(h->dev, 1, h->point_block, 0, h->fp32));
-    h->flux_grid = std::min(flux_grid_blocks(nl),
+    h->flux_grid = std::min(flux_grid_blocks(nl, h->fp32),
                             wave_blocks(h->dev, 2, 128,
                                         h->fp32 ? flux32_smem_bytes(kp) : flux_smem_bytes(kp),
                                         h->fp32));
@@ -1402,7 +1410,8 @@ extern "C" int mfcfd_part_phase(mfcfd_t *h, int phase, int rk, int t, double *va
         b.spd = h->d_spd;
         b.res_part = h->d_res_part;
         b.flux_dbg = h->keep_diag ? h->d_flux_dbg : nullptr;
-        launch_flux(h->geom, h->consts, h->sched, b, rk, rk == h->p.rks, h->flux_grid, s);
+        launch_flux(h->geom, h->consts, h->sched, b, rk, rk == h->p.rks, h->flux_grid,
+                    h->inst_h.ntiles, s);
         h->qcur ^= 1;
         break;
     }

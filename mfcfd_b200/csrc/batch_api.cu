@@ -63,6 +63,7 @@ struct mfcfd_batch {
     unsigned long long *d_mx = nullptr, *d_my = nullptr;
     int *d_hoff = nullptr, *d_hrow = nullptr;  // tile halos of the D and I passes
     unsigned char *d_hloc = nullptr;
+    double *d_fco = nullptr, *d_wsl = nullptr;  // FP64 flux pass: Geom::fco, wsl
     R4 *d_prim[2] = {nullptr, nullptr}, *d_q[2] = {nullptr, nullptr};
     double *d_dq[3] = {nullptr, nullptr, nullptr};
     double *d_qm = nullptr;
@@ -136,7 +137,7 @@ void drop_graphs(mfcfd_batch_t *b) {
 void free_batch(mfcfd_batch_t *b) {
     drop_graphs(b);
     void *bufs[] = {b->d_xy, b->d_nrm, b->d_eps2, b->d_obc, b->d_conn, b->d_nbhs, b->d_mx,
-                    b->d_my, b->d_hoff, b->d_hrow, b->d_hloc, b->d_prim[0], b->d_prim[1], b->d_q[0], b->d_q[1], b->d_dq[0],
+                    b->d_my, b->d_hoff, b->d_hrow, b->d_hloc, b->d_fco, b->d_wsl, b->d_prim[0], b->d_prim[1], b->d_q[0], b->d_q[1], b->d_dq[0],
                     b->d_dq[1], b->d_dq[2], b->d_qm, b->f_prim[0], b->f_prim[1], b->f_q[0], b->f_q[1],
                     b->f_dq[0], b->f_dq[1], b->f_dq[2], b->f_qm, b->f_eps2, b->f_dxy, b->f_w, b->f_lsq,
                     b->f_flsq, b->d_delta, b->d_spd,
@@ -166,7 +167,7 @@ int batch_wave(const mfcfd_batch_t *b, int kind, int block) {
 // of the flux pass ppt chunks of two tiles (ppt 1: every point its thread).
 void set_shape(mfcfd_batch_t *b, int block, int waves, int ppt = 1) {
     b->point_block = block;
-    const int fmax = flux_grid_blocks(b->ntiles * TILE);
+    const int fmax = flux_grid_blocks(b->ntiles * TILE, b->fp32);
     if (waves > 0) {
         b->point_grid = waves * batch_wave(b, 0, block);
         b->inner_grid = waves * batch_wave(b, 1, block);
@@ -207,7 +208,7 @@ void batch_stage(mfcfd_batch_t *b, cudaStream_t s, int rk, int A, int B) {
         sb.spd = b->d_spd;
         sb.res_part = b->d_res_part;
         sb.flux_dbg = nullptr;
-        launch_flux(b->geom, b->consts, b->sched, sb, rk, last, fg, s);
+        launch_flux(b->geom, b->consts, b->sched, sb, rk, last, fg, b->ntiles, s);
     } else {
         const float4 *q_in = b->f_q[b->qcur];
         launch_grad32(b->geom, b->consts, b->geom32, b->sched, q_in, b->d_spd, b->f_dq[0],
@@ -576,6 +577,8 @@ int mfcfd_batch_create(int n_inst, const mfcfd_grid *const *grids, const mfcfd_p
         }
         for (int k = 0; k < 3; ++k) BALLOC(b->d_dq[k], (size_t)8 * N);
         BALLOC(b->d_qm, (size_t)8 * N);
+        BALLOC(b->d_fco, (size_t)8 * N);
+        if (P0.power != 0.0) BALLOC(b->d_wsl, (size_t)kp * N);
     } else {
         BALLOC(b->d_prim[0], N);  // FP64 copy of the state for the force sums
         for (int k = 0; k < 2; ++k) {
@@ -641,6 +644,14 @@ int mfcfd_batch_create(int n_inst, const mfcfd_grid *const *grids, const mfcfd_p
         b->geom.hloc = b->d_hloc;
         b->geom.hkp = halo.hkp;
         b->geom.hc = halo.hc;
+    }
+    if (!b->fp32) {
+        // on the stream of the uploads above, and before the copies below
+        for (const InstInfo &in : info)
+            launch_flux_coef(b->geom, in.base, in.n, in.nw, in.no, P0.power, b->d_fco, b->d_wsl,
+                             nullptr);
+        b->geom.fco = b->d_fco;
+        b->geom.wsl = b->d_wsl;
     }
     b->consts.cfl = P0.cfl;
     b->consts.power = P0.power;
@@ -812,7 +823,7 @@ int mfcfd_batch_set_launch(mfcfd_batch_t *b, int point_block, int point_grid, in
     if (point_grid > 0)
         b->point_grid = b->inner_grid =
             std::min(point_grid, (b->ntot + point_block - 1) / point_block);
-    if (flux_grid > 0) b->flux_grid = std::min(flux_grid, flux_grid_blocks(b->ntiles * TILE));
+    if (flux_grid > 0) b->flux_grid = std::min(flux_grid, flux_grid_blocks(b->ntiles * TILE, b->fp32));
     drop_graphs(b);
     return MFCFD_OK;
 }

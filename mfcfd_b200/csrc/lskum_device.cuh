@@ -56,6 +56,11 @@ struct Geom {
     const int *hrow = nullptr;
     const unsigned char *hloc = nullptr;
     int hkp = 0, hc = 0;
+    // FP64 flux pass, fixed per grid: per point and split list the two
+    // coefficients of the list's least-squares solve ([n][8], launch_flux_coef),
+    // and with power != 0 the weight of every slot ([kp][n]; else nullptr: 1).
+    const double *fco = nullptr;
+    const double *wsl = nullptr;
 };
 // rows a tile halo stages at most (its local row indices are bytes)
 constexpr int HALO_CAP = 64;

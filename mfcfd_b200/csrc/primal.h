@@ -113,9 +113,14 @@ void launch_grad(const Geom &g, const Consts &c, const Sched &s, const R4 *q, co
 // the FP64 dq buffers rotate as dq_src / dq_dst say).
 void launch_inner(const Geom &g, const Consts &c, const Sched &s, const double *dq0,
                   const double *dq_in, double *dq_out, int block, int grid, cudaStream_t st);
-// F pass: flux residual + state update of stage rk (1-based).
+// F pass: flux residual + state update of stage rk (1-based); `tiles` (at
+// least those scheduled) picks the split of the work.
 void launch_flux(const Geom &g, const Consts &c, const Sched &s, const StageBufs &b, int rk,
-                 bool last, int grid, cudaStream_t st);
+                 bool last, int grid, int tiles, cudaStream_t st);
+// Fixed per grid: the list-solve coefficients of points [base, base + n) (wall,
+// outer, interior counts nw, no, rest) and, with wsl, their slots' weights.
+void launch_flux_coef(const Geom &g, int base, int n, int nw, int no, double power, double *fco,
+                      double *wsl, cudaStream_t st);
 // Residual norm and residue of one iteration per instance (hist row i, entry
 // it - it_first), retirement, and the schedule of the next iteration.
 void launch_residual(const InstInfo *inst, int n_inst, const double *res_part, Ctl *ctl,
@@ -125,8 +130,8 @@ void launch_residual(const InstInfo *inst, int n_inst, const double *res_part, C
 cudaError_t init_kernels();
 // tiles (TILE-point schedule units) of n points
 int flux_blocks(int n);
-// flux-pass blocks beyond which some warps would find no chunk of two tiles
-int flux_grid_blocks(int n);
+// flux-pass blocks beyond which some would find no work
+int flux_grid_blocks(int n, bool fp32);
 // resident blocks per SM (kind: 0 D pass, 1 I pass, 2 F pass; fp32 selects
 // the FP32-mixed kernels)
 int batch_occupancy(int kind, bool fp32, int block, size_t smem);

@@ -22,6 +22,7 @@
 #include <algorithm>
 
 #include "batch.cuh"
+#include "flux_math.cuh"
 #include "halo.cuh"
 #include "primal.h"
 
@@ -32,10 +33,9 @@ namespace {
 constexpr int GRAD_BLOCK = 256;  // blocks of the per-point set-up kernels
 constexpr int LPP = 8;                   // lanes per point in the flux pass
 constexpr int FLUX_BLOCK = 128;          // four independent warps
-constexpr int REC = 19;                  // dGxp[4] dGxn[4] dGyp[4] dGyn[4] dels deln w
-#ifndef FLUX_MIN_BLOCKS
-#define FLUX_MIN_BLOCKS 4                // <= 128 registers; shared memory allows 4 blocks
-#endif
+// 4 blocks: 128 registers a thread and all of shared memory but 3.5 KB; at 3
+// (168 registers) 0.420 ms at 1.024M points against 0.389
+constexpr int FLUX_MIN_BLOCKS = 4;
 constexpr double OBT = 1.0 / 3.0;        // state_update.F90:19-20
 constexpr double TBT = 2.0 / 3.0;
 
@@ -330,240 +330,357 @@ kb_grad_h(Geom g, Consts c, Sched s, const R4 *__restrict__ q, const double *__r
 // flux_residual.F90:14-73 cal_flux_residual + state_update.F90:10-141 +
 // q_variables.F90:8-37 on the new state.
 //
-// Work split: a warp owns CHUNK = 32 consecutive points (two tiles) end to
-// end, with no block barrier.  It computes their list derivatives in rounds
-// of PPW = 4 points, eight lanes per point (flux_group), leaving each point's
-// sixteen list derivatives in the warp's shared memory, then updates the 32
-// points with one lane each (update_point) and writes the two tiles'
-// residual partials.
+// Work split: eight lanes a point, one stencil slot a lane, four points a
+// warp round.  A lane reconstructs both states of its slot once (limiter +
+// qtilde -> kinetic state; the reference repeats this per direction list with
+// identical inputs), evaluates the split fluxes of the lists the neighbour
+// belongs to, and adds their differences times the slot's weight in the
+// list's least-squares solve.
 //
-// In flux_group lane l of a point takes stencil slots l, l+8, l+16.  For its
-// neighbour k it reconstructs both states once (limiter + qtilde -> kinetic
-// state, reconstruct_kstate; the reference repeats this per direction list
-// with identical inputs, so sharing it is exact), evaluates the split fluxes
-// of every list the neighbour belongs to, and stores G_k - G_i with the
-// geometry in a record.  Lane pair (2L, 2L+1) then sums list L in slot order
-// -- the reference's loop order -- for components (0,1) and (2,3).  Slots
-// are taken eight at a time: the records of one round of slots are summed
-// before the next round overwrites them, the running sums waiting in shared
-// memory between rounds, so shared memory does not grow with the stencil.
+// The solve is folded into a weight per slot: list L's derivative is
+// (fx sdy2 - fy sdxy) / det with fx = sum dG dels w, fy = sum dG deln w, that
+// is sum dG c with c = (a dels + b deln) w, a = sdy2 / det, b = -sdxy / det (y
+// lists: the roles of dels and deln swapped).  a and b are geometry, formed
+// once per grid (k_flux_coef).  The flux residual is the sum of the list
+// derivatives, so the lists need not be told apart: a lane adds both
+// directions' terms into four sums and eight lanes add theirs by shuffles.
 constexpr int PPW = 32 / LPP;          // points per warp round
-constexpr int CHUNK = 2 * TILE;        // points a warp owns (two tiles)
-constexpr int GST = 17;                // stride of a point's list derivatives (odd: no bank conflicts)
 constexpr int FLUX_WARPS = FLUX_BLOCK / 32;
-// doubles per warp: per point of a round its records and its lanes' parked
-// sums, then the chunk's list derivatives and residual terms
-// (one double of padding puts the four point groups' records on different
-// banks: at 208 doubles, a multiple of 128 bytes, the list-sum reads of the
-// four groups met in the same banks; C2 0.587 -> 0.575 ms)
-constexpr int GROUP_SMEM = LPP * REC + 7 * LPP + 1;
-constexpr int WARP_SMEM = PPW * GROUP_SMEM + CHUNK * GST + CHUNK;
+constexpr int CHUNK_MAX = 2 * TILE;    // points of a chunk
 
+// Per point and split list L: a, b of the list's solve (fco[8 i + 2 L]).
+// *_fluxes.F90 dG*: the sums in slot order; a list the point's kind does not
+// have (wall ypos, outer yneg) and empty rows get zeros.
+__global__ void k_flux_coef(Geom g, int base, int n, int nw, int no, double power,
+                            double *__restrict__ fco, double *__restrict__ wsl) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= n) return;
+    const int i = base + j;
+    const int kind = j < nw ? KIND_WALL : (j < nw + no ? KIND_OUTER : KIND_INTERIOR);
+    const double2 p = g.xy[i], nn = g.nrm[i];
+    const unsigned long long bits[2] = {g.mx[i], g.my[i]};
+    double sxx[4] = {}, syy[4] = {}, sxy[4] = {};
+    for (int r = 0; r < g.nbhs[i]; ++r) {
+        const double2 pk = g.xy[g.conn[(size_t)r * g.n + i]];
+        const double delx = pk.x - p.x, dely = pk.y - p.y;
+        const double dels = delx * nn.y - dely * nn.x, deln = delx * nn.x + dely * nn.y;
+        double w = 1.0;
+        if (wsl) {
+            w = pow(sqrt(delx * delx + dely * dely), power);
+            wsl[(size_t)r * g.n + i] = w;
+        }
+        const double dw = dels * w, nw_ = deln * w;
+#pragma unroll
+        for (int L = 0; L < 4; ++L) {
+            if (!((bits[L >> 1] >> (r + ((L & 1) ? 32 : 0))) & 1ull)) continue;
+            sxx[L] = sxx[L] + dels * dw;
+            syy[L] = syy[L] + deln * nw_;
+            sxy[L] = sxy[L] + dels * nw_;
+        }
+    }
+#pragma unroll
+    for (int L = 0; L < 4; ++L) {
+        const bool none = (kind == KIND_WALL && L == 2) || (kind == KIND_OUTER && L == 3);
+        const double ob = 1.0 / (sxx[L] * syy[L] - sxy[L] * sxy[L]);
+        fco[8 * (size_t)i + 2 * L] = none ? 0.0 : (L < 2 ? syy[L] : sxx[L]) * ob;
+        fco[8 * (size_t)i + 2 * L + 1] = none ? 0.0 : -sxy[L] * ob;
+    }
+}
+
+// Sum of v over the eight lanes of a point: component 2 (bit 2) + (bit 1) of
+// the lane, in a fixed order.
+__device__ __forceinline__ double reduce8(const double v[4], int lane) {
+    const unsigned full = 0xffffffffu;
+    const bool h4 = lane & 4, h2 = lane & 2;
+    const double s0 = __shfl_xor_sync(full, h4 ? v[0] : v[2], 4);
+    const double s1 = __shfl_xor_sync(full, h4 ? v[1] : v[3], 4);
+    const double a0 = (h4 ? v[2] : v[0]) + s0, a1 = (h4 ? v[3] : v[1]) + s1;
+    const double b = (h2 ? a1 : a0) + __shfl_xor_sync(full, h2 ? a0 : a1, 2);
+    return b + __shfl_xor_sync(full, b, 1);
+}
+
+// Shared memory of the unit that computes a tile (a warp, or in the shared
+// split the block): the tile's halo rows (halo.cuh) as one array per 16-byte
+// piece -- q 0-1, dq 2-5, qm 6-9, (x, y) 10 -- at a fixed stride, so that a
+// row's pieces are immediate offsets from its first, and an 8-byte array of
+// eps2; per point of the tile (nx, ny), the membership masks, the list
+// coefficients, local rows and stencil size; the chunk's flux residuals.
+// ROWS is what four blocks an SM leave room for (an O-grid's tiles have 54
+// rows, a point cloud's in RCM order 54 to 60); a larger tile reads its rows
+// from global memory.
+struct FluxSmem {
+    static constexpr int ROWS = 60, HC = ROWS + 1;
+    double2 halo[11][HC];
+    double eps[HC + 1];
+    double2 nrm[TILE];
+    uint4 mask[TILE];              // xpos, xneg, ypos, yneg
+    double2 co[TILE][4];
+    unsigned char loc[TILE * 16];  // hloc rows (of up to 16 bytes)
+    int nbhs[TILE];
+    double G[CHUNK_MAX][4];        // flux residuals, then residual terms
+};
+constexpr int FLUX_SMEM = FLUX_WARPS * sizeof(FluxSmem);
+
+// A scheduled tile: its first point, the points in it (0: no such tile), and
+// the numbers of its points up to which they are wall and outer points.
+struct FluxTile {
+    int i0 = 0, cnt = 0, wall = 0, outer = 0, tile = 0;
+    __device__ __forceinline__ FluxTile() {}
+    __device__ __forceinline__ FluxTile(const Sched &s, int ntiles, int v) {
+        if (v >= ntiles) return;
+        const TileRef t = sched_tile_global(s, v);
+        i0 = t.base + t.j0;
+        cnt = min(TILE, t.n - t.j0);
+        wall = t.nw - t.j0;
+        outer = t.nw + t.no - t.j0;
+        tile = t.tile;
+    }
+    __device__ __forceinline__ int kind(int j) const {
+        return j < wall ? KIND_WALL : (j < outer ? KIND_OUTER : KIND_INTERIOR);
+    }
+};
+
+// The row indices of a tile's halo: lane l holds rows l and l + 32.
+struct FluxHalo {
+    int h0 = 0, hn = 0, k0 = 0, k1 = 0;  // hn 0: no tile, or not staged
+    __device__ __forceinline__ void range(const Geom &g, const FluxTile &t) {
+        h0 = hn = 0;
+        if (t.cnt == 0) return;
+        h0 = __ldg(g.hoff + t.tile);
+        hn = __ldg(g.hoff + t.tile + 1);
+    }
+    __device__ __forceinline__ void rows(const Geom &g, int lane) {
+        hn = hn - h0 <= FluxSmem::ROWS ? hn - h0 : 0;
+        k0 = lane < hn ? __ldg(g.hrow + h0 + lane) : 0;
+        k1 = lane + 32 < hn ? __ldg(g.hrow + h0 + 32 + lane) : 0;
+    }
+    // row u (u / 32 the same for the whole warp)
+    __device__ __forceinline__ int row(int u) const {
+        return __shfl_sync(0xffffffffu, u < 32 ? k0 : k1, u & 31);
+    }
+};
+
+// Copies NP 16-byte pieces of every halo row of an array with the NT threads
+// of the unit, tid of them this one; whole warps.
+template <int NP, int NT>
+__device__ __forceinline__ void stage_rows(const void *src, const FluxHalo &x, double2 *dst,
+                                           int tid) {
+#pragma unroll
+    for (int t = 0; t < HALO_CAP * NP / NT; ++t) {
+        if (NT * t >= NP * x.hn) break;
+        const int u = (NT / NP) * t + tid / NP, part = tid % NP;
+        const int k = x.row(u);
+        if (u < x.hn)
+            halo_cp16(dst + part * FluxSmem::HC + u,
+                      static_cast<const char *>(src) + (size_t)(unsigned)(k * NP + part) * 16);
+    }
+}
+
+// Copies a tile's rows (cp.async).
+template <int NT>
+__device__ __forceinline__ void stage_flux(const Geom &g, const StageBufs &b, const FluxTile &t,
+                                           const FluxHalo &x, FluxSmem &m, int tid) {
+    stage_rows<2, NT>(b.q_in, x, m.halo[0], tid);
+    stage_rows<4, NT>(b.dq, x, m.halo[2], tid);
+    stage_rows<4, NT>(b.qm, x, m.halo[6], tid);
+    if (tid < HALO_CAP) {
+#pragma unroll
+        for (int u0 = 0; u0 < HALO_CAP; u0 += NT < HALO_CAP ? NT : HALO_CAP) {
+            const int u = u0 + tid;
+            const int k = x.row(u);
+            if (u < x.hn) {
+                halo_cp16(&m.halo[10][u], g.xy + k);
+                halo_cp8(&m.eps[u], g.eps2 + k);
+            }
+        }
+    }
+    const double2 *co = reinterpret_cast<const double2 *>(g.fco + 8 * (size_t)t.i0);
+#pragma unroll
+    for (int q = 0; q < (NT < 64 ? 64 / NT : 1); ++q) {
+        const int pc = q * NT + tid;
+        if (pc < 4 * t.cnt) halo_cp16(&m.co[pc >> 2][pc & 3], co + pc);
+    }
+    if (g.hkp <= 16 && tid < g.hkp / 8 * t.cnt)
+        halo_cp8(m.loc + 8 * tid, g.hloc + (size_t)t.i0 * g.hkp + 8 * tid);
+    if (tid < 2 * TILE) {
+        const int j = tid % TILE;
+        if (j < t.cnt) {
+            double *d = reinterpret_cast<double *>(&m.mask[j]);
+            if (tid < TILE) {
+                halo_cp16(&m.nrm[j], g.nrm + t.i0 + j);
+                halo_cp8(d, g.mx + t.i0 + j);
+            } else {
+                halo_cp4(&m.nbhs[j], g.nbhs + t.i0 + j);
+                halo_cp8(d + 1, g.my + t.i0 + j);
+            }
+        }
+    }
+}
+
+// A row in registers: staged (row l of the halo) or from global memory.
+struct FluxRow {
+    double q[4], dx[4], dy[4], qmax[4], qmin[4], eps2;
+    double2 xy;
+    __device__ __forceinline__ void staged(const FluxSmem &m, int l) {
+        double *f[5] = {q, dx, dy, qmax, qmin};
+#pragma unroll
+        for (int a = 0; a < 5; ++a)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const double2 v = m.halo[2 * a + h][l];
+                f[a][2 * h] = v.x;
+                f[a][2 * h + 1] = v.y;
+            }
+        xy = m.halo[10][l];
+        eps2 = m.eps[l];
+    }
+    __device__ __forceinline__ void global(const Geom &g, const StageBufs &b, int k) {
+        const R4 v = ld4w(b.q_in + k);
+        q[0] = v.a; q[1] = v.b; q[2] = v.c; q[3] = v.d;
+        ld8w(b.dq + 8 * (size_t)k, dx, dy);
+        ld8w(b.qm + 8 * (size_t)k, qmax, qmin);
+        xy = g.xy[k];
+        eps2 = g.eps2[k];
+    }
+    __device__ __forceinline__ void qtilde(double delx, double dely, double qt[4]) const {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            qt[c] = limited_qtilde(delx * dx[c] + dely * dy[c], q[c], qmax[c], qmin[c], eps2);
+    }
+};
+
+// One point group of a warp round: the flux residual of point j of tile t
+// (its list-derivative sum) into Gout.  hn: the tile's staged rows (0: none).
 // TAPE: also write both reconstructed kinetic states of every slot to
 // b.kstape (the adjoint's taped re-run; the primal runs TAPE = false).
 template <bool TAPE>
-__device__ __forceinline__ void
-flux_group(const Geom &g, const Consts &c, const StageBufs &b, int i, bool valid, int kind0,
-           double *rec, double *Gout) {
+__device__ __forceinline__ void flux_group(const Geom &g, const StageBufs &b, const FluxTile &t,
+                                           int j, int hn, FluxSmem &m, double *Gout) {
     const int lane = threadIdx.x % LPP;
-    const double inv_gm1 = 1.0 / c.gm1, inv_sqrt_pi = 1.0 / sqrt(c.pi);
-
-    int nb = 0, kind = KIND_INTERIOR;
-    unsigned long long mx = 0, my = 0;
-    double nx = 0.0, ny = 1.0;
-    if (valid) {
-        nb = g.nbhs[i];
-        kind = kind0;
-        mx = g.mx[i];
-        my = g.my[i];
-        const double2 nn = g.nrm[i];
-        nx = nn.x;
-        ny = nn.y;
-    }
-    // x-list flux signs: interior Gxp/Gxn; wall GxII/GxI (A2neg); outer
-    // GxIII/GxIV (A2pos).  y lists: Gyp (+1) / Gyn (-1).
-    const double s2q = kind == KIND_WALL ? -1.0 : 1.0;
-    const int nbw = __reduce_max_sync(0xffffffffu, nb);  // slot rounds of the warp
-    // list-sum role of this lane: list L, components c0, c0+1
-    const int L = lane >> 1, c0 = (lane & 1) * 2;
-    const bool used =
-        valid && !((kind == KIND_WALL && L == 2) || (kind == KIND_OUTER && L == 3));
-    double sdx2 = 0.0, sdy2 = 0.0, sdxy = 0.0;
-    double fx0 = 0.0, fx1 = 0.0, fy0 = 0.0, fy1 = 0.0;
-    double *park = rec + LPP * REC + 7 * lane;  // running sums across slot rounds
-    for (int r0 = 0; r0 < nbw; r0 += LPP) {
-        if (r0 > 0) {
-            // stencils of more than eight slots: the sums wait in shared
-            // memory while the next round's records are computed
-            park[0] = sdx2; park[1] = sdy2; park[2] = sdxy;
-            park[3] = fx0; park[4] = fx1; park[5] = fy0; park[6] = fy1;
+    const double inv_sqrt_pi = 0.56418958354775628695;
+    const int kind = t.kind(j), i = t.i0 + j;
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    const double2 nn = m.nrm[j];
+    const double nx = nn.x, ny = nn.y;
+    const int nb = j < t.cnt ? m.nbhs[j] : 0;
+    for (int r = lane; r < nb; r += LPP) {
+        KState sk, si;
+        double ui[2], uk[2], delx, dely;
+        {
+            double qk[4], qi[4];
+            if (hn > 0) {
+                const unsigned char *gl = g.hloc + (size_t)i * g.hkp, *ml = m.loc + j * g.hkp;
+                const bool in = g.hkp <= 16;
+                const int lk = in ? ml[r] : __ldg(gl + r);
+                const int li = in ? ml[g.hkp - 1] : __ldg(gl + g.hkp - 1);
+                const double2 pi_ = m.halo[10][li], pk = m.halo[10][lk];
+                delx = pk.x - pi_.x;
+                dely = pk.y - pi_.y;
+                FluxRow o;
+                o.staged(m, lk);
+                o.qtilde(delx, dely, qk);
+                o.staged(m, li);
+                o.qtilde(delx, dely, qi);
+            } else {
+                const int k = g.conn[(size_t)r * g.n + i];
+                const double2 pi_ = g.xy[i], pk = g.xy[k];
+                delx = pk.x - pi_.x;
+                dely = pk.y - pi_.y;
+                FluxRow o;
+                o.global(g, b, k);
+                o.qtilde(delx, dely, qk);
+                o.global(g, b, i);
+                o.qtilde(delx, dely, qi);
+            }
+            kstate_pair(qi, qk, nx, ny, inv_sqrt_pi, si, sk, ui, uk);
         }
-        const int r = r0 + lane;
-        if (r < nb) {
-            const int k = g.conn[r * g.n + i];
-            const double2 pi_ = g.xy[i];
-            const double2 pk = g.xy[k];
-            const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
-            // neighbour state first (its gathers are the long-latency loads),
-            // then the point's own state, re-read per slot from L1 so nothing
-            // but the neighbour's kinetic state stays live across the two
-            KState sk, si;
-            double uk[2], ui[2];
-            {
-                const R4 kv = ld4(b.q_in + k);
-                const double qk[4] = {kv.a, kv.b, kv.c, kv.d};
-                double dxk[4], dyk[4], qmaxk[4], qmink[4];
-                ld8w(b.dq + 8 * (size_t)k, dxk, dyk);
-                ld8w(b.qm + 8 * (size_t)k, qmaxk, qmink);
-                sk = reconstruct_kstate(qk, dxk, dyk, qmaxk, qmink, g.eps2[k], delx, dely,
-                                        inv_gm1, nx, ny, inv_sqrt_pi, TAPE ? uk : nullptr);
-            }
-            {
-                const R4 qv = ld4(b.q_in + i);
-                const double qi[4] = {qv.a, qv.b, qv.c, qv.d};
-                double dxi[4], dyi[4], qmaxi[4], qmini[4];
-                ld8w(b.dq + 8 * (size_t)i, dxi, dyi);
-                ld8w(b.qm + 8 * (size_t)i, qmaxi, qmini);
-                si = reconstruct_kstate(qi, dxi, dyi, qmaxi, qmini, g.eps2[i], delx, dely,
-                                        inv_gm1, nx, ny, inv_sqrt_pi, TAPE ? ui : nullptr);
-            }
-            if (TAPE) {
-                // per state rho, p/rho, B1, B2, e1, e2, u1, u2 (ut, un and
-                // |u|^2 follow from u and the point's normal)
-                const double v[KS_TAPE] = {si.rho, si.pbr, si.B1, si.B2, si.e1, si.e2, ui[0],
-                                           ui[1],  sk.rho, sk.pbr, sk.B1, sk.B2, sk.e1, sk.e2,
-                                           uk[0],  uk[1]};
-                double2 *tp = reinterpret_cast<double2 *>(
-                    b.kstape + ((size_t)i * g.kp + r) * KS_TAPE);
+        if (TAPE) {
+            // per state rho, p/rho, B1, B2, e1, e2, u1, u2 (ut, un and |u|^2
+            // follow from u and the point's normal)
+            const double t[KS_TAPE] = {si.rho, si.pbr, si.B1, si.B2, si.e1, si.e2, ui[0], ui[1],
+                                       sk.rho, sk.pbr, sk.B1, sk.B2, sk.e1, sk.e2, uk[0], uk[1]};
+            double2 *tp =
+                reinterpret_cast<double2 *>(b.kstape + ((size_t)i * g.kp + r) * KS_TAPE);
 #pragma unroll
-                for (int h = 0; h < KS_TAPE / 2; ++h) tp[h] = make_double2(v[2 * h], v[2 * h + 1]);
-            }
-            const double tx = ny, ty = -nx;
-            const double dels = delx * tx + dely * ty;
-            const double deln = delx * nx + dely * ny;
-            double w = 1.0;
-            if (!c.power_zero) w = pow(sqrt(dels * dels + deln * deln), c.power);
-            double *e = rec + lane * REC;
-            // Per direction the neighbour is in one list of the pair (in both
-            // only when its projection is exactly 0): one evaluation with the
-            // list's sign taken per lane keeps the warp converged where
-            // neighbours fall in different lists of the pair.
+            for (int h = 0; h < KS_TAPE / 2; ++h) tp[h] = make_double2(t[2 * h], t[2 * h + 1]);
+        }
+        double dels = delx * ny - dely * nx, deln = delx * nx + dely * ny;
+        if (g.wsl) {
+            const double w = g.wsl[(size_t)r * g.n + i];
+            dels *= w;
+            deln *= w;
+        }
+        // Per direction the neighbour is in one list of the pair, in both only
+        // when its projection is exactly 0: the second list is added then.
+        const uint4 mm = m.mask[j];
+        const double w6i = fma(6.0, si.pbr, si.usq), w6k = fma(6.0, sk.pbr, sk.usq);
+        auto add_x = [&](int l, double sg) {
+            const double2 co = m.co[j][l];
+            const double w = fma(co.x, dels, co.y * deln);
             double Gi[4], Gk[4];
-#pragma unroll
-            for (int d = 0; d < 2; ++d) {
-                const unsigned long long bits = d == 0 ? mx : my;
-                const bool in0 = (bits >> r) & 1ull, in1 = (bits >> (r + 32)) & 1ull;
-#pragma unroll
-                for (int pass = 0; pass < 2; ++pass) {
-                    // pass 0: the first list holding the neighbour; pass 1:
-                    // the second list of a neighbour in both
-                    if (pass == 0 ? !(in0 || in1) : !(in0 && in1)) continue;
-                    const int Lx = 2 * d + ((pass == 1 || !in0) ? 1 : 0);
-                    const double sg = (Lx & 1) ? -1.0 : 1.0;
-                    if (d == 0) {
-                        if (kind == KIND_INTERIOR) {
-                            flux_gx(si, sg, Gi);
-                            flux_gx(sk, sg, Gk);
-                        } else {
-                            flux_quad(si, sg, s2q, Gi);
-                            flux_quad(sk, sg, s2q, Gk);
-                        }
-                    } else {
-                        flux_gy(si, sg, Gi);
-                        flux_gy(sk, sg, Gk);
-                    }
-#pragma unroll
-                    for (int m = 0; m < 4; ++m) e[4 * Lx + m] = Gk[m] - Gi[m];
-                }
+            if (kind == KIND_INTERIOR) {
+                flux_split(si, si.ut, si.un, si.B1, si.e1, sg, 0.5 * sg, w6i, Gi);
+                flux_split(sk, sk.ut, sk.un, sk.B1, sk.e1, sg, 0.5 * sg, w6k, Gk);
+            } else {
+                // wall GxII/GxI (A2neg), outer GxIII/GxIV (A2pos)
+                const double s2 = kind == KIND_WALL ? -1.0 : 1.0;
+                flux_quad(si, sg, s2, Gi);
+                flux_quad(sk, sg, s2, Gk);
             }
-            e[16] = dels;
-            e[17] = deln;
-            e[18] = w;
-        }
-        __syncwarp();
-        if (r0 > 0) {
-            sdx2 = park[0]; sdy2 = park[1]; sdxy = park[2];
-            fx0 = park[3]; fx1 = park[4]; fy0 = park[5]; fy1 = park[6];
-        }
-        // list sums of this round's slots, in slot order
-        if (used) {
-            // the list's slots of this round in slot order (lowest bit first):
-            // a lane loops over its own members only
-            const unsigned long long lbits = ((L < 2) ? mx : my) >> ((L & 1) ? 32 : 0);
-            // (a point with fewer slots than r0 has none in this round)
-            const int cnt = min(nb, r0 + LPP) - r0;
-            unsigned rb = cnt > 0 ? (unsigned)(lbits >> r0) & ((1u << cnt) - 1u) : 0u;
-            while (rb) {
-                const int rr = r0 + __ffs(rb) - 1;
-                rb &= rb - 1u;
-                const double *e = rec + (rr - r0) * REC;
-                double dels = e[16], deln = e[17], w = e[18];
-                double dels_w = dels * w, deln_w = deln * w;
-                sdx2 = sdx2 + dels * dels_w;
-                sdy2 = sdy2 + deln * deln_w;
-                sdxy = sdxy + dels * deln_w;
-                double d0 = e[4 * L + c0], d1 = e[4 * L + c0 + 1];
-                fx0 = fx0 + d0 * dels_w;
-                fy0 = fy0 + d0 * deln_w;
-                fx1 = fx1 + d1 * dels_w;
-                fy1 = fy1 + d1 * deln_w;
-            }
-        }
-        __syncwarp();  // the next round overwrites the records
-    }
-    double Gv0 = 0.0, Gv1 = 0.0;
-    if (used) {
-        double det = sdx2 * sdy2 - sdxy * sdxy;
-        double one_by_det = 1.0 / det;
-        if (L < 2) {
-            Gv0 = (fx0 * sdy2 - fy0 * sdxy) * one_by_det;
-            Gv1 = (fx1 * sdy2 - fy1 * sdxy) * one_by_det;
-        } else {
-            Gv0 = (fy0 * sdx2 - fx0 * sdxy) * one_by_det;
-            Gv1 = (fy1 * sdx2 - fx1 * sdxy) * one_by_det;
+#pragma unroll
+            for (int d = 0; d < 4; ++d) v[d] = fma(w, Gk[d] - Gi[d], v[d]);
+        };
+        auto add_y = [&](int l, double sg) {
+            const double2 co = m.co[j][2 + l];
+            const double w = fma(co.x, deln, co.y * dels);
+            double Gi[4], Gk[4];
+            flux_split(si, si.un, si.ut, si.B2, si.e2, sg, 0.5 * sg, w6i, Gi);
+            flux_split(sk, sk.un, sk.ut, sk.B2, sk.e2, sg, 0.5 * sg, w6k, Gk);
+            v[0] = fma(w, Gk[0] - Gi[0], v[0]);
+            v[1] = fma(w, Gk[2] - Gi[2], v[1]);
+            v[2] = fma(w, Gk[1] - Gi[1], v[2]);
+            v[3] = fma(w, Gk[3] - Gi[3], v[3]);
+        };
+        const unsigned bit = 1u << r;
+        const bool x0 = mm.x & bit, y0 = mm.z & bit;
+        add_x(x0 ? 0 : 1, x0 ? 1.0 : -1.0);
+        add_y(y0 ? 0 : 1, y0 ? 1.0 : -1.0);
+        if (((mm.x & mm.y) | (mm.z & mm.w)) & bit) {
+            if (mm.x & mm.y & bit) add_x(1, -1.0);
+            if (mm.z & mm.w & bit) add_y(1, -1.0);
         }
     }
-    // lane 2L+h holds G[L][2h], G[L][2h+1]
-    Gout[2 * lane] = Gv0;
-    Gout[2 * lane + 1] = Gv1;
+    __syncwarp();
+    const double sum = reduce8(v, lane);
+    if (!(lane & 1)) Gout[lane >> 1] = sum;
 }
 
-// state_update.F90:10-141 of one point from its four list derivatives
-// Gs[4L+m]; returns its res_sqr term.
+// state_update.F90:10-141 of one point from the sum of its list derivatives;
+// returns its res_sqr term.
 __device__ __forceinline__ double
 update_point(const Geom &g, const Consts &c, const StageBufs &b, int rk, int last, int i,
              int kind, int orow, const double *Gs) {
-    double G[4][4];
-#pragma unroll
-    for (int L = 0; L < 4; ++L)
-#pragma unroll
-        for (int m = 0; m < 4; ++m) G[L][m] = Gs[4 * L + m];
     const double2 nn = g.nrm[i];
     const double nx = nn.x, ny = nn.y;
     double res_sqr = 0.0;
     {
-        const double delta = b.delta[i];
+                const double delta = b.delta[i];
+        const R4 P = ld4(b.prim_in + i), O = rk == 3 ? ld4(b.prim_old + i) : R4{0, 0, 0, 0};
         double fr[4];
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            if (kind == KIND_WALL) fr[m] = 2.0 * delta * (G[0][m] + G[1][m] + G[3][m]);
-            else if (kind == KIND_OUTER) fr[m] = delta * (G[0][m] + G[1][m] + G[2][m]);
-            else fr[m] = delta * (G[0][m] + G[1][m] + G[2][m] + G[3][m]);
-        }
+        for (int m = 0; m < 4; ++m)
+            fr[m] = (kind == KIND_WALL ? 2.0 * delta : delta) * Gs[m];
         if (b.flux_dbg) st4(reinterpret_cast<R4 *>(b.flux_dbg) + i, fr[0], fr[1], fr[2], fr[3]);
-        R4 P = ld4(b.prim_in + i);
         double U[4], Uo[4] = {0.0, 0.0, 0.0, 0.0};
         if (kind == KIND_OUTER) {
             const double *inf = g.obc + 8 * (size_t)orow;
             conserved_ubar(P.a, P.b, P.c, P.d, nx, ny, inf, c.pi, c.gm1, U);
             if (rk == 3) {
-                R4 O = ld4(b.prim_old + i);
                 conserved_ubar(O.a, O.b, O.c, O.d, nx, ny, inf, c.pi, c.gm1, Uo);
             }
         } else {
             prim_to_conserved(P.a, P.b, P.c, P.d, nx, ny, U);
             if (rk == 3) {
-                R4 O = ld4(b.prim_old + i);
                 prim_to_conserved(O.a, O.b, O.c, O.d, nx, ny, Uo);
             }
         }
@@ -592,72 +709,90 @@ update_point(const Geom &g, const Consts &c, const StageBufs &b, int rk, int las
     return res_sqr;
 }
 
-// F pass: each warp walks chunks of two scheduled tiles with a stride of all
-// warps of the grid.  A tile never straddles two instances and its partial
-// lands in slot (instance's first tile + tile number), summed over its 16
-// points in point order, so an instance's residual sums do not depend on the
-// other instances or on the launch shape.
+// F pass over chunks of `ct` (1 or 2) scheduled tiles.  COOP = false: a warp
+// owns a chunk, computes its points four at a time and updates them with one
+// lane each, with no block barrier.  COOP = true: the block's four warps
+// share a chunk (each a quarter of its points) and its first warp updates it
+// after a barrier.  Both call the same functions on a point, so the split
+// does not change a result.  A tile never straddles two instances and its
+// partial lands in slot (instance's first tile + tile number), summed over
+// its 16 points in point order, so an instance's residual sums do not depend
+// on the other instances or on the launch shape.
+//
+// A tile's rows come through shared memory: its halo (54 rows a 16-point tile
+// of an O-grid, against 144 row reads) is copied with cp.async, the row
+// indices a tile ahead.
 template <bool TAPE>
 __global__ void __launch_bounds__(FLUX_BLOCK, FLUX_MIN_BLOCKS)
-kb_flux(Geom g, Consts c, Sched s, StageBufs b, int rk, int last) {
-    __shared__ double sm[FLUX_WARPS * WARP_SMEM];
-#ifdef FLUX_SCHED_GLOBAL
-    // the schedule stays in global memory: 2 KB more shared memory per block
-    // for the records (one more resident block per SM)
+kb_flux(Geom g, Consts c, Sched s, StageBufs b, int rk, int last, int ct, int coop) {
+    extern __shared__ double2 fsm[];
     const int ntiles = __ldg(s.pre + __ldg(s.nact));
-#define FLUX_TILE(v) sched_tile_global(s, v)
-#else
-    __shared__ SchedSmem ss;
-    load_sched(s, ss);  // the kernel's only block barrier
-    const int ntiles = ss.pre[ss.nact];
-#define FLUX_TILE(v) sched_tile(s, ss, v)
-#endif
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    double *rec = sm + warp * WARP_SMEM;       // PPW groups of GROUP_SMEM
-    double *wG = rec + PPW * GROUP_SMEM;       // CHUNK points x GST
-    double *wres = wG + CHUNK * GST;           // CHUNK residual terms
-    const int nchunks = (ntiles + 1) / 2;
-    for (int ch = blockIdx.x * FLUX_WARPS + warp; ch < nchunks; ch += gridDim.x * FLUX_WARPS) {
-        const bool has1 = 2 * ch + 1 < ntiles;
-        for (int rnd = 0; rnd < CHUNK / PPW; ++rnd) {
-            const int pj = rnd * PPW + lane / LPP;  // point of the chunk
-            const int v = 2 * ch + (pj < TILE ? 0 : 1);
-            bool valid = false;
-            int i = 0, kind = KIND_INTERIOR;
-            if (v < ntiles) {
-                const TileRef t = FLUX_TILE(v);
-                const int j = t.j0 + (pj % TILE);
-                valid = j < t.n;
-                i = t.base + j;
-                kind = j < t.nw ? KIND_WALL : (j < t.nw + t.no ? KIND_OUTER : KIND_INTERIOR);
-            }
-            flux_group<TAPE>(g, c, b, i, valid, kind, rec + (lane / LPP) * GROUP_SMEM,
-                             wG + GST * pj);
+    FluxSmem &m = reinterpret_cast<FluxSmem *>(fsm)[coop ? 0 : warp];
+    const int nchunks = (ntiles + ct - 1) / ct, pts = ct * TILE;
+    const int jw = coop ? warp * PPW : 0, nj = coop ? PPW : TILE;  // the warp's points of a tile
+    const int step = coop ? gridDim.x : gridDim.x * FLUX_WARPS;
+    int ch = coop ? blockIdx.x : blockIdx.x * FLUX_WARPS + warp, u = 0;
+    if (ch >= nchunks) return;  // (coop: the whole block)
+    FluxTile cur(s, ntiles, ct * ch);
+    FluxHalo hx;
+    hx.range(g, cur);
+    hx.rows(g, lane);
+    auto stage = [&] {
+        if (coop) stage_flux<FLUX_BLOCK>(g, b, cur, hx, m, threadIdx.x);
+        else stage_flux<32>(g, b, cur, hx, m, lane);
+    };
+    auto sync = [&] {
+        if (coop) __syncthreads();
+        else __syncwarp();
+    };
+    stage();
+    while (true) {
+        const int hn = hx.hn, done = ct * ch;  // the chunk's first tile
+        const bool end = u + 1 == ct;
+        if (end) ch += step;
+        // the tile after this one: its halo's range now, its row indices once
+        // that has come (after the first round)
+        const FluxTile nxt(s, ntiles, end ? ct * ch : done + u + 1);
+        hx.range(g, nxt);
+        halo_wait();
+        sync();
+        for (int rnd = 0; rnd < nj; rnd += PPW) {
+            const int j = jw + rnd + lane / LPP;
+            flux_group<TAPE>(g, b, cur, j, hn, m, m.G[u * TILE + j]);
+            if (rnd == 0) hx.rows(g, lane);
         }
-        __syncwarp();
+        sync();
+        // the next tile's rows are on their way while this chunk is updated
+        cur = nxt;
+        stage();
+        u = end ? 0 : u + 1;
+        if (!end) continue;
         // the chunk's state updates, one point per lane
-        const int v = 2 * ch + (lane < TILE ? 0 : 1);
-        const TileRef t = FLUX_TILE(v < ntiles ? v : 2 * ch);
-        const int j = t.j0 + (lane % TILE);
-        const bool valid = v < ntiles && j < t.n;
-        double rs = 0.0;
-        if (valid) {
-            const int kind = j < t.nw ? KIND_WALL : (j < t.nw + t.no ? KIND_OUTER : KIND_INTERIOR);
-            rs = update_point(g, c, b, rk, last, t.base + j, kind, t.obc_off + j - t.nw,
-                              wG + GST * lane);
-        }
-        if (last) {
-            wres[lane] = rs;
-            __syncwarp();
-            if ((lane % TILE) == 0 && (lane < TILE || has1)) {
-                double acc = 0.0;
-                for (int q = 0; q < TILE; ++q) acc = acc + wres[lane + q];
-                b.res_part[t.tile] = acc;
+        if (!coop || warp == 0) {
+            const int v = done + lane / TILE;
+            const bool tile = lane < pts && v < ntiles;
+            const TileRef t = sched_tile_global(s, tile ? v : done);
+            const int j = t.j0 + (lane % TILE);
+            double rs = 0.0;
+            if (tile && j < t.n) {
+                const int kind =
+                    j < t.nw ? KIND_WALL : (j < t.nw + t.no ? KIND_OUTER : KIND_INTERIOR);
+                rs = update_point(g, c, b, rk, last, t.base + j, kind, t.obc_off + j - t.nw,
+                                  m.G[lane]);
+            }
+            if (last) {
+                m.G[lane][0] = rs;
+                __syncwarp();
+                if ((lane % TILE) == 0 && tile) {
+                    double acc = 0.0;
+                    for (int q = 0; q < TILE; ++q) acc = acc + m.G[lane + q][0];
+                    b.res_part[t.tile] = acc;
+                }
             }
         }
-        __syncwarp();  // the next chunk reuses wG and wres
+        if (ch >= nchunks) break;
     }
-#undef FLUX_TILE
 }
 
 // Sum of nparts tile partials in a fixed order (deterministic, independent
@@ -867,8 +1002,44 @@ inline int nblk(int n, int b) { return (n + b - 1) / b; }
 }  // namespace
 
 int flux_blocks(int n) { return nblk(n, TILE); }
-// blocks that give every warp of the flux pass one chunk of two tiles
-int flux_grid_blocks(int n) { return nblk(nblk(n, TILE), 2 * FLUX_WARPS); }
+
+namespace {
+int sm_count() {
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return std::max(sms, 1);
+}
+// Split of the FP64 flux pass for `tiles` scheduled tiles.  Up to one tile a
+// resident block, the block's warps share the tile (a round each): 11.4 us
+// against 16.4 at 4,000 points, 17.9 both at 16,000.  Beyond that a warp
+// takes chunks of one tile or, for less idle lanes in the updates (1.15
+// times the rate), of two, whichever its whole number of turns makes cheaper:
+// one against two tiles 45.8 / 52.2 us at 91,000 points, 38.6 / 37.6 at
+// 64,000, 112 / 105 at 256,000, 417 / 389 at 1,024,000.
+struct FluxShape {
+    int ct, coop;
+};
+FluxShape flux_shape(int tiles) {
+    const int blocks = sm_count() * FLUX_MIN_BLOCKS, warps = blocks * FLUX_WARPS;
+    if (tiles <= blocks) return FluxShape{1, 1};
+    const double one = 1.15 * nblk(tiles, warps), two = 2.0 * nblk(tiles, 2 * warps);
+    return FluxShape{one < two ? 1 : 2, 0};
+}
+}  // namespace
+
+// flux-pass blocks that give every chunk its warp (or its block)
+int flux_grid_blocks(int n, bool fp32) {
+    const int tiles = nblk(n, TILE);
+    if (fp32) return nblk(tiles, 2 * FLUX_WARPS);
+    const FluxShape f = flux_shape(tiles);
+    return nblk(nblk(tiles, f.ct), f.coop ? 1 : FLUX_WARPS);
+}
+
+void launch_flux_coef(const Geom &g, int base, int n, int nw, int no, double power, double *fco,
+                      double *wsl, cudaStream_t st) {
+    k_flux_coef<<<nblk(n, GRAD_BLOCK), GRAD_BLOCK, 0, st>>>(g, base, n, nw, no, power, fco, wsl);
+}
 
 // staging memory of a block of the halo kernels: two tiles a warp
 size_t halo_smem_bytes(int kind, int hc) {
@@ -881,6 +1052,12 @@ cudaError_t init_kernels() {
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(kb_inner_h, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)halo_smem_bytes(1, HALO_CAP + 1));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kb_flux<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 FLUX_SMEM);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kb_flux<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 FLUX_SMEM);
     return e;
 }
 
@@ -918,7 +1095,8 @@ int batch_occupancy(int kind, bool fp32, int block, size_t smem) {
     else if (kind == 1)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_inner_h, HALO_BLOCK,
                                                           halo_smem_bytes(1, HALO_CAP + 1));
-    else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_flux<false>, block, smem);
+    else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_flux<false>, block,
+                                                          FLUX_SMEM);
     return e == cudaSuccess ? nb : 1;
 }
 
@@ -950,10 +1128,13 @@ void launch_inner(const Geom &g, const Consts &c, const Sched &s, const double *
 }
 
 void launch_flux(const Geom &g, const Consts &c, const Sched &s, const StageBufs &b, int rk,
-                 bool last, int grid, cudaStream_t st) {
+                 bool last, int grid, int tiles, cudaStream_t st) {
+    const FluxShape f = flux_shape(tiles);
     const int gr = wave(2, FLUX_BLOCK, 0, grid);
-    if (b.kstape) kb_flux<true><<<gr, FLUX_BLOCK, 0, st>>>(g, c, s, b, rk, last ? 1 : 0);
-    else kb_flux<false><<<gr, FLUX_BLOCK, 0, st>>>(g, c, s, b, rk, last ? 1 : 0);
+    constexpr int sm = FLUX_SMEM;
+    if (b.kstape)
+        kb_flux<true><<<gr, FLUX_BLOCK, sm, st>>>(g, c, s, b, rk, last ? 1 : 0, f.ct, f.coop);
+    else kb_flux<false><<<gr, FLUX_BLOCK, sm, st>>>(g, c, s, b, rk, last ? 1 : 0, f.ct, f.coop);
 }
 
 void launch_residual(const InstInfo *inst, int n_inst, const double *res_part, Ctl *ctl,
