@@ -170,7 +170,7 @@ void launch_stage(mfcfd_t *h, cudaStream_t s, int rk, int A, int B, F after) {
         b.res_part = h->d_res_part;
         b.flux_dbg = h->keep_diag ? h->d_flux_dbg : nullptr;
         b.f = h->geom32;
-        launch_flux32(h->geom, h->consts, h->sched, b, rk, last, h->flux_grid, s);
+        launch_flux32(h->geom, h->consts, h->sched, b, rk, last, h->flux_grid, h->inst_h.ntiles, s);
         after();
     }
     h->qcur ^= 1;

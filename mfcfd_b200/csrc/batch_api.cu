@@ -230,7 +230,7 @@ void batch_stage(mfcfd_batch_t *b, cudaStream_t s, int rk, int A, int B) {
         sb.res_part = b->d_res_part;
         sb.flux_dbg = nullptr;
         sb.f = b->geom32;
-        launch_flux32(b->geom, b->consts, b->sched, sb, rk, last, fg, s);
+        launch_flux32(b->geom, b->consts, b->sched, sb, rk, last, fg, b->ntiles, s);
     }
     b->qcur ^= 1;
     b->launches += 2 + m;

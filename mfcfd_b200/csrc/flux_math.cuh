@@ -98,9 +98,11 @@ __device__ __forceinline__ double limited_qtilde(double t, double q, double qmax
     return fma(phi, del_neg, q);
 }
 
-// qtilde -> the state before its exponentials (q_variables.F90:230-256 with
-// the rearrangements of reconstruct_kstate): u, beta^(-5/2) into rho, the
-// density's exponent, |u|^2, sqrt(beta), p/rho.
+// qtilde -> the state before its exponentials (q_variables.F90:230-256).  beta
+// and p/rho come from qtilde itself (beta = -qtilde_4/2, p/rho = 1/(2 beta)),
+// and rho = exp(texp - log(beta)/(gamma-1)) with gamma = 1.4, a constant of
+// the reference (parameter.F90:10), as exp(texp) beta^(-5/2) = exp(texp)
+// (1/beta)^2 / sqrt(beta): no log.
 struct KPre {
     double u1, u2, texp, rb5, sb;
 };

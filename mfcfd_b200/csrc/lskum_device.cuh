@@ -165,7 +165,8 @@ __device__ __forceinline__ KStateT<T> kstate(T u1, T u2, T rho, T pr, T nx, T ny
     return s;
 }
 
-// erf(x) given exp(-x*x).  FP64: the library erf.  FP32: Abramowitz &
+// erf(x) given exp(-x*x).  FP64: the library erf.  FP32 (the flux pass
+// evaluates it on pairs, kstate2 of primal_fp32.cu): Abramowitz &
 // Stegun 7.1.26 (after Hastings), erf(|x|) = 1 - t (a1 + t (a2 + t (a3 + t
 // (a4 + t a5)))) exp(-x^2), t = 1 / (1 + p |x|), absolute error below
 // 1.5e-7 (5.3e-7 evaluated in FP32; tests/test_erf32.py) -- the split
@@ -186,61 +187,6 @@ __device__ __forceinline__ float erf_with_exp<float>(float x, float e) {
     p = p * t - 0.284496736f;
     p = p * t + 0.254829592f;
     return copysignf(1.0f - (p * t) * e, x);
-}
-
-// reconstruct + kstate in one, for the flux passes: the kinetic state of the
-// limited reconstruction towards one neighbour.  beta and p/rho come from
-// qtilde itself (beta = -qtilde_4/2, p/rho = 1/(2 beta)), which the
-// reference's 0.5 rho/p and p/rho of the same state equal in exact
-// arithmetic; 0.5/sqrt(pi beta) is formed as (p/rho) sqrt(beta) / sqrt(pi)
-// and beta**(-1/(gamma-1)) without a log (below).  Five divisions and one
-// reciprocal square root per state instead of ten divisions, two square
-// roots and a log; the results differ from reconstruct + kstate by rounding
-// only.
-template <class T>
-__device__ __forceinline__ KStateT<T> reconstruct_kstate(const T q[4], const T dqx[4],
-                                                         const T dqy[4], const T qmax[4],
-                                                         const T qmin[4], T eps2, T delx, T dely,
-                                                         T inv_gm1, T nx, T ny, T inv_sqrt_pi,
-                                                         T *u_out = nullptr) {
-    T qt[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        T t = delx * dqx[r] + dely * dqy[r];
-        T phi = venkat_phi<T>(q[r] - T(0.5) * t, q[r], qmax[r], qmin[r], eps2);
-        qt[r] = q[r] - T(0.5) * phi * t;
-    }
-    const T beta = -qt[3] * T(0.5);
-    const T temp = T(0.5) / beta;  // p / rho
-    const T u1 = qt[1] * temp, u2 = qt[2] * temp;
-    if (u_out) {  // the adjoint's tape keeps the reconstructed velocity
-        u_out[0] = u1;
-        u_out[1] = u2;
-    }
-    const T temp1 = qt[0] + beta * (u1 * u1 + u2 * u2);
-    KStateT<T> s;
-    // rho = exp(temp1 - log(beta)/(gamma-1)) with gamma = 1.4, a constant of
-    // the reference (parameter.F90:10): beta**(-1/(gamma-1)) = beta**(-2.5)
-    // = (1/beta)**2 / sqrt(beta), 1/beta = 2 p/rho -- no log, and sqrt(beta)
-    // from the same reciprocal square root (C2: 0.705 -> 0.649 ms a flux
-    // pass).  inv_gm1 is kept in the signature for the callers.
-    const T rb = rsqrt(beta);
-    const T sb = beta * rb;
-    s.rho = exp(temp1) * ((T(4.0) * temp * temp) * rb);
-    (void)inv_gm1;
-    const T tx = ny, ty = -nx;
-    s.ut = u1 * tx + u2 * ty;
-    s.un = u1 * nx + u2 * ny;
-    const T S1 = s.ut * sb, S2 = s.un * sb;
-    const T h = temp * sb * inv_sqrt_pi;  // 0.5 / sqrt(pi beta)
-    const T E1 = exp(-S1 * S1), E2 = exp(-S2 * S2);
-    s.B1 = E1 * h;
-    s.B2 = E2 * h;
-    s.e1 = erf_with_exp(S1, E1);
-    s.e2 = erf_with_exp(S2, E2);
-    s.pbr = temp;
-    s.usq = s.ut * s.ut + s.un * s.un;
-    return s;
 }
 
 // split_fluxes.F90:8-96 flux_Gxp (s1 = +1) / flux_Gxn (s1 = -1)

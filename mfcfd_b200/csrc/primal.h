@@ -132,6 +132,12 @@ cudaError_t init_kernels();
 int flux_blocks(int n);
 // flux-pass blocks beyond which some would find no work
 int flux_grid_blocks(int n, bool fp32);
+// Split of a flux pass: tiles a chunk (1 or 2), whether a block's warps share it
+struct FluxShape {
+    int ct, coop;
+};
+FluxShape flux_shape(int tiles, int per_sm);
+int flux32_per_sm();  // resident blocks an SM of the FP32-mixed flux pass
 // resident blocks per SM (kind: 0 D pass, 1 I pass, 2 F pass; fp32 selects
 // the FP32-mixed kernels)
 int batch_occupancy(int kind, bool fp32, int block, size_t smem);
@@ -201,7 +207,7 @@ inline int dq_src(int t) { return dq32_src(t); }
 inline int dq_dst(int t) { return dq32_dst(t); }
 inline int dq_final(int m) { return dq32_final(m); }
 void launch_flux32(const Geom &g, const Consts &c, const Sched &s, const StageBufs32 &b, int rk,
-                   bool last, int grid, cudaStream_t st);
+                   bool last, int grid, int tiles, cudaStream_t st);
 void launch_init_state32(const Geom &g, const float4 *prim, float4 *q, double *spd,
                          cudaStream_t s);
 

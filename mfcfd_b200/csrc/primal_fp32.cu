@@ -2,20 +2,19 @@
 //
 // Stored per point in FP32: prim, q, dq, qm (half the FP64 gather traffic).
 // Computed in FP32: the q-derivative sums of the D and I passes, the
-// per-neighbour work of the flux pass -- limiter, qtilde -> primitive (log,
-// exp), the Maxwellian moments (exp, erf, sqrt) and the split fluxes -- with
-// the flux contributions summed by compensated (Kahan) FP32 addition in slot
-// order.  The 2x2 least-squares normal matrices, ill-conditioned on
-// stretched near-wall stencils, are pure geometry: they are formed and
-// inverted once per grid in FP64 (Geom32) and only applied per iteration.
-// The state update runs in FP32 too (the state is stored in FP32); kept in
-// FP64: the local time step, the list derivatives and flux residual, the
-// residual norm (from the FP64 increment) and the force coefficients.
+// per-neighbour work of the flux pass -- limiter, qtilde -> kinetic state,
+// Maxwellian moments and split fluxes.  The 2x2 least-squares normal
+// matrices, ill-conditioned on stretched near-wall stencils, are pure
+// geometry: they are formed and inverted once per grid in FP64 (Geom32) and
+// only applied per iteration.  Kept in FP64: the sums of the flux
+// contributions and the flux residual, the arithmetic of the state update,
+// the local time step, the residual norm and the force coefficients.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 
 #include "batch.cuh"
+#include "flux_tile.cuh"
 #include "halo.cuh"
 #include "primal.h"
 
@@ -24,12 +23,6 @@ namespace lskum {
 namespace {
 
 constexpr int GRAD_BLOCK = 256;
-constexpr int LPP = 8;
-constexpr int FLUX_BLOCK = 128;  // four independent warps
-constexpr int FREC = 10;  // dGxp..dGyn as 16 floats, then each list's slot weight c_L (20 floats)
-#ifndef FLUX32_MIN_BLOCKS
-#define FLUX32_MIN_BLOCKS 7  // <= 72 registers (8 blocks: 64 registers with spills, 0.370 against 0.364 ms on C2)
-#endif
 constexpr double OBT = 1.0 / 3.0;
 constexpr double TBT = 2.0 / 3.0;
 
@@ -238,309 +231,373 @@ kb_grad32_h(Geom g, Consts c, Geom32 f, Sched s, const float4 *__restrict__ q,
     }
 }
 
-// Compensated FP32 addition (Kahan): s += v with running correction cmp.
-__device__ __forceinline__ void kahan_add(float &s, float &cmp, float v) {
-    float y = __fsub_rn(v, cmp);
-    float t = __fadd_rn(s, y);
-    cmp = __fsub_rn(__fsub_rn(t, s), y);
-    s = t;
+// ---------------------------------------------------------------------------
+// F pass.
+//
+// Pairs of FP32 values in one 64-bit register pair: sm_100 adds, multiplies
+// and fuses both in one instruction (f32x2), and this pass is bound by the
+// instructions it issues.  The limiter works on pairs of components, the
+// kinetic states and split fluxes on the pair of directions (t, n).
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float x, float y) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ F2 f2(float x) { return f2(x, x); }
+__device__ __forceinline__ float lo(F2 a) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+    return x;
+}
+__device__ __forceinline__ float hi(F2 a) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+    return y;
+}
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) {
+    F2 r;
+    asm("sub.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ float rcpf(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rsqf(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float ex2f(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
 }
 
-// cal_flux_residual + state_update + eval_q_variables of the new state, with
-// the per-neighbour work in FP32.  Work split as in the FP64 pass: a warp
-// owns two tiles (32 points) end to end with no block barrier, computes
-// their list derivatives in rounds of four points (eight lanes each, slots
-// taken eight at a time with the lane pairs' Kahan sums parked in shared
-// memory between slot rounds), then updates the 32 points one per lane.
-#ifndef FLUX32_CT
-#define FLUX32_CT 1  // tiles a warp owns: 1 (0.366 ms per C2 launch) or 2 (every lane updates a point; 0.375 ms)
-#endif
-// Arithmetic types of the flux pass: RT for the reconstruction to the
-// kinetic state, FT for the split fluxes and their differences, UT for the
-// state update.  The state is stored in FP32 throughout.  The update runs in
-// FP64: its conversions prim -> U -> prim, four times an iteration, are what
-// moved the FP32-mixed loop away from the FP64 loop (640x400 grid, 2,000
-// iterations from freestream: |dCd| 1.1e-5 with an FP32 update, 2.2e-7 with
-// an FP64 one, at 1.4 % of the pass's time), while FP64 reconstruction or
-// fluxes changed nothing measurable (|dCd| 1.10-1.12e-5 with either).
-#ifndef FLUX32_RT
-#define FLUX32_RT float
-#endif
-#ifndef FLUX32_FT
-#define FLUX32_FT float
-#endif
-#ifndef FLUX32_UT
-#define FLUX32_UT double
-#endif
-using RT = FLUX32_RT;
-using FT = FLUX32_FT;
-using UT = FLUX32_UT;
-template <class D, class S>
-__device__ __forceinline__ KStateT<D> kcast(const KStateT<S> &s) {
-    KStateT<D> d;
-    d.rho = (D)s.rho; d.ut = (D)s.ut; d.un = (D)s.un; d.pbr = (D)s.pbr; d.usq = (D)s.usq;
-    d.B1 = (D)s.B1; d.B2 = (D)s.B2; d.e1 = (D)s.e1; d.e2 = (D)s.e2;
-    return d;
+// venkat_limiter and the limited qtilde of two components (limiters.F90:64-110),
+// mt = -(d . dq): del_neg is mt/2, and its factor common to the quotient's
+// numerator and denominator is cancelled.
+__device__ __forceinline__ F2 limited2(F2 mt, F2 q, F2 qmax, F2 qmin, F2 eps2) {
+    const F2 dn = mt * f2(0.5f);
+    const F2 dp = f2(lo(mt) > 0.f ? lo(qmax) : lo(qmin), hi(mt) > 0.f ? hi(qmax) : hi(qmin)) - q;
+    const F2 a = fma2(dp, dp, eps2);
+    const F2 num = fma2(mt, dp, a), den = fma2(dn, dp + mt, a);
+    const F2 f = num * f2(rcpf(lo(den)), rcpf(hi(den)));
+    constexpr float thr = (float)MFCFD_VENKAT_THR;
+    const F2 phi = f2(fabsf(lo(dn)) <= thr ? 1.0f : fminf(lo(f), 1.0f),
+                      fabsf(hi(dn)) <= thr ? 1.0f : fminf(hi(f), 1.0f));
+    return fma2(phi, dn, q);
 }
-// the reconstructed kinetic state of point p along (dx, dy)
-__device__ __forceinline__ KStateT<FT> kstate32(const StageBufs32 &b, int p, RT dx, RT dy, RT inv_gm1,
-                                                RT nx, RT ny, RT inv_sqrt_pi) {
-    const float4 v = __ldg(b.q_in + p);
-    float dxf[4], dyf[4], qmaxf[4], qminf[4];
-    ldf8w(b.dq + 8 * (size_t)p, dxf, dyf);
-    ldf8w(b.qm + 8 * (size_t)p, qmaxf, qminf);
-    const RT q[4] = {v.x, v.y, v.z, v.w};
-    RT ddx[4], ddy[4], qmax[4], qmin[4];
+
+// A row of the stage's arrays: staged (row l of the halo) or from global memory.
+struct Row32 {
+    F2 q[2], dx[2], dy[2], qmax[2], qmin[2];
+    float eps2;
+    __device__ __forceinline__ void qtilde(F2 mdx, F2 mdy, F2 qt[2]) const {
+        const F2 e = f2(eps2);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        ddx[j] = dxf[j]; ddy[j] = dyf[j]; qmax[j] = qmaxf[j]; qmin[j] = qminf[j];
+        for (int h = 0; h < 2; ++h)
+            qt[h] = limited2(fma2(mdx, dx[h], mdy * dy[h]), q[h], qmax[h], qmin[h], e);
     }
-    return kcast<FT>(reconstruct_kstate<RT>(q, ddx, ddy, qmax, qmin, (RT)b.eps2f[p], dx, dy,
-                                            inv_gm1, nx, ny, inv_sqrt_pi));
-}
-constexpr int PPW = 32 / LPP;
-constexpr int CT = FLUX32_CT;
-constexpr int CHUNK = CT * TILE;
-constexpr int GST = 17;                                  // odd: no bank conflicts
-constexpr int FLUX_WARPS = FLUX_BLOCK / 32;
-constexpr int GROUP_SMEM = LPP * FREC + 4 * LPP;         // records + parked sums (doubles)
-constexpr int WARP_SMEM = PPW * GROUP_SMEM + CHUNK * GST + CHUNK;
+};
 
-__device__ __forceinline__ void
-flux32_group(const Geom &g, const Consts &c, const StageBufs32 &b, int i, bool valid,
-             int kind0, double *rec, double *Gout) {
-    const int lane = threadIdx.x % LPP;
-    int nb = 0, kind = KIND_INTERIOR;
-    unsigned long long mx = 0, my = 0;
-    RT nxf = 0, nyf = 1;
-    if (valid) {
-        nb = g.nbhs[i];
-        kind = kind0;
-        mx = g.mx[i];
-        my = g.my[i];
-        const double2 nn = g.nrm[i];
-        nxf = (RT)nn.x;
-        nyf = (RT)nn.y;
-    }
-    const RT inv_gm1 = (RT)(1.0 / c.gm1), inv_sqrt_pi = (RT)(1.0 / sqrt(c.pi));
-    const FT s2q = kind == KIND_WALL ? FT(-1) : FT(1);
-    const int nbw = __reduce_max_sync(0xffffffffu, nb);
-    const int L = lane >> 1, c0 = (lane & 1) * 2;
-    const bool used =
-        valid && !((kind == KIND_WALL && L == 2) || (kind == KIND_OUTER && L == 3));
-    // Kahan sums of the lane's two list components and their corrections
-    float fx0 = 0.f, fx1 = 0.f, cx0 = 0.f, cx1 = 0.f;
-    float *park = reinterpret_cast<float *>(rec + LPP * FREC) + 8 * lane;
-    for (int r0 = 0; r0 < nbw; r0 += LPP) {
-        if (r0 > 0) {
-            park[0] = fx0; park[1] = fx1; park[2] = cx0; park[3] = cx1;
+// Kinetic state of a limited reconstruction (kstate_pre's forms): the
+// velocity in the point's frame, Maxwellian half-moments and erf as (t, n)
+// pairs.  erf from the exponential the moments take anyway (erf_with_exp).
+struct KState2 {
+    F2 U, B, e;
+    float rho, pbr, usq;
+};
+__device__ __forceinline__ KState2 kstate2(const F2 qt[2], float nx, float ny, float inv_sqrt_pi) {
+    constexpr float log2e = 1.44269504088896340736f;
+    KState2 s;
+    const float nq = -hi(qt[1]), beta = 0.5f * nq;
+    s.pbr = rcpf(nq);
+    const float u1 = hi(qt[0]) * s.pbr, u2 = lo(qt[1]) * s.pbr;
+    s.usq = u1 * u1 + u2 * u2;
+    const float texp = lo(qt[0]) + beta * s.usq;
+    const float rb = rsqf(beta), sb = beta * rb;
+    s.rho = ex2f(texp * log2e) * ((4.0f * s.pbr * s.pbr) * rb);
+    s.U = fma2(f2(u1), f2(ny, nx), f2(u2) * f2(-nx, ny));
+    const F2 S = s.U * f2(sb);
+    const F2 x = (S * S) * f2(-log2e);
+    const F2 E = f2(ex2f(lo(x)), ex2f(hi(x)));
+    s.B = E * f2(s.pbr * sb * inv_sqrt_pi);
+    const F2 d = fma2(f2(fabsf(lo(S)), fabsf(hi(S))), f2(0.3275911f), f2(1.0f));
+    const F2 t = f2(rcpf(lo(d)), rcpf(hi(d)));
+    F2 p = f2(-1.061405429f);
+    p = fma2(p, t, f2(1.453152027f));
+    p = fma2(p, t, f2(-1.421413741f));
+    p = fma2(p, t, f2(0.284496736f));
+    p = fma2(p, t, f2(-0.254829592f));
+    const F2 r = fma2(p * t, E, f2(1.0f));
+    s.e = f2(copysignf(lo(r), lo(S)), copysignf(hi(r), hi(S)));
+    return s;
+}
+
+// split_fluxes.F90 along t (first of each pair) and along n (second), sg the
+// signs of the two lists: mass, momentum along the direction, momentum across
+// it, energy (flux_split of the FP64 pass).
+__device__ __forceinline__ void flux_split2(const KState2 &s, F2 sg, F2 G[4]) {
+    const F2 A = fma2(sg * f2(0.5f), s.e, f2(0.5f));
+    const F2 a = fma2(s.U, A, sg * s.B);
+    const F2 pA = f2(s.pbr) * A;
+    const float w6 = 6.0f * s.pbr + s.usq;
+    G[0] = f2(s.rho) * a;
+    G[1] = f2(s.rho) * fma2(s.U, a, pA);
+    G[2] = f2(hi(s.U), lo(s.U)) * G[0];
+    G[3] = f2(0.5f * s.rho) * fma2(f2(w6), a, s.U * pA);
+}
+
+__device__ __forceinline__ KStateT<float> kstate_plain(const KState2 &s) {
+    KStateT<float> k;
+    k.rho = s.rho; k.ut = lo(s.U); k.un = hi(s.U); k.pbr = s.pbr; k.usq = s.usq;
+    k.B1 = lo(s.B); k.B2 = hi(s.B); k.e1 = lo(s.e); k.e2 = hi(s.e);
+    return k;
+}
+
+// Shared memory of a unit: the tile's halo rows as one array per 16-byte piece
+// (q 0, dq 1-2, qm 3-4, (x, y) 5) and the limiter's eps2, the tile's own
+// points and list coefficients, the chunk's flux residuals.
+struct Flux32Smem {
+    static constexpr int ROWS = HALO_CAP, HC = ROWS + 1;
+    double2 halo[6][HC];
+    float4 co[TILE][2];
+    FluxOwn own;
+    double G[CHUNK_MAX][4];  // flux residuals, then residual terms
+    float eps[HC + 3];
+};
+constexpr int FLUX32_SMEM = FLUX_WARPS * sizeof(Flux32Smem);
+// 96 registers at 5 blocks: 0.214 ms at 1.024M points; 6 blocks spill (0.258),
+// 4 have too few warps (0.223)
+constexpr int FLUX32_MIN_BLOCKS = 5;
+
+// cal_flux_residual + state_update + eval_q_variables of the new state with
+// the per-neighbour work in FP32: the FP64 pass's split of the work
+// (flux_pass) and its pooled list weights; a slot's weighted differences are
+// FP32, their sums over the slots FP64.  Bound by issue (64 % of the slots at
+// 620 instructions a round, 833 with scalar FP32 arithmetic and per-list
+// compensated sums): 0.283 -> 0.214 ms at 1.024M points, 77 -> 65 us at
+// 256,000, 26 -> 14 us at 16,000, 26 -> 10 us at 1,536.
+//
+// The update runs in FP64: its conversions prim -> U -> prim, four times an
+// iteration, are what moved an earlier FP32 update away from the FP64 loop
+// (640x400 grid, 2,000 iterations from freestream: |dCd| 1.1e-5 with an FP32
+// update, 2.2e-7 with an FP64 one), while FP64 reconstruction or fluxes
+// changed nothing measurable.
+struct Flux32 {
+    using Smem = Flux32Smem;
+    const Geom &g;
+    const Consts &c;
+    const StageBufs32 &b;
+    int rk, last;
+
+    template <int NT>
+    __device__ __forceinline__ void stage(const FluxTile &t, const FluxHalo &x, Smem &m, int tid) {
+        stage_rows<1, NT, Smem::HC>(b.q_in, x, m.halo[0], tid);
+        stage_rows<2, NT, Smem::HC>(b.dq, x, m.halo[1], tid);
+        stage_rows<2, NT, Smem::HC>(b.qm, x, m.halo[3], tid);
+        stage_rows<1, NT, Smem::HC>(g.xy, x, m.halo[5], tid);
+        if (tid < HALO_CAP) {
+#pragma unroll
+            for (int u0 = 0; u0 < HALO_CAP; u0 += NT < HALO_CAP ? NT : HALO_CAP) {
+                const int k = x.row(u0 + tid);
+                if (u0 + tid < x.hn) halo_cp4(&m.eps[u0 + tid], b.eps2f + k);
+            }
         }
-        const int r = r0 + lane;
-        if (r < nb) {
-            const int k = g.conn[r * g.n + i];
-            const float2 d = __ldg(b.f.dxy + r * g.n + i);
-            const float dxf = d.x, dyf = d.y;
-            const KStateT<FT> sk = kstate32(b, k, dxf, dyf, inv_gm1, nxf, nyf, inv_sqrt_pi);
-            const KStateT<FT> si = kstate32(b, i, dxf, dyf, inv_gm1, nxf, nyf, inv_sqrt_pi);
-            const float dels = dxf * nyf - dyf * nxf;
-            const float deln = dxf * nxf + dyf * nyf;
-            const float w = b.f.w ? __ldg(b.f.w + r * g.n + i) : 1.0f;
-            float *ef = reinterpret_cast<float *>(rec + lane * FREC);
-            FT Gi[4], Gk[4];
+        if (tid < 2 * t.cnt)
+            halo_cp16(&m.co[0][0] + tid, b.f.flsq + 2 * (size_t)t.i0 + tid);
+        m.own.stage<NT>(g, t, tid);
+    }
+
+    __device__ __forceinline__ void row(const Smem &m, int l, Row32 &o) const {
+        const float4 q = *reinterpret_cast<const float4 *>(&m.halo[0][l]);
+        const float4 x = *reinterpret_cast<const float4 *>(&m.halo[1][l]);
+        const float4 y = *reinterpret_cast<const float4 *>(&m.halo[2][l]);
+        const float4 h = *reinterpret_cast<const float4 *>(&m.halo[3][l]);
+        const float4 w = *reinterpret_cast<const float4 *>(&m.halo[4][l]);
+        o.q[0] = f2(q.x, q.y); o.q[1] = f2(q.z, q.w);
+        o.dx[0] = f2(x.x, x.y); o.dx[1] = f2(x.z, x.w);
+        o.dy[0] = f2(y.x, y.y); o.dy[1] = f2(y.z, y.w);
+        o.qmax[0] = f2(h.x, h.y); o.qmax[1] = f2(h.z, h.w);
+        o.qmin[0] = f2(w.x, w.y); o.qmin[1] = f2(w.z, w.w);
+        o.eps2 = m.eps[l];
+    }
+    __device__ __forceinline__ void row(int k, Row32 &o) const {
+        const float4 q = __ldg(b.q_in + k);
+        float x[4], y[4], h[4], w[4];
+        ldf8w(b.dq + 8 * (size_t)k, x, y);
+        ldf8w(b.qm + 8 * (size_t)k, h, w);
+        o.q[0] = f2(q.x, q.y); o.q[1] = f2(q.z, q.w);
 #pragma unroll
-            for (int dd = 0; dd < 2; ++dd) {
-                // one converged evaluation per direction, as in the FP64 pass
-                const unsigned long long bits = dd == 0 ? mx : my;
-                const bool in0 = (bits >> r) & 1ull, in1 = (bits >> (r + 32)) & 1ull;
-#pragma unroll
-                for (int pass = 0; pass < 2; ++pass) {
-                    if (pass == 0 ? !(in0 || in1) : !(in0 && in1)) continue;
-                    const int Lx = 2 * dd + ((pass == 1 || !in0) ? 1 : 0);
-                    const FT sg = (Lx & 1) ? FT(-1) : FT(1);
-                    if (dd == 0) {
-                        if (kind == KIND_INTERIOR) {
-                            flux_gx<FT>(si, sg, Gi);
-                            flux_gx<FT>(sk, sg, Gk);
-                        } else {
-                            flux_quad<FT>(si, sg, s2q, Gi);
-                            flux_quad<FT>(sk, sg, s2q, Gk);
-                        }
-                    } else {
-                        flux_gy<FT>(si, sg, Gi);
-                        flux_gy<FT>(sk, sg, Gk);
-                    }
-#pragma unroll
-                    for (int m = 0; m < 4; ++m) ef[4 * Lx + m] = (float)(Gk[m] - Gi[m]);
-                }
-            }
+        for (int a = 0; a < 2; ++a) {
+            o.dx[a] = f2(x[2 * a], x[2 * a + 1]);
+            o.dy[a] = f2(y[2 * a], y[2 * a + 1]);
+            o.qmax[a] = f2(h[2 * a], h[2 * a + 1]);
+            o.qmin[a] = f2(w[2 * a], w[2 * a + 1]);
+        }
+        o.eps2 = b.eps2f[k];
+    }
+
+    __device__ __forceinline__ void group(const FluxTile &t, int j, int hn, Smem &m, double *G) {
+        const int lane = threadIdx.x % LPP;
+        const float inv_sqrt_pi = 0.56418958354775628695f;
+        const int kind = t.kind(j), i = t.i0 + j;
+        double v[4] = {0.0, 0.0, 0.0, 0.0};
+        const double2 nn = m.own.nrm[j];
+        const float nx = (float)nn.x, ny = (float)nn.y;
+        const int nb = j < t.cnt ? m.own.nbhs[j] : 0;
+        for (int r = lane; r < nb; r += LPP) {
+            KState2 sk, si;
+            float dx, dy;
             {
-                // the list solves folded into the slot: list L's derivative is
-                // sum_slots d * c_L with c_L = a_L dels w + b_L deln w (x lists)
-                // or a_L deln w + b_L dels w (y lists)
-                const float sw = dels * w, nw = deln * w;
-                const float4 cx = __ldg(b.f.flsq + 2 * (size_t)i);
-                const float4 cy = __ldg(b.f.flsq + 2 * (size_t)i + 1);
-                ef[16] = cx.x * sw + cx.y * nw;
-                ef[17] = cx.z * sw + cx.w * nw;
-                ef[18] = cy.x * nw + cy.y * sw;
-                ef[19] = cy.z * nw + cy.w * sw;
+                F2 qk[2], qi[2];
+                Row32 o;
+                if (hn > 0) {
+                    int lk, li;
+                    m.own.rows(g, i, j, r, lk, li);
+                    const double2 pi_ = m.halo[5][li], pk = m.halo[5][lk];
+                    // rounded as the host rounds the offsets it stores
+                    dx = (float)(pk.x - pi_.x);
+                    dy = (float)(pk.y - pi_.y);
+                    const F2 mdx = f2(-dx), mdy = f2(-dy);
+                    row(m, lk, o);
+                    o.qtilde(mdx, mdy, qk);
+                    row(m, li, o);
+                    o.qtilde(mdx, mdy, qi);
+                } else {
+                    const float2 d = __ldg(b.f.dxy + (size_t)r * g.n + i);
+                    dx = d.x;
+                    dy = d.y;
+                    const F2 mdx = f2(-dx), mdy = f2(-dy);
+                    row(g.conn[(size_t)r * g.n + i], o);
+                    o.qtilde(mdx, mdy, qk);
+                    row(i, o);
+                    o.qtilde(mdx, mdy, qi);
+                }
+                sk = kstate2(qk, nx, ny, inv_sqrt_pi);
+                si = kstate2(qi, nx, ny, inv_sqrt_pi);
             }
+            const float w = b.f.w ? __ldg(b.f.w + (size_t)r * g.n + i) : 1.0f;
+            const float dels = (dx * ny - dy * nx) * w, deln = (dx * nx + dy * ny) * w;
+            // Per direction the neighbour is in one list of the pair, in both
+            // only when its projection is exactly 0: the second list is added
+            // then.
+            const uint4 mm = m.own.mask[j];
+            const float2 *co = reinterpret_cast<const float2 *>(m.co[j]);
+            auto add = [&](int lx, int ly, bool ux, bool uy) {
+                const float2 cx = co[lx], cy = co[2 + ly];
+                const float sx = lx ? -1.0f : 1.0f, sy = ly ? -1.0f : 1.0f;
+                const float wx = ux ? cx.x * dels + cx.y * deln : 0.0f;
+                const float wy = uy ? cy.x * deln + cy.y * dels : 0.0f;
+                F2 Gi[4], Gk[4];
+                flux_split2(si, f2(sx, sy), Gi);
+                flux_split2(sk, f2(sx, sy), Gk);
+                // differences along t and along n, as scalars: a pair built in the
+                // branch below from its own half came out wrong (ptxas 12.9)
+                float X[4], Y[4];
+#pragma unroll
+                for (int d = 0; d < 4; ++d) {
+                    const F2 D = Gk[d] - Gi[d];
+                    X[d] = lo(D);
+                    Y[d] = hi(D);
+                }
+                if (kind != KIND_INTERIOR) {
+                    // wall GxII/GxI (A2neg), outer GxIII/GxIV (A2pos)
+                    const float s2 = kind == KIND_WALL ? -1.0f : 1.0f;
+                    float Qi[4], Qk[4];
+                    flux_quad<float>(kstate_plain(si), sx, s2, Qi);
+                    flux_quad<float>(kstate_plain(sk), sx, s2, Qk);
+#pragma unroll
+                    for (int d = 0; d < 4; ++d) X[d] = Qk[d] - Qi[d];
+                }
+                v[0] += (double)(wx * X[0] + wy * Y[0]);
+                v[1] += (double)(wx * X[1] + wy * Y[2]);
+                v[2] += (double)(wx * X[2] + wy * Y[1]);
+                v[3] += (double)(wx * X[3] + wy * Y[3]);
+            };
+            const unsigned bit = 1u << r;
+            add(mm.x & bit ? 0 : 1, mm.z & bit ? 0 : 1, true, true);
+            const bool tx = mm.x & mm.y & bit, ty = mm.z & mm.w & bit;
+            if (tx || ty) add(1, 1, tx, ty);
         }
         __syncwarp();
-        if (r0 > 0) {
-            fx0 = park[0]; fx1 = park[1]; cx0 = park[2]; cx1 = park[3];
-        }
-        if (used) {
-            // the list's slots of this round in slot order (lowest bit first):
-            // a lane loops over its own members only
-            const unsigned long long lbits = ((L < 2) ? mx : my) >> ((L & 1) ? 32 : 0);
-            // (a point with fewer slots than r0 has none in this round)
-            const int cnt = min(nb, r0 + LPP) - r0;
-            unsigned rb = cnt > 0 ? (unsigned)(lbits >> r0) & ((1u << cnt) - 1u) : 0u;
-            while (rb) {
-                const int rr = r0 + __ffs(rb) - 1;
-                rb &= rb - 1u;
-                const float *ef = reinterpret_cast<const float *>(rec + (rr - r0) * FREC);
-                const float d0 = ef[4 * L + c0], d1 = ef[4 * L + c0 + 1];
-                const float cl = ef[16 + L];
-                kahan_add(fx0, cx0, d0 * cl);
-                kahan_add(fx1, cx1, d1 * cl);
-            }
-        }
-        __syncwarp();  // the next round overwrites the records
+        const double sum = reduce8(v, lane);
+        if (!(lane & 1)) G[lane >> 1] = sum;
     }
-    double Gv0 = 0.0, Gv1 = 0.0;
-    if (used) {
-        Gv0 = (double)fx0 - cx0;
-        Gv1 = (double)fx1 - cx1;
-    }
-    // lane 2L+h holds G[L][2h], G[L][2h+1]
-    Gout[2 * lane] = Gv0;
-    Gout[2 * lane + 1] = Gv1;
-}
 
-// state_update.F90:10-141 of one point from its four list derivatives
-// Gs[4L+m]: FP32 state in and out, arithmetic in UT; returns its res_sqr
-// term (FP64).
-__device__ __forceinline__ double
-update32_point(const Geom &g, const Consts &c, const StageBufs32 &b, int rk, int last, int i,
-               int kind, int orow, const double *Gs) {
-    double G[4][4];
-#pragma unroll
-    for (int L = 0; L < 4; ++L)
-#pragma unroll
-        for (int m = 0; m < 4; ++m) G[L][m] = Gs[4 * L + m];
-    const double2 nn = g.nrm[i];
-    const double nx = nn.x, ny = nn.y;
-    double res_sqr = 0.0;
-    {
-        const double delta = b.delta[i];
+    // state_update.F90:10-141 of one point from the sum of its list
+    // derivatives: FP32 state in and out, FP64 arithmetic; returns its res_sqr
+    // term.
+    __device__ __forceinline__ double update(int i, int kind, int orow, const double *Gs) {
+        const double2 nn = g.nrm[i];
+        const double nx = nn.x, ny = nn.y, delta = b.delta[i];
+        const float4 Pf = b.prim_in[i], Of = rk == 3 ? b.prim_old[i] : Pf;
         double fr[4];
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            if (kind == KIND_WALL) fr[m] = 2.0 * delta * (G[0][m] + G[1][m] + G[3][m]);
-            else if (kind == KIND_OUTER) fr[m] = delta * (G[0][m] + G[1][m] + G[2][m]);
-            else fr[m] = delta * (G[0][m] + G[1][m] + G[2][m] + G[3][m]);
-        }
+        for (int m = 0; m < 4; ++m)
+            fr[m] = (kind == KIND_WALL ? 2.0 * delta : delta) * Gs[m];
         if (b.flux_dbg) st4(reinterpret_cast<R4 *>(b.flux_dbg) + i, fr[0], fr[1], fr[2], fr[3]);
-        // state_update in UT (the state is stored in FP32); the residual
-        // from the increment itself, 0.5 euler fr(1), in FP64, which FP32
-        // differences of U(1) would cancel (last stage: rk != 3)
-        if (kind != KIND_OUTER) res_sqr = (0.5 * c.euler * fr[0]) * (0.5 * c.euler * fr[0]);
-        const UT nxf = (UT)nx, nyf = (UT)ny, pif = (UT)c.pi, gm1f = (UT)c.gm1;
-        UT frf[4] = {(UT)fr[0], (UT)fr[1], (UT)fr[2], (UT)fr[3]};
-        const float4 P = b.prim_in[i];
-        UT U[4], Uo[4] = {0, 0, 0, 0};
+        // the residual from the increment itself, 0.5 euler fr(1), which
+        // differences of the stored FP32 state would cancel (last stage: rk != 3)
+        const double he = 0.5 * c.euler;
+        const double res_sqr = kind != KIND_OUTER ? (he * fr[0]) * (he * fr[0]) : 0.0;
+        double U[4], Uo[4] = {0.0, 0.0, 0.0, 0.0};
         if (kind == KIND_OUTER) {
             const double *inf = g.obc + 8 * (size_t)orow;
-            const UT inff[5] = {(UT)inf[0], (UT)inf[1], (UT)inf[2], (UT)inf[3], (UT)inf[4]};
-            conserved_ubar_t<UT>(P.x, P.y, P.z, P.w, nxf, nyf, inff, pif, gm1f, U);
-            if (rk == 3) {
-                const float4 O = b.prim_old[i];
-                conserved_ubar_t<UT>(O.x, O.y, O.z, O.w, nxf, nyf, inff, pif, gm1f, Uo);
-            }
+            conserved_ubar(Pf.x, Pf.y, Pf.z, Pf.w, nx, ny, inf, c.pi, c.gm1, U);
+            if (rk == 3) conserved_ubar(Of.x, Of.y, Of.z, Of.w, nx, ny, inf, c.pi, c.gm1, Uo);
         } else {
-            prim_to_conserved_t<UT>(P.x, P.y, P.z, P.w, nxf, nyf, U);
-            if (rk == 3) {
-                const float4 O = b.prim_old[i];
-                prim_to_conserved_t<UT>(O.x, O.y, O.z, O.w, nxf, nyf, Uo);
-            }
+            prim_to_conserved(Pf.x, Pf.y, Pf.z, Pf.w, nx, ny, U);
+            if (rk == 3) prim_to_conserved(Of.x, Of.y, Of.z, Of.w, nx, ny, Uo);
         }
-        const UT half_euler = (UT)(0.5 * c.euler);
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
-            if (rk != 3) U[m] = U[m] - half_euler * frf[m];
-            else U[m] = (UT)TBT * Uo[m] + (UT)OBT * (U[m] - UT(0.5) * frf[m]);
+            if (rk != 3) U[m] = U[m] - he * fr[m];
+            else U[m] = TBT * Uo[m] + OBT * (U[m] - 0.5 * fr[m]);
         }
-        if (kind == KIND_WALL) U[2] = 0;
-        const UT U2_rot = U[1], U3_rot = U[2];
-        U[1] = U2_rot * nyf + U3_rot * nxf;
-        U[2] = U3_rot * nyf - U2_rot * nxf;
-        const UT temp = UT(1) / U[0];
+        if (kind == KIND_WALL) U[2] = 0.0;
+        const double U2_rot = U[1], U3_rot = U[2];
+        U[1] = U2_rot * ny + U3_rot * nx;
+        U[2] = U3_rot * ny - U2_rot * nx;
+        const double temp = 1.0 / U[0];
         const float rho = (float)U[0];
         const float u1 = (float)(U[1] * temp);
         const float u2 = (float)(U[2] * temp);
-        const float pr = (float)(UT(0.4) * (U[3] - (UT(0.5) * temp) * (U[1] * U[1] + U[2] * U[2])));
+        const float pr = (float)(0.4 * (U[3] - (0.5 * temp) * (U[1] * U[1] + U[2] * U[2])));
         b.prim_out[i] = make_float4(rho, u1, u2, pr);
         float qn[4];
         q_from_prim_t<float>(rho, u1, u2, pr, qn);
         b.q_out[i] = make_float4(qn[0], qn[1], qn[2], qn[3]);
         if (last) b.spd[i] = (double)(sqrtf(u1 * u1 + u2 * u2) + 3.0f * sqrtf(pr / rho));
+        return res_sqr;
     }
-    return res_sqr;
-}
+};
 
-// Each warp walks chunks of two scheduled tiles with a stride of all warps of
-// the grid; tile partials as in the FP64 pass.
 __global__ void __launch_bounds__(FLUX_BLOCK, FLUX32_MIN_BLOCKS)
-kb_flux32(Geom g, Consts c, Sched s, StageBufs32 b, int rk, int last) {
-    __shared__ double sm[FLUX_WARPS * WARP_SMEM];
-    __shared__ SchedSmem ss;
-    load_sched(s, ss);  // the kernel's only block barrier
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    double *rec = sm + warp * WARP_SMEM;
-    double *wG = rec + PPW * GROUP_SMEM;
-    double *wres = wG + CHUNK * GST;
-    const int ntiles = ss.pre[ss.nact];
-    const int nchunks = (ntiles + CT - 1) / CT;
-    for (int ch = blockIdx.x * FLUX_WARPS + warp; ch < nchunks; ch += gridDim.x * FLUX_WARPS) {
-        for (int rnd = 0; rnd < CHUNK / PPW; ++rnd) {
-            const int pj = rnd * PPW + lane / LPP;
-            const int v = CT * ch + pj / TILE;
-            bool valid = false;
-            int i = 0, kind = KIND_INTERIOR;
-            if (v < ntiles) {
-                const TileRef t = sched_tile(s, ss, v);
-                const int j = t.j0 + (pj % TILE);
-                valid = j < t.n;
-                i = t.base + j;
-                kind = j < t.nw ? KIND_WALL : (j < t.nw + t.no ? KIND_OUTER : KIND_INTERIOR);
-            }
-            flux32_group(g, c, b, i, valid, kind, rec + (lane / LPP) * GROUP_SMEM, wG + GST * pj);
-        }
-        __syncwarp();
-        const int v = CT * ch + lane / TILE;  // lanes past the chunk idle here
-        const bool inchunk = lane < CHUNK && v < ntiles;
-        const TileRef t = sched_tile(s, ss, inchunk ? v : CT * ch);
-        const int j = t.j0 + (lane % TILE);
-        const bool valid = inchunk && j < t.n;
-        double rs = 0.0;
-        if (valid) {
-            const int kind = j < t.nw ? KIND_WALL : (j < t.nw + t.no ? KIND_OUTER : KIND_INTERIOR);
-            rs = update32_point(g, c, b, rk, last, t.base + j, kind, t.obc_off + j - t.nw,
-                                wG + GST * lane);
-        }
-        if (last) {
-            if (lane < CHUNK) wres[lane] = rs;
-            __syncwarp();
-            if ((lane % TILE) == 0 && inchunk) {
-                double acc = 0.0;
-                for (int q = 0; q < TILE; ++q) acc = acc + wres[lane + q];
-                b.res_part[t.tile] = acc;
-            }
-        }
-        __syncwarp();  // the next chunk reuses wG and wres
-    }
+kb_flux32(Geom g, Consts c, Sched s, StageBufs32 b, int rk, int last, int ct, int coop) {
+    extern __shared__ double2 fsm[];
+    Flux32 p{g, c, b, rk, last};
+    flux_pass(p, g, s, reinterpret_cast<Flux32Smem *>(fsm), b.res_part, last, ct, coop);
 }
 
 __global__ void k_init_state32(Geom g, const float4 *__restrict__ prim, float4 *__restrict__ q,
@@ -568,10 +625,11 @@ inline int nblk(int n, int b) { return (n + b - 1) / b; }
 
 
 cudaError_t init_kernels32() {
-    // the FP32 halo D pass stays below the default 48 KB of dynamic shared
-    // memory (at most 25 KB); nothing to set
+    // within the default 48 KB of dynamic shared memory: nothing to set
+    static_assert(FLUX32_SMEM <= 48 * 1024, "");
     return cudaSuccess;
 }
+int flux32_per_sm() { return FLUX32_MIN_BLOCKS; }
 
 namespace {
 // dynamic shared memory of the halo kernels at staging stride hc
@@ -588,8 +646,8 @@ int halo32_wave(int kind, int hc) {
 }
 }  // namespace
 
-// the flux pass's shared memory is static (independent of the stencil size)
-size_t flux32_smem_bytes(int) { return 0; }
+// the flux pass's shared memory does not depend on the stencil size
+size_t flux32_smem_bytes(int) { return FLUX32_SMEM; }
 
 int batch_occupancy32(int kind, int block, size_t smem) {
     int nb = 0;
@@ -630,9 +688,10 @@ void launch_inner32(const Geom &g, const Consts &c, const Geom32 &f, const Sched
 }
 
 void launch_flux32(const Geom &g, const Consts &c, const Sched &s, const StageBufs32 &b,
-                         int rk, bool last, int grid, cudaStream_t st) {
-    kb_flux32<<<wave32(2, FLUX_BLOCK, 0, grid), FLUX_BLOCK, 0, st>>>(g, c, s, b, rk,
-                                                                     last ? 1 : 0);
+                         int rk, bool last, int grid, int tiles, cudaStream_t st) {
+    const FluxShape f = flux_shape(tiles, FLUX32_MIN_BLOCKS);
+    kb_flux32<<<wave32(2, FLUX_BLOCK, FLUX32_SMEM, grid), FLUX_BLOCK, FLUX32_SMEM, st>>>(
+        g, c, s, b, rk, last ? 1 : 0, f.ct, f.coop);
 }
 
 void launch_init_state32(const Geom &g, const float4 *prim, float4 *q, double *spd,

@@ -23,6 +23,7 @@
 
 #include "batch.cuh"
 #include "flux_math.cuh"
+#include "flux_tile.cuh"
 #include "halo.cuh"
 #include "primal.h"
 
@@ -31,8 +32,6 @@ namespace lskum {
 namespace {
 
 constexpr int GRAD_BLOCK = 256;  // blocks of the per-point set-up kernels
-constexpr int LPP = 8;                   // lanes per point in the flux pass
-constexpr int FLUX_BLOCK = 128;          // four independent warps
 // 4 blocks: 128 registers a thread and all of shared memory but 3.5 KB; at 3
 // (168 registers) 0.420 ms at 1.024M points against 0.389
 constexpr int FLUX_MIN_BLOCKS = 4;
@@ -344,10 +343,6 @@ kb_grad_h(Geom g, Consts c, Sched s, const R4 *__restrict__ q, const double *__r
 // once per grid (k_flux_coef).  The flux residual is the sum of the list
 // derivatives, so the lists need not be told apart: a lane adds both
 // directions' terms into four sums and eight lanes add theirs by shuffles.
-constexpr int PPW = 32 / LPP;          // points per warp round
-constexpr int FLUX_WARPS = FLUX_BLOCK / 32;
-constexpr int CHUNK_MAX = 2 * TILE;    // points of a chunk
-
 // Per point and split list L: a, b of the list's solve (fco[8 i + 2 L]).
 // *_fluxes.F90 dG*: the sums in slot order; a list the point's kind does not
 // have (wall ypos, outer yneg) and empty rows get zeros.
@@ -387,18 +382,6 @@ __global__ void k_flux_coef(Geom g, int base, int n, int nw, int no, double powe
     }
 }
 
-// Sum of v over the eight lanes of a point: component 2 (bit 2) + (bit 1) of
-// the lane, in a fixed order.
-__device__ __forceinline__ double reduce8(const double v[4], int lane) {
-    const unsigned full = 0xffffffffu;
-    const bool h4 = lane & 4, h2 = lane & 2;
-    const double s0 = __shfl_xor_sync(full, h4 ? v[0] : v[2], 4);
-    const double s1 = __shfl_xor_sync(full, h4 ? v[1] : v[3], 4);
-    const double a0 = (h4 ? v[2] : v[0]) + s0, a1 = (h4 ? v[3] : v[1]) + s1;
-    const double b = (h2 ? a1 : a0) + __shfl_xor_sync(full, h2 ? a0 : a1, 2);
-    return b + __shfl_xor_sync(full, b, 1);
-}
-
 // Shared memory of the unit that computes a tile (a warp, or in the shared
 // split the block): the tile's halo rows (halo.cuh) as one array per 16-byte
 // piece -- q 0-1, dq 2-5, qm 6-9, (x, y) 10 -- at a fixed stride, so that a
@@ -412,77 +395,19 @@ struct FluxSmem {
     static constexpr int ROWS = 60, HC = ROWS + 1;
     double2 halo[11][HC];
     double eps[HC + 1];
-    double2 nrm[TILE];
-    uint4 mask[TILE];              // xpos, xneg, ypos, yneg
     double2 co[TILE][4];
-    unsigned char loc[TILE * 16];  // hloc rows (of up to 16 bytes)
-    int nbhs[TILE];
-    double G[CHUNK_MAX][4];        // flux residuals, then residual terms
+    FluxOwn own;
+    double G[CHUNK_MAX][4];  // flux residuals, then residual terms
 };
 constexpr int FLUX_SMEM = FLUX_WARPS * sizeof(FluxSmem);
-
-// A scheduled tile: its first point, the points in it (0: no such tile), and
-// the numbers of its points up to which they are wall and outer points.
-struct FluxTile {
-    int i0 = 0, cnt = 0, wall = 0, outer = 0, tile = 0;
-    __device__ __forceinline__ FluxTile() {}
-    __device__ __forceinline__ FluxTile(const Sched &s, int ntiles, int v) {
-        if (v >= ntiles) return;
-        const TileRef t = sched_tile_global(s, v);
-        i0 = t.base + t.j0;
-        cnt = min(TILE, t.n - t.j0);
-        wall = t.nw - t.j0;
-        outer = t.nw + t.no - t.j0;
-        tile = t.tile;
-    }
-    __device__ __forceinline__ int kind(int j) const {
-        return j < wall ? KIND_WALL : (j < outer ? KIND_OUTER : KIND_INTERIOR);
-    }
-};
-
-// The row indices of a tile's halo: lane l holds rows l and l + 32.
-struct FluxHalo {
-    int h0 = 0, hn = 0, k0 = 0, k1 = 0;  // hn 0: no tile, or not staged
-    __device__ __forceinline__ void range(const Geom &g, const FluxTile &t) {
-        h0 = hn = 0;
-        if (t.cnt == 0) return;
-        h0 = __ldg(g.hoff + t.tile);
-        hn = __ldg(g.hoff + t.tile + 1);
-    }
-    __device__ __forceinline__ void rows(const Geom &g, int lane) {
-        hn = hn - h0 <= FluxSmem::ROWS ? hn - h0 : 0;
-        k0 = lane < hn ? __ldg(g.hrow + h0 + lane) : 0;
-        k1 = lane + 32 < hn ? __ldg(g.hrow + h0 + 32 + lane) : 0;
-    }
-    // row u (u / 32 the same for the whole warp)
-    __device__ __forceinline__ int row(int u) const {
-        return __shfl_sync(0xffffffffu, u < 32 ? k0 : k1, u & 31);
-    }
-};
-
-// Copies NP 16-byte pieces of every halo row of an array with the NT threads
-// of the unit, tid of them this one; whole warps.
-template <int NP, int NT>
-__device__ __forceinline__ void stage_rows(const void *src, const FluxHalo &x, double2 *dst,
-                                           int tid) {
-#pragma unroll
-    for (int t = 0; t < HALO_CAP * NP / NT; ++t) {
-        if (NT * t >= NP * x.hn) break;
-        const int u = (NT / NP) * t + tid / NP, part = tid % NP;
-        const int k = x.row(u);
-        if (u < x.hn)
-            halo_cp16(dst + part * FluxSmem::HC + u,
-                      static_cast<const char *>(src) + (size_t)(unsigned)(k * NP + part) * 16);
-    }
-}
 
 // Copies a tile's rows (cp.async).
 template <int NT>
 __device__ __forceinline__ void stage_flux(const Geom &g, const StageBufs &b, const FluxTile &t,
                                            const FluxHalo &x, FluxSmem &m, int tid) {
-    stage_rows<2, NT>(b.q_in, x, m.halo[0], tid);
-    stage_rows<4, NT>(b.dq, x, m.halo[2], tid);
-    stage_rows<4, NT>(b.qm, x, m.halo[6], tid);
+    stage_rows<2, NT, FluxSmem::HC>(b.q_in, x, m.halo[0], tid);
+    stage_rows<4, NT, FluxSmem::HC>(b.dq, x, m.halo[2], tid);
+    stage_rows<4, NT, FluxSmem::HC>(b.qm, x, m.halo[6], tid);
     if (tid < HALO_CAP) {
 #pragma unroll
         for (int u0 = 0; u0 < HALO_CAP; u0 += NT < HALO_CAP ? NT : HALO_CAP) {
@@ -500,21 +425,7 @@ __device__ __forceinline__ void stage_flux(const Geom &g, const StageBufs &b, co
         const int pc = q * NT + tid;
         if (pc < 4 * t.cnt) halo_cp16(&m.co[pc >> 2][pc & 3], co + pc);
     }
-    if (g.hkp <= 16 && tid < g.hkp / 8 * t.cnt)
-        halo_cp8(m.loc + 8 * tid, g.hloc + (size_t)t.i0 * g.hkp + 8 * tid);
-    if (tid < 2 * TILE) {
-        const int j = tid % TILE;
-        if (j < t.cnt) {
-            double *d = reinterpret_cast<double *>(&m.mask[j]);
-            if (tid < TILE) {
-                halo_cp16(&m.nrm[j], g.nrm + t.i0 + j);
-                halo_cp8(d, g.mx + t.i0 + j);
-            } else {
-                halo_cp4(&m.nbhs[j], g.nbhs + t.i0 + j);
-                halo_cp8(d + 1, g.my + t.i0 + j);
-            }
-        }
-    }
+    m.own.stage<NT>(g, t, tid);
 }
 
 // A row in registers: staged (row l of the halo) or from global memory.
@@ -560,19 +471,17 @@ __device__ __forceinline__ void flux_group(const Geom &g, const StageBufs &b, co
     const double inv_sqrt_pi = 0.56418958354775628695;
     const int kind = t.kind(j), i = t.i0 + j;
     double v[4] = {0.0, 0.0, 0.0, 0.0};
-    const double2 nn = m.nrm[j];
+    const double2 nn = m.own.nrm[j];
     const double nx = nn.x, ny = nn.y;
-    const int nb = j < t.cnt ? m.nbhs[j] : 0;
+    const int nb = j < t.cnt ? m.own.nbhs[j] : 0;
     for (int r = lane; r < nb; r += LPP) {
         KState sk, si;
         double ui[2], uk[2], delx, dely;
         {
             double qk[4], qi[4];
             if (hn > 0) {
-                const unsigned char *gl = g.hloc + (size_t)i * g.hkp, *ml = m.loc + j * g.hkp;
-                const bool in = g.hkp <= 16;
-                const int lk = in ? ml[r] : __ldg(gl + r);
-                const int li = in ? ml[g.hkp - 1] : __ldg(gl + g.hkp - 1);
+                int lk, li;
+                m.own.rows(g, i, j, r, lk, li);
                 const double2 pi_ = m.halo[10][li], pk = m.halo[10][lk];
                 delx = pk.x - pi_.x;
                 dely = pk.y - pi_.y;
@@ -612,7 +521,7 @@ __device__ __forceinline__ void flux_group(const Geom &g, const StageBufs &b, co
         }
         // Per direction the neighbour is in one list of the pair, in both only
         // when its projection is exactly 0: the second list is added then.
-        const uint4 mm = m.mask[j];
+        const uint4 mm = m.own.mask[j];
         const double w6i = fma(6.0, si.pbr, si.usq), w6k = fma(6.0, sk.pbr, sk.usq);
         auto add_x = [&](int l, double sg) {
             const double2 co = m.co[j][l];
@@ -709,90 +618,32 @@ update_point(const Geom &g, const Consts &c, const StageBufs &b, int rk, int las
     return res_sqr;
 }
 
-// F pass over chunks of `ct` (1 or 2) scheduled tiles.  COOP = false: a warp
-// owns a chunk, computes its points four at a time and updates them with one
-// lane each, with no block barrier.  COOP = true: the block's four warps
-// share a chunk (each a quarter of its points) and its first warp updates it
-// after a barrier.  Both call the same functions on a point, so the split
-// does not change a result.  A tile never straddles two instances and its
-// partial lands in slot (instance's first tile + tile number), summed over
-// its 16 points in point order, so an instance's residual sums do not depend
-// on the other instances or on the launch shape.
-//
-// A tile's rows come through shared memory: its halo (54 rows a 16-point tile
-// of an O-grid, against 144 row reads) is copied with cp.async, the row
-// indices a tile ahead.
+template <bool TAPE>
+struct Flux64 {
+    using Smem = FluxSmem;
+    const Geom &g;
+    const Consts &c;
+    const StageBufs &b;
+    int rk, last;
+    template <int NT>
+    __device__ __forceinline__ void stage(const FluxTile &t, const FluxHalo &x, Smem &m, int tid) {
+        stage_flux<NT>(g, b, t, x, m, tid);
+    }
+    __device__ __forceinline__ void group(const FluxTile &t, int j, int hn, Smem &m, double *G) {
+        flux_group<TAPE>(g, b, t, j, hn, m, G);
+    }
+    __device__ __forceinline__ double update(int i, int kind, int orow, const double *G) {
+        return update_point(g, c, b, rk, last, i, kind, orow, G);
+    }
+};
+
+// F pass (flux_pass).
 template <bool TAPE>
 __global__ void __launch_bounds__(FLUX_BLOCK, FLUX_MIN_BLOCKS)
 kb_flux(Geom g, Consts c, Sched s, StageBufs b, int rk, int last, int ct, int coop) {
     extern __shared__ double2 fsm[];
-    const int ntiles = __ldg(s.pre + __ldg(s.nact));
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    FluxSmem &m = reinterpret_cast<FluxSmem *>(fsm)[coop ? 0 : warp];
-    const int nchunks = (ntiles + ct - 1) / ct, pts = ct * TILE;
-    const int jw = coop ? warp * PPW : 0, nj = coop ? PPW : TILE;  // the warp's points of a tile
-    const int step = coop ? gridDim.x : gridDim.x * FLUX_WARPS;
-    int ch = coop ? blockIdx.x : blockIdx.x * FLUX_WARPS + warp, u = 0;
-    if (ch >= nchunks) return;  // (coop: the whole block)
-    FluxTile cur(s, ntiles, ct * ch);
-    FluxHalo hx;
-    hx.range(g, cur);
-    hx.rows(g, lane);
-    auto stage = [&] {
-        if (coop) stage_flux<FLUX_BLOCK>(g, b, cur, hx, m, threadIdx.x);
-        else stage_flux<32>(g, b, cur, hx, m, lane);
-    };
-    auto sync = [&] {
-        if (coop) __syncthreads();
-        else __syncwarp();
-    };
-    stage();
-    while (true) {
-        const int hn = hx.hn, done = ct * ch;  // the chunk's first tile
-        const bool end = u + 1 == ct;
-        if (end) ch += step;
-        // the tile after this one: its halo's range now, its row indices once
-        // that has come (after the first round)
-        const FluxTile nxt(s, ntiles, end ? ct * ch : done + u + 1);
-        hx.range(g, nxt);
-        halo_wait();
-        sync();
-        for (int rnd = 0; rnd < nj; rnd += PPW) {
-            const int j = jw + rnd + lane / LPP;
-            flux_group<TAPE>(g, b, cur, j, hn, m, m.G[u * TILE + j]);
-            if (rnd == 0) hx.rows(g, lane);
-        }
-        sync();
-        // the next tile's rows are on their way while this chunk is updated
-        cur = nxt;
-        stage();
-        u = end ? 0 : u + 1;
-        if (!end) continue;
-        // the chunk's state updates, one point per lane
-        if (!coop || warp == 0) {
-            const int v = done + lane / TILE;
-            const bool tile = lane < pts && v < ntiles;
-            const TileRef t = sched_tile_global(s, tile ? v : done);
-            const int j = t.j0 + (lane % TILE);
-            double rs = 0.0;
-            if (tile && j < t.n) {
-                const int kind =
-                    j < t.nw ? KIND_WALL : (j < t.nw + t.no ? KIND_OUTER : KIND_INTERIOR);
-                rs = update_point(g, c, b, rk, last, t.base + j, kind, t.obc_off + j - t.nw,
-                                  m.G[lane]);
-            }
-            if (last) {
-                m.G[lane][0] = rs;
-                __syncwarp();
-                if ((lane % TILE) == 0 && tile) {
-                    double acc = 0.0;
-                    for (int q = 0; q < TILE; ++q) acc = acc + m.G[lane + q][0];
-                    b.res_part[t.tile] = acc;
-                }
-            }
-        }
-        if (ch >= nchunks) break;
-    }
+    Flux64<TAPE> p{g, c, b, rk, last};
+    flux_pass(p, g, s, reinterpret_cast<FluxSmem *>(fsm), b.res_part, last, ct, coop);
 }
 
 // Sum of nparts tile partials in a fixed order (deterministic, independent
@@ -1010,29 +861,26 @@ int sm_count() {
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     return std::max(sms, 1);
 }
-// Split of the FP64 flux pass for `tiles` scheduled tiles.  Up to one tile a
-// resident block, the block's warps share the tile (a round each): 11.4 us
-// against 16.4 at 4,000 points, 17.9 both at 16,000.  Beyond that a warp
-// takes chunks of one tile or, for less idle lanes in the updates (1.15
-// times the rate), of two, whichever its whole number of turns makes cheaper:
-// one against two tiles 45.8 / 52.2 us at 91,000 points, 38.6 / 37.6 at
-// 64,000, 112 / 105 at 256,000, 417 / 389 at 1,024,000.
-struct FluxShape {
-    int ct, coop;
-};
-FluxShape flux_shape(int tiles) {
-    const int blocks = sm_count() * FLUX_MIN_BLOCKS, warps = blocks * FLUX_WARPS;
+}  // namespace
+
+// Split of a flux pass for `tiles` scheduled tiles (`per_sm` resident blocks).
+// Up to one tile a resident block, the block's warps share the tile (a round
+// each): FP64 11.4 us against 16.4 at 4,000 points, 17.9 both at 16,000.
+// Beyond that a warp takes chunks of one tile or, for less idle lanes in the
+// updates (1.15 times the rate), of two, whichever its whole number of turns
+// makes cheaper: FP64, one against two tiles, 45.8 / 52.2 us at 91,000
+// points, 38.6 / 37.6 at 64,000, 112 / 105 at 256,000, 417 / 389 at 1,024,000.
+FluxShape flux_shape(int tiles, int per_sm) {
+    const int blocks = sm_count() * per_sm, warps = blocks * FLUX_WARPS;
     if (tiles <= blocks) return FluxShape{1, 1};
     const double one = 1.15 * nblk(tiles, warps), two = 2.0 * nblk(tiles, 2 * warps);
     return FluxShape{one < two ? 1 : 2, 0};
 }
-}  // namespace
 
 // flux-pass blocks that give every chunk its warp (or its block)
 int flux_grid_blocks(int n, bool fp32) {
     const int tiles = nblk(n, TILE);
-    if (fp32) return nblk(tiles, 2 * FLUX_WARPS);
-    const FluxShape f = flux_shape(tiles);
+    const FluxShape f = flux_shape(tiles, fp32 ? flux32_per_sm() : FLUX_MIN_BLOCKS);
     return nblk(nblk(tiles, f.ct), f.coop ? 1 : FLUX_WARPS);
 }
 
@@ -1129,7 +977,7 @@ void launch_inner(const Geom &g, const Consts &c, const Sched &s, const double *
 
 void launch_flux(const Geom &g, const Consts &c, const Sched &s, const StageBufs &b, int rk,
                  bool last, int grid, int tiles, cudaStream_t st) {
-    const FluxShape f = flux_shape(tiles);
+    const FluxShape f = flux_shape(tiles, FLUX_MIN_BLOCKS);
     const int gr = wave(2, FLUX_BLOCK, 0, grid);
     constexpr int sm = FLUX_SMEM;
     if (b.kstape)

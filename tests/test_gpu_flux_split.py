@@ -39,3 +39,31 @@ def test_flux_pass_paths(ni, nj, flow):
     assert np.allclose(r, ref, rtol=0, atol=1e-9)
     assert max_rel(got, o.prim()) < 1e-10
     o.close()
+
+
+@pytest.mark.parametrize("ni,nj,jitter", [
+    (16, 9, 0.1),      # 9 tiles
+    (33, 17, 0.1),     # a last tile of one point
+    (120, 98, 0.1),    # 735 tiles: a block a tile on 148 SMs
+    (120, 99, 0.1),    # 743: a warp a tile
+    (240, 197, 0.1),   # 2,955: one turn
+    (240, 198, 0.1),   # 2,970: two turns, or two tiles a warp
+    (62, 24, 0.0),     # ties
+])
+def test_fp32_flux_pass_paths(ni, nj, jitter):
+    """flux_res of one stage against the FP64 pass.  Each of the up to 8 slots
+    of a point adds the rounding (6e-8, about ten roundings deep) of two
+    fluxes of order one times delta |c| (the time step over the spacing, at
+    most about 0.1, twice that on the wall): 2e-6."""
+    g = naca_ogrid(ni, nj, seed=7, first_spacing=5e-3, jitter=jitter)
+    wave = 0.05 * np.sin(3 * g.x + 2 * g.y)[:, None] * np.array([1, .5, .3, 1.4])
+    prim = np.array([1, 0.8, 0.01, 1 / 1.4]) * (1 + wave)
+    got = {}
+    for precision in ("fp64", "fp32_mixed"):
+        with Solver(g, cfl=0.2, vl_const=5.0, mach=0.8, aoa=1.5, tscheme="first",
+                    precision=precision) as s:
+            s.keep_diagnostics(True)
+            s.set_state(prim)
+            s.run(1)
+            got[precision] = s.get_array("flux_res")
+    assert np.max(np.abs(got["fp32_mixed"] - got["fp64"])) < 2e-6
