@@ -9,8 +9,8 @@ namespace lskum {
 
 constexpr int ADJ_CW = 22;  // contribution record per (point, slot)
 // flux pass: per (point, slot) the neighbour side's record (adjoint of its
-// reconstructed u1, u2, rho, p; its rho; delx/dely adjoint; padding)
-constexpr int NBREC = 8;
+// limited qtilde, delx/dely adjoint)
+constexpr int NBREC = 6;
 // q-derivative pass: per point the record its neighbours' side reads
 constexpr int GREC = 24;
 enum { ADJ_GATHER_INNER = 1, ADJ_GATHER_GRAD = 2 };
@@ -35,13 +35,13 @@ struct AdjGather {
     const int *nptr, *nsrc;  // normals: 2 j + role, per boundary point
 };
 
-cudaError_t init_adjoint_kernels();
 void launch_update_b(const Geom &g, const Consts &c, const AdjConsts &a, const R4 *prim_in,
                      const R4 *prim_old, const R4 *fr, const double *pb_out, double *pb_in,
                      double *pb_old, double *frb, double *nxb, double *nyb, int rk,
                      cudaStream_t s);
-// kst: the stage's kinetic-state tape of the forward re-run ([n][kp][KS_TAPE],
-// written by the flux pass with StageBufs::kstape), or nullptr to recompute
+// fr: the stage's taped flux residual; kst: its kinetic-state tape of the
+// forward re-run ([n][kp][KS_TAPE], written by the flux pass with
+// StageBufs::kstape), or nullptr to recompute.
 // The flux pass reverses in two kernels: k_flux_b per point (its fluxes,
 // kinetic states and own reconstruction; writes nbrec [n][kp][NBREC]) and
 // k_flux_b_nbr per neighbour over the transposed stencil (the neighbour's
@@ -49,8 +49,8 @@ void launch_update_b(const Geom &g, const Consts &c, const AdjConsts &a, const R
 // belong to the point as well), then k_back_sum adds those to the point.
 // nbrec and back may share the contribution buffer (n*kp*(NBREC+2) <=
 // n*kp*ADJ_CW doubles).
-void launch_flux_b(const Geom &g, const Consts &c, const R4 *q_in, const double *dq,
-                   const double *qm, const double *delta, const double *frb, double *qb,
+void launch_flux_b(const Geom &g, const R4 *q_in, const double *dq, const double *qm,
+                   const double *delta, const R4 *fr, const double *frb, double *qb,
                    double *dqb, double *qmb, double *xb, double *yb, double *nxb, double *nyb,
                    double *deltab, double *nbrec, double *back, const int *tptr,
                    const int *tlist, const double *kst, cudaStream_t s);

@@ -50,6 +50,7 @@ struct AdjointState {
     // kinetic-state tape of the re-run (rks stages of [n][kp][KS_TAPE]); null
     // when it did not fit, and the reverse flux pass recomputes the states
     double *tks = nullptr;
+    double *d_fcg = nullptr;
     double *hist = nullptr;
     int hist_cap = 0;
     std::vector<R4 *> snaps;  // snapshot rows (n points each) in one device block
@@ -204,8 +205,11 @@ int adj_setup(mfcfd_t *h) {
     }
     CK(dmalloc(&a->snap0, n));
     CK(dmalloc(&a->fin, n));
-    cudaError_t e = init_adjoint_kernels();
-    if (e != cudaSuccess) return cuda_fail(h, e, "init_adjoint_kernels");
+    // the third entry of every list's inverse normal matrix (Geom::fcg)
+    CK(dmalloc(&a->d_fcg, (size_t)4 * n));
+    launch_flux_coef(h->geom, 0, n, h->nw, h->no, 0.0, h->d_fco, nullptr, a->d_fcg, h->stream);
+    CK(cudaGetLastError());
+    h->geom.fcg = a->d_fcg;
     return MFCFD_OK;
 }
 
@@ -286,11 +290,9 @@ int reverse_taped(mfcfd_t *h, AdjointState *a) {
         if (rk != 1) CK(cudaMemsetAsync(pb_in, 0, sizeof(double) * 4 * n, s));
         launch_update_b(h->geom, h->consts, ac, a->tprim[rk - 1], a->tprim[0], a->tfr[rk - 1],
                         pb_out, pb_in, a->pbA, a->frb, a->nxb, a->nyb, rk, s);
-        CK(cudaMemsetAsync(a->qb, 0, sizeof(double) * 4 * n, s));
-        CK(cudaMemsetAsync(a->qmb, 0, sizeof(double) * 8 * n, s));
-        CK(cudaMemsetAsync(a->dqb[m & 1], 0, sizeof(double) * 8 * n, s));
-        launch_flux_b(h->geom, h->consts, a->tq[rk - 1], dq_at(a, rk, m), qm_at(a, rk), a->tdelta,
-                      a->frb, a->qb, a->dqb[m & 1], a->qmb, a->xb, a->yb, a->nxb, a->nyb,
+        // (writes qb, qmb and dqb[m & 1])
+        launch_flux_b(h->geom, a->tq[rk - 1], dq_at(a, rk, m), qm_at(a, rk), a->tdelta,
+                      a->tfr[rk - 1], a->frb, a->qb, a->dqb[m & 1], a->qmb, a->xb, a->yb, a->nxb, a->nyb,
                       a->deltab, a->contrib, a->contrib + (size_t)n * a->kp * NBREC, a->d_tptr,
                       a->d_tlist, ks_at(a, rk), s);
         for (int t = m; t >= 1; --t) {
@@ -390,7 +392,7 @@ void lskum_host::free_adjoint(mfcfd_t *h) {
                     a->d_nsrc, a->tdq, a->tqm, a->tdelta, a->tspd,
                     a->pb[0], a->pb[1], a->pbA, a->qb, a->dqb[0], a->dqb[1], a->qmb,
                     a->deltab, a->frb, a->xb, a->yb, a->nxb, a->nyb, a->contrib, a->hist,
-                    a->snap0, a->fin, a->tks};
+                    a->snap0, a->fin, a->tks, a->d_fcg};
     for (void *b : bufs)
         if (b) cudaFree(b);
     for (int s = 0; s < 5; ++s) {

@@ -22,6 +22,7 @@
 #include <algorithm>
 
 #include "adjoint.h"
+#include "flux_tile.cuh"
 #include "lskum_adjoint.cuh"
 
 namespace lskum {
@@ -29,9 +30,7 @@ namespace lskum {
 namespace {
 
 constexpr int BLK = 128;
-constexpr int LPP = 8;
 constexpr int GROUPS = BLK / LPP;
-constexpr int BREC = 44;  // dG[16] dels deln si[9] sk[9] prim_i[4] prim_k[4]
 constexpr double OBT = 1.0 / 3.0;
 constexpr double TBT = 2.0 / 3.0;
 
@@ -50,12 +49,8 @@ __device__ __forceinline__ void ld4nc(const double *p, double v[4]) {
         : "l"(p));
 }
 
-__device__ __forceinline__ void kst_store(double *e, const KState &s) {
-    e[0] = s.rho; e[1] = s.ut; e[2] = s.un; e[3] = s.pbr; e[4] = s.usq;
-    e[5] = s.B1; e[6] = s.B2; e[7] = s.e1; e[8] = s.e2;
-}
 // A kinetic state from its tape entry (rho, p/rho, B1, B2, e1, e2, u1, u2)
-// and the point's normal, as reconstruct_kstate forms ut, un and |u|^2.
+// and the point's normal, as kstate_pair forms ut, un and |u|^2.
 __device__ __forceinline__ KState kst_taped(const double *v, double nx, double ny) {
     KState s;
     const double tx = ny, ty = -nx;
@@ -67,16 +62,9 @@ __device__ __forceinline__ KState kst_taped(const double *v, double nx, double n
     s.e2 = v[5];
     s.ut = v[6] * tx + v[7] * ty;
     s.un = v[6] * nx + v[7] * ny;
-    s.usq = s.ut * s.ut + s.un * s.un;
+    s.usq = fma(v[6], v[6], v[7] * v[7]);
     return s;
 }
-__device__ __forceinline__ KState kst_load(const double *e) {
-    KState s;
-    s.rho = e[0]; s.ut = e[1]; s.un = e[2]; s.pbr = e[3]; s.usq = e[4];
-    s.B1 = e[5]; s.B2 = e[6]; s.e1 = e[7]; s.e2 = e[8];
-    return s;
-}
-
 // state_update_b (state_update.F90:10-141, reverse)
 // Stores n (even) doubles as 16-byte pairs; dst is 16-byte aligned (records
 // are ADJ_CW = 22 doubles = 176 bytes from an aligned base).
@@ -193,306 +181,326 @@ k_update_b(Geom g, Consts c, AdjConsts a, const R4 *__restrict__ prim_in,
     nyb[i] += nybv;
 }
 
-// cal_flux_residual_b: same lane layout as the forward flux pass.
-#ifndef FLUXB_MIN_BLOCKS
-#define FLUXB_MIN_BLOCKS 3  // 168 registers; 4 blocks (128) spill (C3: 6.39 against 6.68 ms per reversed iteration)
-#endif
+// cal_flux_residual_b, eight lanes a point, one slot a lane, as in the forward
+// flux pass.  With the list solves folded into slot weights (c = p . d, p the
+// list's two coefficients, d = (dels, deln)), the flux residual is coef times
+// the sum of c dG over slots and lists, so its reverse needs no list sums of
+// the fluxes: with F = coef times the residual's adjoint, a slot's fluxes
+// receive c F (the neighbour's) and -c F (the point's), and c receives F . dG.
+// The time step's adjoint is the residual's dotted with the taped residual
+// over the step.  The weights' own adjoint goes back through M p = e (M = sum
+// d d^T over the list): with pb = sum cb d and z = M^-1 pb, each d receives
+// -z c - p (z . d), two numbers a list summed over the point's lanes.
+//
+// Everything a warp's round reads but the neighbours' coordinates is copied to
+// shared memory (cp.async) at its start, so the loads' latency is met once.
+// Bound by latency: 488 us at 256,000 points when the list sums and the
+// reconstructions' primitive states went through shared-memory records, 404
+// with the folded weights, 226 with the copies; 3 blocks (168 registers)
+// against 269 us at 4 (spills).
+constexpr int FLUXB_MIN_BLOCKS = 3;
+// A warp's shared memory: the taped states of its 32 slots (128 bytes padded
+// to 144: a lane's pieces on distinct banks), its four points' rows, the
+// slots' partial offset adjoints, z of each list.
+struct FluxBSmem {
+    double2 tape[32][KS_TAPE / 2 + 1];
+    double2 q[4][2], dq[4][5], qm[4][5], co[4][4], fcg[4][2];
+    double part[4][20][4];
+    double z[4][8];
+};
 __global__ void __launch_bounds__(BLK, FLUXB_MIN_BLOCKS)
-k_flux_b(Geom g, Consts c, const R4 *__restrict__ q_in, const double *__restrict__ dq,
+k_flux_b(Geom g, const R4 *__restrict__ q_in, const double *__restrict__ dq,
          const double *__restrict__ qm, const double *__restrict__ delta,
-         const double *__restrict__ frb, double *__restrict__ qb, double *__restrict__ dqb,
-         double *__restrict__ qmb, double *__restrict__ xb, double *__restrict__ yb,
-         double *__restrict__ nxb, double *__restrict__ nyb, double *__restrict__ deltab,
-         double *__restrict__ nbrec, const double *__restrict__ kst) {
-    extern __shared__ double sm[];
-    __shared__ double lb[GROUPS][4][11];  // fx_b[4] fy_b[4] sdx2_b sdy2_b sdxy_b per list
-    const int grp = threadIdx.x / LPP, lane = threadIdx.x % LPP;
-    const int i = blockIdx.x * GROUPS + grp;
+         const double *__restrict__ fr, const double *__restrict__ frb, double *__restrict__ qb,
+         double *__restrict__ dqb, double *__restrict__ qmb, double *__restrict__ xb,
+         double *__restrict__ yb, double *__restrict__ nxb, double *__restrict__ nyb,
+         double *__restrict__ deltab, double *__restrict__ nbrec,
+         const double *__restrict__ kst) {
+    __shared__ FluxBSmem smem[BLK / 32];
+    FluxBSmem &m = smem[threadIdx.x / 32];
+    const int wl = threadIdx.x % 32, pg = wl / LPP, lane = wl % LPP;
+    const int i0 = (blockIdx.x * BLK + threadIdx.x - wl) / LPP;  // the warp's first point
+    const int i = i0 + pg;
     const bool valid = i < g.n;
-    double *rec = sm + (size_t)grp * g.kp * BREC;
-    int nb = 0, kind = KIND_INTERIOR;
-    unsigned long long mx = 0, my = 0;
-    double nx = 0.0, ny = 1.0;
-    double2 pi_ = make_double2(0.0, 0.0);
+    // copies
+    if (kst) {
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            const int pc = 32 * t + wl, slot = pc / 8, part = pc % 8;
+            const int p = i0 + slot / LPP, r = slot % LPP;
+            if (p < g.n && r < g.kp)
+                halo_cp16(&m.tape[slot][part], kst + ((size_t)p * g.kp + r) * KS_TAPE + 2 * part);
+        }
+    }
+    {
+        const int p = i0 + wl / 8, part = wl % 8;  // 8 pieces a point
+        if (p < g.n) {
+            const int h = part & 3;
+            if (part < 4) {
+                halo_cp16(&m.dq[wl / 8][h], dq + 8 * (size_t)p + 2 * h);
+                halo_cp16(&m.co[wl / 8][h], g.fco + 8 * (size_t)p + 2 * h);
+            } else {
+                halo_cp16(&m.qm[wl / 8][h], qm + 8 * (size_t)p + 2 * h);
+                if (h < 2)
+                    halo_cp16(&m.q[wl / 8][h], reinterpret_cast<const double *>(q_in + p) + 2 * h);
+                else halo_cp16(&m.fcg[wl / 8][h - 2], g.fcg + 4 * (size_t)p + 2 * (h - 2));
+            }
+        }
+    }
+    int nb = 0, kind = KIND_INTERIOR, k0 = 0;
+    double nx = 0.0, ny = 1.0, eps2 = 0.0, geo_old = 0.0;
+    double2 pi_ = make_double2(0.0, 0.0), pk0 = pi_;
+    uint4 mm = make_uint4(0, 0, 0, 0);
+    double F[4] = {0.0, 0.0, 0.0, 0.0};
+    double *geo = (lane & 4 ? (lane & 2 ? nyb : nxb) : (lane & 2 ? yb : xb)) + i;
     if (valid) {
         nb = g.nbhs[i];
+        if (lane < g.kp) k0 = g.conn[(size_t)lane * g.n + i];  // (unused slots name i)
         kind = i < g.nw ? KIND_WALL : (i < g.nw + g.no ? KIND_OUTER : KIND_INTERIOR);
-        mx = g.mx[i];
-        my = g.my[i];
+        const unsigned long long mx = g.mx[i], my = g.my[i];
+        mm = make_uint4((unsigned)mx, (unsigned)(mx >> 32), (unsigned)my, (unsigned)(my >> 32));
         const double2 nn = g.nrm[i];
         nx = nn.x;
         ny = nn.y;
         pi_ = g.xy[i];
-    }
-    const double s2q = kind == KIND_WALL ? -1.0 : 1.0;
-    // phase A: forward per slot
-    if (valid) {
-        for (int r = lane; r < nb; r += LPP) {
-            const int k = g.conn[r * g.n + i];
-            const double2 pk = g.xy[k];
-            const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
-            double e_[8];
-            KState si, sk;
-            if (kst) {
-                // the forward re-run taped both reconstructions of this slot
-                // (128 contiguous bytes, in four 256-bit loads)
-                const double *tp = kst + ((size_t)i * g.kp + r) * KS_TAPE;
-                double v[KS_TAPE];
+        eps2 = g.eps2[i];
+        if (!(lane & 1)) geo_old = *geo;
+        double b4[4];
+        ld4nc(frb + 4 * (size_t)i, b4);
+        const double dl = delta[i];
+        pk0 = g.xy[k0];
 #pragma unroll
-                for (int hh = 0; hh < KS_TAPE / 4; ++hh) ld4nc(tp + 4 * hh, v + 4 * hh);
-                si = kst_taped(v, nx, ny);
-                sk = kst_taped(v + 8, nx, ny);
-                e_[0] = v[6]; e_[1] = v[7]; e_[2] = si.rho; e_[3] = si.rho * si.pbr;
-                e_[4] = v[14]; e_[5] = v[15]; e_[6] = sk.rho; e_[7] = sk.rho * sk.pbr;
-            } else {
-                const R4 qv = ld4(q_in + i), kv = ld4(q_in + k);
-                const double qi[4] = {qv.a, qv.b, qv.c, qv.d}, qk[4] = {kv.a, kv.b, kv.c, kv.d};
-                double dxi[4], dyi[4], qmaxi[4], qmini[4], dxk[4], dyk[4], qmaxk[4], qmink[4];
-                ld8a(dq + 8 * (size_t)i, dxi, dyi);
-                ld8a(qm + 8 * (size_t)i, qmaxi, qmini);
-                ld8a(dq + 8 * (size_t)k, dxk, dyk);
-                ld8a(qm + 8 * (size_t)k, qmaxk, qmink);
-                reconstruct(qi, dxi, dyi, qmaxi, qmini, g.eps2[i], delx, dely, c.gm1, e_[0],
-                            e_[1], e_[2], e_[3]);
-                reconstruct(qk, dxk, dyk, qmaxk, qmink, g.eps2[k], delx, dely, c.gm1, e_[4],
-                            e_[5], e_[6], e_[7]);
-                si = kstate(e_[0], e_[1], e_[2], e_[3], nx, ny, c.pi);
-                sk = kstate(e_[4], e_[5], e_[6], e_[7], nx, ny, c.pi);
-            }
-            double *e = rec + r * BREC;
-            // one converged evaluation per direction and list holding the
-            // neighbour (two only at a zero projection), lists in ascending
-            // order, as in the forward kb_flux
-            for (int d = 0; d < 2; ++d) {
-                const unsigned long long bits = d == 0 ? mx : my;
-                const bool in0 = (bits >> r) & 1ull, in1 = (bits >> (r + 32)) & 1ull;
-                for (int pass = 0; pass < 2; ++pass) {
-                    if (pass == 0 ? !(in0 || in1) : !(in0 && in1)) continue;
-                    const int L = 2 * d + ((pass == 1 || !in0) ? 1 : 0);
-                    const double sg = (L & 1) ? -1.0 : 1.0;
-                    double Gi[4], Gk[4];
-                    if (d == 0) {
-                        if (kind == KIND_INTERIOR) {
-                            flux_gx(si, sg, Gi);
-                            flux_gx(sk, sg, Gk);
-                        } else {
-                            flux_quad(si, sg, s2q, Gi);
-                            flux_quad(sk, sg, s2q, Gk);
+        for (int c = 0; c < 4; ++c) F[c] = (kind == KIND_WALL ? 2.0 * dl : dl) * b4[c];
+        if (lane == 0) {
+            double f4[4];
+            ld4nc(fr + 4 * (size_t)i, f4);
+            deltab[i] += (b4[0] * f4[0] + b4[1] * f4[1] + (b4[2] * f4[2] + b4[3] * f4[3])) / dl;
+        }
+    }
+    const double2 *co = m.co[pg];
+    double pb[8] = {}, nxs = 0.0, nys = 0.0, acc[3] = {};
+    halo_wait();
+    __syncwarp();
+    const unsigned full = 0xffffffffu;
+    const int nbw = __reduce_max_sync(full, nb);
+    for (int r0 = 0; r0 < nbw; r0 += LPP) {
+        const int r = r0 + lane;
+        // a lane without a slot carries a zero adjoint through limited_b
+        double delx = 0.0, dely = 0.0, delxb = 0.0, delyb = 0.0, delsb = 0.0, delnb = 0.0;
+        double qtb[4] = {0.0, 0.0, 0.0, 0.0};
+        if (r < nb) {
+            const int k = r0 ? g.conn[(size_t)r * g.n + i] : k0;
+            const double2 pk = r0 ? g.xy[k] : pk0;
+            delx = pk.x - pi_.x;
+            dely = pk.y - pi_.y;
+            const double dels = delx * ny - dely * nx, deln = delx * nx + dely * ny;
+            // the lists holding the neighbour: one of each direction (lx, ly), in
+            // both only when its projection is exactly 0 (tx, ty)
+            const unsigned bit = 1u << r;
+            const int lx = mm.x & bit ? 0 : 1, ly = mm.z & bit ? 0 : 1;
+            const bool tx = mm.x & mm.y & bit, ty = mm.z & mm.w & bit;
+            const double2 px = co[lx], py = co[2 + ly];
+            const double cx = fma(px.x, dels, px.y * deln), cy = fma(py.x, deln, py.y * dels);
+            double cbx = 0.0, cby = 0.0, cbx1 = 0.0, cby1 = 0.0;
+            // the neighbour's state (h = 0), then the point's (h = 1), one at a
+            // time: both at once need more registers than three blocks leave
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                const double sgn = h ? -1.0 : 1.0;
+                KState s;
+                double u1, u2;
+                if (kst) {
+                    // the forward re-run taped both reconstructions of this slot
+                    double v[KS_TAPE / 2];
+                    const int o = h ? 0 : KS_TAPE / 2;
+                    if (r0 == 0) {
+#pragma unroll
+                        for (int c = 0; c < KS_TAPE / 4; ++c) {
+                            const double2 t = m.tape[wl][o / 2 + c];
+                            v[2 * c] = t.x;
+                            v[2 * c + 1] = t.y;
                         }
                     } else {
-                        flux_gy(si, sg, Gi);
-                        flux_gy(sk, sg, Gk);
+                        const double *tp = kst + ((size_t)i * g.kp + r) * KS_TAPE + o;
+                        ld4nc(tp, v);
+                        ld4nc(tp + 4, v + 4);
                     }
-                    for (int m = 0; m < 4; ++m) e[4 * L + m] = Gk[m] - Gi[m];
-                }
-            }
-            e[16] = delx * ny - dely * nx;
-            e[17] = delx * nx + dely * ny;
-            kst_store(e + 18, si);
-            kst_store(e + 27, sk);
-            for (int m = 0; m < 8; ++m) e[36 + m] = e_[m];
-        }
-    }
-    __syncwarp();
-    // phase B: list sums, forward G and the list-level adjoints
-    double Gv0 = 0.0, Gv1 = 0.0;
-    const int L = lane >> 1, c0 = (lane & 1) * 2;
-    const bool used = valid && !((kind == KIND_WALL && L == 2) || (kind == KIND_OUTER && L == 3));
-    const unsigned long long lbits = ((L < 2) ? mx : my) >> ((L & 1) ? 32 : 0);
-    double sdx2 = 0.0, sdy2 = 0.0, sdxy = 0.0, fx[2] = {0.0, 0.0}, fy[2] = {0.0, 0.0};
-    double obd = 0.0;
-    if (used) {
-        // the list's slots in slot order (lowest bit first): a lane loops
-        // over its own members only (nb <= 20)
-        unsigned rb = (unsigned)lbits & ((1u << nb) - 1u);
-        while (rb) {
-            const int r = __ffs(rb) - 1;
-            rb &= rb - 1u;
-            const double *e = rec + r * BREC;
-            const double dels = e[16], deln = e[17];
-            sdx2 = sdx2 + dels * dels;
-            sdy2 = sdy2 + deln * deln;
-            sdxy = sdxy + dels * deln;
-            for (int h = 0; h < 2; ++h) {
-                fx[h] = fx[h] + e[4 * L + c0 + h] * dels;
-                fy[h] = fy[h] + e[4 * L + c0 + h] * deln;
-            }
-        }
-        obd = 1.0 / (sdx2 * sdy2 - sdxy * sdxy);
-        if (L < 2) {
-            Gv0 = (fx[0] * sdy2 - fy[0] * sdxy) * obd;
-            Gv1 = (fx[1] * sdy2 - fy[1] * sdxy) * obd;
-        } else {
-            Gv0 = (fy[0] * sdx2 - fx[0] * sdxy) * obd;
-            Gv1 = (fy[1] * sdx2 - fx[1] * sdxy) * obd;
-        }
-    }
-    double G[4][4];
-    for (int LL = 0; LL < 4; ++LL)
-        for (int h = 0; h < 2; ++h) {
-            G[LL][2 * h] = __shfl_sync(0xffffffffu, Gv0, 2 * LL + h, LPP);
-            G[LL][2 * h + 1] = __shfl_sync(0xffffffffu, Gv1, 2 * LL + h, LPP);
-        }
-    double frbv[4] = {0.0, 0.0, 0.0, 0.0}, dl = 0.0;
-    if (valid) {
-        for (int m = 0; m < 4; ++m) frbv[m] = frb[4 * (size_t)i + m];
-        dl = delta[i];
-    }
-    const double coef = kind == KIND_WALL ? 2.0 * dl : dl;
-    double sx2b = 0.0, sy2b = 0.0, sxyb = 0.0, obdb = 0.0, fxb[2] = {0.0, 0.0},
-           fyb[2] = {0.0, 0.0};
-    if (used) {
-        for (int h = 0; h < 2; ++h) {
-            const double Gb = coef * frbv[c0 + h];
-            if (L < 2) {
-                fxb[h] = Gb * sdy2 * obd;
-                fyb[h] = -Gb * sdxy * obd;
-                sy2b += Gb * fx[h] * obd;
-                sxyb += -Gb * fy[h] * obd;
-                obdb += Gb * (fx[h] * sdy2 - fy[h] * sdxy);
-            } else {
-                fyb[h] = Gb * sdx2 * obd;
-                fxb[h] = -Gb * sdxy * obd;
-                sx2b += Gb * fy[h] * obd;
-                sxyb += -Gb * fx[h] * obd;
-                obdb += Gb * (fy[h] * sdx2 - fx[h] * sdxy);
-            }
-        }
-    }
-    // combine the lane pair (components 0,1 and 2,3 of list L)
-    sx2b += __shfl_xor_sync(0xffffffffu, sx2b, 1, LPP);
-    sy2b += __shfl_xor_sync(0xffffffffu, sy2b, 1, LPP);
-    sxyb += __shfl_xor_sync(0xffffffffu, sxyb, 1, LPP);
-    obdb += __shfl_xor_sync(0xffffffffu, obdb, 1, LPP);
-    if (used) {
-        const double detb = -obdb * obd * obd;
-        sx2b += detb * sdy2;
-        sy2b += detb * sdx2;
-        sxyb += -2.0 * detb * sdxy;
-        for (int h = 0; h < 2; ++h) {
-            lb[grp][L][c0 + h] = fxb[h];
-            lb[grp][L][4 + c0 + h] = fyb[h];
-        }
-        if ((lane & 1) == 0) {
-            lb[grp][L][8] = sx2b;
-            lb[grp][L][9] = sy2b;
-            lb[grp][L][10] = sxyb;
-        }
-    }
-    if (valid && lane == 0) {
-        double db = 0.0;
-        for (int m = 0; m < 4; ++m) {
-            double sg;
-            if (kind == KIND_WALL) sg = 2.0 * (G[0][m] + G[1][m] + G[3][m]);
-            else if (kind == KIND_OUTER) sg = G[0][m] + G[1][m] + G[2][m];
-            else sg = G[0][m] + G[1][m] + G[2][m] + G[3][m];
-            db += frbv[m] * sg;
-        }
-        deltab[i] += db;
-    }
-    __syncwarp();
-    // phase C: per slot reverse of the fluxes, kinetic states and the
-    // point's own reconstruction; the neighbour's reconstruction is left to
-    // k_flux_b_nbr
-    if (valid) {
-        for (int r = lane; r < nb; r += LPP) {
-            const int k = g.conn[r * g.n + i];
-            const double2 pk = g.xy[k];
-            const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
-            double *e = rec + r * BREC;
-            const double dels = e[16], deln = e[17];
-            const KState si = kst_load(e + 18), sk = kst_load(e + 27);
-            double pr_[8];
-            for (int m = 0; m < 8; ++m) pr_[m] = e[36 + m];
-            double delsb = 0.0, delnb = 0.0;
-            KStateB sib, skb;
-            kzero(sib);
-            kzero(skb);
-            for (int slot = 0; slot < 4; ++slot) {
-                // (direction, pass) as in phase A: the lists holding the
-                // neighbour in ascending order, one converged pass each
-                const int d = slot >> 1, pass = slot & 1;
-                const unsigned long long bits = d == 0 ? mx : my;
-                const bool in0 = (bits >> r) & 1ull, in1 = (bits >> (r + 32)) & 1ull;
-                if (pass == 0 ? !(in0 || in1) : !(in0 && in1)) continue;
-                const int LL = 2 * d + ((pass == 1 || !in0) ? 1 : 0);
-                if ((kind == KIND_WALL && LL == 2) || (kind == KIND_OUTER && LL == 3)) continue;
-                const double sg = (LL & 1) ? -1.0 : 1.0;
-                double dGb[4], mdGb[4];
-                for (int m = 0; m < 4; ++m) {
-                    const double fxbm = lb[grp][LL][m], fybm = lb[grp][LL][4 + m];
-                    dGb[m] = fxbm * dels + fybm * deln;
-                    mdGb[m] = -dGb[m];
-                    delsb += fxbm * e[4 * LL + m];
-                    delnb += fybm * e[4 * LL + m];
-                }
-                const double s2b = lb[grp][LL][8], n2b = lb[grp][LL][9], snb = lb[grp][LL][10];
-                delsb += 2.0 * dels * s2b + deln * snb;
-                delnb += 2.0 * deln * n2b + dels * snb;
-                if (d == 0) {
-                    if (kind == KIND_INTERIOR) {
-                        flux_gx_b(sk, sg, dGb, skb);
-                        flux_gx_b(si, sg, mdGb, sib);
-                    } else {
-                        flux_quad_b(sk, sg, s2q, dGb, skb);
-                        flux_quad_b(si, sg, s2q, mdGb, sib);
-                    }
+                    s = kst_taped(v, nx, ny);
+                    u1 = v[6];
+                    u2 = v[7];
                 } else {
-                    flux_gy_b(sk, sg, dGb, skb);
-                    flux_gy_b(si, sg, mdGb, sib);
+                    const int p = h ? i : k;
+                    const R4 v = ld4(q_in + p);
+                    const double q[4] = {v.a, v.b, v.c, v.d};
+                    double dx[4], dy[4], hi[4], lo[4], qt[4], u[2], w[2];
+                    ld8a(dq + 8 * (size_t)p, dx, dy);
+                    ld8a(qm + 8 * (size_t)p, hi, lo);
+#pragma unroll
+                    for (int m = 0; m < 4; ++m)
+                        qt[m] = limited_qtilde(delx * dx[m] + dely * dy[m], q[m], hi[m], lo[m],
+                                               g.eps2[p]);
+                    KState same;
+                    kstate_pair(qt, qt, nx, ny, 0.56418958354775628695, s, same, u, w);
+                    u1 = u[0];
+                    u2 = u[1];
                 }
+                const double w6 = fma(6.0, s.pbr, s.usq);
+                KStateB b;
+                kzero(b);
+                // reverse of sgn c (F . G) of list l along t; returns sgn F . G
+                auto along_t = [&](int l, double c) {
+                    const double sg = l ? -1.0 : 1.0;
+                    if (kind == KIND_INTERIOR)
+                        return sgn * flux_split_b(s, s.ut, s.un, s.B1, s.e1, sg, w6, F, c, b.ut, b.un,
+                                                  b.B1, b.e1, b);
+                    const double s2 = kind == KIND_WALL ? -1.0 : 1.0;
+                    double G[4], cF[4], d = 0.0;
+                    flux_quad(s, sg, s2, G);
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        d = fma(F[m], G[m], d);
+                        cF[m] = c * F[m];
+                    }
+                    flux_quad_b(s, sg, s2, cF, b);
+                    return sgn * d;
+                };
+                auto along_n = [&](int l, double c) {
+                    const double sg = l ? -1.0 : 1.0;
+                    const double Fn[4] = {F[0], F[2], F[1], F[3]};
+                    return sgn * flux_split_b(s, s.un, s.ut, s.B2, s.e2, sg, w6, Fn, c, b.un, b.ut,
+                                              b.B2, b.e2, b);
+                };
+                cbx += along_t(lx, sgn * cx);
+                cby += along_n(ly, sgn * cy);
+                if (tx) {
+                    const double2 p = co[1];
+                    cbx1 += along_t(1, sgn * fma(p.x, dels, p.y * deln));
+                }
+                if (ty) {
+                    const double2 p = co[3];
+                    cby1 += along_n(1, sgn * fma(p.x, deln, p.y * dels));
+                }
+                kstate_qt_b(s, u1, u2, nx, ny, b, qtb, nxs, nys);
+                // from this k_flux_b_nbr reverses the neighbour's reconstruction
+                if (h == 0) st_pairs(nbrec + ((size_t)i * g.kp + r) * NBREC, qtb, 4);
             }
-            double nxbv = 0.0, nybv = 0.0;
-            double piu1b = 0.0, piu2b = 0.0, pirb = 0.0, pipb = 0.0;
-            double pku1b = 0.0, pku2b = 0.0, pkrb = 0.0, pkpb = 0.0;
-            kstate_b_s(si, pr_[0], pr_[1], nx, ny, sib, piu1b, piu2b, pirb, pipb, nxbv, nybv);
-            kstate_b_s(sk, pr_[4], pr_[5], nx, ny, skb, pku1b, pku2b, pkrb, pkpb, nxbv, nybv);
-            double delxb = delsb * ny + delnb * nx;
-            double delyb = -delsb * nx + delnb * ny;
-            nxbv += -delsb * dely + delnb * delx;
-            nybv += delsb * delx + delnb * dely;
-            const R4 qv = ld4(q_in + i);
-            const double qi[4] = {qv.a, qv.b, qv.c, qv.d};
-            double dxi[4], dyi[4], qmaxi[4], qmini[4];
-            ld8a(dq + 8 * (size_t)i, dxi, dyi);
-            ld8a(qm + 8 * (size_t)i, qmaxi, qmini);
-            double qib[4] = {0, 0, 0, 0}, dxib[4] = {0, 0, 0, 0}, dyib[4] = {0, 0, 0, 0},
-                   qmaxib[4] = {0, 0, 0, 0}, qminib[4] = {0, 0, 0, 0};
-            reconstruct_b(qi, dxi, dyi, qmaxi, qmini, g.eps2[i], delx, dely, c.gm1, pr_[2], piu1b,
-                          piu2b, pirb, pipb, qib, dxib, dyib, qmaxib, qminib, delxb, delyb);
-            // the neighbour's side: its reconstruction is reversed by
-            // k_flux_b_nbr from this record (the adjoint of its reconstructed
-            // primitive state, its density, and delx/dely's adjoint so far)
-            {
-                const double v[NBREC] = {pku1b, pku2b, pkrb, pkpb, pr_[6], delxb, delyb, 0.0};
-                st_pairs(nbrec + ((size_t)i * g.kp + r) * NBREC, v, NBREC);
+            // the slot weights' adjoint: cb d to each list's pb, cb p to d
+            delsb = fma(cbx, px.x, cby * py.y);
+            delnb = fma(cbx, px.y, cby * py.x);
+#pragma unroll
+            for (int l = 0; l < 2; ++l) {
+                const double wx = l == lx ? cbx : (l == 1 ? cbx1 : 0.0);
+                const double wy = l == ly ? cby : (l == 1 ? cby1 : 0.0);
+                pb[2 * l] = fma(wx, dels, pb[2 * l]);
+                pb[2 * l + 1] = fma(wx, deln, pb[2 * l + 1]);
+                pb[4 + 2 * l] = fma(wy, dels, pb[4 + 2 * l]);
+                pb[5 + 2 * l] = fma(wy, deln, pb[5 + 2 * l]);
             }
-            // self contribution of this slot, summed in slot order below
-            for (int m = 0; m < 4; ++m) {
-                e[m] = qib[m];
-                e[4 + m] = dxib[m];
-                e[8 + m] = dyib[m];
-                e[12 + m] = qmaxib[m];
-                e[16 + m] = qminib[m];
+            if (tx) {
+                delsb = fma(cbx1, co[1].x, delsb);
+                delnb = fma(cbx1, co[1].y, delnb);
             }
-            e[20] = -delxb;
-            e[21] = -delyb;
-            e[22] = nxbv;
-            e[23] = nybv;
+            if (ty) {
+                delsb = fma(cby1, co[3].y, delsb);
+                delnb = fma(cby1, co[3].x, delnb);
+            }
         }
+        double own[24] = {};
+        {
+            double qi[4], dxi[4], dyi[4], qmaxi[4], qmini[4];
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const double2 a = m.q[pg][c], x = m.dq[pg][c], y = m.dq[pg][2 + c],
+                          hi = m.qm[pg][c], lo = m.qm[pg][2 + c];
+                qi[2 * c] = a.x; qi[2 * c + 1] = a.y;
+                dxi[2 * c] = x.x; dxi[2 * c + 1] = x.y;
+                dyi[2 * c] = y.x; dyi[2 * c + 1] = y.y;
+                qmaxi[2 * c] = hi.x; qmaxi[2 * c + 1] = hi.y;
+                qmini[2 * c] = lo.x; qmini[2 * c + 1] = lo.y;
+            }
+            limited_b(qi, dxi, dyi, qmaxi, qmini, eps2, delx, dely, qtb, own, own + 4,
+                      own + 8, own + 12, own + 16, delxb, delyb);
+        }
+        if (r < nb) {
+            double2 *pt = reinterpret_cast<double2 *>(m.part[pg][r]);
+            pt[0] = make_double2(delsb, delnb);
+            pt[1] = make_double2(delxb, delyb);
+        }
+        // the round's own-point sums: lane t keeps fields 3 t .. 3 t + 2
+        const bool h4 = lane & 4, h2 = lane & 2, h1 = lane & 1;
+        double a[12], b[6];
+#pragma unroll
+        for (int f = 0; f < 12; ++f)
+            a[f] = (h4 ? own[12 + f] : own[f]) +
+                   __shfl_xor_sync(full, h4 ? own[f] : own[12 + f], 4);
+#pragma unroll
+        for (int f = 0; f < 6; ++f)
+            b[f] = (h2 ? a[6 + f] : a[f]) + __shfl_xor_sync(full, h2 ? a[f] : a[6 + f], 2);
+#pragma unroll
+        for (int f = 0; f < 3; ++f)
+            acc[f] += (h1 ? b[3 + f] : b[f]) + __shfl_xor_sync(full, h1 ? b[f] : b[3 + f], 1);
+    }
+    // pb summed over the point's lanes: lane 2 L + h holds component h of list
+    // L, then z's component
+    {
+        const bool h4 = lane & 4, h2 = lane & 2, h1 = lane & 1;
+        double a[4], b[2];
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            a[c] = (h4 ? pb[4 + c] : pb[c]) + __shfl_xor_sync(full, h4 ? pb[c] : pb[4 + c], 4);
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+            b[c] = (h2 ? a[2 + c] : a[c]) + __shfl_xor_sync(full, h2 ? a[c] : a[2 + c], 2);
+        const double v = (h1 ? b[1] : b[0]) + __shfl_xor_sync(full, h1 ? b[0] : b[1], 1);
+        const double w = __shfl_xor_sync(full, v, 1);
+        const int L = lane >> 1;
+        const double2 p = co[L];
+        const double gg = reinterpret_cast<const double *>(m.fcg[pg])[L];
+        // the diagonal entry of M^-1 of this lane's component
+        m.z[pg][lane] = fma((L < 2) == !h1 ? p.x : gg, v, p.y * w);
     }
     __syncwarp();
+    double sums[4] = {0.0, 0.0, 0.0, 0.0};  // of x, y, nx, ny
+    for (int r = lane; r < nb; r += LPP) {
+        const double2 pk = r >= LPP ? g.xy[g.conn[(size_t)r * g.n + i]] : pk0;
+        const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
+        const double dels = delx * ny - dely * nx, deln = delx * nx + dely * ny;
+        const double *pt = m.part[pg][r];
+        double delsb = pt[0], delnb = pt[1];
+        const unsigned bit = 1u << r;
+        const unsigned in[4] = {mm.x, mm.y, mm.z, mm.w};
+#pragma unroll
+        for (int L = 0; L < 4; ++L) {
+            if (!(in[L] & bit)) continue;
+            const double2 c2 = co[L];
+            const double ps = L < 2 ? c2.x : c2.y, pn = L < 2 ? c2.y : c2.x;
+            const double zs = m.z[pg][2 * L], zn = m.z[pg][2 * L + 1];
+            const double c = ps * dels + pn * deln, zd = zs * dels + zn * deln;
+            delsb -= zs * c + ps * zd;
+            delnb -= zn * c + pn * zd;
+        }
+        const double delxb = pt[2] + (delsb * ny + delnb * nx);
+        const double delyb = pt[3] + (delnb * ny - delsb * nx);
+        nxs += delnb * delx - delsb * dely;
+        nys += delsb * delx + delnb * dely;
+        reinterpret_cast<double2 *>(nbrec + ((size_t)i * g.kp + r) * NBREC)[2] =
+            make_double2(delxb, delyb);
+        sums[0] -= delxb;
+        sums[1] -= delyb;
+    }
+    sums[2] = nxs;
+    sums[3] = nys;
+    __syncwarp();
+    const double sum = reduce8(sums, lane);
     if (!valid) return;
-    for (int f = lane; f < 24; f += LPP) {
-        double s = 0.0;
-        for (int r = 0; r < nb; ++r) s = s + rec[r * BREC + f];
-        if (f < 4) qb[4 * (size_t)i + f] += s;
-        else if (f < 12) dqb[8 * (size_t)i + (f - 4)] += s;
-        else if (f < 20) qmb[8 * (size_t)i + (f - 12)] += s;
-        else if (f == 20) xb[i] += s;
-        else if (f == 21) yb[i] += s;
-        else if (f == 22) nxb[i] += s;
-        else nyb[i] += s;
+    if (!(lane & 1)) *geo = geo_old + sum;
+    // the stage's first contributions to q, dq and qm: stored, not added
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const int f = 3 * lane + c;
+        if (f < 4) qb[4 * (size_t)i + f] = acc[c];
+        else if (f < 12) dqb[8 * (size_t)i + (f - 4)] = acc[c];
+        else if (f < 20) qmb[8 * (size_t)i + (f - 12)] = acc[c];
     }
 }
 
@@ -504,11 +512,11 @@ k_flux_b(Geom g, Consts c, const R4 *__restrict__ q_in, const double *__restrict
 // reconstruction adds belongs to point i as well (delx = x_k - x_i): it is
 // left in back[(i, r)] for k_back_sum.
 constexpr int NBR_BLK = 128;
-#ifndef NBR_MIN_BLOCKS
-#define NBR_MIN_BLOCKS 3  // 168 registers (4: 128 with spills, 1 % slower)
-#endif
+// 128 registers (256,000 points: 74 us, 79 at 3 blocks; 91 when the record held
+// the adjoint of the primitive state)
+constexpr int NBR_MIN_BLOCKS = 4;
 __global__ void __launch_bounds__(NBR_BLK, NBR_MIN_BLOCKS)
-k_flux_b_nbr(Geom g, Consts c, const R4 *__restrict__ q_in, const double *__restrict__ dq,
+k_flux_b_nbr(Geom g, const R4 *__restrict__ q_in, const double *__restrict__ dq,
              const double *__restrict__ qm, const int *__restrict__ tptr,
              const int *__restrict__ tlist, const double *__restrict__ nbrec,
              double *__restrict__ qb, double *__restrict__ dqb, double *__restrict__ qmb,
@@ -531,14 +539,15 @@ k_flux_b_nbr(Geom g, Consts c, const R4 *__restrict__ q_in, const double *__rest
         const int i = slot / g.kp;
         const double2 pi_ = g.xy[i];
         const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
-        // the record: (u1b, u2b), (rhob, prb), (rho, delxb), (delyb, 0)
+        // the record: the adjoint of k's limited qtilde, delx/dely's so far
         const double2 *rv = reinterpret_cast<const double2 *>(nbrec + (size_t)slot * NBREC);
-        const double2 ub = __ldg(rv), pb = __ldg(rv + 1), rd = __ldg(rv + 2), dy = __ldg(rv + 3);
+        const double2 v0 = __ldg(rv), v1 = __ldg(rv + 1), dd = __ldg(rv + 2);
+        const double qtb[4] = {v0.x, v0.y, v1.x, v1.y};
         double dxr = 0.0, dyr = 0.0;
-        reconstruct_b(qk, dxk, dyk, qmaxk, qmink, eps2, delx, dely, c.gm1, rd.x, ub.x, ub.y, pb.x,
-                      pb.y, qkb, dxkb, dykb, qmaxkb, qminkb, dxr, dyr);
-        xkb += rd.y + dxr;
-        ykb += dy.x + dyr;
+        limited_b(qk, dxk, dyk, qmaxk, qmink, eps2, delx, dely, qtb, qkb, dxkb, dykb, qmaxkb,
+                  qminkb, dxr, dyr);
+        xkb += dd.x + dxr;
+        ykb += dd.y + dyr;
         back[slot] = make_double2(dxr, dyr);
     }
     add_pairs(qb + 4 * (size_t)k, qkb, 4);
@@ -1060,11 +1069,6 @@ inline int nblk(int n, int b) { return (n + b - 1) / b; }
 
 }  // namespace
 
-cudaError_t init_adjoint_kernels() {
-    return cudaFuncSetAttribute(k_flux_b, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                GROUPS * 20 * BREC * (int)sizeof(double));
-}
-
 void launch_update_b(const Geom &g, const Consts &c, const AdjConsts &a, const R4 *prim_in,
                      const R4 *prim_old, const R4 *fr, const double *pb_out, double *pb_in,
                      double *pb_old, double *frb, double *nxb, double *nyb, int rk,
@@ -1073,16 +1077,16 @@ void launch_update_b(const Geom &g, const Consts &c, const AdjConsts &a, const R
                                              pb_old, frb, nxb, nyb, rk);
 }
 
-void launch_flux_b(const Geom &g, const Consts &c, const R4 *q_in, const double *dq,
-                   const double *qm, const double *delta, const double *frb, double *qb,
+void launch_flux_b(const Geom &g, const R4 *q_in, const double *dq, const double *qm,
+                   const double *delta, const R4 *fr, const double *frb, double *qb,
                    double *dqb, double *qmb, double *xb, double *yb, double *nxb, double *nyb,
                    double *deltab, double *nbrec, double *back, const int *tptr,
                    const int *tlist, const double *kst, cudaStream_t s) {
-    size_t smem = (size_t)GROUPS * g.kp * BREC * sizeof(double);
-    k_flux_b<<<nblk(g.n, GROUPS), BLK, smem, s>>>(g, c, q_in, dq, qm, delta, frb, qb, dqb, qmb,
-                                                  xb, yb, nxb, nyb, deltab, nbrec, kst);
+    k_flux_b<<<nblk(g.n, GROUPS), BLK, 0, s>>>(g, q_in, dq, qm, delta,
+                                               reinterpret_cast<const double *>(fr), frb, qb,
+                                               dqb, qmb, xb, yb, nxb, nyb, deltab, nbrec, kst);
     double2 *bk = reinterpret_cast<double2 *>(back);
-    k_flux_b_nbr<<<nblk(g.n, NBR_BLK), NBR_BLK, 0, s>>>(g, c, q_in, dq, qm, tptr, tlist, nbrec,
+    k_flux_b_nbr<<<nblk(g.n, NBR_BLK), NBR_BLK, 0, s>>>(g, q_in, dq, qm, tptr, tlist, nbrec,
                                                        qb, dqb, qmb, xb, yb, bk);
     k_back_sum<<<nblk(g.n, 256), 256, 0, s>>>(g, bk, xb, yb);
 }

@@ -884,7 +884,7 @@ static int create_handle(const mfcfd_grid *grid, const mfcfd_params *params, int
     }
     if (!h->fp32) {
         // on the stream of the uploads above, and before the copies below
-        launch_flux_coef(h->geom, 0, nl, nw, no, P.power, h->d_fco, h->d_wsl, nullptr);
+        launch_flux_coef(h->geom, 0, nl, nw, no, P.power, h->d_fco, h->d_wsl, nullptr, nullptr);
         h->geom.fco = h->d_fco;
         h->geom.wsl = h->d_wsl;
     }

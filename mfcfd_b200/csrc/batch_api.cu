@@ -649,7 +649,7 @@ int mfcfd_batch_create(int n_inst, const mfcfd_grid *const *grids, const mfcfd_p
         // on the stream of the uploads above, and before the copies below
         for (const InstInfo &in : info)
             launch_flux_coef(b->geom, in.base, in.n, in.nw, in.no, P0.power, b->d_fco, b->d_wsl,
-                             nullptr);
+                             nullptr, nullptr);
         b->geom.fco = b->d_fco;
         b->geom.wsl = b->d_wsl;
     }

@@ -39,7 +39,7 @@ __device__ __forceinline__ double rsqrt_h3(double x) {
 constexpr double EXP_MAX = 700.0;
 // The polynomials' coefficients sit in constant memory: as literals each cost
 // two moves into registers at every use.
-__constant__ double c_exp[14] = {
+static __constant__ double c_exp[14] = {
     0x1.71547652b82fep+0, 6755399441055744.0 /* 1.5 2^52 */, -0x1.62e42fefa39efp-1,
     -0x1.abc9e3b39803fp-56,
     0x1.af38a9b0ec855p-26, 0x1.289185613a3d6p-22, 0x1.71de0dae63bb3p-19, 0x1.a019b90d2ae7ap-16,
@@ -64,7 +64,7 @@ __device__ __forceinline__ double exp_mid(double x) {
 // x Q at most 2.5e-17).  1.25 covers |u| sqrt(beta) up to Mach 1.49 along a
 // direction; beyond it the library's erf is taken.
 constexpr double ERF_MAX = 1.25;
-__constant__ double c_erf[14] = {
+static __constant__ double c_erf[14] = {
     -0x1.cd03490bc5835p-39, 0x1.5daf7ab4a9346p-34, -0x1.46f41e3907e41p-30,
     0x1.fa4fba2e1e1b8p-27, -0x1.5f42a98f93ce9p-23, 0x1.b9e1480408c3dp-20,
     -0x1.f4d1ed44b13b7p-17, 0x1.f9a320de78f7ap-14, -0x1.c02db3c5bcce0p-11,
@@ -77,8 +77,8 @@ __device__ __forceinline__ double erf_mid(double x, double z) {
     return x * p;
 }
 
-__device__ __noinline__ double exp_any(double x) { return exp(x); }
-__device__ __noinline__ double erf_any(double x) { return erf(x); }
+static __device__ __noinline__ double exp_any(double x) { return exp(x); }
+static __device__ __noinline__ double erf_any(double x) { return erf(x); }
 
 __device__ __forceinline__ int abs_hi(double x) { return __double2hiint(x) & 0x7fffffff; }
 

@@ -8,6 +8,7 @@
 // (e.g. src_mpi_adjoint/sensitivity_files/limiters_b.F90:43-165).
 #pragma once
 
+#include "flux_math.cuh"
 #include "lskum_device.cuh"
 
 namespace lskum {
@@ -22,82 +23,31 @@ __device__ __forceinline__ void kzero(KStateB &b) {
     b.rho = b.ut = b.un = b.pbr = b.usq = b.B1 = b.B2 = b.e1 = b.e2 = 0.0;
 }
 
-// split_fluxes_b: flux_Gxp / flux_Gxn (s1 = +-1)
-__device__ __forceinline__ void flux_gx_b(const KState &s, double s1, const double Gb[4],
-                                          KStateB &b) {
-    const double A1 = 0.5 * (1.0 + s1 * s.e1);
-    double A1b = 0.0;
-    const double t1 = s.pbr + s.ut * s.ut;
-    const double t2 = t1 * A1 + s1 * (s.ut * s.B1);
-    const double t3 = s.ut * s.un * A1 + s1 * (s.un * s.B1);
-    const double t7 = (7.0 * s.pbr) + s.usq;
-    const double t4 = 0.5 * s.ut * t7 * A1;
-    const double t6 = (6.0 * s.pbr) + s.usq;
-    b.rho += Gb[0] * (s.ut * A1 + s1 * s.B1) + Gb[1] * t2 + Gb[2] * t3 +
-             Gb[3] * (t4 + s1 * (0.5 * t6 * s.B1));
-    const double a0 = s.rho * Gb[0];
-    b.ut += a0 * A1;
-    A1b += a0 * s.ut;
-    b.B1 += a0 * s1;
-    const double a1 = s.rho * Gb[1];
-    const double t1b = a1 * A1;
-    A1b += a1 * t1;
-    b.ut += a1 * s1 * s.B1 + 2.0 * s.ut * t1b;
-    b.B1 += a1 * s1 * s.ut;
-    b.pbr += t1b;
-    const double a2 = s.rho * Gb[2];
-    b.ut += a2 * s.un * A1;
-    b.un += a2 * (s.ut * A1 + s1 * s.B1);
-    A1b += a2 * s.ut * s.un;
-    b.B1 += a2 * s1 * s.un;
-    const double a3 = s.rho * Gb[3];
-    const double t7b = a3 * 0.5 * s.ut * A1;
-    const double t6b = a3 * s1 * 0.5 * s.B1;
-    b.ut += a3 * 0.5 * t7 * A1;
-    A1b += a3 * 0.5 * s.ut * t7;
-    b.B1 += a3 * s1 * 0.5 * t6;
-    b.pbr += 7.0 * t7b + 6.0 * t6b;
-    b.usq += t7b + t6b;
-    b.e1 += 0.5 * s1 * A1b;
-}
-
-// split_fluxes_b: flux_Gyp / flux_Gyn (s2 = +-1)
-__device__ __forceinline__ void flux_gy_b(const KState &s, double s2, const double Gb[4],
-                                          KStateB &b) {
-    const double A2 = 0.5 * (1.0 + s2 * s.e2);
-    double A2b = 0.0;
-    const double t1 = s.pbr + s.un * s.un;
-    const double t2 = t1 * A2 + s2 * (s.un * s.B2);
-    const double t3 = s.ut * s.un * A2 + s2 * (s.ut * s.B2);
-    const double t7 = (7.0 * s.pbr) + s.usq;
-    const double t4 = 0.5 * s.un * t7 * A2;
-    const double t6 = (6.0 * s.pbr) + s.usq;
-    b.rho += Gb[0] * (s.un * A2 + s2 * s.B2) + Gb[2] * t2 + Gb[1] * t3 +
-             Gb[3] * (t4 + s2 * (0.5 * t6 * s.B2));
-    const double a0 = s.rho * Gb[0];
-    b.un += a0 * A2;
-    A2b += a0 * s.un;
-    b.B2 += a0 * s2;
-    const double a2 = s.rho * Gb[2];
-    const double t1b = a2 * A2;
-    A2b += a2 * t1;
-    b.un += a2 * s2 * s.B2 + 2.0 * s.un * t1b;
-    b.B2 += a2 * s2 * s.un;
-    b.pbr += t1b;
-    const double a1 = s.rho * Gb[1];
-    b.un += a1 * s.ut * A2;
-    b.ut += a1 * (s.un * A2 + s2 * s.B2);
-    A2b += a1 * s.ut * s.un;
-    b.B2 += a1 * s2 * s.ut;
-    const double a3 = s.rho * Gb[3];
-    const double t7b = a3 * 0.5 * s.un * A2;
-    const double t6b = a3 * s2 * 0.5 * s.B2;
-    b.un += a3 * 0.5 * t7 * A2;
-    A2b += a3 * 0.5 * s.un * t7;
-    b.B2 += a3 * s2 * 0.5 * t6;
-    b.pbr += 7.0 * t7b + 6.0 * t6b;
-    b.usq += t7b + t6b;
-    b.e2 += 0.5 * s2 * A2b;
+// split_fluxes_b in the forms of flux_split (flux_math.cuh): for a direction
+// with velocity u along and o across it, moments B and e, list sign sg and w6
+// = 6 p/rho + |u|^2, the reverse of c (F . G) for F over (mass, momentum along,
+// momentum across, energy).  Returns F . G.
+__device__ __forceinline__ double flux_split_b(const KState &s, double u, double o, double B,
+                                               double e, double sg, double w6, const double F[4],
+                                               double c, double &ub, double &ob, double &Bb,
+                                               double &eb, KStateB &b) {
+    const double A = fma(0.5 * sg, e, 0.5);
+    const double a = fma(u, A, sg * B);
+    const double pA = s.pbr * A;
+    const double oF = fma(o, F[2], F[0]), hF = 0.5 * F[3];
+    const double t = fma(F[1], fma(u, a, pA), fma(hF, fma(w6, a, u * pA), oF * a));
+    b.rho = fma(c, t, b.rho);
+    const double cr = c * s.rho, r1 = cr * F[1], r3 = cr * hF;
+    const double ab = fma(r3, w6, fma(r1, u, cr * oF));
+    const double pAb = fma(r3, u, r1);
+    ub = fma(ab, A, fma(r3, pA, fma(r1, a, ub)));
+    ob = fma(cr * F[2], a, ob);
+    const double w6b = r3 * a;
+    b.pbr = fma(6.0, w6b, fma(pAb, A, b.pbr));
+    b.usq += w6b;
+    Bb = fma(sg, ab, Bb);
+    eb = fma(0.5 * sg, fma(ab, u, pAb * s.pbr), eb);
+    return s.rho * t;
 }
 
 // quadrant_fluxes_b: GxI..GxIV
@@ -155,170 +105,69 @@ __device__ __forceinline__ void flux_quad_b(const KState &s, double s1, double s
     b.e2 += 0.5 * s2 * A2b;
 }
 
-// kstate_b: adjoint of the kinetic state w.r.t. (u1, u2, rho, pr) and the
-// point's normal (nx, ny), which sets the (t, n) frame.
-__device__ __forceinline__ void kstate_b(double u1, double u2, double rho, double pr, double nx,
-                                         double ny, double pi, KStateB sb_, double &u1b,
-                                         double &u2b, double &rhob, double &prb, double &nxb,
-                                         double &nyb) {
-    const double ut = u1 * ny - u2 * nx;
-    const double un = u1 * nx + u2 * ny;
-    const double beta = 0.5 * rho / pr;
-    const double sb = sqrt(beta);
-    const double S1 = ut * sb, S2 = un * sb;
-    const double spb = sqrt(pi * beta);
-    const double E1 = exp(-S1 * S1), E2 = exp(-S2 * S2);
-    const double B1 = 0.5 * E1 / spb, B2 = 0.5 * E2 / spb;
-    double utb = sb_.ut + 2.0 * ut * sb_.usq;
-    double unb = sb_.un + 2.0 * un * sb_.usq;
-    prb += sb_.pbr / rho;
-    rhob += sb_.rho - sb_.pbr * (pr / rho) / rho;
-    const double S1b = sb_.e1 * MFCFD_TWO_OVER_SQRT_PI * E1 + sb_.B1 * B1 * (-2.0 * S1);
-    const double S2b = sb_.e2 * MFCFD_TWO_OVER_SQRT_PI * E2 + sb_.B2 * B2 * (-2.0 * S2);
-    const double spbb = -(sb_.B1 * B1 + sb_.B2 * B2) / spb;
-    double betab = spbb * pi / (2.0 * spb);
-    utb += S1b * sb;
-    unb += S2b * sb;
-    const double sbb = S1b * ut + S2b * un;
-    betab += sbb / (2.0 * sb);
-    rhob += betab * 0.5 / pr;
-    prb += -betab * beta / pr;
-    u1b += utb * ny + unb * nx;
-    u2b += -utb * nx + unb * ny;
-    nxb += -utb * u2 + unb * u1;
+// kstate_pre / kstate_pair (flux_math.cuh) reversed: the adjoint b of a kinetic
+// state s with velocity (u1, u2) to that of its limited qtilde, added to the
+// normal's.  exp(-S^2) comes back from the moments (B = exp(-S^2) / (2 sqrt(pi
+// beta))), so one reciprocal and one reciprocal square root are all it takes.
+__device__ __forceinline__ void kstate_qt_b(const KState &s, double u1, double u2, double nx,
+                                            double ny, const KStateB &b, double qtb[4],
+                                            double &nxb, double &nyb) {
+    const double beta = 0.5 * rcp_h3(s.pbr);
+    const double sb = beta * rsqrt_h3(beta);
+    const double S1 = s.ut * sb, S2 = s.un * sb;
+    const double S1b = s.B1 * (4.0 * sb * b.e1 - 2.0 * S1 * b.B1);
+    const double S2b = s.B2 * (4.0 * sb * b.e2 - 2.0 * S2 * b.B2);
+    const double utb = fma(S1b, sb, b.ut), unb = fma(S2b, sb, b.un);
+    const double texpb = b.rho * s.rho;
+    const double usqb = fma(texpb, beta, b.usq);
+    const double u1b = fma(2.0 * u1, usqb, utb * ny + unb * nx);
+    const double u2b = fma(2.0 * u2, usqb, unb * ny - utb * nx);
+    nxb += unb * u1 - utb * u2;
     nyb += utb * u1 + unb * u2;
+    // p/rho = 1/(2 beta), u = qtilde_2,3 p/rho
+    const double pbrb = fma(2.0 * beta, u1b * u1 + u2b * u2, b.pbr);
+    double betab = fma(texpb, s.usq - 5.0 * s.pbr, -2.0 * s.pbr * s.pbr * pbrb);
+    betab = fma(s.pbr, sb * (S1b * s.ut + S2b * s.un) - (b.B1 * s.B1 + b.B2 * s.B2), betab);
+    qtb[0] = texpb;
+    qtb[1] = u1b * s.pbr;
+    qtb[2] = u2b * s.pbr;
+    qtb[3] = -0.5 * betab;
 }
 
-// kstate_b from the forward's own kinetic state s (its rho, ut, un, p/rho,
-// B1, B2): exp(-S^2) / sqrt(pi beta) = 2 B and (2/sqrt(pi)) exp(-S^2) =
-// 4 B sqrt(beta), so the adjoint needs one square root and two divisions
-// instead of kstate_b's two exponentials, two square roots and seven
-// divisions.  (u1, u2) is the state's velocity.
-__device__ __forceinline__ void kstate_b_s(const KState &s, double u1, double u2, double nx,
-                                           double ny, const KStateB &sb_, double &u1b,
-                                           double &u2b, double &rhob, double &prb, double &nxb,
-                                           double &nyb) {
-    const double ut = s.ut, un = s.un, pbr = s.pbr;
-    const double beta = 0.5 / pbr;
-    const double ir = 1.0 / s.rho;
-    const double sb = sqrt(beta);
-    const double S1 = ut * sb, S2 = un * sb;
-    double utb = sb_.ut + 2.0 * ut * sb_.usq;
-    double unb = sb_.un + 2.0 * un * sb_.usq;
-    prb += sb_.pbr * ir;
-    rhob += sb_.rho - sb_.pbr * pbr * ir;
-    const double S1b = s.B1 * (4.0 * sb * sb_.e1 - 2.0 * S1 * sb_.B1);
-    const double S2b = s.B2 * (4.0 * sb * sb_.e2 - 2.0 * S2 * sb_.B2);
-    double betab = -(sb_.B1 * s.B1 + sb_.B2 * s.B2) * pbr;
-    utb += S1b * sb;
-    unb += S2b * sb;
-    betab += (S1b * ut + S2b * un) * sb * pbr;  // d sqrt(beta) / d beta = sqrt(beta) p/rho
-    // beta = rho / (2 pr): d/drho = beta / rho, d/dpr = -beta / pr = -2 beta^2 / rho
-    rhob += betab * beta * ir;
-    prb += -betab * 2.0 * beta * beta * ir;
-    u1b += utb * ny + unb * nx;
-    u2b += -utb * nx + unb * ny;
-    nxb += -utb * u2 + unb * u1;
-    nyb += utb * u1 + unb * u2;
-}
-
-// qtilde_to_primitive_b (one division: 1/beta; 1/gm1 is loop-invariant
-// where this is inlined)
-__device__ __forceinline__ void qtilde_to_primitive_b(const double qt[4], double gm1, double rho,
-                                                      double u1b, double u2b, double rhob,
-                                                      double prb, double qtb[4]) {
-    const double beta = -qt[3] * 0.5;
-    const double ib = 1.0 / beta;
-    const double igm1 = 1.0 / gm1;
-    const double temp = 0.5 * ib;
-    const double u1 = qt[1] * temp, u2 = qt[2] * temp;
-    rhob += prb * temp;
-    double tempb = prb * rho;
-    const double temp2b = rhob * rho;
-    const double temp1b = temp2b;
-    double betab = -temp2b * ib * igm1;
-    qtb[0] += temp1b;
-    betab += temp1b * (u1 * u1 + u2 * u2);
-    u1b += temp1b * 2.0 * beta * u1;
-    u2b += temp1b * 2.0 * beta * u2;
-    qtb[1] += u1b * temp;
-    qtb[2] += u2b * temp;
-    tempb += u1b * qt[1] + u2b * qt[2];
-    betab += -tempb * temp * ib;
-    qtb[3] += -0.5 * betab;
-}
-
-// reconstruct_b: adjoint of the limited reconstruction to primitive
-// variables.  The Venkatakrishnan limiter of each component (its forward
-// value and venkat_limiter_b) shares one reciprocal of its denominator:
-// phi = num (1/den), num_b = phi_b (1/den), den_b = -phi_b phi (1/den).
-__device__ __forceinline__ void reconstruct_b(const double q[4], const double dqx[4],
-                                              const double dqy[4], const double qmax[4],
-                                              const double qmin[4], double eps2, double delx,
-                                              double dely, double gm1, double rho, double u1b,
-                                              double u2b, double rhob, double prb, double qb[4],
-                                              double dqxb[4], double dqyb[4], double qmaxb[4],
-                                              double qminb[4], double &delxb, double &delyb) {
-    double qt[4], t[4], phi[4], idn[4];
-    unsigned active = 0;  // bit r: the limiter of component r is below 1
+// limited_qtilde (flux_math.cuh) of a row reversed, all four components: the
+// adjoint qtb of the limited qtilde towards (delx, dely), added to the row's
+// adjoints and the offset's (limiters_b.F90:43-165).
+__device__ __forceinline__ void limited_b(const double q[4], const double dqx[4],
+                                          const double dqy[4], const double qmax[4],
+                                          const double qmin[4], double eps2, double delx,
+                                          double dely, const double qtb[4], double qb[4],
+                                          double dqxb[4], double dqyb[4], double qmaxb[4],
+                                          double qminb[4], double &delxb, double &delyb) {
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-        t[r] = delx * dqx[r] + dely * dqy[r];
-        const double dn = (q[r] - 0.5 * t[r]) - q[r];
-        phi[r] = 1.0;
-        idn[r] = 0.0;
-        if (fabs(dn) > MFCFD_VENKAT_THR) {
-            const double dp = dn > 0.0 ? qmax[r] - q[r] : qmin[r] - q[r];
-            const double num = ((dp * dp) + eps2) * dn + 2.0 * dn * dn * dp;
-            const double den = ((dp * dp + 2.0 * dn * dn) + dn * dp + eps2) * dn;
-            const double id = 1.0 / den;
-            const double temp = num * id;
-            if (temp < 1.0) {
-                phi[r] = temp;
-                idn[r] = id;
-                active |= 1u << r;
-            }
-        }
-        qt[r] = q[r] - 0.5 * phi[r] * t[r];
-    }
-    double qtb[4] = {0.0, 0.0, 0.0, 0.0};
-    qtilde_to_primitive_b(qt, gm1, rho, u1b, u2b, rhob, prb, qtb);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
+        const double t = delx * dqx[r] + dely * dqy[r];
+        const double dn = -0.5 * t;
+        const bool up = dn > 0.0;
+        const double dp = (up ? qmax[r] : qmin[r]) - q[r];
+        const double a = fma(dp, dp, eps2);
+        const double id = rcp_h3(fma(dn, dp - t, a));
+        const double f = fma(-t, dp, a) * id;
+        const bool act = f < 1.0 && fabs(dn) > MFCFD_VENKAT_THR;
         qb[r] += qtb[r];
-        double tb = -0.5 * phi[r] * qtb[r];
-        if ((active >> r) & 1u) {
-            // venkat_limiter_b of component r
-            const double phib = -0.5 * t[r] * qtb[r];
-            const double dn = (q[r] - 0.5 * t[r]) - q[r];
-            const bool up = dn > 0.0;
-            const double dp = up ? qmax[r] - q[r] : qmin[r] - q[r];
-            const double num1 = (dp * dp) + eps2;
-            const double den1 = dp * dp + 2.0 * dn * dn;
-            const double den2 = den1 + dn * dp + eps2;
-            const double numb = phib * idn[r];
-            const double denb = -phib * phi[r] * idn[r];
-            const double den2b = denb * dn;
-            double dnb = denb * den2;
-            const double den1b = den2b;
-            dnb += den2b * dp;
-            double dpb = den2b * dn;
-            dpb += den1b * 2.0 * dp;
-            dnb += den1b * 4.0 * dn;
-            const double num1b = numb * dn;
-            dnb += numb * (num1 + 4.0 * dn * dp);
-            dpb += numb * 2.0 * dn * dn;
-            dpb += num1b * 2.0 * dp;
+        double dnb = qtb[r];
+        if (act) {
+            const double numb = qtb[r] * dn * id, denb = -numb * f;
+            const double dpb = 2.0 * numb * (dp + dn) + denb * fma(2.0, dp, dn);
+            dnb = fma(f, qtb[r], 2.0 * numb * dp + denb * fma(4.0, dn, dp));
             if (up) qmaxb[r] += dpb;
             else qminb[r] += dpb;
             qb[r] -= dpb;
-            // dn = qt0 - q with qt0 = q - t/2: q's two shares of dnb cancel
-            tb += -0.5 * dnb;
         }
-        delxb += tb * dqx[r];
-        delyb += tb * dqy[r];
-        dqxb[r] += tb * delx;
-        dqyb[r] += tb * dely;
+        const double tb = -0.5 * dnb;
+        delxb = fma(tb, dqx[r], delxb);
+        delyb = fma(tb, dqy[r], delyb);
+        dqxb[r] = fma(tb, delx, dqxb[r]);
+        dqyb[r] = fma(tb, dely, dqyb[r]);
     }
 }
 

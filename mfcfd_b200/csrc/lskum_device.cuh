@@ -61,6 +61,8 @@ struct Geom {
     // and with power != 0 the weight of every slot ([kp][n]; else nullptr: 1).
     const double *fco = nullptr;
     const double *wsl = nullptr;
+    // reverse flux pass: the third entry of each list's inverse matrix ([n][4])
+    const double *fcg = nullptr;
 };
 // rows a tile halo stages at most (its local row indices are bytes)
 constexpr int HALO_CAP = 64;

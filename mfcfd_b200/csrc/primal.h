@@ -118,9 +118,10 @@ void launch_inner(const Geom &g, const Consts &c, const Sched &s, const double *
 void launch_flux(const Geom &g, const Consts &c, const Sched &s, const StageBufs &b, int rk,
                  bool last, int grid, int tiles, cudaStream_t st);
 // Fixed per grid: the list-solve coefficients of points [base, base + n) (wall,
-// outer, interior counts nw, no, rest) and, with wsl, their slots' weights.
+// outer, interior counts nw, no, rest) and, with wsl, their slots' weights
+// and, with fcg, the third entries of the lists' inverse matrices.
 void launch_flux_coef(const Geom &g, int base, int n, int nw, int no, double power, double *fco,
-                      double *wsl, cudaStream_t st);
+                      double *wsl, double *fcg, cudaStream_t st);
 // Residual norm and residue of one iteration per instance (hist row i, entry
 // it - it_first), retirement, and the schedule of the next iteration.
 void launch_residual(const InstInfo *inst, int n_inst, const double *res_part, Ctl *ctl,

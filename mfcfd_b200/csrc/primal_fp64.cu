@@ -345,9 +345,11 @@ kb_grad_h(Geom g, Consts c, Sched s, const R4 *__restrict__ q, const double *__r
 // directions' terms into four sums and eight lanes add theirs by shuffles.
 // Per point and split list L: a, b of the list's solve (fco[8 i + 2 L]).
 // *_fluxes.F90 dG*: the sums in slot order; a list the point's kind does not
-// have (wall ypos, outer yneg) and empty rows get zeros.
+// have (wall ypos, outer yneg) gets zeros.  fcg: the third entry of the list's
+// inverse normal matrix (the reverse pass).
 __global__ void k_flux_coef(Geom g, int base, int n, int nw, int no, double power,
-                            double *__restrict__ fco, double *__restrict__ wsl) {
+                            double *__restrict__ fco, double *__restrict__ wsl,
+                            double *__restrict__ fcg) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const int i = base + j;
@@ -379,6 +381,7 @@ __global__ void k_flux_coef(Geom g, int base, int n, int nw, int no, double powe
         const double ob = 1.0 / (sxx[L] * syy[L] - sxy[L] * sxy[L]);
         fco[8 * (size_t)i + 2 * L] = none ? 0.0 : (L < 2 ? syy[L] : sxx[L]) * ob;
         fco[8 * (size_t)i + 2 * L + 1] = none ? 0.0 : -sxy[L] * ob;
+        if (fcg) fcg[4 * (size_t)i + L] = none ? 0.0 : (L < 2 ? sxx[L] : syy[L]) * ob;
     }
 }
 
@@ -885,8 +888,9 @@ int flux_grid_blocks(int n, bool fp32) {
 }
 
 void launch_flux_coef(const Geom &g, int base, int n, int nw, int no, double power, double *fco,
-                      double *wsl, cudaStream_t st) {
-    k_flux_coef<<<nblk(n, GRAD_BLOCK), GRAD_BLOCK, 0, st>>>(g, base, n, nw, no, power, fco, wsl);
+                      double *wsl, double *fcg, cudaStream_t st) {
+    k_flux_coef<<<nblk(n, GRAD_BLOCK), GRAD_BLOCK, 0, st>>>(g, base, n, nw, no, power, fco, wsl,
+                                                            fcg);
 }
 
 // staging memory of a block of the halo kernels: two tiles a warp
