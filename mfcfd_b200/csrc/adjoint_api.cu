@@ -72,6 +72,7 @@ double *qm_at(AdjointState *a, int rk) { return a->tqm + (size_t)(rk - 1) * 8 * 
 
 int adj_setup(mfcfd_t *h) {
     if (h->adj) return MFCFD_OK;
+    lskum_host::drop_tangent(h);  // its memory may be what the tape needs
     AdjointState *a = new AdjointState();
     h->adj = a;
     const int n = h->n, kp = h->kp, m = h->p.inner_iterations, rks = h->p.rks;
@@ -437,6 +438,7 @@ int adjoint_prepare(mfcfd_t *h, int objective, int n_iters, size_t ckpt_bytes, i
     const long long want = ckpt_bytes > row ? (long long)(ckpt_bytes / row) - 1 : 0;
     *nsnap = (int)std::min<long long>(want, n_iters - 1);
     if ((int)a->snaps.size() < *nsnap + 1) {  // + one scratch row; one allocation
+        lskum_host::drop_tangent(h);
         if (a->snap_pool) cudaFree(a->snap_pool);
         a->snap_pool = nullptr;
         a->snaps.clear();

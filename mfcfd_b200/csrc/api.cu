@@ -61,6 +61,7 @@ namespace {
 
 void free_all(mfcfd_t *h) {
     lskum_host::free_adjoint(h);
+    lskum_host::drop_tangent(h);
     for (auto &row : h->pair_exec)
         for (auto &g : row)
             if (g) cudaGraphExecDestroy(g);
@@ -68,7 +69,7 @@ void free_all(mfcfd_t *h) {
         for (auto &g : row)
             if (g) cudaGraphExecDestroy(g);
     void *bufs[] = {h->d_xy, h->d_nrm, h->d_eps2, h->d_obc, h->d_conn, h->d_nbhs, h->d_mx,
-                    h->d_my, h->d_hoff, h->d_hrow, h->d_hloc, h->d_fco, h->d_wsl, h->d_prim[0], h->d_prim[1], h->d_q[0], h->d_q[1], h->d_dq[0],
+                    h->d_my, h->d_hoff, h->d_hrow, h->d_hloc, h->d_fco, h->d_wsl, h->d_perm, h->d_prim[0], h->d_prim[1], h->d_q[0], h->d_q[1], h->d_dq[0],
                     h->d_dq[1], h->d_dq[2], h->d_qm, h->d_delta, h->d_spd, h->d_res_part, h->d_flux_dbg,
                     h->d_hist, h->d_forces, h->d_ctl, h->d_sh_idx, h->d_sh_shape, h->d_sh_geo,
                     h->d_sh_my, h->f_prim[0], h->f_prim[1], h->f_q[0], h->f_q[1],
@@ -799,6 +800,7 @@ static int create_handle(const mfcfd_grid *grid, const mfcfd_params *params, int
     ALLOC(h->d_obc, hobc.size());
     ALLOC(h->d_conn, (size_t)kp * n);
     ALLOC(h->d_nbhs, n);
+    ALLOC(h->d_perm, n);
     ALLOC(h->d_mx, n);
     ALLOC(h->d_my, n);
     {
@@ -855,7 +857,7 @@ static int create_handle(const mfcfd_grid *grid, const mfcfd_params *params, int
     }
     if ((st = up(h->d_xy, hxy)) || (st = up(h->d_nrm, hnrm)) || (st = up(h->d_eps2, heps)) ||
         (st = up(h->d_obc, hobc)) || (st = up(h->d_conn, hconn)) || (st = up(h->d_nbhs, hnb)) ||
-        (st = up(h->d_mx, hmx)) || (st = up(h->d_my, hmy)))
+        (st = up(h->d_mx, hmx)) || (st = up(h->d_my, hmy)) || (st = up(h->d_perm, h->perm)))
         goto fail_create;
     if (h->d_hoff && ((st = up(h->d_hoff, halo.off)) || (st = up(h->d_hrow, halo.rows)) ||
                       (st = up(h->d_hloc, halo.loc))))

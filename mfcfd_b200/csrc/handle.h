@@ -12,7 +12,8 @@
 
 using namespace lskum;
 
-struct AdjointState;  // adjoint buffers (adjoint_api.cu), created on first use
+struct AdjointState;
+struct TanWork;  // adjoint buffers (adjoint_api.cu), created on first use
 
 struct mfcfd {
     int dev = 0;
@@ -79,6 +80,8 @@ struct mfcfd {
     std::string err;
     std::vector<double> shape_cp;
     AdjointState *adj = nullptr;
+    TanWork *tan = nullptr;     // mfcfd_tangent's device workspace
+    int *d_perm = nullptr;      // perm on the device
     // device address of the fixed residue-history array of mfcfd_run_noalloc
     // on this handle's device, resolved by mfcfd_create (nullptr if that
     // lookup failed; noalloc_err then says why)
@@ -135,6 +138,7 @@ int upload_state_aux(mfcfd_t *h);
 // (enqueued on the handle's stream).
 int reset_run(mfcfd_t *h, int it_first);
 void free_adjoint(mfcfd_t *h);
+void drop_tangent(mfcfd_t *h);  // frees mfcfd_tangent's workspace
 template <class T>
 inline cudaError_t dmalloc(T **p, size_t count) {
     return cudaMalloc(reinterpret_cast<void **>(p), count * sizeof(T) + (count == 0 ? 16 : 0));

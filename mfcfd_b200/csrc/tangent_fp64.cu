@@ -10,25 +10,29 @@
 // that direction.  For the reverse-mode gradient g of mfcfd_adjoint,
 // dJ/de = <g, (dx, dy)> (the dot-product test).
 //
-// The kernels are plain thread-per-point passes over the same device
-// templates as the primal (reconstruct, kstate, split/quadrant fluxes,
-// q_from_prim, prim_to_conserved, conserved_ubar) instantiated on Dual, with
-// each list sum in slot order; min_dist is data, as in the reference.
+// The D and I passes and the state update are thread-per-point passes over the
+// primal's device templates (q_from_prim, prim_to_conserved, conserved_ubar)
+// instantiated on Dual; the flux pass has the primal's split of the work and
+// forms (flux_math.cuh), differentiated.  min_dist is data, as in the
+// reference.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <new>
+#include <type_traits>
 #include <vector>
 
 // handle.h (and through it the primal device templates) comes before
 // dual.cuh: the templates' double instantiations must see only the libm
 // overloads, and the Dual ones are found by argument-dependent lookup.
 #include "handle.h"
+#include "flux_math.cuh"
+#include "flux_tile.cuh"
 #include "dual.cuh"
 #include "objective.h"
 
 using namespace lskum;
 using lskum_host::cuda_fail;
-using lskum_host::dmalloc;
 using lskum_host::fail;
 
 namespace {
@@ -186,86 +190,201 @@ k_t_inner(Geom g, TanState s, int qc, int a) {
     st_dual8(s.dqv[a ^ 1], s.dqt[a ^ 1], i, dx, dy);
 }
 
-// cal_flux_residual_d + state_update_d + eval_q_variables_d of the new state.
-// Each list is summed over its slots in slot order (the reference's order);
-// the states of a neighbour in two lists are recomputed per list.
+// The split lists' solve coefficients (k_flux_coef of the primal) as Duals:
+// per point and list a, b of the slot weight c = a dels + b deln (y lists: the
+// roles swapped).  Geometry: once per call.
 __global__ void __launch_bounds__(TB)
-k_t_flux(Geom g, Consts c, TanState s, int A, int B, int qc, int dqa, int rk, int last) {
+k_t_coef(Geom g, TanState s, Dual *__restrict__ co) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.n) return;
     const int kind = i < g.nw ? KIND_WALL : (i < g.nw + g.no ? KIND_OUTER : KIND_INTERIOR);
     Dual xi, yi;
     xy_dual(g, s, i, xi, yi);
     const Dual nx(g.nrm[i].x, s.nrm_t[i].x), ny(g.nrm[i].y, s.nrm_t[i].y);
-    const Dual pi_c(c.pi), gm1(c.gm1), eps2i(g.eps2[i]);
-    Dual qi[4], dxi[4], dyi[4], qmaxi[4], qmini[4];
-    ld_dual4(s.qv[qc], s.qt[qc], i, qi);
-    ld_dual8(s.dqv[dqa], s.dqt[dqa], i, dxi, dyi);
-    ld_dual8(s.qmv, s.qmt, i, qmaxi, qmini);
-    const int nb = g.nbhs[i];
-    const unsigned long long mx = g.mx[i], my = g.my[i];
-    const Dual s2q(kind == KIND_WALL ? -1.0 : 1.0);
-    const Dual tx = ny, ty = -nx;
-    Dual G[4][4];
+    const unsigned long long bits[2] = {g.mx[i], g.my[i]};
+    Dual sxx[4], syy[4], sxy[4];
+    for (int r = 0; r < g.nbhs[i]; ++r) {
+        Dual xk, yk;
+        xy_dual(g, s, g.conn[(size_t)r * g.n + i], xk, yk);
+        const Dual delx = xk - xi, dely = yk - yi;
+        const Dual dels = delx * ny - dely * nx, deln = delx * nx + dely * ny;
+        const Dual a = dels * dels, b = deln * deln, c = dels * deln;
+#pragma unroll
+        for (int L = 0; L < 4; ++L) {
+            if (!((bits[L >> 1] >> (r + ((L & 1) ? 32 : 0))) & 1ull)) continue;
+            sxx[L] += a;
+            syy[L] += b;
+            sxy[L] += c;
+        }
+    }
+#pragma unroll
     for (int L = 0; L < 4; ++L) {
-        if ((kind == KIND_WALL && L == 2) || (kind == KIND_OUTER && L == 3)) continue;
-        const unsigned long long bits = ((L < 2) ? mx : my) >> ((L & 1) ? 32 : 0);
-        const Dual sg((L & 1) ? -1.0 : 1.0);
-        Dual sdx2, sdy2, sdxy, fx[4], fy[4];
-        for (int r = 0; r < nb; ++r) {
-            if (!((bits >> r) & 1ull)) continue;
-            const int k = g.conn[r * g.n + i];
-            Dual xk, yk;
-            xy_dual(g, s, k, xk, yk);
-            const Dual delx = xk - xi, dely = yk - yi;
-            Dual qk[4], dxk[4], dyk[4], qmaxk[4], qmink[4];
-            ld_dual4(s.qv[qc], s.qt[qc], k, qk);
-            ld_dual8(s.dqv[dqa], s.dqt[dqa], k, dxk, dyk);
-            ld_dual8(s.qmv, s.qmt, k, qmaxk, qmink);
-            Dual u1, u2, rho, pr;
-            reconstruct<Dual>(qk, dxk, dyk, qmaxk, qmink, Dual(g.eps2[k]), delx, dely, gm1, u1,
-                              u2, rho, pr);
-            const KStateT<Dual> sk = kstate<Dual>(u1, u2, rho, pr, nx, ny, pi_c);
-            reconstruct<Dual>(qi, dxi, dyi, qmaxi, qmini, eps2i, delx, dely, gm1, u1, u2, rho,
-                              pr);
-            const KStateT<Dual> si = kstate<Dual>(u1, u2, rho, pr, nx, ny, pi_c);
-            Dual Gi[4], Gk[4];
-            if (L < 2) {
+        const bool none = (kind == KIND_WALL && L == 2) || (kind == KIND_OUTER && L == 3);
+        const Dual ob = Dual(1.0) / (sxx[L] * syy[L] - sxy[L] * sxy[L]);
+        co[8 * (size_t)i + 2 * L] = none ? Dual() : (L < 2 ? syy[L] : sxx[L]) * ob;
+        co[8 * (size_t)i + 2 * L + 1] = none ? Dual() : -(sxy[L] * ob);
+    }
+}
+
+// limited_qtilde (flux_math.cuh) on Duals.
+__device__ __forceinline__ Dual limited_dual(Dual t, Dual q, Dual qmax, Dual qmin, double eps2) {
+    const Dual dn(-0.5 * t.v, -0.5 * t.d);
+    const Dual dp = (dn.v > 0.0 ? qmax : qmin) - q;
+    const Dual a = dp * dp + Dual(eps2);
+    const Dual num = a - t * dp, den = a + dn * (dp - t);
+    const double id = rcp_h3(den.v), f = num.v * id;
+    const bool act = f < 1.0 && ::fabs(dn.v) > MFCFD_VENKAT_THR;
+    const Dual phi(act ? f : 1.0, act ? (num.d - f * den.d) * id : 0.0);
+    return q + phi * dn;
+}
+
+// The derivative of a kinetic state (values s, velocity u) from its limited
+// qtilde's (kstate_pre / kstate_pair of flux_math.cuh, differentiated).
+__device__ __forceinline__ KStateT<Dual> kstate_dual(const KState &s, const double u[2],
+                                                     const Dual qt[4], Dual nx, Dual ny) {
+    const double beta = -0.5 * qt[3].v, dbeta = -0.5 * qt[3].d;
+    const double sb = beta * rsqrt_h3(beta), dsb = sb * s.pbr * dbeta;
+    const double dpbr = s.pbr * s.pbr * qt[3].d;
+    const double du1 = qt[1].d * s.pbr + qt[1].v * dpbr, du2 = qt[2].d * s.pbr + qt[2].v * dpbr;
+    KStateT<Dual> k;
+    k.pbr = Dual(s.pbr, dpbr);
+    k.usq = Dual(s.usq, 2.0 * (u[0] * du1 + u[1] * du2));
+    const double dtexp = qt[0].d + dbeta * s.usq + beta * k.usq.d;
+    k.rho = Dual(s.rho, s.rho * (dtexp - 5.0 * s.pbr * dbeta));  // 2.5 / beta = 5 p/rho
+    k.ut = Dual(s.ut, du1 * ny.v + u[0] * ny.d - (du2 * nx.v + u[1] * nx.d));
+    k.un = Dual(s.un, du1 * nx.v + u[0] * nx.d + (du2 * ny.v + u[1] * ny.d));
+    const double S1 = s.ut * sb, S2 = s.un * sb;
+    const double dS1 = k.ut.d * sb + s.ut * dsb, dS2 = k.un.d * sb + s.un * dsb;
+    // B = E h with h = 1 / (2 sqrt(pi beta)), so E = 2 sqrt(pi) sb B and dh = -h p/rho dbeta;
+    // d erf(S) = 2/sqrt(pi) E dS = 4 sb B dS
+    k.B1 = Dual(s.B1, -s.B1 * (2.0 * S1 * dS1 + s.pbr * dbeta));
+    k.B2 = Dual(s.B2, -s.B2 * (2.0 * S2 * dS2 + s.pbr * dbeta));
+    k.e1 = Dual(s.e1, 4.0 * sb * s.B1 * dS1);
+    k.e2 = Dual(s.e2, 4.0 * sb * s.B2 * dS2);
+    return k;
+}
+
+// flux_split (flux_math.cuh) on Duals.
+__device__ __forceinline__ void flux_split_dual(const KStateT<Dual> &s, Dual u, Dual o, Dual B,
+                                                Dual e, double sg, Dual G[4]) {
+    const Dual A(0.5 + 0.5 * sg * e.v, 0.5 * sg * e.d);
+    const Dual a = u * A + Dual(sg * B.v, sg * B.d);
+    const Dual pA = s.pbr * A;
+    const Dual w6(6.0 * s.pbr.v + s.usq.v, 6.0 * s.pbr.d + s.usq.d);
+    G[0] = s.rho * a;
+    G[1] = s.rho * (u * a + pA);
+    G[2] = o * G[0];
+    G[3] = Dual(0.5 * s.rho.v, 0.5 * s.rho.d) * (w6 * a + u * pA);
+}
+
+// cal_flux_residual_d: eight lanes a point, one slot a lane, and the pooled
+// slot weights of the primal flux pass; the sum of the list derivatives as
+// four values, then four derivatives, into fs [n][8].  94 us at 64,000 points;
+// a thread a point, with both states recomputed for each list and four list
+// sums of Duals, spilled at 255 registers and took 354.  Bound by latency at 8
+// warps an SM.
+__global__ void __launch_bounds__(TB)
+k_t_flux(Geom g, TanState s, int qc, int dqa, const Dual *__restrict__ coef,
+         double *__restrict__ fs) {
+    const int lane = threadIdx.x % LPP;
+    const int i = (blockIdx.x * TB + threadIdx.x) / LPP;
+    const bool valid = i < g.n;
+    const int nb = valid ? g.nbhs[i] : 0;
+    Dual v[4];
+    for (int r = lane; r < nb; r += LPP) {
+        const int kind = i < g.nw ? KIND_WALL : (i < g.nw + g.no ? KIND_OUTER : KIND_INTERIOR);
+        const int k = g.conn[(size_t)r * g.n + i];
+        Dual xi, yi, xk, yk;
+        xy_dual(g, s, i, xi, yi);
+        xy_dual(g, s, k, xk, yk);
+        const Dual nx(g.nrm[i].x, s.nrm_t[i].x), ny(g.nrm[i].y, s.nrm_t[i].y);
+        const Dual delx = xk - xi, dely = yk - yi;
+        Dual qt[2][4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int p = h ? k : i;
+            Dual q[4], dx[4], dy[4], hi[4], lo[4];
+            ld_dual4(s.qv[qc], s.qt[qc], p, q);
+            ld_dual8(s.dqv[dqa], s.dqt[dqa], p, dx, dy);
+            ld_dual8(s.qmv, s.qmt, p, hi, lo);
+            const double eps2 = g.eps2[p];
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+                qt[h][m] = limited_dual(delx * dx[m] + dely * dy[m], q[m], hi[m], lo[m], eps2);
+        }
+        KStateT<Dual> si, sk;
+        {
+            const double qi[4] = {qt[0][0].v, qt[0][1].v, qt[0][2].v, qt[0][3].v};
+            const double qk[4] = {qt[1][0].v, qt[1][1].v, qt[1][2].v, qt[1][3].v};
+            KState vi, vk;
+            double ui[2], uk[2];
+            kstate_pair(qi, qk, nx.v, ny.v, 0.56418958354775628695, vi, vk, ui, uk);
+            si = kstate_dual(vi, ui, qt[0], nx, ny);
+            sk = kstate_dual(vk, uk, qt[1], nx, ny);
+        }
+        const Dual dels = delx * ny - dely * nx, deln = delx * nx + dely * ny;
+        const Dual *co = coef + 8 * (size_t)i;
+        // the lists holding the neighbour, two of a direction only when its
+        // projection is exactly 0
+        const unsigned long long mx = g.mx[i], my = g.my[i];
+#pragma unroll 1
+        for (int l = 0; l < 2; ++l) {
+            const double sg = l ? -1.0 : 1.0;
+            if ((mx >> (r + 32 * l)) & 1ull) {
+                const Dual w = co[2 * l] * dels + co[2 * l + 1] * deln;
+                Dual Gi[4], Gk[4];
                 if (kind == KIND_INTERIOR) {
-                    flux_gx<Dual>(si, sg, Gi);
-                    flux_gx<Dual>(sk, sg, Gk);
+                    flux_split_dual(si, si.ut, si.un, si.B1, si.e1, sg, Gi);
+                    flux_split_dual(sk, sk.ut, sk.un, sk.B1, sk.e1, sg, Gk);
                 } else {
-                    flux_quad<Dual>(si, sg, s2q, Gi);
-                    flux_quad<Dual>(sk, sg, s2q, Gk);
+                    const Dual s2(kind == KIND_WALL ? -1.0 : 1.0);
+                    flux_quad<Dual>(si, Dual(sg), s2, Gi);
+                    flux_quad<Dual>(sk, Dual(sg), s2, Gk);
                 }
-            } else {
-                flux_gy<Dual>(si, sg, Gi);
-                flux_gy<Dual>(sk, sg, Gk);
+#pragma unroll
+                for (int m = 0; m < 4; ++m) v[m] += w * (Gk[m] - Gi[m]);
             }
-            const Dual dels = delx * tx + dely * ty;
-            const Dual deln = delx * nx + dely * ny;
-            sdx2 = sdx2 + dels * dels;
-            sdy2 = sdy2 + deln * deln;
-            sdxy = sdxy + dels * deln;
-            for (int m = 0; m < 4; ++m) {
-                const Dual d = Gk[m] - Gi[m];
-                fx[m] = fx[m] + d * dels;
-                fy[m] = fy[m] + d * deln;
+            if ((my >> (r + 32 * l)) & 1ull) {
+                const Dual w = co[4 + 2 * l] * deln + co[5 + 2 * l] * dels;
+                Dual Gi[4], Gk[4];
+                flux_split_dual(si, si.un, si.ut, si.B2, si.e2, sg, Gi);
+                flux_split_dual(sk, sk.un, sk.ut, sk.B2, sk.e2, sg, Gk);
+                v[0] += w * (Gk[0] - Gi[0]);
+                v[1] += w * (Gk[2] - Gi[2]);
+                v[2] += w * (Gk[1] - Gi[1]);
+                v[3] += w * (Gk[3] - Gi[3]);
             }
         }
-        const Dual one_by_det = Dual(1.0) / (sdx2 * sdy2 - sdxy * sdxy);
-        for (int m = 0; m < 4; ++m)
-            G[L][m] = L < 2 ? (fx[m] * sdy2 - fy[m] * sdxy) * one_by_det
-                            : (fy[m] * sdx2 - fx[m] * sdxy) * one_by_det;
     }
-    // state_update_d (state_update_d.F90)
-    const Dual delta(s.dlv[i], s.dlt[i]);
+    __syncwarp();
+    // lane t of a point gets entry t of (four values, four derivatives)
+    const unsigned full = 0xffffffffu;
+    const bool h4 = lane & 4, h2 = lane & 2, h1 = lane & 1;
+    double a[4], b[2];
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+        a[m] = (h4 ? v[m].d : v[m].v) + __shfl_xor_sync(full, h4 ? v[m].v : v[m].d, 4);
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+        b[m] = (h2 ? a[2 + m] : a[m]) + __shfl_xor_sync(full, h2 ? a[m] : a[2 + m], 2);
+    const double sum = (h1 ? b[1] : b[0]) + __shfl_xor_sync(full, h1 ? b[0] : b[1], 1);
+    if (valid) fs[8 * (size_t)i + lane] = sum;
+}
+
+// state_update_d (state_update_d.F90) + eval_q_variables_d of the new state.
+__global__ void __launch_bounds__(TB)
+k_t_update(Geom g, Consts c, TanState s, const double *__restrict__ fs, int A, int B, int qc,
+           int rk, int last) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= g.n) return;
+    const int kind = i < g.nw ? KIND_WALL : (i < g.nw + g.no ? KIND_OUTER : KIND_INTERIOR);
+    const Dual nx(g.nrm[i].x, s.nrm_t[i].x), ny(g.nrm[i].y, s.nrm_t[i].y);
+    const Dual pi_c(c.pi), gm1(c.gm1);
+    Dual delta(s.dlv[i], s.dlt[i]);
+    if (kind == KIND_WALL) delta = Dual(2.0) * delta;
     Dual fr[4];
-    for (int m = 0; m < 4; ++m) {
-        if (kind == KIND_WALL) fr[m] = Dual(2.0) * delta * (G[0][m] + G[1][m] + G[3][m]);
-        else if (kind == KIND_OUTER) fr[m] = delta * (G[0][m] + G[1][m] + G[2][m]);
-        else fr[m] = delta * (G[0][m] + G[1][m] + G[2][m] + G[3][m]);
-    }
+    for (int m = 0; m < 4; ++m)
+        fr[m] = delta * Dual(fs[8 * (size_t)i + m], fs[8 * (size_t)i + 4 + m]);
     Dual P[4], U[4], Uo[4];
     ld_dual4(rk == 1 ? s.pv[A] : s.pv[B], rk == 1 ? s.pt[A] : s.pt[B], i, P);
     if (kind == KIND_OUTER) {
@@ -313,38 +432,95 @@ struct TanShape {
     const int *idx, *left, *right, *shape;
 };
 
-// compute_cl_cd_cm_d (compute_force_coeffs_d.F90), one thread, shape points
-// in grid order: out[0] = J, out[1] = dJ/de.
-__global__ void k_t_forces(Geom g, TanState s, TanShape t, int cur, double mach, double cos_t,
-                           double sin_t, int objective, double *out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// compute_cl_cd_cm_d (compute_force_coeffs_d.F90): out[0] = J, out[1] =
+// dJ/de.  One block: the points' terms in parallel, thread 0 adds them shape by
+// shape in grid order (the reference's).
+constexpr int TF = 512;
+__global__ void __launch_bounds__(TF)
+k_t_forces(Geom g, TanState s, TanShape t, int cur, double mach, double cos_t, double sin_t,
+           int objective, double *out) {
+    __shared__ Dual th[TF], tv[TF];
+    __shared__ int ts[TF];
     const double pr_inf = 1.0 / 1.4;
     const Dual temp(0.5 * 1.0 * mach * mach);
     Dual J;
     for (int sh = 0; sh < t.shapes; ++sh) {
         Dual H, V;
-        for (int j = 0; j < t.npts; ++j) {
-            if (t.shape[j] != sh) continue;
-            const int m = t.idx[j], l = t.left[j], r = t.right[j];
-            Dual lx, ly, mxx, myy, rx, ry;
-            xy_dual(g, s, l, lx, ly);
-            xy_dual(g, s, m, mxx, myy);
-            xy_dual(g, s, r, rx, ry);
-            const Dual ds1 = sqrt((mxx - lx) * (mxx - lx) + (myy - ly) * (myy - ly));
-            const Dual ds2 = sqrt((rx - mxx) * (rx - mxx) + (ry - myy) * (ry - myy));
-            const Dual ds = Dual(0.5) * (ds1 + ds2);
-            const Dual nx(g.nrm[m].x, s.nrm_t[m].x), ny(g.nrm[m].y, s.nrm_t[m].y);
-            Dual cp = Dual(s.pv[cur][m].d, s.pt[cur][m].d) - Dual(pr_inf);
-            cp = -cp / temp;
-            H = H + cp * nx * ds;
-            V = V + cp * ny * ds;
+        for (int j0 = 0; j0 < t.npts; j0 += TF) {
+            const int j = j0 + threadIdx.x;
+            if (j < t.npts) {
+                const int m = t.idx[j], l = t.left[j], r = t.right[j];
+                Dual lx, ly, mxx, myy, rx, ry;
+                xy_dual(g, s, l, lx, ly);
+                xy_dual(g, s, m, mxx, myy);
+                xy_dual(g, s, r, rx, ry);
+                const Dual ds1 = sqrt((mxx - lx) * (mxx - lx) + (myy - ly) * (myy - ly));
+                const Dual ds2 = sqrt((rx - mxx) * (rx - mxx) + (ry - myy) * (ry - myy));
+                const Dual ds = Dual(0.5) * (ds1 + ds2);
+                const Dual nx(g.nrm[m].x, s.nrm_t[m].x), ny(g.nrm[m].y, s.nrm_t[m].y);
+                Dual cp = Dual(s.pv[cur][m].d, s.pt[cur][m].d) - Dual(pr_inf);
+                cp = -cp / temp;
+                th[threadIdx.x] = cp * nx * ds;
+                tv[threadIdx.x] = cp * ny * ds;
+                ts[threadIdx.x] = t.shape[j];
+            }
+            __syncthreads();
+            if (threadIdx.x == 0)
+                for (int q = 0; q < min(TF, t.npts - j0); ++q)
+                    if (ts[q] == sh) {
+                        H += th[q];
+                        V += tv[q];
+                    }
+            __syncthreads();
         }
         const Dual cl = V * Dual(cos_t) - H * Dual(sin_t);
         const Dual cd = H * Dual(cos_t) + V * Dual(sin_t);
         J = J + (objective == 1 ? cd : cl);
     }
-    out[0] = J.v;
-    out[1] = J.d;
+    if (threadIdx.x == 0) {
+        out[0] = J.v;
+        out[1] = J.d;
+    }
+}
+
+// The seed in the handle's point order, d the caller-order directions (dx, then
+// dy; a missing one is zero).
+__global__ void k_t_seed(int n, const int *__restrict__ perm, const double *__restrict__ d,
+                         double2 *__restrict__ xy_t, double2 *__restrict__ nrm_t) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    xy_t[p] = make_double2(d[perm[p]], d[n + perm[p]]);
+    nrm_t[p] = make_double2(0.0, 0.0);
+}
+
+// point_normals_d.F90 of the boundary points and, of the outer ones, the
+// freestream half of Ubar (state_update.F90:248-263) with its derivative.
+__global__ void k_t_normals(Geom g, TanState s, const int *__restrict__ left,
+                            const int *__restrict__ right, double u1_inf, double u2_inf,
+                            double pi, double2 *__restrict__ nrm_t, Dual *__restrict__ obc) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= g.nw + g.no) return;
+    Dual lx, ly, mx, my, rx, ry;
+    xy_dual(g, s, left[p], lx, ly);
+    xy_dual(g, s, p, mx, my);
+    xy_dual(g, s, right[p], rx, ry);
+    const Dual vx = Dual(0.5) * ((my - ly) + (ry - my)), vy = Dual(0.5) * ((mx - lx) + (rx - mx));
+    const Dual det = sqrt(vx * vx + vy * vy);
+    const Dual dnx = -vx / det, dny = vy / det;
+    nrm_t[p] = make_double2(dnx.d, dny.d);
+    if (p < g.nw) return;
+    const double pr_inf = 1.0 / 1.4, rho_inf = 1.0, gamma = 1.4;
+    const Dual nx(g.nrm[p].x, dnx.d), ny(g.nrm[p].y, dny.d);
+    const Dual u1r = Dual(u1_inf) * ny - Dual(u2_inf) * nx;
+    const Dual u2r = Dual(u1_inf) * nx + Dual(u2_inf) * ny;
+    const double beta = (0.5 * rho_inf) / pr_inf;
+    const Dual S2 = u2r * Dual(::sqrt(beta));
+    Dual *o = obc + 8 * (size_t)(p - g.nw);
+    o[0] = u1r;
+    o[1] = u2r;
+    o[2] = Dual(pr_inf / (rho_inf * (gamma - 1.0))) + Dual(0.5) * (u1r * u1r + u2r * u2r);
+    o[3] = Dual(0.5) * (Dual(1.0) - erf(S2));
+    o[4] = exp(-S2 * S2) / Dual(2.0 * ::sqrt(pi * beta));
 }
 
 // Per-point terms of the secondary objectives (compute_entropy.F90:21-27,
@@ -399,6 +575,110 @@ inline int nblk(int n, int b) { return (n + b - 1) / b; }
 
 }  // namespace
 
+// Device workspace of mfcfd_tangent, kept with the handle: one allocation,
+// made by the first call (27 allocations and frees a call took longer than ten
+// iterations of 64,000 points) and given back by mfcfd_destroy or when the
+// adjoint needs the memory (drop_tangent).
+struct TanWork {
+    char *block = nullptr;
+    TanState s{};
+    double2 *xy_t = nullptr, *nrm_t = nullptr;
+    Dual *obc = nullptr, *coef = nullptr;
+    double *fs = nullptr, *dir = nullptr, *out = nullptr;
+    int *left = nullptr, *right = nullptr;  // ring neighbours of the boundary points
+    int *si = nullptr, *sl = nullptr, *sr = nullptr, *ss = nullptr;  // shape points, grid order
+    int nshape = 0;
+};
+
+void lskum_host::drop_tangent(mfcfd_t *h) {
+    if (!h->tan) return;
+    if (h->tan->block) cudaFree(h->tan->block);
+    delete h->tan;
+    h->tan = nullptr;
+}
+
+namespace {
+
+int tan_setup(mfcfd_t *h) {
+    if (h->tan) return MFCFD_OK;
+    const int n = h->n, nw = h->nw, no = h->no;
+    std::vector<int> inv(n);
+    for (int p = 0; p < n; ++p) inv[h->perm[p]] = p;
+    std::vector<int> idx[6];  // left, right, si, sl, sr, ss
+    for (int p = 0; p < nw + no; ++p) {
+        idx[0].push_back(inv[h->left0[h->perm[p]] - 1]);
+        idx[1].push_back(inv[h->right0[h->perm[p]] - 1]);
+    }
+    for (int i = 0; i < n; ++i) {
+        if (h->flag2_0[i] <= 0) continue;
+        idx[2].push_back(inv[i]);
+        idx[3].push_back(inv[h->left0[i] - 1]);
+        idx[4].push_back(inv[h->right0[i] - 1]);
+        idx[5].push_back(h->flag2_0[i] - 1);
+    }
+    TanWork *w = new (std::nothrow) TanWork();
+    if (!w) return fail(h, MFCFD_ERR_OOM, "host allocation failed");
+    w->nshape = (int)idx[2].size();
+    // the same walk sizes the block, then hands out its parts
+    size_t bytes = 0;
+    for (int pass = 0; pass < 2; ++pass) {
+        size_t at = 0;
+        auto take = [&](auto *&p, size_t count) {
+            using T = std::remove_reference_t<decltype(*p)>;
+            if (pass) p = reinterpret_cast<T *>(w->block + at);
+            at += (count * sizeof(T) + 255) / 256 * 256;
+        };
+        TanState &s = w->s;
+        for (int b = 0; b < 2; ++b) {
+            take(s.pv[b], n);
+            take(s.pt[b], n);
+            take(s.qv[b], n);
+            take(s.qt[b], n);
+            take(s.dqv[b], (size_t)8 * n);
+            take(s.dqt[b], (size_t)8 * n);
+        }
+        take(s.qmv, (size_t)8 * n);
+        take(s.qmt, (size_t)8 * n);
+        take(s.dlv, n);
+        take(s.dlt, n);
+        take(s.spv, n);
+        take(s.spt, n);
+        take(w->xy_t, n);
+        take(w->nrm_t, n);
+        take(w->obc, (size_t)8 * std::max(no, 1));
+        take(w->coef, (size_t)8 * n);
+        take(w->fs, (size_t)8 * n);
+        take(w->dir, (size_t)2 * n);
+        take(w->out, 2);
+        int **ints[6] = {&w->left, &w->right, &w->si, &w->sl, &w->sr, &w->ss};
+        for (int a = 0; a < 6; ++a) take(*ints[a], std::max<size_t>(idx[a].size(), 1));
+        if (pass) break;
+        bytes = at;
+        cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&w->block), bytes);
+        if (e != cudaSuccess) {
+            delete w;
+            return cuda_fail(h, e, "mfcfd_tangent cudaMalloc");
+        }
+    }
+    w->s.xy_t = w->xy_t;
+    w->s.nrm_t = w->nrm_t;
+    w->s.obc = w->obc;
+    h->tan = w;
+    int *dst[6] = {w->left, w->right, w->si, w->sl, w->sr, w->ss};
+    for (int a = 0; a < 6; ++a)
+        if (!idx[a].empty()) {
+            cudaError_t e = cudaMemcpy(dst[a], idx[a].data(), idx[a].size() * sizeof(int),
+                                       cudaMemcpyHostToDevice);
+            if (e != cudaSuccess) {
+                lskum_host::drop_tangent(h);
+                return cuda_fail(h, e, "mfcfd_tangent cudaMemcpy");
+            }
+        }
+    return MFCFD_OK;
+}
+
+}  // namespace
+
 extern "C" int mfcfd_tangent(mfcfd_t *h, int objective, int n_iters, const double *dx,
                              const double *dy, double *J, double *dJ) {
     if (!h) return MFCFD_ERR_ARG;
@@ -408,177 +688,75 @@ extern "C" int mfcfd_tangent(mfcfd_t *h, int objective, int n_iters, const doubl
     if (h->fp32 || h->p.power != 0.0)
         return fail(h, MFCFD_ERR_ARG, "mfcfd_tangent needs an FP64 handle with power = 0");
     const int n = h->n, nw = h->nw, no = h->no, m = h->p.inner_iterations, rks = h->p.rks;
+    DevGuard dg(h->dev);
+    CK(dg.err);
     CK(cudaStreamSynchronize(h->stream));
-    std::vector<int> inv(n);
-    for (int p = 0; p < n; ++p) inv[h->perm[p]] = p;
-    // seed and geometry derivatives (point_normals_d.F90 on the host)
-    std::vector<double2> hxy(n), hnrm(n), xy_t(n), nrm_t(n, make_double2(0.0, 0.0));
-    CK(cudaMemcpy(hxy.data(), h->d_xy, n * sizeof(double2), cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(hnrm.data(), h->d_nrm, n * sizeof(double2), cudaMemcpyDeviceToHost));
-    for (int p = 0; p < n; ++p)
-        xy_t[p] = make_double2(dx ? dx[h->perm[p]] : 0.0, dy ? dy[h->perm[p]] : 0.0);
-    auto X = [&](int p) { return Dual(hxy[p].x, xy_t[p].x); };
-    auto Y = [&](int p) { return Dual(hxy[p].y, xy_t[p].y); };
-    std::vector<Dual> obc((size_t)8 * std::max(no, 1));
-    const double pi = h->pi;
-    for (int p = 0; p < nw + no; ++p) {
-        const int l = inv[h->left0[h->perm[p]] - 1], r = inv[h->right0[h->perm[p]] - 1];
-        const Dual nx1 = Y(p) - Y(l), nx2 = Y(r) - Y(p), ny1 = X(p) - X(l), ny2 = X(r) - X(p);
-        const Dual vx = Dual(0.5) * (nx1 + nx2), vy = Dual(0.5) * (ny1 + ny2);
-        const Dual det = sqrt(vx * vx + vy * vy);
-        const Dual nx = -vx / det, ny = vy / det;
-        nrm_t[p] = make_double2(nx.d, ny.d);
-        if (p >= nw) {
-            // state_update.F90:248-263, the freestream half of Ubar
-            const double pr_inf = 1.0 / 1.4, rho_inf = 1.0, gamma = 1.4;
-            const Dual u1_inf(h->q_inf[1]), u2_inf(h->q_inf[2]);
-            const Dual tx = Dual(hnrm[p].y, nrm_t[p].y), ty = -Dual(hnrm[p].x, nrm_t[p].x);
-            const Dual nxd(hnrm[p].x, nrm_t[p].x), nyd(hnrm[p].y, nrm_t[p].y);
-            const Dual u1r = u1_inf * tx + u2_inf * ty;
-            const Dual u2r = u1_inf * nxd + u2_inf * nyd;
-            const Dual temp1 = (u1r * u1r + u2r * u2r);
-            const Dual e_inf = Dual(pr_inf / (rho_inf * (gamma - 1.0))) + Dual(0.5) * temp1;
-            const double beta = (0.5 * rho_inf) / pr_inf;
-            const Dual S2 = u2r * Dual(::sqrt(beta));
-            const Dual B2_inf = exp(-S2 * S2) / Dual(2.0 * ::sqrt(pi * beta));
-            const Dual A2n_inf = Dual(0.5) * (Dual(1.0) - erf(S2));
-            Dual *o = &obc[(size_t)8 * (p - nw)];
-            o[0] = u1r;
-            o[1] = u2r;
-            o[2] = e_inf;
-            o[3] = A2n_inf;
-            o[4] = B2_inf;
+    if (int st = tan_setup(h)) return st;
+    const TanWork &w = *h->tan;
+    const TanState &s = w.s;
+    cudaStream_t str = h->stream;
+    // the seed and the geometry's derivatives
+    if (dx) CK(cudaMemcpyAsync(w.dir, dx, sizeof(double) * n, cudaMemcpyHostToDevice, str));
+    else CK(cudaMemsetAsync(w.dir, 0, sizeof(double) * n, str));
+    if (dy) CK(cudaMemcpyAsync(w.dir + n, dy, sizeof(double) * n, cudaMemcpyHostToDevice, str));
+    else CK(cudaMemsetAsync(w.dir + n, 0, sizeof(double) * n, str));
+    k_t_seed<<<nblk(n, 256), 256, 0, str>>>(n, h->d_perm, w.dir, w.xy_t, w.nrm_t);
+    if (nw + no > 0)
+        k_t_normals<<<nblk(nw + no, 128), 128, 0, str>>>(h->geom, s, w.left, w.right, h->q_inf[1],
+                                                         h->q_inf[2], h->pi, w.nrm_t, w.obc);
+    k_t_coef<<<nblk(n, TB), TB, 0, str>>>(h->geom, s, w.coef);
+    // the handle's state (held fixed: derivative 0)
+    CK(cudaMemcpyAsync(s.pv[0], h->d_prim[h->cur], sizeof(R4) * n, cudaMemcpyDeviceToDevice, str));
+    CK(cudaMemsetAsync(s.pt[0], 0, sizeof(R4) * n, str));
+    int cur = 0, qc = 0;
+    k_t_init<<<nblk(n, 256), 256, 0, str>>>(n, s, cur, qc);
+    h->launches += 4;
+    for (int it = 0; it < n_iters; ++it) {
+        const int A = cur, B = cur ^ 1;
+        for (int rk = 1; rk <= rks; ++rk) {
+            k_t_grad<<<nblk(n, TB), TB, 0, str>>>(h->geom, h->consts, s, qc, rk == 1 ? 1 : 0);
+            for (int t = 1; t <= m; ++t)
+                k_t_inner<<<nblk(n, TB), TB, 0, str>>>(h->geom, s, qc, (t - 1) & 1);
+            k_t_flux<<<nblk(n, TB / LPP), TB, 0, str>>>(h->geom, s, qc, m & 1, w.coef, w.fs);
+            k_t_update<<<nblk(n, TB), TB, 0, str>>>(h->geom, h->consts, s, w.fs, A, B, qc, rk,
+                                                   rk == rks ? 1 : 0);
+            qc ^= 1;
+            h->launches += 3 + m;
         }
+        cur = B;
+        CK(cudaGetLastError());
     }
-    // shape points in grid order
-    std::vector<int> si, sl, sr, ss;
-    for (int i = 0; i < n; ++i) {
-        if (h->flag2_0[i] <= 0) continue;
-        si.push_back(inv[i]);
-        sl.push_back(inv[h->left0[i] - 1]);
-        sr.push_back(inv[h->right0[i] - 1]);
-        ss.push_back(h->flag2_0[i] - 1);
+    if (objective >= MFCFD_OBJ_ENTROPY) {
+        // secondary objectives: per-point Dual terms, summed in caller order
+        double *d_tv = w.fs, *d_td = w.fs + n;  // (the flux sums are done with)
+        const double gp = lskum_host::stagnation_gamma_power();
+        const double p0_inf = lskum_host::stagnation_p0_inf(h->p.mach);
+        k_t_obj_terms<<<nblk(n, 256), 256, 0, str>>>(h->geom, s, cur, objective, gp, p0_inf, d_tv,
+                                                     d_td);
+        h->launches += 1;
+        CK(cudaGetLastError());
+        std::vector<double> tv(n), td(n);
+        CK(cudaMemcpyAsync(tv.data(), d_tv, sizeof(double) * n, cudaMemcpyDeviceToHost, str));
+        CK(cudaMemcpyAsync(td.data(), d_td, sizeof(double) * n, cudaMemcpyDeviceToHost, str));
+        CK(cudaStreamSynchronize(str));
+        std::vector<int> inv(n);
+        for (int p = 0; p < n; ++p) inv[h->perm[p]] = p;
+        Dual sum;
+        for (int k = 0; k < n; ++k) sum = sum + Dual(tv[inv[k]], td[inv[k]]);
+        if (objective == MFCFD_OBJ_STAGNATION) sum = sum * Dual(1 / (p0_inf * p0_inf * n));
+        if (J) *J = sum.v;
+        if (dJ) *dJ = sum.d;
+        return MFCFD_OK;
     }
-    const size_t ns = std::max<size_t>(si.size(), 1);
-
-    // device buffers (freed on return)
-    std::vector<void *> owned;
-    auto take = [&](auto **p, size_t cnt) -> cudaError_t {
-        cudaError_t e = dmalloc(p, cnt);
-        if (e == cudaSuccess) owned.push_back(*p);
-        return e;
-    };
-    int st = MFCFD_OK;
-    TanState s{};
-    double2 *d_xyt = nullptr, *d_nrmt = nullptr;
-    Dual *d_obc = nullptr;
-    int *d_si = nullptr, *d_sl = nullptr, *d_sr = nullptr, *d_ss = nullptr;
-    double *d_out = nullptr;
-    cudaError_t e = take(&d_xyt, n);
-    if (e == cudaSuccess) e = take(&d_nrmt, n);
-    if (e == cudaSuccess) e = take(&d_obc, obc.size());
-    for (int b = 0; b < 2 && e == cudaSuccess; ++b) {
-        e = take(&s.pv[b], n);
-        if (e == cudaSuccess) e = take(&s.pt[b], n);
-        if (e == cudaSuccess) e = take(&s.qv[b], n);
-        if (e == cudaSuccess) e = take(&s.qt[b], n);
-        if (e == cudaSuccess) e = take(&s.dqv[b], (size_t)8 * n);
-        if (e == cudaSuccess) e = take(&s.dqt[b], (size_t)8 * n);
-    }
-    if (e == cudaSuccess) e = take(&s.qmv, (size_t)8 * n);
-    if (e == cudaSuccess) e = take(&s.qmt, (size_t)8 * n);
-    if (e == cudaSuccess) e = take(&s.dlv, n);
-    if (e == cudaSuccess) e = take(&s.dlt, n);
-    if (e == cudaSuccess) e = take(&s.spv, n);
-    if (e == cudaSuccess) e = take(&s.spt, n);
-    if (e == cudaSuccess) e = take(&d_si, ns);
-    if (e == cudaSuccess) e = take(&d_sl, ns);
-    if (e == cudaSuccess) e = take(&d_sr, ns);
-    if (e == cudaSuccess) e = take(&d_ss, ns);
-    if (e == cudaSuccess) e = take(&d_out, 2);
-    if (e != cudaSuccess) st = cuda_fail(h, e, "mfcfd_tangent cudaMalloc");
-    auto up = [&](void *d, const void *src, size_t bytes) {
-        if (st == MFCFD_OK && bytes) {
-            cudaError_t u = cudaMemcpy(d, src, bytes, cudaMemcpyHostToDevice);
-            if (u != cudaSuccess) st = cuda_fail(h, u, "mfcfd_tangent cudaMemcpy");
-        }
-    };
-    up(d_xyt, xy_t.data(), n * sizeof(double2));
-    up(d_nrmt, nrm_t.data(), n * sizeof(double2));
-    up(d_obc, obc.data(), obc.size() * sizeof(Dual));
-    up(d_si, si.data(), si.size() * sizeof(int));
-    up(d_sl, sl.data(), sl.size() * sizeof(int));
-    up(d_sr, sr.data(), sr.size() * sizeof(int));
-    up(d_ss, ss.data(), ss.size() * sizeof(int));
-    if (st == MFCFD_OK) {
-        s.xy_t = d_xyt;
-        s.nrm_t = d_nrmt;
-        s.obc = d_obc;
-        cudaStream_t str = h->stream;
-        // the handle's state (held fixed: derivative 0)
-        cudaError_t c1 = cudaMemcpyAsync(s.pv[0], h->d_prim[h->cur], sizeof(R4) * n,
-                                         cudaMemcpyDeviceToDevice, str);
-        if (c1 == cudaSuccess) c1 = cudaMemsetAsync(s.pt[0], 0, sizeof(R4) * n, str);
-        if (c1 != cudaSuccess) st = cuda_fail(h, c1, "mfcfd_tangent state copy");
-        int cur = 0, qc = 0;
-        if (st == MFCFD_OK) k_t_init<<<nblk(n, 256), 256, 0, str>>>(n, s, cur, qc);
-        for (int it = 0; it < n_iters && st == MFCFD_OK; ++it) {
-            const int A = cur, B = cur ^ 1;
-            for (int rk = 1; rk <= rks; ++rk) {
-                k_t_grad<<<nblk(n, TB), TB, 0, str>>>(h->geom, h->consts, s, qc, rk == 1 ? 1 : 0);
-                for (int t = 1; t <= m; ++t)
-                    k_t_inner<<<nblk(n, TB), TB, 0, str>>>(h->geom, s, qc, (t - 1) & 1);
-                k_t_flux<<<nblk(n, TB), TB, 0, str>>>(h->geom, h->consts, s, A, B, qc, m & 1, rk,
-                                                     rk == rks ? 1 : 0);
-                qc ^= 1;
-                h->launches += 2 + m;
-            }
-            cur = B;
-            cudaError_t le = cudaGetLastError();
-            if (le != cudaSuccess) st = cuda_fail(h, le, "mfcfd_tangent launch");
-        }
-        if (st == MFCFD_OK && objective >= MFCFD_OBJ_ENTROPY) {
-            // secondary objectives: per-point Dual terms, summed in caller order
-            double *d_tv = nullptr, *d_td = nullptr;
-            cudaError_t c2 = take(&d_tv, n);
-            if (c2 == cudaSuccess) c2 = take(&d_td, n);
-            const double gp = lskum_host::stagnation_gamma_power();
-            const double p0_inf = lskum_host::stagnation_p0_inf(h->p.mach);
-            if (c2 == cudaSuccess) {
-                k_t_obj_terms<<<nblk(n, 256), 256, 0, str>>>(h->geom, s, cur, objective, gp, p0_inf,
-                                                             d_tv, d_td);
-                h->launches += 1;
-                c2 = cudaGetLastError();
-            }
-            std::vector<double> tv(n), td(n);
-            if (c2 == cudaSuccess)
-                c2 = cudaMemcpyAsync(tv.data(), d_tv, sizeof(double) * n, cudaMemcpyDeviceToHost, str);
-            if (c2 == cudaSuccess)
-                c2 = cudaMemcpyAsync(td.data(), d_td, sizeof(double) * n, cudaMemcpyDeviceToHost, str);
-            if (c2 == cudaSuccess) c2 = cudaStreamSynchronize(str);
-            if (c2 != cudaSuccess) {
-                st = cuda_fail(h, c2, "mfcfd_tangent objective");
-            } else {
-                Dual sum;
-                for (int k = 0; k < n; ++k) sum = sum + Dual(tv[inv[k]], td[inv[k]]);
-                if (objective == MFCFD_OBJ_STAGNATION) sum = sum * Dual(1 / (p0_inf * p0_inf * n));
-                if (J) *J = sum.v;
-                if (dJ) *dJ = sum.d;
-            }
-        } else if (st == MFCFD_OK) {
-            TanShape ts{(int)si.size(), h->shapes, d_si, d_sl, d_sr, d_ss};
-            k_t_forces<<<1, 32, 0, str>>>(h->geom, s, ts, cur, h->p.mach, h->cos_t, h->sin_t,
-                                          objective, d_out);
-            h->launches += 2;
-            double o[2] = {0.0, 0.0};
-            cudaError_t c2 = cudaMemcpyAsync(o, d_out, sizeof(o), cudaMemcpyDeviceToHost, str);
-            if (c2 == cudaSuccess) c2 = cudaStreamSynchronize(str);
-            if (c2 != cudaSuccess) st = cuda_fail(h, c2, "mfcfd_tangent result");
-            if (J) *J = o[0];
-            if (dJ) *dJ = o[1];
-        }
-    }
-    cudaStreamSynchronize(h->stream);
-    for (void *p : owned) cudaFree(p);
-    return st;
+    const TanShape ts{w.nshape, h->shapes, w.si, w.sl, w.sr, w.ss};
+    k_t_forces<<<1, TF, 0, str>>>(h->geom, s, ts, cur, h->p.mach, h->cos_t, h->sin_t, objective,
+                                  w.out);
+    h->launches += 1;
+    CK(cudaGetLastError());
+    double o[2] = {0.0, 0.0};
+    CK(cudaMemcpyAsync(o, w.out, sizeof(o), cudaMemcpyDeviceToHost, str));
+    CK(cudaStreamSynchronize(str));
+    if (J) *J = o[0];
+    if (dJ) *dJ = o[1];
+    return MFCFD_OK;
 }
