@@ -127,7 +127,8 @@ struct HaloRows {
 // q_variables.F90:41-112 eval_q_derivatives and state_update.F90:190-236
 // func_delta over the rows of R, in slot order.
 template <class Rows>
-__device__ __forceinline__ void grad_sums(const Consts &c, const Rows &R, int nb, int with_delta,
+__device__ __forceinline__ void grad_sums(const Consts &c, const Geom &g, int i, const Rows &R,
+                                          int nb, int with_delta,
                                           double dx[4], double dy[4], double qmax[4],
                                           double qmin[4], double &min_delt) {
     const int me = R.self();
@@ -151,7 +152,7 @@ __device__ __forceinline__ void grad_sums(const Consts &c, const Rows &R, int nb
         }
         double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
         double dist = sqrt(delx * delx + dely * dely);
-        double w = c.power_zero ? 1.0 : pow(dist, c.power);
+        const double w = g.wsl ? __ldg(g.wsl + (size_t)r * g.n + i) : 1.0;
         sdx2 = sdx2 + delx * delx * w;
         sdy2 = sdy2 + dely * dely * w;
         sdxy = sdxy + delx * dely * w;
@@ -186,7 +187,7 @@ __device__ __forceinline__ void grad_sums(const Consts &c, const Rows &R, int nb
 // dq0y: the point's D-pass derivatives; the point's own dq_i and the
 // neighbours' come through R.
 template <class Rows>
-__device__ __forceinline__ void inner_sums(const Consts &c, const Rows &R, int nb,
+__device__ __forceinline__ void inner_sums(const Geom &g, int i, const Rows &R, int nb,
                                            const double dq0x[4], const double dq0y[4],
                                            double dx[4], double dy[4]) {
     const int me = R.self();
@@ -199,8 +200,7 @@ __device__ __forceinline__ void inner_sums(const Consts &c, const Rows &R, int n
         R.dqrow(k, dxk, dyk);
         const double2 pk = R.xy(k);
         double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
-        double w = 1.0;
-        if (!c.power_zero) w = pow(sqrt(delx * delx + dely * dely), c.power);
+        const double w = g.wsl ? __ldg(g.wsl + (size_t)r * g.n + i) : 1.0;
         sdx2 = sdx2 + delx * delx * w;
         sdy2 = sdy2 + dely * dely * w;
         sdxy = sdxy + delx * dely * w;
@@ -264,7 +264,7 @@ __device__ __forceinline__ void stage_halo(const Geom &g, const R4 *q, const dou
 // barrier but the schedule load; the lanes of a warp meet at __syncwarp
 // before the rows are read and before they are overwritten.
 __global__ void __launch_bounds__(HALO_BLOCK, HALO_MIN_BLOCKS_I)
-kb_inner_h(Geom g, Consts c, Sched s, const double *__restrict__ dq0,
+kb_inner_h(Geom g, Sched s, const double *__restrict__ dq0,
            const double *__restrict__ dq_in, double *__restrict__ dq_out) {
     extern __shared__ double2 hsm[];
     __shared__ SchedSmem ss;
@@ -284,10 +284,10 @@ kb_inner_h(Geom g, Consts c, Sched s, const double *__restrict__ dq0,
         __syncwarp();
         if (cur.i >= 0) {
             double dx[4], dy[4];
-            if (cur.hn > 0) inner_sums(c, hr, cur.nb, ax, ay, dx, dy);
+            if (cur.hn > 0) inner_sums(g, cur.i, hr, cur.nb, ax, ay, dx, dy);
             else
-                inner_sums(c, GlobalRows{g, nullptr, dq_in, nullptr, cur.i}, cur.nb, ax, ay, dx,
-                           dy);
+                inner_sums(g, cur.i, GlobalRows{g, nullptr, dq_in, nullptr, cur.i}, cur.nb, ax,
+                           ay, dx, dy);
             st8w(dq_out + 8 * (size_t)cur.i, dx, dy);
         }
         __syncwarp();
@@ -314,10 +314,11 @@ kb_grad_h(Geom g, Consts c, Sched s, const R4 *__restrict__ q, const double *__r
         __syncwarp();
         if (cur.i >= 0) {
             double dx[4], dy[4], qmax[4], qmin[4], min_delt;
-            if (cur.hn > 0) grad_sums(c, hr, cur.nb, with_delta, dx, dy, qmax, qmin, min_delt);
+            if (cur.hn > 0)
+                grad_sums(c, g, cur.i, hr, cur.nb, with_delta, dx, dy, qmax, qmin, min_delt);
             else
-                grad_sums(c, GlobalRows{g, q, nullptr, spd, cur.i}, cur.nb, with_delta, dx, dy,
-                          qmax, qmin, min_delt);
+                grad_sums(c, g, cur.i, GlobalRows{g, q, nullptr, spd, cur.i}, cur.nb, with_delta,
+                          dx, dy, qmax, qmin, min_delt);
             st8w(dq + 8 * (size_t)cur.i, dx, dy);
             st8w(qm + 8 * (size_t)cur.i, qmax, qmin);
             if (with_delta) delta[cur.i] = min_delt;
@@ -799,56 +800,51 @@ __global__ void k_init_state(Geom g, const R4 *__restrict__ prim, R4 *__restrict
     spd[i] = sqrt(P.b * P.b + P.c * P.c) + 3.0 * sqrt(P.d / P.a);
 }
 
-// compute_force_coeffs.F90:11-102, one thread, shape points in grid order.
-// One block of FORCE_BLOCK threads: per chunk of FORCE_BLOCK shape points the
-// threads form cp and the point's three terms in parallel, then thread 0
-// adds them to its shape's sums in point order (the reference's loop order),
-// so the sums do not depend on the launch.
-constexpr int FORCE_BLOCK = 1024;
+// compute_force_coeffs.F90:11-102.  One block of FORCE_BLOCK threads, so the
+// sums do not depend on the launch: a thread adds its points j, j +
+// FORCE_BLOCK, ... of a shape in grid order, then a tree over the block adds
+// the threads.  (Thread 0 adding every point in turn took 108 us at 1,280
+// shape points, 17 at 160; now 7 and 6.)
+constexpr int FORCE_BLOCK = 512;
 
 __global__ void __launch_bounds__(FORCE_BLOCK)
 k_forces(ShapeTab t, const R4 *__restrict__ prim, double mach, double cos_t, double sin_t,
          double *out) {
-    __shared__ double th[FORCE_BLOCK], tv[FORCE_BLOCK], tm[FORCE_BLOCK];
-    __shared__ int ts[FORCE_BLOCK];
+    __shared__ double sm[3][FORCE_BLOCK / 32];
     const double rho_inf = 1.0, pr_inf = 1.0 / 1.4;
-    double *H = out, *V = out + t.shapes, *PM = out + 2 * t.shapes;
     double *cp_out = out + 3 * t.shapes;
-    if (threadIdx.x == 0)
-        for (int s = 0; s < t.shapes; ++s) H[s] = V[s] = PM[s] = 0.0;
     const double temp = 0.5 * rho_inf * mach * mach;
-    for (int j0 = 0; j0 < t.npts; j0 += FORCE_BLOCK) {
-        const int j = j0 + threadIdx.x;
-        if (j < t.npts) {
-            const int m = t.idx[j];
+    const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+    for (int s = 0; s < t.shapes; ++s) {
+        double v[3] = {0.0, 0.0, 0.0};  // H, V, pitching moment
+        for (int j = threadIdx.x; j < t.npts; j += FORCE_BLOCK) {
+            if (t.shape[j] != s) continue;
             const double nx = t.geo[4 * j], ny = t.geo[4 * j + 1], ds = t.geo[4 * j + 2];
             const double mx = t.geo[4 * j + 3], my = t.my[j];
-            double cp = prim[m].d - pr_inf;
+            double cp = prim[t.idx[j]].d - pr_inf;
             cp = -cp / temp;
             cp_out[j] = cp;
-            th[threadIdx.x] = cp * nx * ds;
-            tv[threadIdx.x] = cp * ny * ds;
-            tm[threadIdx.x] = -cp * ny * ds * (mx - 0.25) + cp * nx * ds * (my);
-            ts[threadIdx.x] = t.shape[j];
+            v[0] = v[0] + cp * nx * ds;
+            v[1] = v[1] + cp * ny * ds;
+            v[2] = v[2] + (-cp * ny * ds * (mx - 0.25) + cp * nx * ds * (my));
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            for (int w = 16; w > 0; w >>= 1) v[c] = v[c] + __shfl_xor_sync(0xffffffffu, v[c], w);
+            if (lane == 0) sm[c][warp] = v[c];
         }
         __syncthreads();
         if (threadIdx.x == 0) {
-            const int nj = min(FORCE_BLOCK, t.npts - j0);
-            for (int q = 0; q < nj; ++q) {
-                const int s = ts[q];
-                H[s] = H[s] + th[q];
-                V[s] = V[s] + tv[q];
-                PM[s] = PM[s] + tm[q];
+            for (int c = 0; c < 3; ++c) {
+                v[c] = 0.0;
+                for (int w = 0; w < FORCE_BLOCK / 32; ++w) v[c] = v[c] + sm[c][w];
             }
+            out[s] = v[1] * cos_t - v[0] * sin_t;                // Cl
+            out[t.shapes + s] = v[0] * cos_t + v[1] * sin_t;     // Cd
+            out[2 * t.shapes + s] = v[2];
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0)
-        for (int s = 0; s < t.shapes; ++s) {
-            double h = H[s], v = V[s];
-            H[s] = v * cos_t - h * sin_t;  // Cl
-            V[s] = h * cos_t + v * sin_t;  // Cd
-        }
 }
 
 inline int nblk(int n, int b) { return (n + b - 1) / b; }
@@ -975,8 +971,9 @@ void launch_grad(const Geom &g, const Consts &c, const Sched &s, const R4 *q, co
 void launch_inner(const Geom &g, const Consts &c, const Sched &s, const double *dq0,
                   const double *dq_in, double *dq_out, int block, int grid, cudaStream_t st) {
     (void)block;
+    (void)c;
     kb_inner_h<<<grid > 0 ? grid : halo_wave(1, g.hc), HALO_BLOCK, halo_smem_bytes(1, g.hc), st>>>(
-        g, c, s, dq0, dq_in, dq_out);
+        g, s, dq0, dq_in, dq_out);
 }
 
 void launch_flux(const Geom &g, const Consts &c, const Sched &s, const StageBufs &b, int rk,
