@@ -208,7 +208,8 @@ int adj_setup(mfcfd_t *h) {
     CK(dmalloc(&a->fin, n));
     // the third entry of every list's inverse normal matrix (Geom::fcg)
     CK(dmalloc(&a->d_fcg, (size_t)4 * n));
-    launch_flux_coef(h->geom, 0, n, h->nw, h->no, 0.0, h->d_fco, nullptr, a->d_fcg, h->stream);
+    launch_flux_coef(h->geom, 0, n, h->nw, h->no, 0.0, h->d_fco, nullptr, a->d_fcg, nullptr,
+                     h->stream);
     CK(cudaGetLastError());
     h->geom.fcg = a->d_fcg;
     return MFCFD_OK;

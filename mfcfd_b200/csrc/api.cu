@@ -69,7 +69,7 @@ void free_all(mfcfd_t *h) {
         for (auto &g : row)
             if (g) cudaGraphExecDestroy(g);
     void *bufs[] = {h->d_xy, h->d_nrm, h->d_eps2, h->d_obc, h->d_conn, h->d_nbhs, h->d_mx,
-                    h->d_my, h->d_hoff, h->d_hrow, h->d_hloc, h->d_fco, h->d_wsl, h->d_perm, h->d_prim[0], h->d_prim[1], h->d_q[0], h->d_q[1], h->d_dq[0],
+                    h->d_my, h->d_hoff, h->d_hrow, h->d_hloc, h->d_fco, h->d_wsl, h->d_minv, h->d_perm, h->d_prim[0], h->d_prim[1], h->d_q[0], h->d_q[1], h->d_dq[0],
                     h->d_dq[1], h->d_dq[2], h->d_qm, h->d_delta, h->d_spd, h->d_res_part, h->d_flux_dbg,
                     h->d_hist, h->d_forces, h->d_ctl, h->d_sh_idx, h->d_sh_shape, h->d_sh_geo,
                     h->d_sh_my, h->f_prim[0], h->f_prim[1], h->f_q[0], h->f_q[1],
@@ -817,6 +817,7 @@ static int create_handle(const mfcfd_grid *grid, const mfcfd_params *params, int
         for (int b = 0; b < 3; ++b) ALLOC(h->d_dq[b], (size_t)8 * n);
         ALLOC(h->d_qm, (size_t)8 * n);
         ALLOC(h->d_fco, (size_t)8 * n);
+        ALLOC(h->d_minv, (size_t)4 * n);
         if (P.power != 0.0) ALLOC(h->d_wsl, (size_t)kp * n);
     } else {
         ALLOC(h->d_prim[0], n);  // FP64 copy of the state for forces/diagnostics
@@ -886,9 +887,11 @@ static int create_handle(const mfcfd_grid *grid, const mfcfd_params *params, int
     }
     if (!h->fp32) {
         // on the stream of the uploads above, and before the copies below
-        launch_flux_coef(h->geom, 0, nl, nw, no, P.power, h->d_fco, h->d_wsl, nullptr, nullptr);
+        launch_flux_coef(h->geom, 0, nl, nw, no, P.power, h->d_fco, h->d_wsl, nullptr, h->d_minv,
+                         nullptr);
         h->geom.fco = h->d_fco;
         h->geom.wsl = h->d_wsl;
+        h->geom.minv = h->d_minv;
     }
     h->consts.cfl = P.cfl;
     h->consts.power = P.power;
@@ -902,7 +905,7 @@ static int create_handle(const mfcfd_grid *grid, const mfcfd_params *params, int
     // resident blocks per pass (measured 3% faster at 1M points than a
     // block per tile, which reloads the schedule in every block)
     h->inst_h = InstInfo{0, nl, nw, no, 0, 0, flux_blocks(nl), 0};
-    h->sched = sched_view(h->d_inst, h->d_sched);
+    h->sched = sched_view(h->d_inst, h->d_sched, &h->inst_h);
     h->point_block = default_point_block(h->fp32);
     h->point_grid = std::min((nl + h->point_block - 1) / h->point_block,
                              wave_blocks(h->dev, 0, h->point_block, 0, h->fp32));

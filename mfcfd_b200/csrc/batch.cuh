@@ -28,6 +28,14 @@ __device__ __forceinline__ void load_sched(const Sched &s, SchedSmem &ss) {
     __syncthreads();
 }
 
+// Whole block: the scheduled tiles; a schedule of several instances is copied
+// into shared memory.
+__device__ __forceinline__ int sched_begin(const Sched &s, SchedSmem &ss) {
+    if (s.single) return __ldg(s.nact) ? s.one.ntiles : 0;
+    load_sched(s, ss);
+    return ss.pre[ss.nact];
+}
+
 // Active slot holding virtual tile v: the largest a with pre[a] <= v.
 __device__ __forceinline__ int find_slot(const SchedSmem &ss, int v) {
     int lo = 0, hi = ss.nact - 1;
@@ -45,34 +53,34 @@ struct TileRef {
     int j0;                        // instance-local index of the tile's first point
 };
 
-__device__ __forceinline__ TileRef sched_tile(const Sched &s, const SchedSmem &ss, int v) {
-    const int a = find_slot(ss, v);
-    const InstInfo &in = s.inst[ss.act[a]];
-    const int k = v - ss.pre[a];
+__device__ __forceinline__ TileRef tile_of(const InstInfo &in, int k) {
     return TileRef{in.base, in.n, in.nw, in.no, in.obc_off, in.tile0 + k, k * TILE};
+}
+
+__device__ __forceinline__ TileRef sched_tile(const Sched &s, const SchedSmem &ss, int v) {
+    if (s.single) return tile_of(s.one, v);
+    const int a = find_slot(ss, v);
+    return tile_of(s.inst[ss.act[a]], v - ss.pre[a]);
 }
 
 // sched_tile with the schedule read from global memory (through L1) instead
 // of a shared-memory copy: for kernels whose shared memory bounds residency.
 __device__ __forceinline__ TileRef sched_tile_global(const Sched &s, int v) {
+    if (s.single) return tile_of(s.one, v);
     int lo = 0, hi = __ldg(s.nact) - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (__ldg(s.pre + mid) <= v) lo = mid;
         else hi = mid - 1;
     }
-    const InstInfo &in = s.inst[__ldg(s.act + lo)];
-    const int k = v - __ldg(s.pre + lo);
-    return TileRef{in.base, in.n, in.nw, in.no, in.obc_off, in.tile0 + k, k * TILE};
+    return tile_of(s.inst[__ldg(s.act + lo)], v - __ldg(s.pre + lo));
 }
 
 // Global point of virtual point vp, or -1 for a padding point.
 __device__ __forceinline__ int sched_point(const Sched &s, const SchedSmem &ss, int vp) {
-    const int v = vp / TILE;
-    const int a = find_slot(ss, v);
-    const InstInfo &in = s.inst[ss.act[a]];
-    const int j = (v - ss.pre[a]) * TILE + vp % TILE;
-    return j < in.n ? in.base + j : -1;
+    const TileRef t = sched_tile(s, ss, vp / TILE);
+    const int j = t.j0 + vp % TILE;
+    return j < t.n ? t.base + j : -1;
 }
 
 }  // namespace lskum

@@ -63,7 +63,7 @@ struct mfcfd_batch {
     unsigned long long *d_mx = nullptr, *d_my = nullptr;
     int *d_hoff = nullptr, *d_hrow = nullptr;  // tile halos of the D and I passes
     unsigned char *d_hloc = nullptr;
-    double *d_fco = nullptr, *d_wsl = nullptr;  // FP64 flux pass: Geom::fco, wsl
+    double *d_fco = nullptr, *d_wsl = nullptr, *d_minv = nullptr;  // Geom::fco, wsl, minv (FP64)
     R4 *d_prim[2] = {nullptr, nullptr}, *d_q[2] = {nullptr, nullptr};
     double *d_dq[3] = {nullptr, nullptr, nullptr};
     double *d_qm = nullptr;
@@ -137,7 +137,7 @@ void drop_graphs(mfcfd_batch_t *b) {
 void free_batch(mfcfd_batch_t *b) {
     drop_graphs(b);
     void *bufs[] = {b->d_xy, b->d_nrm, b->d_eps2, b->d_obc, b->d_conn, b->d_nbhs, b->d_mx,
-                    b->d_my, b->d_hoff, b->d_hrow, b->d_hloc, b->d_fco, b->d_wsl, b->d_prim[0], b->d_prim[1], b->d_q[0], b->d_q[1], b->d_dq[0],
+                    b->d_my, b->d_hoff, b->d_hrow, b->d_hloc, b->d_fco, b->d_wsl, b->d_minv, b->d_prim[0], b->d_prim[1], b->d_q[0], b->d_q[1], b->d_dq[0],
                     b->d_dq[1], b->d_dq[2], b->d_qm, b->f_prim[0], b->f_prim[1], b->f_q[0], b->f_q[1],
                     b->f_dq[0], b->f_dq[1], b->f_dq[2], b->f_qm, b->f_eps2, b->f_dxy, b->f_w, b->f_lsq,
                     b->f_flsq, b->d_delta, b->d_spd,
@@ -582,6 +582,7 @@ int mfcfd_batch_create(int n_inst, const mfcfd_grid *const *grids, const mfcfd_p
         for (int k = 0; k < 3; ++k) BALLOC(b->d_dq[k], (size_t)8 * N);
         BALLOC(b->d_qm, (size_t)8 * N);
         BALLOC(b->d_fco, (size_t)8 * N);
+        BALLOC(b->d_minv, (size_t)4 * N);
         if (P0.power != 0.0) BALLOC(b->d_wsl, (size_t)kp * N);
     } else {
         BALLOC(b->d_prim[0], N);  // FP64 copy of the state for the force sums
@@ -653,9 +654,10 @@ int mfcfd_batch_create(int n_inst, const mfcfd_grid *const *grids, const mfcfd_p
         // on the stream of the uploads above, and before the copies below
         for (const InstInfo &in : info)
             launch_flux_coef(b->geom, in.base, in.n, in.nw, in.no, P0.power, b->d_fco, b->d_wsl,
-                             nullptr, nullptr);
+                             nullptr, b->d_minv, nullptr);
         b->geom.fco = b->d_fco;
         b->geom.wsl = b->d_wsl;
+        b->geom.minv = b->d_minv;
     }
     b->consts.cfl = P0.cfl;
     b->consts.power = P0.power;

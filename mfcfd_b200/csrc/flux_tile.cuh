@@ -140,7 +140,7 @@ template <class P>
 __device__ __forceinline__ void flux_pass(P &p, const Geom &g, const Sched &s,
                                           typename P::Smem *sm, double *res_part, int last, int ct,
                                           int coop) {
-    const int ntiles = __ldg(s.pre + __ldg(s.nact));
+    const int live = __ldg(s.nact), ntiles = s.single ? s.one.ntiles : __ldg(s.pre + live);
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     typename P::Smem &m = sm[coop ? 0 : warp];
     constexpr int ROWS = P::Smem::ROWS;
@@ -153,6 +153,7 @@ __device__ __forceinline__ void flux_pass(P &p, const Geom &g, const Sched &s,
     FluxHalo hx;
     hx.range(g, cur);
     hx.rows(g, lane, ROWS);
+    if (!live) return;  // (retired)
     auto stage = [&] {
         if (coop) p.template stage<FLUX_BLOCK>(cur, hx, m, threadIdx.x);
         else p.template stage<32>(cur, hx, m, lane);

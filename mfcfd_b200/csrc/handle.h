@@ -36,7 +36,7 @@ struct mfcfd {
     unsigned long long *d_mx = nullptr, *d_my = nullptr;
     int *d_hoff = nullptr, *d_hrow = nullptr;  // tile halos of the D and I passes
     unsigned char *d_hloc = nullptr;
-    double *d_fco = nullptr, *d_wsl = nullptr;  // FP64 flux pass: Geom::fco, wsl
+    double *d_fco = nullptr, *d_wsl = nullptr, *d_minv = nullptr;  // Geom::fco, wsl, minv (FP64)
     R4 *d_prim[2] = {nullptr, nullptr}, *d_q[2] = {nullptr, nullptr};
     double *d_dq[3] = {nullptr, nullptr, nullptr};  // D-pass result, then the inner iterations'
     double *d_qm = nullptr, *d_delta = nullptr, *d_spd = nullptr, *d_res_part = nullptr;

@@ -63,6 +63,9 @@ struct Geom {
     const double *wsl = nullptr;
     // reverse flux pass: the third entry of each list's inverse matrix ([n][4])
     const double *fcg = nullptr;
+    // FP64 D and I passes: the inverse of the full stencil's normal matrix, [n][4]
+    // (xx, xy, yy, unused)
+    const double *minv = nullptr;
 };
 // rows a tile halo stages at most (its local row indices are bytes)
 constexpr int HALO_CAP = 64;

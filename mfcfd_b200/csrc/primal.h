@@ -52,9 +52,14 @@ struct Sched {
     const int *pre;
     const int *act;
     const int *nact;
+    // A schedule of one instance (a single grid's) carries it in the kernel's
+    // parameters: only whether it still runs (*nact) is read from memory.
+    InstInfo one;
+    int single;
 };
-inline Sched sched_view(const InstInfo *inst, const int *blk) {
-    return Sched{inst, blk + SCHED_PRE, blk + SCHED_ACT, blk + SCHED_NACT};
+inline Sched sched_view(const InstInfo *inst, const int *blk, const InstInfo *one = nullptr) {
+    return Sched{inst, blk + SCHED_PRE, blk + SCHED_ACT, blk + SCHED_NACT,
+                 one ? *one : InstInfo{}, one ? 1 : 0};
 }
 // Host: the schedule of the instances with active[i] != 0, in instance order.
 inline void sched_fill(int *blk, const InstInfo *inst, const int *active, int n_inst) {
@@ -119,9 +124,10 @@ void launch_flux(const Geom &g, const Consts &c, const Sched &s, const StageBufs
                  bool last, int grid, int tiles, cudaStream_t st);
 // Fixed per grid: the list-solve coefficients of points [base, base + n) (wall,
 // outer, interior counts nw, no, rest) and, with wsl, their slots' weights
-// and, with fcg, the third entries of the lists' inverse matrices.
+// and, with fcg, the third entries of the lists' inverse matrices; with minv,
+// the inverse of the full stencil's normal matrix.
 void launch_flux_coef(const Geom &g, int base, int n, int nw, int no, double power, double *fco,
-                      double *wsl, double *fcg, cudaStream_t st);
+                      double *wsl, double *fcg, double *minv, cudaStream_t st);
 // Residual norm and residue of one iteration per instance (hist row i, entry
 // it - it_first), retirement, and the schedule of the next iteration.
 void launch_residual(const InstInfo *inst, int n_inst, const double *res_part, Ctl *ctl,

@@ -87,8 +87,7 @@ __global__ void __launch_bounds__(GRAD_BLOCK)
 kb_inner32(Geom g, Geom32 f, Sched s, const float *__restrict__ dq0,
            const float *__restrict__ dq_in, float *__restrict__ dq_out) {
     __shared__ SchedSmem ss;
-    load_sched(s, ss);
-    const int total = ss.pre[ss.nact] * TILE;
+    const int total = sched_begin(s, ss) * TILE;
     for (int vp = blockIdx.x * blockDim.x + threadIdx.x; vp < total;
          vp += gridDim.x * blockDim.x) {
         const int i = sched_point(s, ss, vp);
@@ -199,8 +198,7 @@ kb_grad32_h(Geom g, Consts c, Geom32 f, Sched s, const float4 *__restrict__ q,
             double *__restrict__ delta, int with_delta) {
     extern __shared__ double2 hsm[];
     __shared__ SchedSmem ss;
-    load_sched(s, ss);
-    const int ntiles = ss.pre[ss.nact];
+    const int ntiles = sched_begin(s, ss);
     const int wpb = blockDim.x / 32, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int half = lane / TILE, stride = gridDim.x * wpb;
     using H = HaloRows32;

@@ -135,9 +135,9 @@ __device__ __forceinline__ void grad_sums(const Consts &c, const Geom &g, int i,
     const double2 pi_ = R.xy(me);
     double qi[4];
     R.qrow(me, qi);
+    const R4 M = ld4w(reinterpret_cast<const R4 *>(g.minv) + i);
 #pragma unroll
     for (int m = 0; m < 4; ++m) qmax[m] = qmin[m] = qi[m];
-    double sdx2 = 0.0, sdy2 = 0.0, sdxy = 0.0;
     double sdxq[4] = {0.0, 0.0, 0.0, 0.0}, sdyq[4] = {0.0, 0.0, 0.0, 0.0};
     min_delt = 1.0;
     for (int r = 0; r < nb; ++r) {
@@ -145,34 +145,26 @@ __device__ __forceinline__ void grad_sums(const Consts &c, const Geom &g, int i,
         double qk[4];
         R.qrow(k, qk);
         const double2 pk = R.xy(k);
-#pragma unroll
-        for (int mm = 0; mm < 4; ++mm) {
-            if (qk[mm] > qmax[mm]) qmax[mm] = qk[mm];
-            if (qk[mm] < qmin[mm]) qmin[mm] = qk[mm];
-        }
-        double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
-        double dist = sqrt(delx * delx + dely * dely);
+        const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
         const double w = g.wsl ? __ldg(g.wsl + (size_t)r * g.n + i) : 1.0;
-        sdx2 = sdx2 + delx * delx * w;
-        sdy2 = sdy2 + dely * dely * w;
-        sdxy = sdxy + delx * dely * w;
+        const double wx = w * delx, wy = w * dely;
 #pragma unroll
-        for (int mm = 0; mm < 4; ++mm) {
-            sdxq[mm] = sdxq[mm] + w * delx * (qk[mm] - qi[mm]);
-            sdyq[mm] = sdyq[mm] + w * dely * (qk[mm] - qi[mm]);
+        for (int m = 0; m < 4; ++m) {
+            if (qk[m] > qmax[m]) qmax[m] = qk[m];
+            if (qk[m] < qmin[m]) qmin[m] = qk[m];
+            sdxq[m] = sdxq[m] + wx * (qk[m] - qi[m]);
+            sdyq[m] = sdyq[m] + wy * (qk[m] - qi[m]);
         }
         if (with_delta) {
-            double delta_t = dist / R.spdv(k);
+            double delta_t = sqrt(delx * delx + dely * dely) / R.spdv(k);
             delta_t = c.cfl * delta_t;
             if (min_delt > delta_t) min_delt = delta_t;
         }
     }
-    double det = sdx2 * sdy2 - sdxy * sdxy;
-    double one_by_det = 1.0 / det;
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
-        dx[m] = (sdxq[m] * sdy2 - sdyq[m] * sdxy) * one_by_det;
-        dy[m] = (sdyq[m] * sdx2 - sdxq[m] * sdxy) * one_by_det;
+        dx[m] = M.a * sdxq[m] + M.b * sdyq[m];
+        dy[m] = M.b * sdxq[m] + M.c * sdyq[m];
     }
 }
 
@@ -192,18 +184,15 @@ __device__ __forceinline__ void inner_sums(const Geom &g, int i, const Rows &R, 
                                            double dx[4], double dy[4]) {
     const int me = R.self();
     const double2 pi_ = R.xy(me);
-    double sdx2 = 0.0, sdy2 = 0.0, sdxy = 0.0;
+    const R4 M = ld4w(reinterpret_cast<const R4 *>(g.minv) + i);
     double sA[4] = {0.0, 0.0, 0.0, 0.0}, sB[4] = {0.0, 0.0, 0.0, 0.0};
     for (int r = 0; r < nb; ++r) {
         const int k = R.nbr(r);
         double dxk[4], dyk[4];
         R.dqrow(k, dxk, dyk);
         const double2 pk = R.xy(k);
-        double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
+        const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
         const double w = g.wsl ? __ldg(g.wsl + (size_t)r * g.n + i) : 1.0;
-        sdx2 = sdx2 + delx * delx * w;
-        sdy2 = sdy2 + dely * dely * w;
-        sdxy = sdxy + delx * dely * w;
         const double wx = w * delx, wy = w * dely;
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
@@ -214,12 +203,10 @@ __device__ __forceinline__ void inner_sums(const Geom &g, int i, const Rows &R, 
     }
     double dxi[4], dyi[4];
     R.dqrow(me, dxi, dyi);
-    double det = sdx2 * sdy2 - sdxy * sdxy;
-    double one_by_det = 1.0 / det;
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
-        const double Lx = one_by_det * (sA[m] * sdy2 - sB[m] * sdxy);
-        const double Ly = one_by_det * (sB[m] * sdx2 - sA[m] * sdxy);
+        const double Lx = M.a * sA[m] + M.b * sB[m];
+        const double Ly = M.b * sA[m] + M.c * sB[m];
         dx[m] = (dq0x[m] + 0.5 * dxi[m]) - 0.5 * Lx;
         dy[m] = (dq0y[m] + 0.5 * dyi[m]) - 0.5 * Ly;
     }
@@ -268,8 +255,7 @@ kb_inner_h(Geom g, Sched s, const double *__restrict__ dq0,
            const double *__restrict__ dq_in, double *__restrict__ dq_out) {
     extern __shared__ double2 hsm[];
     __shared__ SchedSmem ss;
-    load_sched(s, ss);
-    const int ntiles = ss.pre[ss.nact];
+    const int ntiles = sched_begin(s, ss);
     const int wpb = blockDim.x / 32, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int half = lane / TILE, stride = gridDim.x * wpb;
     double2 *sm0 = hsm + (size_t)(2 * warp) * HA_I * g.hc, *sm1 = sm0 + HA_I * g.hc;
@@ -300,8 +286,7 @@ kb_grad_h(Geom g, Consts c, Sched s, const R4 *__restrict__ q, const double *__r
           int with_delta) {
     extern __shared__ double2 hsm[];
     __shared__ SchedSmem ss;
-    load_sched(s, ss);
-    const int ntiles = ss.pre[ss.nact];
+    const int ntiles = sched_begin(s, ss);
     const int wpb = blockDim.x / 32, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int half = lane / TILE, stride = gridDim.x * wpb;
     double2 *sm0 = hsm + (size_t)(2 * warp) * HA_D * g.hc, *sm1 = sm0 + HA_D * g.hc;
@@ -347,17 +332,17 @@ kb_grad_h(Geom g, Consts c, Sched s, const R4 *__restrict__ q, const double *__r
 // Per point and split list L: a, b of the list's solve (fco[8 i + 2 L]).
 // *_fluxes.F90 dG*: the sums in slot order; a list the point's kind does not
 // have (wall ypos, outer yneg) gets zeros.  fcg: the third entry of the list's
-// inverse normal matrix (the reverse pass).
+// inverse normal matrix (the reverse pass); minv: the full stencil's.
 __global__ void k_flux_coef(Geom g, int base, int n, int nw, int no, double power,
                             double *__restrict__ fco, double *__restrict__ wsl,
-                            double *__restrict__ fcg) {
+                            double *__restrict__ fcg, double *__restrict__ minv) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const int i = base + j;
     const int kind = j < nw ? KIND_WALL : (j < nw + no ? KIND_OUTER : KIND_INTERIOR);
     const double2 p = g.xy[i], nn = g.nrm[i];
     const unsigned long long bits[2] = {g.mx[i], g.my[i]};
-    double sxx[4] = {}, syy[4] = {}, sxy[4] = {};
+    double sxx[4] = {}, syy[4] = {}, sxy[4] = {}, mxx = 0.0, myy = 0.0, mxy = 0.0;
     for (int r = 0; r < g.nbhs[i]; ++r) {
         const double2 pk = g.xy[g.conn[(size_t)r * g.n + i]];
         const double delx = pk.x - p.x, dely = pk.y - p.y;
@@ -367,6 +352,9 @@ __global__ void k_flux_coef(Geom g, int base, int n, int nw, int no, double powe
             w = pow(sqrt(delx * delx + dely * dely), power);
             wsl[(size_t)r * g.n + i] = w;
         }
+        mxx = mxx + delx * delx * w;
+        myy = myy + dely * dely * w;
+        mxy = mxy + delx * dely * w;
         const double dw = dels * w, nw_ = deln * w;
 #pragma unroll
         for (int L = 0; L < 4; ++L) {
@@ -375,6 +363,10 @@ __global__ void k_flux_coef(Geom g, int base, int n, int nw, int no, double powe
             syy[L] = syy[L] + deln * nw_;
             sxy[L] = sxy[L] + dels * nw_;
         }
+    }
+    if (minv) {
+        const double ob = 1.0 / (mxx * myy - mxy * mxy);
+        st4(reinterpret_cast<R4 *>(minv) + i, myy * ob, -mxy * ob, mxx * ob, 0.0);
     }
 #pragma unroll
     for (int L = 0; L < 4; ++L) {
@@ -884,9 +876,9 @@ int flux_grid_blocks(int n, bool fp32) {
 }
 
 void launch_flux_coef(const Geom &g, int base, int n, int nw, int no, double power, double *fco,
-                      double *wsl, double *fcg, cudaStream_t st) {
+                      double *wsl, double *fcg, double *minv, cudaStream_t st) {
     k_flux_coef<<<nblk(n, GRAD_BLOCK), GRAD_BLOCK, 0, st>>>(g, base, n, nw, no, power, fco, wsl,
-                                                            fcg);
+                                                            fcg, minv);
 }
 
 // staging memory of a block of the halo kernels: two tiles a warp
