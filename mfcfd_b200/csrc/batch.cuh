@@ -29,9 +29,13 @@ __device__ __forceinline__ void load_sched(const Sched &s, SchedSmem &ss) {
 }
 
 // Whole block: the scheduled tiles; a schedule of several instances is copied
-// into shared memory.
-__device__ __forceinline__ int sched_begin(const Sched &s, SchedSmem &ss) {
-    if (s.single) return __ldg(s.nact) ? s.one.ntiles : 0;
+// into shared memory.  live: 0 once every instance has retired (no tiles then;
+// of a one-instance schedule the tiles are returned all the same, so that a
+// pass can start its first loads before the flag has come: it checks live
+// before it writes).
+__device__ __forceinline__ int sched_begin(const Sched &s, SchedSmem &ss, int &live) {
+    live = __ldg(s.nact);
+    if (s.single) return s.one.ntiles;
     load_sched(s, ss);
     return ss.pre[ss.nact];
 }

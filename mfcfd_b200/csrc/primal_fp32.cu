@@ -87,11 +87,12 @@ __global__ void __launch_bounds__(GRAD_BLOCK)
 kb_inner32(Geom g, Geom32 f, Sched s, const float *__restrict__ dq0,
            const float *__restrict__ dq_in, float *__restrict__ dq_out) {
     __shared__ SchedSmem ss;
-    const int total = sched_begin(s, ss) * TILE;
+    int live;
+    const int total = sched_begin(s, ss, live) * TILE;
     for (int vp = blockIdx.x * blockDim.x + threadIdx.x; vp < total;
          vp += gridDim.x * blockDim.x) {
         const int i = sched_point(s, ss, vp);
-        if (i >= 0) inner32_point(g, f, dq0, dq_in, dq_out, i);
+        if (i >= 0 && live) inner32_point(g, f, dq0, dq_in, dq_out, i);
     }
 }
 
@@ -198,7 +199,8 @@ kb_grad32_h(Geom g, Consts c, Geom32 f, Sched s, const float4 *__restrict__ q,
             double *__restrict__ delta, int with_delta) {
     extern __shared__ double2 hsm[];
     __shared__ SchedSmem ss;
-    const int ntiles = sched_begin(s, ss);
+    int live;
+    const int ntiles = sched_begin(s, ss, live);
     const int wpb = blockDim.x / 32, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int half = lane / TILE, stride = gridDim.x * wpb;
     using H = HaloRows32;
@@ -206,6 +208,7 @@ kb_grad32_h(Geom g, Consts c, Geom32 f, Sched s, const float4 *__restrict__ q,
     HaloChunk cur;
     for (int ch = blockIdx.x * wpb + warp; 2 * ch < ntiles; ch += stride) {
         halo_chunk(g, s, ss, ntiles, ch, lane, cur);
+        if (!live) return;
         stage_array<1>(q, 16, cur.x, lane, sm0, sm1, g.hc, H::OQ);
         stage_array<1>(g.xy, 16, cur.x, lane, sm0, sm1, g.hc, H::OXY);
         if (with_delta) stage_array8(spd, cur.x, lane, sm0, sm1, g.hc, H::OSPD);

@@ -255,13 +255,15 @@ kb_inner_h(Geom g, Sched s, const double *__restrict__ dq0,
            const double *__restrict__ dq_in, double *__restrict__ dq_out) {
     extern __shared__ double2 hsm[];
     __shared__ SchedSmem ss;
-    const int ntiles = sched_begin(s, ss);
+    int live;
+    const int ntiles = sched_begin(s, ss, live);
     const int wpb = blockDim.x / 32, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int half = lane / TILE, stride = gridDim.x * wpb;
     double2 *sm0 = hsm + (size_t)(2 * warp) * HA_I * g.hc, *sm1 = sm0 + HA_I * g.hc;
     HaloChunk cur;
     for (int ch = blockIdx.x * wpb + warp; 2 * ch < ntiles; ch += stride) {
         halo_chunk(g, s, ss, ntiles, ch, lane, cur);
+        if (!live) return;
         stage_halo<HA_I>(g, nullptr, dq_in, nullptr, cur.x, lane, sm0, sm1);
         const HaloRows<HA_I> hr(g, half ? sm1 : sm0, cur.hn > 0 ? cur.i : -1);
         double ax[4], ay[4];
@@ -286,13 +288,15 @@ kb_grad_h(Geom g, Consts c, Sched s, const R4 *__restrict__ q, const double *__r
           int with_delta) {
     extern __shared__ double2 hsm[];
     __shared__ SchedSmem ss;
-    const int ntiles = sched_begin(s, ss);
+    int live;
+    const int ntiles = sched_begin(s, ss, live);
     const int wpb = blockDim.x / 32, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int half = lane / TILE, stride = gridDim.x * wpb;
     double2 *sm0 = hsm + (size_t)(2 * warp) * HA_D * g.hc, *sm1 = sm0 + HA_D * g.hc;
     HaloChunk cur;
     for (int ch = blockIdx.x * wpb + warp; 2 * ch < ntiles; ch += stride) {
         halo_chunk(g, s, ss, ntiles, ch, lane, cur);
+        if (!live) return;
         stage_halo<HA_D>(g, q, nullptr, with_delta ? spd : nullptr, cur.x, lane, sm0, sm1);
         const HaloRows<HA_D> hr(g, half ? sm1 : sm0, cur.hn > 0 ? cur.i : -1);
         halo_wait();
@@ -644,16 +648,18 @@ kb_flux(Geom g, Consts c, Sched s, StageBufs b, int rk, int last, int ct, int co
 
 // Sum of nparts tile partials in a fixed order (deterministic, independent
 // of the launch shape of the passes that wrote them): thread t of a block of
-// 1024 keeps eight accumulators over partials t + 1024 j (j mod 8 picks the
-// accumulator, so the loads of one thread are independent), adds them
-// pairwise, and a tree over the block adds the threads.  The result is in
-// s[0] for every thread.
-__device__ __forceinline__ void sum_parts_block(const double *__restrict__ part, int nparts,
-                                                double *s) {
-    constexpr int U = 8;
-    const int T = blockDim.x;
-    double acc[U] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+// RES_BLOCK keeps sixteen accumulators over partials t + RES_BLOCK j (j mod 16
+// picks the accumulator, so the loads of one thread are independent), adds them
+// pairwise, and trees over the warps and over their sums add the threads.  The
+// result is returned to warp 0; s: one double a warp.  One block an instance:
+// bound by the latency of its loads.
+constexpr int RES_BLOCK = 512;
+__device__ __forceinline__ double sum_parts_block(const double *__restrict__ part, int nparts,
+                                                  double *s) {
+    constexpr int U = 16, T = RES_BLOCK;
+    double acc[U] = {};
     int t = threadIdx.x;
+#pragma unroll 2
     for (; t + (U - 1) * T < nparts; t += U * T) {
 #pragma unroll
         for (int j = 0; j < U; ++j) acc[j] = acc[j] + __ldg(part + t + j * T);
@@ -661,21 +667,28 @@ __device__ __forceinline__ void sum_parts_block(const double *__restrict__ part,
 #pragma unroll
     for (int j = 0; j < U; ++j)
         if (t + j * T < nparts) acc[j] = acc[j] + __ldg(part + t + j * T);
-    s[threadIdx.x] = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
+#pragma unroll
+    for (int w = U / 2; w > 0; w >>= 1)
+#pragma unroll
+        for (int j = 0; j < w; ++j) acc[j] = acc[j] + acc[j + w];
+    double v = acc[0];
+    for (int w = 16; w > 0; w >>= 1) v = v + __shfl_xor_sync(0xffffffffu, v, w);
+    if (threadIdx.x % 32 == 0) s[threadIdx.x / 32] = v;
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) s[threadIdx.x] = s[threadIdx.x] + s[threadIdx.x + w];
-        __syncthreads();
+    if (threadIdx.x < 32) {
+        v = threadIdx.x < T / 32 ? s[threadIdx.x] : 0.0;
+        for (int w = 16; w > 0; w >>= 1) v = v + __shfl_xor_sync(0xffffffffu, v, w);
     }
+    return v;
 }
 
 // fpi_solver.F90:57-70: res_new = sqrt(sum res_sqr)/plen and the residue.
-// Whole block of 1024 threads; the residue is returned on thread 0.
+// Whole block of RES_BLOCK threads; the residue is returned on thread 0.
 __device__ __forceinline__ double residual_block(const double *__restrict__ part, int nparts,
                                                  Ctl *ctl, double *hist, double *s) {
-    sum_parts_block(part, nparts, s);
+    const double sum = sum_parts_block(part, nparts, s);
     if (threadIdx.x == 0) {
-        double res_new = sqrt(s[0]) / ctl->plen;
+        double res_new = sqrt(sum) / ctl->plen;
         int it = ctl->it;
         double residue;
         if (it <= 2 && ctl->restart == 0) {
@@ -694,13 +707,13 @@ __device__ __forceinline__ double residual_block(const double *__restrict__ part
 }
 
 // Sum of nparts tile partials in the fixed order of residual_block (one
-// block of 1024 threads): a partitioned grid's share of the residual, which
+// block of RES_BLOCK threads): a partitioned grid's share of the residual, which
 // the host adds over the ranks before the norm.
-__global__ void __launch_bounds__(1024)
+__global__ void __launch_bounds__(RES_BLOCK)
 k_sum_parts(const double *__restrict__ part, int nparts, double *out) {
-    __shared__ double s[1024];
-    sum_parts_block(part, nparts, s);
-    if (threadIdx.x == 0) *out = s[0];
+    __shared__ double s[RES_BLOCK / 32];
+    const double sum = sum_parts_block(part, nparts, s);
+    if (threadIdx.x == 0) *out = sum;
 }
 
 // Per-instance residual (block b = instance b): the instance's tile partials
@@ -710,18 +723,19 @@ k_sum_parts(const double *__restrict__ part, int nparts, double *out) {
 // schedule from Ctl::active for the next iteration's passes: a stable
 // compaction of the running instances and the prefix sums of their tile
 // counts (Hillis-Steele scans over MAX_BATCH slots).
-__global__ void __launch_bounds__(1024)
+__global__ void __launch_bounds__(RES_BLOCK)
 kb_residual(const InstInfo *__restrict__ inst, int n_inst, const double *__restrict__ part,
             Ctl *ctl, double *hist, int hist_ld, const BatchRun *__restrict__ run,
             int *sched) {
-    __shared__ double s[1024];
-    __shared__ int s_active, s_last;
+    __shared__ double s[RES_BLOCK / 32];
+    __shared__ int s_last;
     __shared__ int cnt[MAX_BATCH], til[MAX_BATCH];
     Ctl *c = ctl + blockIdx.x;
-    if (threadIdx.x == 0) s_active = c->active;
-    __syncthreads();
-    if (s_active) {
-        const InstInfo in = inst[blockIdx.x];
+    const InstInfo in = inst[blockIdx.x];
+    // (thread 0 changes it behind the barrier of the sum, which the whole block
+    // meets or, if it is 0, skips)
+    const int active = c->active;
+    if (active) {
         const double residue =
             residual_block(part + in.tile0, in.ntiles, c, hist + (size_t)blockIdx.x * hist_ld, s);
         if (threadIdx.x == 0) {
@@ -736,6 +750,17 @@ kb_residual(const InstInfo *__restrict__ inst, int n_inst, const double *__restr
                 c->state = BATCH_MAX_ITERS;
             }
         }
+    }
+    int *pre = sched + SCHED_PRE, *act = sched + SCHED_ACT;
+    if (gridDim.x == 1) {  // one instance: its own schedule
+        if (threadIdx.x == 0) {
+            const int on = c->active ? 1 : 0;
+            sched[SCHED_NACT] = on;
+            pre[0] = 0;
+            pre[on] = on ? in.ntiles : 0;
+            act[0] = 0;
+        }
+        return;
     }
     int *counter = sched + SCHED_COUNTER;
     if (threadIdx.x == 0) {
@@ -767,7 +792,6 @@ kb_residual(const InstInfo *__restrict__ inst, int n_inst, const double *__restr
         }
         __syncthreads();
     }
-    int *pre = sched + SCHED_PRE, *act = sched + SCHED_ACT;
     if (a) {
         act[cnt[t] - 1] = t;
         pre[cnt[t] - 1] = til[t] - nt;
@@ -981,7 +1005,7 @@ void launch_flux(const Geom &g, const Consts &c, const Sched &s, const StageBufs
 void launch_residual(const InstInfo *inst, int n_inst, const double *res_part, Ctl *ctl,
                      double *hist, int hist_ld, const BatchRun *run, int *sched,
                      cudaStream_t st) {
-    kb_residual<<<n_inst, 1024, 0, st>>>(inst, n_inst, res_part, ctl, hist, hist_ld, run, sched);
+    kb_residual<<<n_inst, RES_BLOCK, 0, st>>>(inst, n_inst, res_part, ctl, hist, hist_ld, run, sched);
 }
 
 void launch_init_state(const Geom &g, const R4 *prim, R4 *q, double *spd, cudaStream_t s) {
@@ -995,7 +1019,7 @@ void launch_init_rows(const Geom &g, const R4 *prim, R4 *q, double *spd, int i0,
 }
 
 void launch_sum_parts(const double *part, int nparts, double *out, cudaStream_t s) {
-    k_sum_parts<<<1, 1024, 0, s>>>(part, nparts, out);
+    k_sum_parts<<<1, RES_BLOCK, 0, s>>>(part, nparts, out);
 }
 
 void launch_forces(const ShapeTab &t, const R4 *prim, double mach, double cos_t, double sin_t,
