@@ -508,10 +508,9 @@ __device__ __forceinline__ void flux_group(const Geom &g, const StageBufs &b, co
             // follow from u and the point's normal)
             const double t[KS_TAPE] = {si.rho, si.pbr, si.B1, si.B2, si.e1, si.e2, ui[0], ui[1],
                                        sk.rho, sk.pbr, sk.B1, sk.B2, sk.e1, sk.e2, uk[0], uk[1]};
-            double2 *tp =
-                reinterpret_cast<double2 *>(b.kstape + ((size_t)i * g.kp + r) * KS_TAPE);
-#pragma unroll
-            for (int h = 0; h < KS_TAPE / 2; ++h) tp[h] = make_double2(t[2 * h], t[2 * h + 1]);
+            double *tp = b.kstape + ((size_t)i * g.kp + r) * KS_TAPE;
+            st8w(tp, t, t + 4);
+            st8w(tp + 8, t + 8, t + 12);
         }
         double dels = delx * ny - dely * nx, deln = delx * nx + dely * ny;
         if (g.wsl) {
