@@ -194,20 +194,28 @@ k_update_b(Geom g, Consts c, AdjConsts a, const R4 *__restrict__ prim_in,
 //
 // Everything a warp's round reads but the neighbours' coordinates is copied to
 // shared memory (cp.async) at its start, so the loads' latency is met once.
-// Bound by latency: 488 us at 256,000 points when the list sums and the
-// reconstructions' primitive states went through shared-memory records, 404
-// with the folded weights, 226 with the copies; 3 blocks (168 registers)
-// against 269 us at 4 (spills).
+// 488 us at 256,000 points when the list sums and the reconstructions'
+// primitive states went through shared-memory records, 404 with the folded
+// weights, 226 with the copies, 214 with the own-point sums through shared
+// memory instead of shuffles.  Bound by issue and by the one exposed load
+// latency at 12 warps an SM (3 blocks of 168 registers; 4 spill: 269 us).
 constexpr int FLUXB_MIN_BLOCKS = 3;
 // A warp's shared memory: the taped states of its 32 slots (128 bytes padded
 // to 144: a lane's pieces on distinct banks), its four points' rows, the
 // slots' partial offset adjoints, z of each list.
 struct FluxBSmem {
     double2 tape[32][KS_TAPE / 2 + 1];
+    double2 more[80];  // (with the tape: the slots' own-point records)
     double2 q[4][2], dq[4][5], qm[4][5], co[4][4], fcg[4][2];
     double part[4][20][4];
     double z[4][8];
+    // the own-point record of a slot: 20 doubles at a stride of 22, and 8 more
+    // between points (a warp's stores and loads on distinct banks)
+    __device__ __forceinline__ double2 *rec(int slot) {
+        return &tape[0][0] + 11 * slot + 4 * (slot / LPP);
+    }
 };
+static_assert(11 * 32 + 4 * 3 <= 32 * 9 + 80, "");
 __global__ void __launch_bounds__(BLK, FLUXB_MIN_BLOCKS)
 k_flux_b(Geom g, const R4 *__restrict__ q_in, const double *__restrict__ dq,
          const double *__restrict__ qm, const double *__restrict__ delta,
@@ -223,28 +231,31 @@ k_flux_b(Geom g, const R4 *__restrict__ q_in, const double *__restrict__ dq,
     const int i = i0 + pg;
     const bool valid = i < g.n;
     // copies
+    const int part = wl % 8, sub = wl / 8;
     if (kst) {
+        // piece `part` of slots 4 h + sub of points i0 + t
+        const size_t row = (size_t)g.kp * KS_TAPE;
+        const double *src = kst + i0 * row + sub * KS_TAPE + 2 * part;
+        double2 *dst = &m.tape[sub][part];
+        constexpr int TS = sizeof(m.tape[0]) / sizeof(double2);
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            const int pc = 32 * t + wl, slot = pc / 8, part = pc % 8;
-            const int p = i0 + slot / LPP, r = slot % LPP;
-            if (p < g.n && r < g.kp)
-                halo_cp16(&m.tape[slot][part], kst + ((size_t)p * g.kp + r) * KS_TAPE + 2 * part);
+        for (int t = 0; t < 4; ++t, src += row) {
+            if (i0 + t >= g.n) break;
+            if (sub < g.kp) halo_cp16(dst + (8 * t) * TS, src);
+            if (4 + sub < g.kp) halo_cp16(dst + (8 * t + 4) * TS, src + 4 * KS_TAPE);
         }
     }
-    {
-        const int p = i0 + wl / 8, part = wl % 8;  // 8 pieces a point
-        if (p < g.n) {
-            const int h = part & 3;
-            if (part < 4) {
-                halo_cp16(&m.dq[wl / 8][h], dq + 8 * (size_t)p + 2 * h);
-                halo_cp16(&m.co[wl / 8][h], g.fco + 8 * (size_t)p + 2 * h);
-            } else {
-                halo_cp16(&m.qm[wl / 8][h], qm + 8 * (size_t)p + 2 * h);
-                if (h < 2)
-                    halo_cp16(&m.q[wl / 8][h], reinterpret_cast<const double *>(q_in + p) + 2 * h);
-                else halo_cp16(&m.fcg[wl / 8][h - 2], g.fcg + 4 * (size_t)p + 2 * (h - 2));
-            }
+    if (i0 + sub < g.n) {
+        const size_t o8 = 8 * (size_t)(i0 + sub);
+        const int h = part & 3;
+        if (part < 4) {
+            halo_cp16(&m.dq[sub][h], dq + o8 + 2 * h);
+            halo_cp16(&m.co[sub][h], g.fco + o8 + 2 * h);
+        } else {
+            halo_cp16(&m.qm[sub][h], qm + o8 + 2 * h);
+            const double *q = reinterpret_cast<const double *>(q_in);
+            if (h < 2) halo_cp16(&m.q[sub][h], q + o8 / 2 + 2 * h);
+            else halo_cp16(&m.fcg[sub][h - 2], g.fcg + o8 / 2 + 2 * (h - 2));
         }
     }
     int nb = 0, kind = KIND_INTERIOR, k0 = 0;
@@ -351,8 +362,8 @@ k_flux_b(Geom g, const R4 *__restrict__ q_in, const double *__restrict__ dq,
                 auto along_t = [&](int l, double c) {
                     const double sg = l ? -1.0 : 1.0;
                     if (kind == KIND_INTERIOR)
-                        return sgn * flux_split_b(s, s.ut, s.un, s.B1, s.e1, sg, w6, F, c, b.ut, b.un,
-                                                  b.B1, b.e1, b);
+                        return sgn * flux_split_b(s, s.ut, s.un, s.B1, s.e1, sg, w6, F, c, b.ut,
+                                                  b.un, b.B1, b.e1, b);
                     const double s2 = kind == KIND_WALL ? -1.0 : 1.0;
                     double G[4], cF[4], d = 0.0;
                     flux_quad(s, sg, s2, G);
@@ -405,7 +416,7 @@ k_flux_b(Geom g, const R4 *__restrict__ q_in, const double *__restrict__ dq,
                 delnb = fma(cby1, co[3].x, delnb);
             }
         }
-        double own[24] = {};
+        double own[20] = {};
         {
             double qi[4], dxi[4], dyi[4], qmaxi[4], qmini[4];
 #pragma unroll
@@ -426,19 +437,21 @@ k_flux_b(Geom g, const R4 *__restrict__ q_in, const double *__restrict__ dq,
             pt[0] = make_double2(delsb, delnb);
             pt[1] = make_double2(delxb, delyb);
         }
-        // the round's own-point sums: lane t keeps fields 3 t .. 3 t + 2
-        const bool h4 = lane & 4, h2 = lane & 2, h1 = lane & 1;
-        double a[12], b[6];
+        // the round's own-point sums, in lane order: lane t adds fields t, t + 8
+        // and t + 16 of its point's eight lanes
+        __syncwarp();  // (the rows lie over the tape, which has been read)
+        double2 *mine = m.rec(wl);
 #pragma unroll
-        for (int f = 0; f < 12; ++f)
-            a[f] = (h4 ? own[12 + f] : own[f]) +
-                   __shfl_xor_sync(full, h4 ? own[f] : own[12 + f], 4);
+        for (int f = 0; f < 10; ++f) mine[f] = make_double2(own[2 * f], own[2 * f + 1]);
+        __syncwarp();
 #pragma unroll
-        for (int f = 0; f < 6; ++f)
-            b[f] = (h2 ? a[6 + f] : a[f]) + __shfl_xor_sync(full, h2 ? a[f] : a[6 + f], 2);
-#pragma unroll
-        for (int f = 0; f < 3; ++f)
-            acc[f] += (h1 ? b[3 + f] : b[f]) + __shfl_xor_sync(full, h1 ? b[f] : b[3 + f], 1);
+        for (int t = 0; t < LPP; ++t) {
+            const double *row = reinterpret_cast<const double *>(m.rec(LPP * pg + t)) + lane;
+            acc[0] += row[0];
+            acc[1] += row[8];
+            if (lane < 4) acc[2] += row[16];
+        }
+        __syncwarp();
     }
     // pb summed over the point's lanes: lane 2 L + h holds component h of list
     // L, then z's component
@@ -495,13 +508,15 @@ k_flux_b(Geom g, const R4 *__restrict__ q_in, const double *__restrict__ dq,
     if (!valid) return;
     if (!(lane & 1)) *geo = geo_old + sum;
     // the stage's first contributions to q, dq and qm: stored, not added
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const int f = 3 * lane + c;
-        if (f < 4) qb[4 * (size_t)i + f] = acc[c];
-        else if (f < 12) dqb[8 * (size_t)i + (f - 4)] = acc[c];
-        else if (f < 20) qmb[8 * (size_t)i + (f - 12)] = acc[c];
+    // (fields: q 4, dq 8, qm 8)
+    if (lane < 4) {
+        qb[4 * (size_t)i + lane] = acc[0];
+        qmb[8 * (size_t)i + 4 + lane] = acc[2];
+    } else {
+        dqb[8 * (size_t)i + lane - 4] = acc[0];
     }
+    if (lane < 4) dqb[8 * (size_t)i + 4 + lane] = acc[1];
+    else qmb[8 * (size_t)i + lane - 4] = acc[1];
 }
 
 // The neighbour side of cal_flux_residual_b, one thread per neighbour k:
