@@ -137,9 +137,9 @@ struct HaloLoc {
         const unsigned long long last = g.hkp > 16 ? w2 : (g.hkp > 8 ? w1 : w0);
         own = (int)(last >> 56);
     }
-    __device__ __forceinline__ int slot(int r) const {
-        const unsigned long long w = r < 8 ? w0 : (r < 16 ? w1 : w2);
-        return (int)((w >> (8 * (r & 7))) & 0xffull);
+    // the rows of slots r0 .. r0 + 7 (r0 0, 8 or 16), a byte each
+    __device__ __forceinline__ unsigned long long word(int r0) const {
+        return r0 == 0 ? w0 : (r0 == 8 ? w1 : w2);
     }
 };
 

@@ -107,9 +107,9 @@ kb_inner32(Geom g, Geom32 f, Sched s, const float *__restrict__ dq0,
 // staging only (x, y) and the row indices, 0.064 ms.)
 constexpr int HALO32_BLOCK = 128;
 constexpr int HA32 = 3;  // staged arrays
-#ifndef HALO32_MIN_BLOCKS
-#define HALO32_MIN_BLOCKS 8
-#endif
+// 64 registers and 8 blocks an SM: 52.1 us at 1.024M points (54.1 at 7, 56.2 at
+// 6, 59.8 at 9, which spills); 55.6 with the slot loop not unrolled
+constexpr int HALO32_MIN_BLOCKS = 8;
 
 struct GlobalRows32 {
     const Geom &g;
@@ -119,8 +119,13 @@ struct GlobalRows32 {
     int i;
     __device__ __forceinline__ void begin() {}
     __device__ __forceinline__ int self() const { return i; }
-    __device__ __forceinline__ int nbr(int r) const { return g.conn[r * g.n + i]; }
-    __device__ __forceinline__ float2 off(int r, int) const { return __ldg(f.dxy + r * g.n + i); }
+    __device__ __forceinline__ unsigned long long word(int) const { return 0ull; }
+    __device__ __forceinline__ int nbr(int r, unsigned long long, int) const {
+        return g.conn[(size_t)r * g.n + i];
+    }
+    __device__ __forceinline__ float2 off(int r, int) const {
+        return __ldg(f.dxy + (size_t)r * g.n + i);
+    }
     __device__ __forceinline__ float4 qrow(int k) const { return __ldg(q + k); }
     __device__ __forceinline__ double spdv(int k) const { return spd[k]; }
 };
@@ -129,14 +134,18 @@ struct GlobalRows32 {
 struct HaloRows32 {
     static constexpr int OQ = 0, OXY = 1, OSPD = 2;
     const double2 *sm;
-    int hc;
+    int hc;  // the grid's staging stride
     HaloLoc loc;
     double2 pi;
     __device__ __forceinline__ HaloRows32(const Geom &g, const double2 *sm_, int i)
         : sm(sm_), hc(g.hc), loc(g, i), pi(make_double2(0.0, 0.0)) {}
     __device__ __forceinline__ void begin() { pi = sm[OXY * hc + loc.own]; }
     __device__ __forceinline__ int self() const { return loc.own; }
-    __device__ __forceinline__ int nbr(int r) const { return loc.slot(r); }
+    __device__ __forceinline__ unsigned long long word(int r0) const { return loc.word(r0); }
+    // slot r0 + j of word(r0)
+    __device__ __forceinline__ int nbr(int, unsigned long long w, int j) const {
+        return (int)((w >> (8 * j)) & 0xffull);
+    }
     __device__ __forceinline__ float2 off(int, int l) const {
         const double2 pk = sm[OXY * hc + l];
         return make_float2((float)(pk.x - pi.x), (float)(pk.y - pi.y));
@@ -160,29 +169,35 @@ __device__ __forceinline__ void grad32_sums(const Consts &c, const Geom32 &f, in
     for (int m = 0; m < 4; ++m) qmax[m] = qmin[m] = qi[m];
     float sx[4] = {0.f, 0.f, 0.f, 0.f}, sy[4] = {0.f, 0.f, 0.f, 0.f};
     min_delt = 1.0;
-    for (int r = 0; r < nb; ++r) {
-        const int k = R.nbr(r);
-        const float4 kv = R.qrow(k);
-        const float2 gs = R.off(r, k);
-        const float qk[4] = {kv.x, kv.y, kv.z, kv.w};
-        const float w = f.w ? __ldg(f.w + r * n + i) : 1.0f;
+    for (int r0 = 0; r0 < nb; r0 += 8) {
+        const unsigned long long word = R.word(r0);
 #pragma unroll
-        for (int mm = 0; mm < 4; ++mm) {
-            if (qk[mm] > qmax[mm]) qmax[mm] = qk[mm];
-            if (qk[mm] < qmin[mm]) qmin[mm] = qk[mm];
-        }
-        const float wdx = w * gs.x, wdy = w * gs.y;
+        for (int j = 0; j < 8; ++j) {
+            const int r = r0 + j;
+            if (r >= nb) break;
+            const int k = R.nbr(r, word, j);
+            const float4 kv = R.qrow(k);
+            const float2 gs = R.off(r, k);
+            const float qk[4] = {kv.x, kv.y, kv.z, kv.w};
+            const float w = f.w ? __ldg(f.w + (size_t)r * n + i) : 1.0f;
 #pragma unroll
-        for (int mm = 0; mm < 4; ++mm) {
-            const float dqm = qk[mm] - qi[mm];
-            sx[mm] = sx[mm] + wdx * dqm;
-            sy[mm] = sy[mm] + wdy * dqm;
-        }
-        if (with_delta) {
-            const double dist = (double)sqrtf(gs.x * gs.x + gs.y * gs.y);
-            double delta_t = dist / R.spdv(k);
-            delta_t = c.cfl * delta_t;
-            if (min_delt > delta_t) min_delt = delta_t;
+            for (int mm = 0; mm < 4; ++mm) {
+                if (qk[mm] > qmax[mm]) qmax[mm] = qk[mm];
+                if (qk[mm] < qmin[mm]) qmin[mm] = qk[mm];
+            }
+            const float wdx = w * gs.x, wdy = w * gs.y;
+#pragma unroll
+            for (int mm = 0; mm < 4; ++mm) {
+                const float dqm = qk[mm] - qi[mm];
+                sx[mm] = sx[mm] + wdx * dqm;
+                sy[mm] = sy[mm] + wdy * dqm;
+            }
+            if (with_delta) {
+                const double dist = (double)sqrtf(gs.x * gs.x + gs.y * gs.y);
+                double delta_t = dist / R.spdv(k);
+                delta_t = c.cfl * delta_t;
+                if (min_delt > delta_t) min_delt = delta_t;
+            }
         }
     }
     const float4 L = __ldg(f.lsq + i);
@@ -204,7 +219,7 @@ kb_grad32_h(Geom g, Consts c, Geom32 f, Sched s, const float4 *__restrict__ q,
     const int wpb = blockDim.x / 32, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int half = lane / TILE, stride = gridDim.x * wpb;
     using H = HaloRows32;
-    double2 *sm0 = hsm + (size_t)(2 * warp) * HA32 * g.hc, *sm1 = sm0 + HA32 * g.hc;
+    double2 *sm0 = hsm + (2 * warp) * HA32 * g.hc, *sm1 = sm0 + HA32 * g.hc;
     HaloChunk cur;
     for (int ch = blockIdx.x * wpb + warp; 2 * ch < ntiles; ch += stride) {
         halo_chunk(g, s, ss, ntiles, ch, lane, cur);

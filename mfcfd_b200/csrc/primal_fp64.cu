@@ -69,7 +69,10 @@ struct GlobalRows {
     const double *spd;  // D pass
     int i;
     __device__ __forceinline__ int self() const { return i; }
-    __device__ __forceinline__ int nbr(int r) const { return g.conn[r * g.n + i]; }
+    __device__ __forceinline__ unsigned long long word(int) const { return 0ull; }
+    __device__ __forceinline__ int nbr(int r, unsigned long long, int) const {
+        return g.conn[(size_t)r * g.n + i];
+    }
     __device__ __forceinline__ double2 xy(int k) const { return g.xy[k]; }
     __device__ __forceinline__ void qrow(int k, double v[4]) const {
         const R4 a = ld4w(q + k);
@@ -81,56 +84,70 @@ struct GlobalRows {
     __device__ __forceinline__ double spdv(int k) const { return spd[k]; }
 };
 
-// Shared-memory arrays of a staged tile halo, hc rows each (hc is the
-// staging stride, one more than a multiple of eight, so that the arrays of a
-// row start on different banks): D pass q[0..1], q[2..3], (x, y), (spd, -);
+// Shared-memory arrays of a staged tile halo, HaloStride rows each (one more
+// than a multiple of eight, so that the arrays of a row start on different
+// banks): D pass q[0..1], q[2..3], (x, y), (spd, -);
 // I pass (x, y), dq/dx[0..1], dq/dx[2..3], dq/dy[0..1], dq/dy[2..3].  One
 // 16-byte array per pair keeps a warp's reads of neighbouring rows on
 // distinct banks.
 constexpr int HA_I = 5, HA_D = 4;
+// Stride of the staged arrays.  Fixed in the D pass, so that a row's pieces are
+// immediate offsets from its first (with the slots' loop unrolled 0.088 ->
+// 0.076 ms at 1.024M points at 5 blocks an SM); the I pass, whose rows are
+// larger, takes the grid's own: what shared memory it leaves is L1, where the
+// tiles' common rows are found (0.082 ms, 0.090 with the fixed stride).
+template <int nA>
+struct HaloStride;
+template <>
+struct HaloStride<HA_D> {
+    static constexpr int hc = HALO_CAP + 1;
+    __host__ __device__ constexpr HaloStride(int) {}
+};
+template <>
+struct HaloStride<HA_I> {
+    int hc;
+    __host__ __device__ constexpr HaloStride(int h) : hc(h) {}
+};
 constexpr int HALO_BLOCK = 128;  // four warps, a half-warp per tile
-// resident blocks per SM the register budget allows, measured at C2: the D
-// pass 0.090 ms at 4 (128 registers), 0.102 at 5, 0.132 at 6; the I pass
-// 0.119 ms at 4, 0.087 at 5 (96 registers), 0.092 at 6
-#ifndef HALO_MIN_BLOCKS_D
-#define HALO_MIN_BLOCKS_D 4
-#endif
-#ifndef HALO_MIN_BLOCKS_I
-#define HALO_MIN_BLOCKS_I 5
-#endif
+// resident blocks per SM (96 registers), measured at 1.024M points: the D pass
+// 0.082 ms at 4, 0.076 at 5, 0.089 at 6; the I pass 0.089, 0.082, 0.097
+constexpr int HALO_MIN_BLOCKS_D = 5, HALO_MIN_BLOCKS_I = 5;
 
 template <int nA>
 struct HaloRows {
     static constexpr int OXY = nA == HA_I ? 0 : 2, ODQ = 1, OSPD = 3;
     const double2 *sm;
-    int hc;
+    HaloStride<nA> st;
     HaloLoc loc;
     // i < 0: no point (nothing is loaded)
     __device__ __forceinline__ HaloRows(const Geom &g, const double2 *sm_, int i)
-        : sm(sm_), hc(g.hc), loc(g, i) {}
+        : sm(sm_), st(g.hc), loc(g, i) {}
     __device__ __forceinline__ int self() const { return loc.own; }
-    __device__ __forceinline__ int nbr(int r) const { return loc.slot(r); }
-    __device__ __forceinline__ double2 xy(int l) const { return sm[OXY * hc + l]; }
+    __device__ __forceinline__ unsigned long long word(int r0) const { return loc.word(r0); }
+    // slot r0 + j of word(r0)
+    __device__ __forceinline__ int nbr(int, unsigned long long w, int j) const {
+        return (int)((w >> (8 * j)) & 0xffull);
+    }
+    __device__ __forceinline__ double2 xy(int l) const { return sm[OXY * st.hc + l]; }
     __device__ __forceinline__ void qrow(int l, double v[4]) const {
-        const double2 a = sm[l], b = sm[hc + l];
+        const double2 a = sm[l], b = sm[st.hc + l];
         v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
     }
     __device__ __forceinline__ void dqrow(int l, double x[4], double y[4]) const {
-        const double2 a = sm[ODQ * hc + l], b = sm[(ODQ + 1) * hc + l],
-                      e = sm[(ODQ + 2) * hc + l], f = sm[(ODQ + 3) * hc + l];
+        const double2 a = sm[ODQ * st.hc + l], b = sm[(ODQ + 1) * st.hc + l],
+                      e = sm[(ODQ + 2) * st.hc + l], f = sm[(ODQ + 3) * st.hc + l];
         x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
         y[0] = e.x; y[1] = e.y; y[2] = f.x; y[3] = f.y;
     }
-    __device__ __forceinline__ double spdv(int l) const { return sm[OSPD * hc + l].x; }
+    __device__ __forceinline__ double spdv(int l) const { return sm[OSPD * st.hc + l].x; }
 };
 
 // q_variables.F90:41-112 eval_q_derivatives and state_update.F90:190-236
 // func_delta over the rows of R, in slot order.
 template <class Rows>
 __device__ __forceinline__ void grad_sums(const Consts &c, const Geom &g, int i, const Rows &R,
-                                          int nb, int with_delta,
-                                          double dx[4], double dy[4], double qmax[4],
-                                          double qmin[4], double &min_delt) {
+                                          int nb, int with_delta, double dx[4], double dy[4],
+                                          double qmax[4], double qmin[4], double &min_delt) {
     const int me = R.self();
     const double2 pi_ = R.xy(me);
     double qi[4];
@@ -140,25 +157,31 @@ __device__ __forceinline__ void grad_sums(const Consts &c, const Geom &g, int i,
     for (int m = 0; m < 4; ++m) qmax[m] = qmin[m] = qi[m];
     double sdxq[4] = {0.0, 0.0, 0.0, 0.0}, sdyq[4] = {0.0, 0.0, 0.0, 0.0};
     min_delt = 1.0;
-    for (int r = 0; r < nb; ++r) {
-        const int k = R.nbr(r);
-        double qk[4];
-        R.qrow(k, qk);
-        const double2 pk = R.xy(k);
-        const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
-        const double w = g.wsl ? __ldg(g.wsl + (size_t)r * g.n + i) : 1.0;
-        const double wx = w * delx, wy = w * dely;
+    for (int r0 = 0; r0 < nb; r0 += 8) {
+        const unsigned long long word = R.word(r0);
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            if (qk[m] > qmax[m]) qmax[m] = qk[m];
-            if (qk[m] < qmin[m]) qmin[m] = qk[m];
-            sdxq[m] = sdxq[m] + wx * (qk[m] - qi[m]);
-            sdyq[m] = sdyq[m] + wy * (qk[m] - qi[m]);
-        }
-        if (with_delta) {
-            double delta_t = sqrt(delx * delx + dely * dely) / R.spdv(k);
-            delta_t = c.cfl * delta_t;
-            if (min_delt > delta_t) min_delt = delta_t;
+        for (int j = 0; j < 8; ++j) {
+            const int r = r0 + j;
+            if (r >= nb) break;
+            const int k = R.nbr(r, word, j);
+            double qk[4];
+            R.qrow(k, qk);
+            const double2 pk = R.xy(k);
+            const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
+            const double w = g.wsl ? __ldg(g.wsl + (size_t)r * g.n + i) : 1.0;
+            const double wx = w * delx, wy = w * dely;
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                if (qk[m] > qmax[m]) qmax[m] = qk[m];
+                if (qk[m] < qmin[m]) qmin[m] = qk[m];
+                sdxq[m] = sdxq[m] + wx * (qk[m] - qi[m]);
+                sdyq[m] = sdyq[m] + wy * (qk[m] - qi[m]);
+            }
+            if (with_delta) {
+                double delta_t = sqrt(delx * delx + dely * dely) / R.spdv(k);
+                delta_t = c.cfl * delta_t;
+                if (min_delt > delta_t) min_delt = delta_t;
+            }
         }
     }
 #pragma unroll
@@ -186,19 +209,25 @@ __device__ __forceinline__ void inner_sums(const Geom &g, int i, const Rows &R, 
     const double2 pi_ = R.xy(me);
     const R4 M = ld4w(reinterpret_cast<const R4 *>(g.minv) + i);
     double sA[4] = {0.0, 0.0, 0.0, 0.0}, sB[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int r = 0; r < nb; ++r) {
-        const int k = R.nbr(r);
-        double dxk[4], dyk[4];
-        R.dqrow(k, dxk, dyk);
-        const double2 pk = R.xy(k);
-        const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
-        const double w = g.wsl ? __ldg(g.wsl + (size_t)r * g.n + i) : 1.0;
-        const double wx = w * delx, wy = w * dely;
+    for (int r0 = 0; r0 < nb; r0 += 8) {
+        const unsigned long long word = R.word(r0);
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            const double t = delx * dxk[m] + dely * dyk[m];
-            sA[m] = sA[m] + wx * t;
-            sB[m] = sB[m] + wy * t;
+        for (int j = 0; j < 8; ++j) {
+            const int r = r0 + j;
+            if (r >= nb) break;
+            const int k = R.nbr(r, word, j);
+            double dxk[4], dyk[4];
+            R.dqrow(k, dxk, dyk);
+            const double2 pk = R.xy(k);
+            const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
+            const double w = g.wsl ? __ldg(g.wsl + (size_t)r * g.n + i) : 1.0;
+            const double wx = w * delx, wy = w * dely;
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                const double t = delx * dxk[m] + dely * dyk[m];
+                sA[m] = sA[m] + wx * t;
+                sB[m] = sB[m] + wy * t;
+            }
         }
     }
     double dxi[4], dyi[4];
@@ -239,10 +268,11 @@ __device__ __forceinline__ void stage_halo(const Geom &g, const R4 *q, const dou
                                            const double *spd, const HaloIdx &x, int lane,
                                            double2 *sm0, double2 *sm1) {
     using H = HaloRows<nA>;
-    if (nA == HA_D) stage_array<2>(q, 32, x, lane, sm0, sm1, g.hc, 0);
-    stage_array<1>(g.xy, 16, x, lane, sm0, sm1, g.hc, H::OXY);
-    if (nA == HA_I) stage_array<4>(dq, 64, x, lane, sm0, sm1, g.hc, H::ODQ);
-    else if (spd) stage_array8(spd, x, lane, sm0, sm1, g.hc, H::OSPD);
+    const HaloStride<nA> st(g.hc);
+    if (nA == HA_D) stage_array<2>(q, 32, x, lane, sm0, sm1, st.hc, 0);
+    stage_array<1>(g.xy, 16, x, lane, sm0, sm1, st.hc, H::OXY);
+    if (nA == HA_I) stage_array<4>(dq, 64, x, lane, sm0, sm1, st.hc, H::ODQ);
+    else if (spd) stage_array8(spd, x, lane, sm0, sm1, st.hc, H::OSPD);
 }
 
 // The D and I passes with tile halos (halo.cuh): a warp stages two tiles'
@@ -259,7 +289,7 @@ kb_inner_h(Geom g, Sched s, const double *__restrict__ dq0,
     const int ntiles = sched_begin(s, ss, live);
     const int wpb = blockDim.x / 32, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int half = lane / TILE, stride = gridDim.x * wpb;
-    double2 *sm0 = hsm + (size_t)(2 * warp) * HA_I * g.hc, *sm1 = sm0 + HA_I * g.hc;
+    double2 *sm0 = hsm + (2 * warp) * HA_I * g.hc, *sm1 = sm0 + HA_I * g.hc;
     HaloChunk cur;
     for (int ch = blockIdx.x * wpb + warp; 2 * ch < ntiles; ch += stride) {
         halo_chunk(g, s, ss, ntiles, ch, lane, cur);
@@ -292,7 +322,8 @@ kb_grad_h(Geom g, Consts c, Sched s, const R4 *__restrict__ q, const double *__r
     const int ntiles = sched_begin(s, ss, live);
     const int wpb = blockDim.x / 32, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int half = lane / TILE, stride = gridDim.x * wpb;
-    double2 *sm0 = hsm + (size_t)(2 * warp) * HA_D * g.hc, *sm1 = sm0 + HA_D * g.hc;
+    double2 *sm0 = hsm + (2 * warp) * HA_D * HaloStride<HA_D>::hc,
+            *sm1 = sm0 + HA_D * HaloStride<HA_D>::hc;
     HaloChunk cur;
     for (int ch = blockIdx.x * wpb + warp; 2 * ch < ntiles; ch += stride) {
         halo_chunk(g, s, ss, ntiles, ch, lane, cur);
@@ -906,7 +937,8 @@ void launch_flux_coef(const Geom &g, int base, int n, int nw, int no, double pow
 
 // staging memory of a block of the halo kernels: two tiles a warp
 size_t halo_smem_bytes(int kind, int hc) {
-    return halo_bytes(HALO_BLOCK / 32, kind == 0 ? HA_D : HA_I, hc);
+    return kind == 0 ? halo_bytes(HALO_BLOCK / 32, HA_D, HaloStride<HA_D>::hc)
+                     : halo_bytes(HALO_BLOCK / 32, HA_I, hc);
 }
 
 cudaError_t init_kernels() {
