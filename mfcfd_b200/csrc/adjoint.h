@@ -7,13 +7,25 @@
 
 namespace lskum {
 
-constexpr int ADJ_CW = 22;  // contribution record per (point, slot)
+// the enstrophy objective's record per (point, slot): the neighbour's u1, u2, x
+// and y adjoints
+constexpr int OBJREC = 4;
 // flux pass: per (point, slot) the neighbour side's record (adjoint of its
 // limited qtilde, delx/dely adjoint)
 constexpr int NBREC = 6;
-// q-derivative pass: per point the record its neighbours' side reads
-constexpr int GREC = 24;
-enum { ADJ_GATHER_INNER = 1, ADJ_GATHER_GRAD = 2 };
+// doubles per (point, slot) of the buffer that holds the flux pass's records and
+// back sums, or the objective's
+constexpr int ADJ_CW = NBREC + 2;
+// per point, of the least-squares solve being reversed: what its neighbours'
+// side reads (LsqIn)
+constexpr int LREC = 12;
+
+// The rows of dq that made the solve's result: with inner iterations the
+// D pass's dq0 and the previous iteration's; null for the D pass itself.
+struct LsqIn {
+    const double *dq0 = nullptr, *prev = nullptr;
+    __host__ __device__ bool inner() const { return prev != nullptr; }
+};
 
 struct AdjConsts {
     double q_inf[4];
@@ -47,29 +59,34 @@ void launch_update_b(const Geom &g, const Consts &c, const AdjConsts &a, const R
 // k_flux_b_nbr per neighbour over the transposed stencil (the neighbour's
 // reconstruction; writes back [n][kp] (delx, dely) adjoint parts that
 // belong to the point as well), then k_back_sum adds those to the point.
-// nbrec and back may share the contribution buffer (n*kp*(NBREC+2) <=
-// n*kp*ADJ_CW doubles).
+// nbrec and back share one buffer of n*kp*(NBREC+2) doubles.  dqb and rec
+// receive dq's adjoint (with inner iterations; otherwise the record holds all
+// that is needed of it) and the records of the solve that made dq.
 void launch_flux_b(const Geom &g, const R4 *q_in, const double *dq, const double *qm,
-                   const double *delta, const R4 *fr, const double *frb, double *qb,
+                   const double *delta, const R4 *fr, const double *frb, LsqIn in, double *qb,
                    double *dqb, double *qmb, double *xb, double *yb, double *nxb, double *nyb,
                    double *deltab, double *nbrec, double *back, const int *tptr,
-                   const int *tlist, const double *kst, cudaStream_t s);
-void launch_inner_b(const Geom &g, const R4 *q, const double *dq_in, const double *dqb_out,
-                    double *dqb_in, double *qb, double *xb, double *yb, double *contrib,
-                    cudaStream_t s);
-// spdA: |u| + 3 sqrt(p/rho) of primA as the forward pass used it (taped).
-// Two kernels: k_grad_b per point (its own side; writes grec [n][GREC], which
-// may share the contribution buffer) and k_grad_b_nbr per neighbour over the
-// transposed stencil (adds to qb, pb = primA's adjoint, xb, yb).
-void launch_grad_b(const Geom &g, const Consts &c, const R4 *q, const R4 *primA,
-                   const double *spdA, const double *dqb, const double *qmb,
-                   const double *deltab, bool with_delta, double *qb, double *pb, double *xb,
-                   double *yb, double *grec, const int *tptr, const int *tlist,
-                   cudaStream_t s);
-void launch_gather(int n, int kp, const int *tptr, const int *tlist, const double *contrib,
-                   int mode, double *a4, double *a8, double *b8, double *xb, double *yb,
-                   cudaStream_t s);
-void launch_qvar_b(int n, const R4 *prim, const double *qb, double *pb, cudaStream_t s);
+                   const int *tlist, const double *kst, double *rec, cudaStream_t s);
+// One inner iteration, dq_in -> dq_out: dqb holds dq_out's adjoint on entry and
+// dq_in's on exit; rec its records on entry, rec_out those of the solve `in`
+// that made dq_in.  dq0b adds up the outputs' adjoints (dq0 enters every inner
+// iteration's result): `first` (the last iteration, reversed first) stores.
+// With in.inner() false dq_in is dq0 itself, and rec_out has the total.
+void launch_inner_b(const Geom &g, const double *dq_in, LsqIn in, bool first, double *dqb,
+                    double *dq0b, const double *rec, double *rec_out, double *xb, double *yb,
+                    const int *tptr, const int *tlist, cudaStream_t s);
+// spdA: |u| + 3 sqrt(p/rho) of the stage's input state prim as the forward pass
+// used it (taped; read with with_delta only).  Two kernels: k_grad_b per point
+// (its own side, completing rec) and k_grad_b_nbr per neighbour over the
+// transposed stencil (adds to pb = prim's adjoint, xb, yb; q's adjoint qb ends
+// there).
+void launch_grad_b(const Geom &g, const Consts &c, const R4 *q, const R4 *prim,
+                   const double *spdA, const double *qmb, const double *deltab,
+                   bool with_delta, const double *back, double *qb, double *pb, double *xb,
+                   double *yb, double *rec, const int *tptr, const int *tlist, cudaStream_t s);
+// Adds the enstrophy objective's records to the neighbours' pb, xb, yb.
+void launch_gather(int n, const int *tptr, const int *tlist, const double *contrib, double *pb,
+                   double *xb, double *yb, cudaStream_t s);
 void launch_forces_b(const AdjShape &t, const AdjGather &gth, const R4 *prim, const double2 *xy,
                      double mach, double cos_t, double sin_t, int objective, double *pb,
                      double *xb, double *yb, double *nxb, double *nyb, cudaStream_t s);

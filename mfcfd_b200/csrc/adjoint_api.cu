@@ -44,9 +44,9 @@ struct AdjointState {
     R4 *tfr[4] = {nullptr, nullptr, nullptr, nullptr};
     double *tdq = nullptr, *tqm = nullptr, *tdelta = nullptr, *tspd = nullptr;
     double *pb[2] = {nullptr, nullptr}, *pbA = nullptr;
-    double *qb = nullptr, *dqb[2] = {nullptr, nullptr}, *qmb = nullptr, *deltab = nullptr;
+    double *qb = nullptr, *dqb = nullptr, *dq0b = nullptr, *qmb = nullptr, *deltab = nullptr;
     double *frb = nullptr, *xb = nullptr, *yb = nullptr, *nxb = nullptr, *nyb = nullptr;
-    double *contrib = nullptr;
+    double *contrib = nullptr, *rec[2] = {nullptr, nullptr};
     // kinetic-state tape of the re-run (rks stages of [n][kp][KS_TAPE]); null
     // when it did not fit, and the reverse flux pass recomputes the states
     double *tks = nullptr;
@@ -188,8 +188,10 @@ int adj_setup(mfcfd_t *h) {
     CK(dmalloc(&a->tspd, n));
     for (int b = 0; b < 2; ++b) {
         CK(dmalloc(&a->pb[b], (size_t)4 * n));
-        CK(dmalloc(&a->dqb[b], (size_t)8 * n));
+        if (b <= m) CK(dmalloc(&a->rec[b], (size_t)LREC * n));
     }
+    CK(dmalloc(&a->dqb, (size_t)8 * n));
+    if (m > 1) CK(dmalloc(&a->dq0b, (size_t)8 * n));
     CK(dmalloc(&a->pbA, (size_t)4 * n));
     CK(dmalloc(&a->qb, (size_t)4 * n));
     CK(dmalloc(&a->qmb, (size_t)8 * n));
@@ -289,25 +291,25 @@ int reverse_taped(mfcfd_t *h, AdjointState *a) {
     for (int rk = rks; rk >= 1; --rk) {
         double *pb_out = a->pb[out];
         double *pb_in = rk == 1 ? a->pbA : a->pb[out ^ 1];
-        if (rk != 1) CK(cudaMemsetAsync(pb_in, 0, sizeof(double) * 4 * n, s));
         launch_update_b(h->geom, h->consts, ac, a->tprim[rk - 1], a->tprim[0], a->tfr[rk - 1],
                         pb_out, pb_in, a->pbA, a->frb, a->nxb, a->nyb, rk, s);
-        // (writes qb, qmb and dqb[m & 1])
+        // what the solve behind dq_t read
+        auto made = [&](int t) {
+            return t > 0 ? LsqIn{dq_at(a, rk, 0), dq_at(a, rk, t - 1)} : LsqIn{};
+        };
+        double *back = a->contrib + (size_t)n * a->kp * NBREC;
         launch_flux_b(h->geom, a->tq[rk - 1], dq_at(a, rk, m), qm_at(a, rk), a->tdelta,
-                      a->tfr[rk - 1], a->frb, a->qb, a->dqb[m & 1], a->qmb, a->xb, a->yb, a->nxb, a->nyb,
-                      a->deltab, a->contrib, a->contrib + (size_t)n * a->kp * NBREC, a->d_tptr,
-                      a->d_tlist, ks_at(a, rk), s);
-        for (int t = m; t >= 1; --t) {
-            launch_inner_b(h->geom, a->tq[rk - 1], dq_at(a, rk, t - 1), a->dqb[t & 1],
-                           a->dqb[(t - 1) & 1], a->qb, a->xb, a->yb, a->contrib, s);
-            launch_gather(n, a->kp, a->d_tptr, a->d_tlist, a->contrib, ADJ_GATHER_INNER, a->qb,
-                          a->dqb[(t - 1) & 1], nullptr, a->xb, a->yb, s);
-        }
-        launch_grad_b(h->geom, h->consts, a->tq[rk - 1], a->tprim[0], a->tspd, a->dqb[0],
-                      a->qmb, a->deltab, rk == 1, a->qb, a->pbA, a->xb, a->yb, a->contrib,
+                      a->tfr[rk - 1], a->frb, made(m), a->qb, a->dqb, a->qmb, a->xb, a->yb,
+                      a->nxb, a->nyb, a->deltab, a->contrib, back, a->d_tptr, a->d_tlist,
+                      ks_at(a, rk), a->rec[m & 1], s);
+        for (int t = m; t >= 1; --t)
+            launch_inner_b(h->geom, dq_at(a, rk, t - 1), made(t - 1), t == m, a->dqb, a->dq0b,
+                           a->rec[t & 1], a->rec[(t - 1) & 1], a->xb, a->yb, a->d_tptr,
+                           a->d_tlist, s);
+        launch_grad_b(h->geom, h->consts, a->tq[rk - 1], a->tprim[rk - 1], a->tspd, a->qmb,
+                      a->deltab, rk == 1, back, a->qb, pb_in, a->xb, a->yb, a->rec[0],
                       a->d_tptr, a->d_tlist, s);
-        launch_qvar_b(n, a->tprim[rk - 1], a->qb, pb_in, s);
-        h->launches += 7 + 2LL * m;
+        h->launches += 5 + m;
         out ^= 1;
     }
     CK(cudaMemcpyAsync(a->pb[0], a->pbA, sizeof(double) * 4 * n, cudaMemcpyDeviceToDevice, s));
@@ -334,8 +336,7 @@ int reverse_iteration(mfcfd_t *h, AdjointState *a, int k, const R4 *state) {
             lskum_host::launch_objective_b(h, a->objective, a->tprim[a->rks], a->pb[0], a->xb,
                                            a->yb, a->contrib, s);
             if (a->objective == MFCFD_OBJ_ENSTROPHY) {
-                launch_gather(n, a->kp, a->d_tptr, a->d_tlist, a->contrib, ADJ_GATHER_GRAD, a->qb,
-                              nullptr, a->pb[0], a->xb, a->yb, s);
+                launch_gather(n, a->d_tptr, a->d_tlist, a->contrib, a->pb[0], a->xb, a->yb, s);
                 h->launches += 1;
             }
         }
@@ -392,7 +393,7 @@ void lskum_host::free_adjoint(mfcfd_t *h) {
     void *bufs[] = {a->d_tptr, a->d_tlist, a->d_sidx, a->d_sleft, a->d_sright, a->d_snx,
                     a->d_sny, a->d_bleft, a->d_bright, a->d_fptr, a->d_fsrc, a->d_nptr,
                     a->d_nsrc, a->tdq, a->tqm, a->tdelta, a->tspd,
-                    a->pb[0], a->pb[1], a->pbA, a->qb, a->dqb[0], a->dqb[1], a->qmb,
+                    a->pb[0], a->pb[1], a->pbA, a->qb, a->dqb, a->dq0b, a->rec[0], a->rec[1], a->qmb,
                     a->deltab, a->frb, a->xb, a->yb, a->nxb, a->nyb, a->contrib, a->hist,
                     a->snap0, a->fin, a->tks, a->d_fcg};
     for (void *b : bufs)

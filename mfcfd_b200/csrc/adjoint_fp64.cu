@@ -4,19 +4,16 @@
 //   k_update_b   state_update_b      prim_out_b -> prim_in_b, prim_old_b, flux_res_b, n_b
 //   k_flux_b     cal_flux_residual_b flux_res_b -> q_b, dq_b, qm_b, x_b, y_b, n_b, delta_b
 //   k_inner_b    eval_q_inner_loop_b (per inner iteration, last first)
-//   k_grad_b     eval_q_derivatives_b + func_delta_b (first stage)
-//   k_qvar_b     eval_q_variables_b  q_b -> prim_in_b
+//   k_grad_b     eval_q_derivatives_b + func_delta_b (first stage), and
+//                eval_q_variables_b  q_b -> prim_in_b
 // (the stage-by-stage order of the reference's FPI_SOLVER_B,
 // src_mpi_adjoint/sensitivity_files/fpi_solver_b.F90:28-156).
 //
-// A point's adjoint flows to its neighbours, without atomics.  The q-
-// derivative reverses write their contribution for neighbour slot r of
-// point i into contrib[(i*kp + r)*CW + field] and k_gather adds them per
-// neighbour in the fixed (i, r) order of the transposed stencil.  The flux
-// reverse, whose neighbour side is most of the work, pulls instead:
-// k_flux_b leaves a short record per slot and k_flux_b_nbr, one thread per
-// neighbour, reverses the neighbour's reconstruction of each slot naming it
-// in that same order.  Results are deterministic either way.
+// A point's adjoint flows to its neighbours without atomics: one thread per
+// neighbour pulls it over the slots (i, r) naming it, in the fixed (i, r) order
+// of the transposed stencil, from what the slot's point left behind -- a record
+// per slot in the flux reverse, a record per point in the least-squares
+// reverses.  Results are deterministic.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -67,7 +64,7 @@ __device__ __forceinline__ KState kst_taped(const double *v, double nx, double n
 }
 // state_update_b (state_update.F90:10-141, reverse)
 // Stores n (even) doubles as 16-byte pairs; dst is 16-byte aligned (records
-// are ADJ_CW = 22 doubles = 176 bytes from an aligned base).
+// are an even number of doubles from an aligned base).
 __device__ __forceinline__ void st_pairs(double *dst, const double *v, int n) {
     double2 *d2 = reinterpret_cast<double2 *>(dst);
 #pragma unroll
@@ -171,7 +168,9 @@ k_update_b(Geom g, Consts c, AdjConsts a, const R4 *__restrict__ prim_in,
         if (rk == 3) prim_to_conserved_b(O.a, O.b, O.c, O.d, nx, ny, Uob, pbo, nxbv, nybv);
     }
     double *pin = pb_in + 4 * (size_t)i;
-    for (int m = 0; m < 4; ++m) pin[m] += pbi[m];
+    // a middle stage's input adjoint begins here; the first stage's, which the
+    // third stage has added to, is accumulated
+    for (int m = 0; m < 4; ++m) pin[m] = rk == 1 ? pin[m] + pbi[m] : pbi[m];
     if (rk == 3) {
         double *pold = pb_old + 4 * (size_t)i;
         for (int m = 0; m < 4; ++m) pold[m] += pbo[m];
@@ -519,23 +518,60 @@ k_flux_b(Geom g, const R4 *__restrict__ q_in, const double *__restrict__ dq,
     else qmb[8 * (size_t)i + lane - 4] = acc[1];
 }
 
+// The record of the least-squares solve whose result o = L s (L the inverse of
+// the stencil's normal matrix M, s = sum of d times the slots' differences) has
+// the adjoint ob: z = L ob, s's adjoint, and M's, -z o^T, as the sums of dx^2,
+// dy^2 and dx dy receive it.  An inner iteration solves
+// dq_t = dq0 + dq_(t-1) / 2 - L s / 2 (inner_sums), so its z and o carry the
+// factor.  Fields: zx[4], zy[4], M's three, one left for k_grad_b.
+__device__ __forceinline__ void lsq_record(const Geom &g, const LsqIn &in, int i,
+                                           const double outx[4], const double outy[4],
+                                           const double obx[4], const double oby[4],
+                                           double *__restrict__ rec) {
+    double L[4], x0[4], y0[4], xp[4], yp[4];
+    ld4nc(g.minv + 4 * (size_t)i, L);
+    if (in.inner()) {
+        ld8a(in.dq0 + 8 * (size_t)i, x0, y0);
+        ld8a(in.prev + 8 * (size_t)i, xp, yp);
+    }
+    const double f = in.inner() ? -0.5 : 1.0;
+    double v[LREC];
+    v[8] = v[9] = v[10] = v[11] = 0.0;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        const double zx = L[0] * obx[m] + L[1] * oby[m], zy = L[1] * obx[m] + L[2] * oby[m];
+        double ox = outx[m], oy = outy[m];
+        if (in.inner()) {  // the solve's own part of the result
+            ox = ox - x0[m] - 0.5 * xp[m];
+            oy = oy - y0[m] - 0.5 * yp[m];
+        }
+        v[m] = f * zx;
+        v[4 + m] = f * zy;
+        v[8] -= zx * ox;
+        v[9] -= zy * oy;
+        v[10] -= zx * oy + zy * ox;
+    }
+    st_pairs(rec + (size_t)i * LREC, v, LREC);
+}
+
 // The neighbour side of cal_flux_residual_b, one thread per neighbour k:
 // over the slots (i, r) that name k (the transposed stencil, in (i, r)
 // order) it reverses k's reconstruction of that slot from k_flux_b's record
 // and adds the results to k's own adjoints in registers: no scatter and no
 // gather of contribution records.  The part of delx/dely's adjoint that this
 // reconstruction adds belongs to point i as well (delx = x_k - x_i): it is
-// left in back[(i, r)] for k_back_sum.
+// left in back[r][i] for k_grad_b.
 constexpr int NBR_BLK = 128;
-// 128 registers (256,000 points: 74 us, 79 at 3 blocks; 91 when the record held
-// the adjoint of the primitive state)
+// 128 registers (256,000 points: 77 us with the solve's records; before those 74,
+// 79 at 3 blocks, 91 with a record of the primitive state's adjoint)
 constexpr int NBR_MIN_BLOCKS = 4;
 __global__ void __launch_bounds__(NBR_BLK, NBR_MIN_BLOCKS)
 k_flux_b_nbr(Geom g, const R4 *__restrict__ q_in, const double *__restrict__ dq,
              const double *__restrict__ qm, const int *__restrict__ tptr,
-             const int *__restrict__ tlist, const double *__restrict__ nbrec,
+             const int *__restrict__ tlist, const double *__restrict__ nbrec, LsqIn in,
              double *__restrict__ qb, double *__restrict__ dqb, double *__restrict__ qmb,
-             double *__restrict__ xb, double *__restrict__ yb, double2 *__restrict__ back) {
+             double *__restrict__ xb, double *__restrict__ yb, double2 *__restrict__ back,
+             double *__restrict__ rec) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= g.n) return;
     const R4 kv = ld4(q_in + k);
@@ -551,7 +587,7 @@ k_flux_b_nbr(Geom g, const R4 *__restrict__ q_in, const double *__restrict__ dq,
     const int e1 = tptr[k + 1];
     for (int e = tptr[k]; e < e1; ++e) {
         const int slot = tlist[e];
-        const int i = slot / g.kp;
+        const int i = slot / g.kp, r = slot - i * g.kp;
         const double2 pi_ = g.xy[i];
         const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
         // the record: the adjoint of k's limited qtilde, delx/dely's so far
@@ -563,15 +599,11 @@ k_flux_b_nbr(Geom g, const R4 *__restrict__ q_in, const double *__restrict__ dq,
                   qminkb, dxr, dyr);
         xkb += dd.x + dxr;
         ykb += dd.y + dyr;
-        back[slot] = make_double2(dxr, dyr);
+        back[(size_t)r * g.n + i] = make_double2(dxr, dyr);
     }
     add_pairs(qb + 4 * (size_t)k, qkb, 4);
     double v8[8];
-    for (int m = 0; m < 4; ++m) {
-        v8[m] = dxkb[m];
-        v8[4 + m] = dykb[m];
-    }
-    add_pairs(dqb + 8 * (size_t)k, v8, 8);
+#pragma unroll
     for (int m = 0; m < 4; ++m) {
         v8[m] = qmaxkb[m];
         v8[4 + m] = qminkb[m];
@@ -579,294 +611,259 @@ k_flux_b_nbr(Geom g, const R4 *__restrict__ q_in, const double *__restrict__ dq,
     add_pairs(qmb + 8 * (size_t)k, v8, 8);
     xb[k] += xkb;
     yb[k] += ykb;
-}
-
-// x_i, y_i receive minus the delx/dely adjoint parts of their slots'
-// neighbour reconstructions, in slot order.
-__global__ void __launch_bounds__(256)
-k_back_sum(Geom g, const double2 *__restrict__ back, double *__restrict__ xb,
-           double *__restrict__ yb) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= g.n) return;
-    const int nb = g.nbhs[i];
-    double sx = 0.0, sy = 0.0;
-    for (int r = 0; r < nb; ++r) {
-        const double2 v = __ldg(back + (size_t)i * g.kp + r);
-        sx = sx + v.x;
-        sy = sy + v.y;
-    }
-    xb[i] -= sx;
-    yb[i] -= sy;
-}
-
-// eval_q_inner_loop_b: one inner iteration; dqb_out is the adjoint of its
-// output, dqb_in receives the point's own share of the input adjoint.
-__global__ void __launch_bounds__(BLK, ADJ_MIN_BLOCKS)
-k_inner_b(Geom g, const R4 *__restrict__ q, const double *__restrict__ dq_in,
-          const double *__restrict__ dqb_out, double *__restrict__ dqb_in, double *__restrict__ qb,
-          double *__restrict__ xb, double *__restrict__ yb, double *__restrict__ contrib) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= g.n) return;
-    const double2 pi_ = g.xy[i];
-    const R4 qv = ld4(q + i);
-    const double qi[4] = {qv.a, qv.b, qv.c, qv.d};
-    double dxi[4], dyi[4];
-    ld8a(dq_in + 8 * (size_t)i, dxi, dyi);
-    const int nb = g.nbhs[i];
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, sx[4] = {0, 0, 0, 0}, sy[4] = {0, 0, 0, 0};
-    for (int r = 0; r < nb; ++r) {
-        const int k = g.conn[r * g.n + i];
-        const R4 kv = ld4(q + k);
-        const double qk[4] = {kv.a, kv.b, kv.c, kv.d};
-        double dxk[4], dyk[4];
-        ld8a(dq_in + 8 * (size_t)k, dxk, dyk);
-        const double2 pk = g.xy[k];
-        const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
-        s0 = s0 + delx * delx;
-        s1 = s1 + dely * dely;
-        s2 = s2 + delx * dely;
-        for (int m = 0; m < 4; ++m) {
-            const double t1 = qi[m] - 0.5 * (delx * dxi[m] + dely * dyi[m]);
-            const double t2 = qk[m] - 0.5 * (delx * dxk[m] + dely * dyk[m]);
-            sx[m] = sx[m] + delx * (t2 - t1);
-            sy[m] = sy[m] + dely * (t2 - t1);
-        }
-    }
-    const double obd = 1.0 / (s0 * s1 - s2 * s2);
-    double dxb[4], dyb[4];
-    ld8a(dqb_out + 8 * (size_t)i, dxb, dyb);
-    double sxb[4], syb[4], s0b = 0.0, s1b = 0.0, s2b = 0.0, obdb = 0.0;
+    // dq's adjoint is complete: what the last least-squares solve's reverse needs
+    double dxo[4], dyo[4];
+    ld8a(dqb + 8 * (size_t)k, dxo, dyo);
+#pragma unroll
     for (int m = 0; m < 4; ++m) {
-        sxb[m] = (dxb[m] * s1 - dyb[m] * s2) * obd;
-        syb[m] = (-dxb[m] * s2 + dyb[m] * s0) * obd;
-        s1b += dxb[m] * sx[m] * obd;
-        s0b += dyb[m] * sy[m] * obd;
-        s2b += (-dxb[m] * sy[m] - dyb[m] * sx[m]) * obd;
-        obdb += dxb[m] * (sx[m] * s1 - sy[m] * s2) + dyb[m] * (sy[m] * s0 - sx[m] * s2);
+        dxkb[m] += dxo[m];
+        dykb[m] += dyo[m];
     }
-    const double detb = -obdb * obd * obd;
-    s0b += detb * s1;
-    s1b += detb * s0;
-    s2b += -2.0 * detb * s2;
-    double qib[4] = {0, 0, 0, 0}, dxib[4] = {0, 0, 0, 0}, dyib[4] = {0, 0, 0, 0};
-    double xib = 0.0, yib = 0.0;
-    for (int r = 0; r < nb; ++r) {
-        const int k = g.conn[r * g.n + i];
-        const R4 kv = ld4(q + k);
-        const double qk[4] = {kv.a, kv.b, kv.c, kv.d};
-        double dxk[4], dyk[4];
-        ld8a(dq_in + 8 * (size_t)k, dxk, dyk);
-        const double2 pk = g.xy[k];
-        const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
-        double delxb = 2.0 * delx * s0b + dely * s2b;
-        double delyb = 2.0 * dely * s1b + delx * s2b;
-        double *cb = contrib + ((size_t)i * g.kp + r) * ADJ_CW;
-        double v[14];  // the record, stored as 16-byte pairs at the end
-        for (int m = 0; m < 4; ++m) {
-            const double t1 = qi[m] - 0.5 * (delx * dxi[m] + dely * dyi[m]);
-            const double t2 = qk[m] - 0.5 * (delx * dxk[m] + dely * dyk[m]);
-            const double d = t2 - t1;
-            const double db = sxb[m] * delx + syb[m] * dely;
-            delxb += sxb[m] * d;
-            delyb += syb[m] * d;
-            v[m] = db;
-            v[4 + m] = -0.5 * delx * db;
-            v[8 + m] = -0.5 * dely * db;
-            delxb += -0.5 * dxk[m] * db + 0.5 * dxi[m] * db;
-            delyb += -0.5 * dyk[m] * db + 0.5 * dyi[m] * db;
-            qib[m] -= db;
-            dxib[m] += 0.5 * delx * db;
-            dyib[m] += 0.5 * dely * db;
-        }
-        v[12] = delxb;
-        v[13] = delyb;
-        st_pairs(cb, v, 14);
-        xib -= delxb;
-        yib -= delyb;
+    if (in.inner()) {
+        st_pairs(dqb + 8 * (size_t)k, dxkb, 4);
+        st_pairs(dqb + 8 * (size_t)k + 4, dykb, 4);
     }
-    add_pairs(qb + 4 * (size_t)i, qib, 4);
-    st_pairs(dqb_in + 8 * (size_t)i, dxib, 4);
-    st_pairs(dqb_in + 8 * (size_t)i + 4, dyib, 4);
-    xb[i] += xib;
-    yb[i] += yib;
+    lsq_record(g, in, k, dxk, dyk, dxkb, dykb, rec);
 }
 
-// eval_q_derivatives_b (+ func_delta_b on the first stage)
-// eval_q_derivatives_b + func_delta_b, the point's own side.  The
-// neighbours' side reads the point's record grec[i] (GREC doubles: sxb[4],
-// syb[4], s0b, s1b, s2b, deltab, qmaxb[4], qminb[4], the packed arg-max /
-// arg-min slots, the time-step minimum's slot) in k_grad_b_nbr.
-__global__ void __launch_bounds__(BLK, ADJ_MIN_BLOCKS)
-k_grad_b(Geom g, Consts c, const R4 *__restrict__ q, const R4 *__restrict__ primA,
-         const double *__restrict__ spdA, const double *__restrict__ dqb,
-         const double *__restrict__ qmb,
-         const double *__restrict__ deltab, int with_delta, double *__restrict__ qb,
-         double *__restrict__ xb, double *__restrict__ yb, double *__restrict__ grec) {
+// eval_q_inner_loop_b: one inner iteration, dq_out = dq0 + dq_in / 2 - L s / 2,
+// s = sum of d (d . dq_k) (inner_sums).  Half the warps take the points' own
+// slots, of which only x and y's adjoints need the neighbours' rows; the other
+// half the slots naming the points, which give dq_in's.
+// Bound by the rows' gathers.  48 us at 256,000 points (6 blocks an SM; 51 at
+// 5, 50 at 7); 293 as a pass that formed the sums again from q and dq and left
+// a record of 14 doubles per slot, and a pass that gathered the records.
+constexpr int INB_BLK = 128, INB_PTS = INB_BLK / 2;
+__global__ void __launch_bounds__(INB_BLK, 6)
+k_inner_b(Geom g, const double *__restrict__ dq_in, LsqIn in, int first,
+          double *__restrict__ dqb, double *__restrict__ dq0b, const double *__restrict__ rec,
+          double *__restrict__ rec_out, double *__restrict__ xb, double *__restrict__ yb,
+          const int *__restrict__ tptr, const int *__restrict__ tlist) {
+    __shared__ double2 own[INB_PTS];
+    const int t = threadIdx.x % INB_PTS, i = blockIdx.x * INB_PTS + t;
+    const bool pull = threadIdx.x >= INB_PTS;
+    double dxb[4] = {0, 0, 0, 0}, dyb[4] = {0, 0, 0, 0}, gx = 0.0, gy = 0.0;
+    double dxi[4], dyi[4];
+    if (i < g.n) {
+        const double2 pi_ = g.xy[i];
+        if (pull) {
+            ld4nc(dq_in + 8 * (size_t)i, dxi);
+            ld4nc(dq_in + 8 * (size_t)i + 4, dyi);
+            const int e1 = tptr[i + 1];
+            for (int e = tptr[i]; e < e1; ++e) {
+                const int j = tlist[e] / g.kp;  // a point whose neighbour i is
+                double zx[4], zy[4], M[4];
+                ld4nc(rec + (size_t)j * LREC, zx);
+                ld4nc(rec + (size_t)j * LREC + 4, zy);
+                ld4nc(rec + (size_t)j * LREC + 8, M);
+                const double2 pj = g.xy[j];
+                const double dx = pi_.x - pj.x, dy = pi_.y - pj.y;
+                gx += 2.0 * dx * M[0] + dy * M[2];
+                gy += 2.0 * dy * M[1] + dx * M[2];
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const double sb = zx[m] * dx + zy[m] * dy;  // of d . dq_i
+                    const double s = dx * dxi[m] + dy * dyi[m];
+                    gx += zx[m] * s + sb * dxi[m];
+                    gy += zy[m] * s + sb * dyi[m];
+                    dxb[m] += dx * sb;
+                    dyb[m] += dy * sb;
+                }
+            }
+        } else {
+            double zx[4], zy[4], M[4], sx = 0.0, sy = 0.0;
+            ld4nc(rec + (size_t)i * LREC, zx);
+            ld4nc(rec + (size_t)i * LREC + 4, zy);
+            ld4nc(rec + (size_t)i * LREC + 8, M);
+            const int nb = g.nbhs[i];
+#pragma unroll 2
+            for (int r = 0; r < nb; ++r) {
+                const int k = g.conn[(size_t)r * g.n + i];
+                double dxk[4], dyk[4];
+                ld4nc(dq_in + 8 * (size_t)k, dxk);
+                ld4nc(dq_in + 8 * (size_t)k + 4, dyk);
+                const double2 pk = g.xy[k];
+                const double dx = pk.x - pi_.x, dy = pk.y - pi_.y;
+                sx += dx;
+                sy += dy;
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const double sb = zx[m] * dx + zy[m] * dy;
+                    const double s = dx * dxk[m] + dy * dyk[m];
+                    gx -= zx[m] * s + sb * dxk[m];
+                    gy -= zy[m] * s + sb * dyk[m];
+                }
+            }
+            gx -= 2.0 * sx * M[0] + sy * M[2];
+            gy -= 2.0 * sy * M[1] + sx * M[2];
+            own[t] = make_double2(gx, gy);
+        }
+    }
+    __syncthreads();
+    if (!pull || i >= g.n) return;
+    xb[i] += gx + own[t].x;
+    yb[i] += gy + own[t].y;
+    double ox[4], oy[4];
+    ld8a(dqb + 8 * (size_t)i, ox, oy);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        dxb[m] += 0.5 * ox[m];
+        dyb[m] += 0.5 * oy[m];
+    }
+    // dq0's adjoint so far
+    if (!first) {
+        double ax[4], ay[4];
+        ld8a(dq0b + 8 * (size_t)i, ax, ay);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            ox[m] += ax[m];
+            oy[m] += ay[m];
+        }
+    }
+    if (in.inner()) {
+        st_pairs(dq0b + 8 * (size_t)i, ox, 4);
+        st_pairs(dq0b + 8 * (size_t)i + 4, oy, 4);
+        st_pairs(dqb + 8 * (size_t)i, dxb, 4);
+        st_pairs(dqb + 8 * (size_t)i + 4, dyb, 4);
+    } else {
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            dxb[m] += ox[m];
+            dyb[m] += oy[m];
+        }
+    }
+    lsq_record(g, in, i, dxi, dyi, dxb, dyb, rec_out);
+}
+
+// eval_q_derivatives_b + func_delta_b, the point's own side: its sums over the
+// neighbours (the solve's adjoint z comes in the record), the neighbours that
+// gave qmax, qmin and the time step -- left packed in the record's last field,
+// 5 bits each and 0 for none, for k_grad_b_nbr -- and the parts of delx/dely's
+// adjoint that k_flux_b_nbr left in back.  33 us at 256,000 points, 45 with the
+// time step (7 blocks an SM; 83 and 55 at 6, 38 and 56 at 8); 66 and a pass of
+// 12 for back when it summed the solve again and wrote a record of 24 doubles.
+template <bool with_delta>
+__global__ void __launch_bounds__(BLK, 7)
+k_grad_b(Geom g, Consts c, const R4 *__restrict__ q, const double *__restrict__ spdA,
+         const double *__restrict__ qmb, const double *__restrict__ deltab,
+         const double2 *__restrict__ back, double *__restrict__ qb, double *__restrict__ xb,
+         double *__restrict__ yb, double *__restrict__ rec) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.n) return;
     const double2 pi_ = g.xy[i];
-    const R4 qv = ld4(q + i);
-    const double qi[4] = {qv.a, qv.b, qv.c, qv.d};
+    double qi[4], qmax[4], qmin[4], sq[4] = {0, 0, 0, 0};
+    ld4nc(reinterpret_cast<const double *>(q + i), qi);
     const int nb = g.nbhs[i];
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, sx[4] = {0, 0, 0, 0}, sy[4] = {0, 0, 0, 0};
-    double qmax[4] = {qi[0], qi[1], qi[2], qi[3]}, qmin[4] = {qi[0], qi[1], qi[2], qi[3]};
-    int amax[4] = {-1, -1, -1, -1}, amin[4] = {-1, -1, -1, -1};
-    double min_delt = 1.0;
-    int amd = -1;
+    // arg-max, arg-min: slot + 1, 0 for the point itself
+    int amax[4] = {0, 0, 0, 0}, amin[4] = {0, 0, 0, 0}, amd = 0;
+    double min_delt = 1.0, sx = 0.0, sy = 0.0, bx = 0.0, by = 0.0;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) qmax[m] = qmin[m] = qi[m];
+#pragma unroll 2
     for (int r = 0; r < nb; ++r) {
-        const int k = g.conn[r * g.n + i];
-        const R4 kv = ld4(q + k);
-        const double qk[4] = {kv.a, kv.b, kv.c, kv.d};
-        for (int m = 0; m < 4; ++m) {
-            if (qk[m] > qmax[m]) { qmax[m] = qk[m]; amax[m] = r; }
-            if (qk[m] < qmin[m]) { qmin[m] = qk[m]; amin[m] = r; }
-        }
-        const double2 pk = g.xy[k];
+        const int k = g.conn[(size_t)r * g.n + i];
+        double qk[4];
+        ld4nc(reinterpret_cast<const double *>(q + k), qk);
+        const double2 pk = g.xy[k], v = back[(size_t)r * g.n + i];
         const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
-        s0 = s0 + delx * delx;
-        s1 = s1 + dely * dely;
-        s2 = s2 + delx * dely;
+        sx += delx;
+        sy += dely;
+        bx += v.x;
+        by += v.y;
+#pragma unroll
         for (int m = 0; m < 4; ++m) {
-            sx[m] = sx[m] + delx * (qk[m] - qi[m]);
-            sy[m] = sy[m] + dely * (qk[m] - qi[m]);
+            sq[m] += qk[m] - qi[m];
+            if (qk[m] > qmax[m]) { qmax[m] = qk[m]; amax[m] = r + 1; }
+            if (qk[m] < qmin[m]) { qmin[m] = qk[m]; amin[m] = r + 1; }
         }
         if (with_delta) {
             // the taped spd of the stage's input state: the forward's own values
             const double dist = sqrt(delx * delx + dely * dely);
             double delta_t = dist / spdA[k];
             delta_t = c.cfl * delta_t;
-            if (min_delt > delta_t) { min_delt = delta_t; amd = r; }
+            if (min_delt > delta_t) { min_delt = delta_t; amd = r + 1; }
         }
     }
-    const double obd = 1.0 / (s0 * s1 - s2 * s2);
-    double dxb[4], dyb[4], qmxb[4], qmnb[4];
-    ld8a(dqb + 8 * (size_t)i, dxb, dyb);
-    ld8a(qmb + 8 * (size_t)i, qmxb, qmnb);
-    double sxb[4], syb[4], s0b = 0.0, s1b = 0.0, s2b = 0.0, obdb = 0.0;
+    double *ri = rec + (size_t)i * LREC;
+    double zx[4], zy[4], qib[4], qxb[4], qnb[4];
+    ld8a(ri, zx, zy);
+    ld8a(qmb + 8 * (size_t)i, qxb, qnb);
+    const double s0b = ri[8], s1b = ri[9], s2b = ri[10];
+    double xib = bx + 2.0 * sx * s0b + sy * s2b, yib = by + 2.0 * sy * s1b + sx * s2b;
+    long long code = 0;
+#pragma unroll
     for (int m = 0; m < 4; ++m) {
-        sxb[m] = (dxb[m] * s1 - dyb[m] * s2) * obd;
-        syb[m] = (-dxb[m] * s2 + dyb[m] * s0) * obd;
-        s1b += dxb[m] * sx[m] * obd;
-        s0b += dyb[m] * sy[m] * obd;
-        s2b += (-dxb[m] * sy[m] - dyb[m] * sx[m]) * obd;
-        obdb += dxb[m] * (sx[m] * s1 - sy[m] * s2) + dyb[m] * (sy[m] * s0 - sx[m] * s2);
+        xib += zx[m] * sq[m];
+        yib += zy[m] * sq[m];
+        qib[m] = -(zx[m] * sx + zy[m] * sy);
+        if (!amax[m]) qib[m] += qxb[m];
+        if (!amin[m]) qib[m] += qnb[m];
+        code |= (long long)amax[m] << (5 * m) | (long long)amin[m] << (20 + 5 * m);
     }
-    const double detb = -obdb * obd * obd;
-    s0b += detb * s1;
-    s1b += detb * s0;
-    s2b += -2.0 * detb * s2;
-    const double dlb = with_delta ? deltab[i] : 0.0;
-    const int amd_used = (with_delta && dlb != 0.0) ? amd : -1;
-    {
-        // the record: slots packed 5 bits each (+1, so -1 -> 0), arg-max in
-        // bits 0-19, arg-min in bits 20-39
-        long long code = 0;
-        for (int m = 0; m < 4; ++m) {
-            code |= (long long)(amax[m] + 1) << (5 * m);
-            code |= (long long)(amin[m] + 1) << (20 + 5 * m);
-        }
-        double v[GREC];
-        for (int m = 0; m < 4; ++m) {
-            v[m] = sxb[m];
-            v[4 + m] = syb[m];
-            v[12 + m] = qmxb[m];
-            v[16 + m] = qmnb[m];
-        }
-        v[8] = s0b;
-        v[9] = s1b;
-        v[10] = s2b;
-        v[11] = dlb;
-        v[20] = __longlong_as_double(code);
-        v[21] = (double)amd_used;
-        v[22] = 0.0;
-        v[23] = 0.0;
-        st_pairs(grec + (size_t)i * GREC, v, GREC);
-    }
-    double qib[4] = {0, 0, 0, 0}, xib = 0.0, yib = 0.0;
-    for (int m = 0; m < 4; ++m) {
-        if (amax[m] < 0) qib[m] += qmxb[m];
-        if (amin[m] < 0) qib[m] += qmnb[m];
-    }
-    for (int r = 0; r < nb; ++r) {
-        const int k = g.conn[r * g.n + i];
-        const R4 kv = ld4(q + k);
-        const double qk[4] = {kv.a, kv.b, kv.c, kv.d};
-        const double2 pk = g.xy[k];
-        const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
-        double delxb = 2.0 * delx * s0b + dely * s2b;
-        double delyb = 2.0 * dely * s1b + delx * s2b;
-        for (int m = 0; m < 4; ++m) {
-            const double t = sxb[m] * delx + syb[m] * dely;
-            qib[m] -= t;
-            delxb += sxb[m] * (qk[m] - qi[m]);
-            delyb += syb[m] * (qk[m] - qi[m]);
-        }
-        if (r == amd_used) {
-            const R4 P = ld4(primA + k);
-            const double modu = sqrt(P.b * P.b + P.c * P.c);
-            const double cs = sqrt(P.d / P.a);
-            const double spd = modu + 3.0 * cs;
+    if (with_delta && amd) {
+        const double dlb = deltab[i];
+        if (dlb != 0.0) {
+            const int k = g.conn[(size_t)(amd - 1) * g.n + i];
+            const double2 pk = g.xy[k];
+            const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
             const double dist = sqrt(delx * delx + dely * dely);
-            const double distb = dlb * c.cfl / spd;
-            delxb += distb * delx / dist;
-            delyb += distb * dely / dist;
+            const double distb = dlb * c.cfl / spdA[k];
+            xib += distb * delx / dist;
+            yib += distb * dely / dist;
+            code |= (long long)amd << 40;
         }
-        xib -= delxb;
-        yib -= delyb;
     }
-    for (int m = 0; m < 4; ++m) qb[4 * (size_t)i + m] += qib[m];
-    xb[i] += xib;
-    yb[i] += yib;
+    ri[11] = __longlong_as_double(code);
+    add_pairs(qb + 4 * (size_t)i, qib, 4);
+    xb[i] -= xib;
+    yb[i] -= yib;
 }
 
 // The neighbours' side of eval_q_derivatives_b + func_delta_b, one thread
 // per neighbour k over the slots (i, r) naming it, in the transposed
 // stencil's (i, r) order: q_k's adjoint from the point's least-squares sums
-// and max/min, the time-step minimum's adjoint through k's taped state, and
+// and max/min, the time-step minimum's adjoint through k's state, and
 // delx/dely's (the point's side takes the same value with the other sign).
-__global__ void __launch_bounds__(BLK)
-k_grad_b_nbr(Geom g, Consts c, const R4 *__restrict__ q, const R4 *__restrict__ primA,
+// q's adjoint is complete then, and goes on to the primitive state
+// (eval_q_variables_b).  40 us at 256,000 points (5 blocks an SM; 45 at 4, 49 at
+// 6); 62 and a pass of 10 for the primitive state with the longer record.
+__global__ void __launch_bounds__(BLK, 5)
+k_grad_b_nbr(Geom g, Consts c, const R4 *__restrict__ q, const R4 *__restrict__ prim,
+             const double *__restrict__ qmb, const double *__restrict__ deltab,
              const int *__restrict__ tptr, const int *__restrict__ tlist,
-             const double *__restrict__ grec, double *__restrict__ qb, double *__restrict__ pb,
-             double *__restrict__ xb, double *__restrict__ yb) {
+             const double *__restrict__ rec, const double *__restrict__ qb,
+             double *__restrict__ pb, double *__restrict__ xb, double *__restrict__ yb) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= g.n) return;
-    const R4 kv = ld4(q + k);
-    const double qk[4] = {kv.a, kv.b, kv.c, kv.d};
+    double qk[4], qkb[4], pkb[4] = {0, 0, 0, 0}, xkb = 0.0, ykb = 0.0;
+    ld4nc(reinterpret_cast<const double *>(q + k), qk);
+    ld4nc(qb + 4 * (size_t)k, qkb);
+    const R4 P = ld4(prim + k);
     const double2 pk = g.xy[k];
-    double qkb[4] = {0, 0, 0, 0}, pkb[4] = {0, 0, 0, 0}, xkb = 0.0, ykb = 0.0;
     const int e1 = tptr[k + 1];
     for (int e = tptr[k]; e < e1; ++e) {
         const int slot = tlist[e];
         const int i = slot / g.kp, r = slot - i * g.kp;
-        const double2 *rv = reinterpret_cast<const double2 *>(grec + (size_t)i * GREC);
-        double v[GREC];
-#pragma unroll
-        for (int h = 0; h < 6; ++h) {  // sxb, syb, s0b..s2b, deltab
-            const double2 t2 = __ldg(rv + h);
-            v[2 * h] = t2.x;
-            v[2 * h + 1] = t2.y;
-        }
-        const double2 cd = __ldg(rv + 10);
-        const long long code = __double_as_longlong(cd.x);
-        const int amd = (int)cd.y;
-        const R4 qv = ld4(q + i);
-        const double qi[4] = {qv.a, qv.b, qv.c, qv.d};
+        double zx[4], zy[4], M[4], qi[4];
+        ld4nc(rec + (size_t)i * LREC, zx);
+        ld4nc(rec + (size_t)i * LREC + 4, zy);
+        ld4nc(rec + (size_t)i * LREC + 8, M);
+        ld4nc(reinterpret_cast<const double *>(q + i), qi);
         const double2 pi_ = g.xy[i];
+        const long long code = __double_as_longlong(M[3]);
         const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
-        double delxb = 2.0 * delx * v[8] + dely * v[10];
-        double delyb = 2.0 * dely * v[9] + delx * v[10];
+        double delxb = 2.0 * delx * M[0] + dely * M[2];
+        double delyb = 2.0 * dely * M[1] + delx * M[2];
+#pragma unroll
         for (int m = 0; m < 4; ++m) {
-            qkb[m] += v[m] * delx + v[4 + m] * dely;
-            if ((int)((code >> (5 * m)) & 31) == r + 1) qkb[m] += grec[(size_t)i * GREC + 12 + m];
-            if ((int)((code >> (20 + 5 * m)) & 31) == r + 1)
-                qkb[m] += grec[(size_t)i * GREC + 16 + m];
-            delxb += v[m] * (qk[m] - qi[m]);
-            delyb += v[4 + m] * (qk[m] - qi[m]);
+            qkb[m] += zx[m] * delx + zy[m] * dely;
+            if ((int)((code >> (5 * m)) & 31) == r + 1) qkb[m] += qmb[8 * (size_t)i + m];
+            if ((int)((code >> (20 + 5 * m)) & 31) == r + 1) qkb[m] += qmb[8 * (size_t)i + 4 + m];
+            delxb += zx[m] * (qk[m] - qi[m]);
+            delyb += zy[m] * (qk[m] - qi[m]);
         }
-        if (r == amd) {
-            const double dlb = v[11];
-            const R4 P = ld4(primA + k);
+        if ((int)(code >> 40) == r + 1) {
+            const double dlb = deltab[i];
             const double modu = sqrt(P.b * P.b + P.c * P.c);
             const double cs = sqrt(P.d / P.a);
             const double spd = modu + 3.0 * cs;
@@ -886,56 +883,32 @@ k_grad_b_nbr(Geom g, Consts c, const R4 *__restrict__ q, const R4 *__restrict__ 
         xkb += delxb;
         ykb += delyb;
     }
-    add_pairs(qb + 4 * (size_t)k, qkb, 4);
+    q_from_prim_b(P.a, P.b, P.c, P.d, qkb, pkb);
     add_pairs(pb + 4 * (size_t)k, pkb, 4);
     xb[k] += xkb;
     yb[k] += ykb;
 }
 
-// Adds the neighbour contributions per point in the fixed transposed order.
-// MODE fixes the record width (14 inner, 10 grad fields) so the
-// accumulators stay in registers; records are read as 16-byte pairs.
-template <int MODE>
+// Adds the enstrophy objective's records (u1, u2, x, y of the neighbour) per
+// point, in the transposed stencil's order.
 __global__ void __launch_bounds__(256)
 k_gather(int n, const int *__restrict__ tptr, const int *__restrict__ tlist,
-         const double *__restrict__ contrib, double *__restrict__ a4, double *__restrict__ a8,
-         double *__restrict__ b8, double *__restrict__ xb, double *__restrict__ yb) {
-    constexpr int NF = MODE == ADJ_GATHER_INNER ? 14 : 10;
+         const double *__restrict__ contrib, double *__restrict__ pb, double *__restrict__ xb,
+         double *__restrict__ yb) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    double acc[NF];
-#pragma unroll
-    for (int f = 0; f < NF; ++f) acc[f] = 0.0;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
     const int e1 = tptr[k + 1];
     for (int e = tptr[k]; e < e1; ++e) {
-        const double2 *cb = reinterpret_cast<const double2 *>(contrib + (size_t)tlist[e] * ADJ_CW);
+        double v[4];
+        ld4nc(contrib + (size_t)tlist[e] * OBJREC, v);
 #pragma unroll
-        for (int f = 0; f < NF / 2; ++f) {
-            const double2 v = __ldg(cb + f);
-            acc[2 * f] = acc[2 * f] + v.x;
-            acc[2 * f + 1] = acc[2 * f + 1] + v.y;
-        }
+        for (int f = 0; f < 4; ++f) acc[f] = acc[f] + v[f];
     }
-    add_pairs(a4 + 4 * (size_t)k, acc, 4);
-    if constexpr (MODE == ADJ_GATHER_INNER) {
-        add_pairs(a8 + 8 * (size_t)k, acc + 4, 8);
-    } else {
-        add_pairs(b8 + 4 * (size_t)k, acc + 4, 4);
-    }
-    xb[k] += acc[NF - 2];
-    yb[k] += acc[NF - 1];
-}
-
-// eval_q_variables_b: pb += (dq/dprim)^T qb
-__global__ void __launch_bounds__(256)
-k_qvar_b(int n, const R4 *__restrict__ prim, const double *__restrict__ qb,
-         double *__restrict__ pb) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const R4 P = ld4(prim + i);
-    double p[4] = {0.0, 0.0, 0.0, 0.0};
-    q_from_prim_b(P.a, P.b, P.c, P.d, qb + 4 * (size_t)i, p);
-    for (int m = 0; m < 4; ++m) pb[4 * (size_t)i + m] += p[m];
+    pb[4 * (size_t)k + 1] += acc[0];
+    pb[4 * (size_t)k + 2] += acc[1];
+    xb[k] += acc[2];
+    yb[k] += acc[3];
 }
 
 // compute_force_coeffs_b: J = sum over shapes of Cl (objective 0) or Cd (1).
@@ -1093,50 +1066,41 @@ void launch_update_b(const Geom &g, const Consts &c, const AdjConsts &a, const R
 }
 
 void launch_flux_b(const Geom &g, const R4 *q_in, const double *dq, const double *qm,
-                   const double *delta, const R4 *fr, const double *frb, double *qb,
+                   const double *delta, const R4 *fr, const double *frb, LsqIn in, double *qb,
                    double *dqb, double *qmb, double *xb, double *yb, double *nxb, double *nyb,
                    double *deltab, double *nbrec, double *back, const int *tptr,
-                   const int *tlist, const double *kst, cudaStream_t s) {
+                   const int *tlist, const double *kst, double *rec, cudaStream_t s) {
     k_flux_b<<<nblk(g.n, GROUPS), BLK, 0, s>>>(g, q_in, dq, qm, delta,
                                                reinterpret_cast<const double *>(fr), frb, qb,
                                                dqb, qmb, xb, yb, nxb, nyb, deltab, nbrec, kst);
     double2 *bk = reinterpret_cast<double2 *>(back);
-    k_flux_b_nbr<<<nblk(g.n, NBR_BLK), NBR_BLK, 0, s>>>(g, q_in, dq, qm, tptr, tlist, nbrec,
-                                                       qb, dqb, qmb, xb, yb, bk);
-    k_back_sum<<<nblk(g.n, 256), 256, 0, s>>>(g, bk, xb, yb);
+    k_flux_b_nbr<<<nblk(g.n, NBR_BLK), NBR_BLK, 0, s>>>(g, q_in, dq, qm, tptr, tlist, nbrec, in,
+                                                       qb, dqb, qmb, xb, yb, bk, rec);
 }
 
-void launch_inner_b(const Geom &g, const R4 *q, const double *dq_in, const double *dqb_out,
-                    double *dqb_in, double *qb, double *xb, double *yb, double *contrib,
-                    cudaStream_t s) {
-    k_inner_b<<<nblk(g.n, BLK), BLK, 0, s>>>(g, q, dq_in, dqb_out, dqb_in, qb, xb, yb, contrib);
+void launch_inner_b(const Geom &g, const double *dq_in, LsqIn in, bool first, double *dqb,
+                    double *dq0b, const double *rec, double *rec_out, double *xb, double *yb,
+                    const int *tptr, const int *tlist, cudaStream_t s) {
+    k_inner_b<<<nblk(g.n, INB_PTS), INB_BLK, 0, s>>>(g, dq_in, in, first ? 1 : 0, dqb, dq0b, rec,
+                                                     rec_out, xb, yb, tptr, tlist);
 }
 
-void launch_grad_b(const Geom &g, const Consts &c, const R4 *q, const R4 *primA,
-                   const double *spdA, const double *dqb, const double *qmb,
-                   const double *deltab, bool with_delta, double *qb, double *pb, double *xb,
-                   double *yb, double *grec, const int *tptr, const int *tlist,
-                   cudaStream_t s) {
-    k_grad_b<<<nblk(g.n, BLK), BLK, 0, s>>>(g, c, q, primA, spdA, dqb, qmb, deltab,
-                                           with_delta ? 1 : 0, qb, xb, yb, grec);
-    k_grad_b_nbr<<<nblk(g.n, BLK), BLK, 0, s>>>(g, c, q, primA, tptr, tlist, grec, qb, pb, xb,
-                                               yb);
-}
-
-void launch_gather(int n, int kp, const int *tptr, const int *tlist, const double *contrib,
-                   int mode, double *a4, double *a8, double *b8, double *xb, double *yb,
-                   cudaStream_t s) {
-    (void)kp;
-    if (mode == ADJ_GATHER_INNER)
-        k_gather<ADJ_GATHER_INNER><<<nblk(n, 256), 256, 0, s>>>(n, tptr, tlist, contrib, a4, a8,
-                                                               b8, xb, yb);
+void launch_grad_b(const Geom &g, const Consts &c, const R4 *q, const R4 *prim,
+                   const double *spdA, const double *qmb, const double *deltab,
+                   bool with_delta, const double *back, double *qb, double *pb, double *xb,
+                   double *yb, double *rec, const int *tptr, const int *tlist, cudaStream_t s) {
+    const double2 *bk = reinterpret_cast<const double2 *>(back);
+    const int nb = nblk(g.n, BLK);
+    if (with_delta)
+        k_grad_b<true><<<nb, BLK, 0, s>>>(g, c, q, spdA, qmb, deltab, bk, qb, xb, yb, rec);
     else
-        k_gather<ADJ_GATHER_GRAD><<<nblk(n, 256), 256, 0, s>>>(n, tptr, tlist, contrib, a4, a8, b8,
-                                                              xb, yb);
+        k_grad_b<false><<<nb, BLK, 0, s>>>(g, c, q, spdA, qmb, deltab, bk, qb, xb, yb, rec);
+    k_grad_b_nbr<<<nb, BLK, 0, s>>>(g, c, q, prim, qmb, deltab, tptr, tlist, rec, qb, pb, xb, yb);
 }
 
-void launch_qvar_b(int n, const R4 *prim, const double *qb, double *pb, cudaStream_t s) {
-    k_qvar_b<<<nblk(n, 256), 256, 0, s>>>(n, prim, qb, pb);
+void launch_gather(int n, const int *tptr, const int *tlist, const double *contrib, double *pb,
+                   double *xb, double *yb, cudaStream_t s) {
+    k_gather<<<nblk(n, 256), 256, 0, s>>>(n, tptr, tlist, contrib, pb, xb, yb);
 }
 
 void launch_forces_b(const AdjShape &t, const AdjGather &gth, const R4 *prim, const double2 *xy,

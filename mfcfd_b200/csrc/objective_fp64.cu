@@ -90,8 +90,8 @@ __global__ void k_obj_terms(Geom g, Consts c, const R4 *__restrict__ prim, int k
 // Seeds of the reverse sweep (the adjoints of the Tapenade _b routines of
 // the objectives): pb += dJ/dprim of each point; for the enstrophy also the
 // coordinates (xb, yb of the point itself, and per stencil slot a
-// contribution record for the neighbour: fields 4..7 its prim adjoint, 8..9
-// its x, y adjoint, added by the gather in the transposed-stencil order).
+// record of the neighbour's u1, u2, x and y adjoints, added by the gather in
+// the transposed-stencil order).
 __global__ void k_obj_seed_b(Geom g, const R4 *__restrict__ prim, int kind, double gamma_power,
                              double p0_inf, double scale, double *__restrict__ pb,
                              double *__restrict__ xb, double *__restrict__ yb,
@@ -152,14 +152,11 @@ __global__ void k_obj_seed_b(Geom g, const R4 *__restrict__ prim, int kind, doub
             const double dyb = 2.0 * dy * syyb + dx * sxyb + du1 * syu1b + du2 * syu2b;
             const double du1b = dx * sxu1b + dy * syu1b;
             const double du2b = dx * sxu2b + dy * syu2b;
-            double *cb = contrib + ((size_t)i * g.kp + r) * ADJ_CW;
-            cb[0] = cb[1] = cb[2] = cb[3] = 0.0;
-            cb[4] = 0.0;
-            cb[5] = du1b;
-            cb[6] = du2b;
-            cb[7] = 0.0;
-            cb[8] = dxb;
-            cb[9] = dyb;
+            double *cb = contrib + ((size_t)i * g.kp + r) * OBJREC;
+            cb[0] = du1b;
+            cb[1] = du2b;
+            cb[2] = dxb;
+            cb[3] = dyb;
             u1ib -= du1b;
             u2ib -= du2b;
             xib -= dxb;
