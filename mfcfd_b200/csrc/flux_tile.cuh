@@ -15,6 +15,14 @@ constexpr int FLUX_BLOCK = 128;              // four warps
 constexpr int FLUX_WARPS = FLUX_BLOCK / 32;
 constexpr int CHUNK_MAX = 2 * TILE;          // points of a chunk
 
+// The small grids' D and I passes: a point's eight lanes leave their slots'
+// fields in shared memory, SLOT_F elements a field and SLOT_P a point, so that
+// a warp's stores and loads fall on distinct banks.
+constexpr int SLOT_BLOCK = 128, SLOT_PTS = SLOT_BLOCK / LPP, SLOT_F = 9, SLOT_P = 68;
+__device__ __forceinline__ int slot_point(const Sched &s, const SchedSmem &ss, int total, int vp) {
+    return vp < total ? sched_point(s, ss, vp) : -1;
+}
+
 // Sum of v over the eight lanes of a point: component 2 (bit 2) + (bit 1) of
 // the lane, in a fixed order.
 __device__ __forceinline__ double reduce8(const double v[4], int lane) {

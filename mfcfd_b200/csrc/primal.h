@@ -105,6 +105,9 @@ struct StageBufs {
 // then the neighbour's reconstruction rho p/rho B1 B2 erf1 erf2 u1 u2
 constexpr int KS_TAPE = 16;
 
+// whether the D and I passes of a grid of n points go by slots
+bool slot_passes(int n);
+
 // The passes of one stage.  Each is a grid-stride kernel over the tiles of
 // the scheduled instances; `block` threads per block for the point passes
 // and `grid` blocks (0 = one wave of resident blocks).

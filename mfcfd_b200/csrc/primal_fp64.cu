@@ -174,11 +174,11 @@ __device__ __forceinline__ void grad_sums(const Consts &c, const Geom &g, int i,
             for (int m = 0; m < 4; ++m) {
                 if (qk[m] > qmax[m]) qmax[m] = qk[m];
                 if (qk[m] < qmin[m]) qmin[m] = qk[m];
-                sdxq[m] = sdxq[m] + wx * (qk[m] - qi[m]);
-                sdyq[m] = sdyq[m] + wy * (qk[m] - qi[m]);
+                sdxq[m] = fma(wx, qk[m] - qi[m], sdxq[m]);
+                sdyq[m] = fma(wy, qk[m] - qi[m], sdyq[m]);
             }
             if (with_delta) {
-                double delta_t = sqrt(delx * delx + dely * dely) / R.spdv(k);
+                double delta_t = sqrt(fma(delx, delx, dely * dely)) / R.spdv(k);
                 delta_t = c.cfl * delta_t;
                 if (min_delt > delta_t) min_delt = delta_t;
             }
@@ -186,8 +186,8 @@ __device__ __forceinline__ void grad_sums(const Consts &c, const Geom &g, int i,
     }
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
-        dx[m] = M.a * sdxq[m] + M.b * sdyq[m];
-        dy[m] = M.b * sdxq[m] + M.c * sdyq[m];
+        dx[m] = fma(M.a, sdxq[m], M.b * sdyq[m]);
+        dy[m] = fma(M.b, sdxq[m], M.c * sdyq[m]);
     }
 }
 
@@ -224,9 +224,9 @@ __device__ __forceinline__ void inner_sums(const Geom &g, int i, const Rows &R, 
             const double wx = w * delx, wy = w * dely;
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
-                const double t = delx * dxk[m] + dely * dyk[m];
-                sA[m] = sA[m] + wx * t;
-                sB[m] = sB[m] + wy * t;
+                const double t = fma(delx, dxk[m], dely * dyk[m]);
+                sA[m] = fma(wx, t, sA[m]);
+                sB[m] = fma(wy, t, sB[m]);
             }
         }
     }
@@ -234,10 +234,10 @@ __device__ __forceinline__ void inner_sums(const Geom &g, int i, const Rows &R, 
     R.dqrow(me, dxi, dyi);
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
-        const double Lx = M.a * sA[m] + M.b * sB[m];
-        const double Ly = M.b * sA[m] + M.c * sB[m];
-        dx[m] = (dq0x[m] + 0.5 * dxi[m]) - 0.5 * Lx;
-        dy[m] = (dq0y[m] + 0.5 * dyi[m]) - 0.5 * Ly;
+        const double Lx = fma(M.a, sA[m], M.b * sB[m]);
+        const double Ly = fma(M.b, sA[m], M.c * sB[m]);
+        dx[m] = fma(-0.5, Lx, fma(0.5, dxi[m], dq0x[m]));
+        dy[m] = fma(-0.5, Ly, fma(0.5, dyi[m], dq0y[m]));
     }
 }
 
@@ -344,6 +344,145 @@ kb_grad_h(Geom g, Consts c, Sched s, const R4 *__restrict__ q, const double *__r
             if (with_delta) delta[cur.i] = min_delt;
         }
         __syncwarp();
+    }
+}
+
+// The D and I passes of a small grid (slot_passes): eight lanes a point, a
+// stencil slot a lane, four points a warp.  With few points the passes wait,
+// they do not compute: the halo form's chain (halo range, row indices, copies,
+// then eight slots in turn) becomes index, row, eight sums.  A slot's lane
+// leaves its row in shared memory and lane l sums field l over the slots in
+// slot order, the halo form's own operations, so a grid gets the same values
+// from either (the products' contractions are spelled out in both).
+// D and I pass at 1,536 points, one inner iteration: an iteration 65.2 ->
+// 48.2 us; at 16,000 points 97.0 -> 87.8.
+__global__ void __launch_bounds__(SLOT_BLOCK)
+kb_grad_s(Geom g, Consts c, Sched s, const R4 *__restrict__ q, const double *__restrict__ spd,
+          double *__restrict__ dq, double *__restrict__ qm, double *__restrict__ delta,
+          int with_delta) {
+    __shared__ SchedSmem ss;
+    __shared__ double sm[SLOT_PTS * SLOT_P];
+    int live;
+    const int total = sched_begin(s, ss, live) * TILE;
+    const int p = threadIdx.x / LPP, l = threadIdx.x % LPP, m = l & 3;
+    double *row = sm + p * SLOT_P;  // fields qk[4], w dx, w dy
+    for (int v0 = blockIdx.x * SLOT_PTS; v0 < total; v0 += gridDim.x * SLOT_PTS) {
+        const int i = slot_point(s, ss, total, v0 + p);
+        int nb = 0, k = 0;
+        double2 pi_ = make_double2(0.0, 0.0);
+        double qi = 0.0, M0 = 0.0, M1 = 0.0;
+        if (i >= 0) {
+            nb = __ldg(g.nbhs + i);
+            if (l < g.kp) k = __ldg(g.conn + (size_t)l * g.n + i);
+            pi_ = g.xy[i];
+            qi = __ldg(reinterpret_cast<const double *>(q + i) + m);
+            // dx = a sx + b sy, dy = b sx + c sy: the factors of this lane's sums
+            M0 = __ldg(g.minv + 4 * (size_t)i + (l < 4 ? 0 : 2));
+            M1 = __ldg(g.minv + 4 * (size_t)i + 1);
+        }
+        if (!live) return;
+        double sum = 0.0, ext = qi, dmin = 1.0;
+        const int nbw = __reduce_max_sync(0xffffffffu, nb);
+        for (int r0 = 0; r0 < nbw; r0 += LPP) {
+            const int r = r0 + l;
+            if (r0 > 0 && r < nb) k = __ldg(g.conn + (size_t)r * g.n + i);
+            if (r < nb) {
+                double qk[4];
+                const R4 a = ld4w(q + k);
+                qk[0] = a.a; qk[1] = a.b; qk[2] = a.c; qk[3] = a.d;
+                const double2 pk = g.xy[k];
+                const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
+                const double w = g.wsl ? __ldg(g.wsl + (size_t)r * g.n + i) : 1.0;
+#pragma unroll
+                for (int f = 0; f < 4; ++f) row[f * SLOT_F + l] = qk[f];
+                row[4 * SLOT_F + l] = w * delx;
+                row[5 * SLOT_F + l] = w * dely;
+                if (with_delta) {
+                    double delta_t = sqrt(fma(delx, delx, dely * dely)) / spd[k];
+                    delta_t = c.cfl * delta_t;
+                    if (dmin > delta_t) dmin = delta_t;
+                }
+            }
+            __syncwarp();
+            const double *qf = row + m * SLOT_F, *wf = row + (4 + l / 4) * SLOT_F;
+#pragma unroll
+            for (int j = 0; j < LPP; ++j) {
+                if (r0 + j >= nb) break;
+                const double qk = qf[j], wd = wf[j];
+                if (l < 4 ? qk > ext : qk < ext) ext = qk;
+                sum = fma(wd, qk - qi, sum);
+            }
+            __syncwarp();
+        }
+        // lanes 0-3 hold sx and qmax, 4-7 sy and qmin
+        const double other = __shfl_xor_sync(0xffffffffu, sum, 4);
+        if (with_delta) {
+#pragma unroll
+            for (int o = 4; o; o >>= 1) {
+                const double d = __shfl_xor_sync(0xffffffffu, dmin, o);
+                if (dmin > d) dmin = d;
+            }
+        }
+        if (i >= 0) {
+            dq[8 * (size_t)i + l] = l < 4 ? fma(M0, sum, M1 * other) : fma(M1, other, M0 * sum);
+            qm[8 * (size_t)i + l] = ext;
+            if (with_delta && l == 0) delta[i] = dmin;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(SLOT_BLOCK)
+kb_inner_s(Geom g, Sched s, const double *__restrict__ dq0, const double *__restrict__ dq_in,
+           double *__restrict__ dq_out) {
+    __shared__ SchedSmem ss;
+    __shared__ double sm[SLOT_PTS * SLOT_P];
+    int live;
+    const int total = sched_begin(s, ss, live) * TILE;
+    const int p = threadIdx.x / LPP, l = threadIdx.x % LPP, m = l & 3;
+    double *row = sm + p * SLOT_P;  // fields d . dq_k [4], w dx, w dy
+    for (int v0 = blockIdx.x * SLOT_PTS; v0 < total; v0 += gridDim.x * SLOT_PTS) {
+        const int i = slot_point(s, ss, total, v0 + p);
+        int nb = 0, k = 0;
+        double2 pi_ = make_double2(0.0, 0.0);
+        double a0 = 0.0, di = 0.0, M0 = 0.0, M1 = 0.0;
+        if (i >= 0) {
+            nb = __ldg(g.nbhs + i);
+            if (l < g.kp) k = __ldg(g.conn + (size_t)l * g.n + i);
+            pi_ = g.xy[i];
+            a0 = __ldg(dq0 + 8 * (size_t)i + l);
+            di = __ldg(dq_in + 8 * (size_t)i + l);
+            M0 = __ldg(g.minv + 4 * (size_t)i + (l < 4 ? 0 : 2));
+            M1 = __ldg(g.minv + 4 * (size_t)i + 1);
+        }
+        if (!live) return;
+        double sum = 0.0;
+        const int nbw = __reduce_max_sync(0xffffffffu, nb);
+        for (int r0 = 0; r0 < nbw; r0 += LPP) {
+            const int r = r0 + l;
+            if (r0 > 0 && r < nb) k = __ldg(g.conn + (size_t)r * g.n + i);
+            if (r < nb) {
+                double dxk[4], dyk[4];
+                ld8w(dq_in + 8 * (size_t)k, dxk, dyk);
+                const double2 pk = g.xy[k];
+                const double delx = pk.x - pi_.x, dely = pk.y - pi_.y;
+                const double w = g.wsl ? __ldg(g.wsl + (size_t)r * g.n + i) : 1.0;
+#pragma unroll
+                for (int f = 0; f < 4; ++f) row[f * SLOT_F + l] = fma(delx, dxk[f], dely * dyk[f]);
+                row[4 * SLOT_F + l] = w * delx;
+                row[5 * SLOT_F + l] = w * dely;
+            }
+            __syncwarp();
+            const double *tf = row + m * SLOT_F, *wf = row + (4 + l / 4) * SLOT_F;
+#pragma unroll
+            for (int j = 0; j < LPP; ++j) {
+                if (r0 + j >= nb) break;
+                sum = fma(wf[j], tf[j], sum);
+            }
+            __syncwarp();
+        }
+        const double other = __shfl_xor_sync(0xffffffffu, sum, 4);
+        const double L = l < 4 ? fma(M0, sum, M1 * other) : fma(M1, other, M0 * sum);
+        if (i >= 0) dq_out[8 * (size_t)i + l] = fma(-0.5, L, fma(0.5, di, a0));
     }
 }
 
@@ -922,6 +1061,13 @@ FluxShape flux_shape(int tiles, int per_sm) {
     return FluxShape{one < two ? 1 : 2, 0};
 }
 
+// The D and I passes by slots (kb_grad_s, kb_inner_s, and FP32) while their
+// blocks are one wave, nine an SM: beyond it the halo form's fewer loads win
+// (an iteration with one inner iteration on 148 SMs, by slots / halos: FP64
+// 20,000 points 101.6 / 108.3 us, 24,000 112.4 / 109.4; FP32 20,000 points
+// 70.4 / 79.5, 24,000 76.4 / 77.6, 32,000 86.7 / 86.7).
+bool slot_passes(int n) { return nblk(n, SLOT_PTS) <= 9 * sm_count(); }
+
 // flux-pass blocks that give every chunk its warp (or its block)
 int flux_grid_blocks(int n, bool fp32) {
     const int tiles = nblk(n, TILE);
@@ -1011,6 +1157,11 @@ void launch_grad(const Geom &g, const Consts &c, const Sched &s, const R4 *q, co
                  double *dq, double *qm, double *delta, bool with_delta, int block, int grid,
                  cudaStream_t st) {
     (void)block;  // the halo kernels' blocks are HALO_BLOCK threads
+    if (slot_passes(g.n)) {
+        kb_grad_s<<<nblk(g.n, SLOT_PTS), SLOT_BLOCK, 0, st>>>(g, c, s, q, spd, dq, qm, delta,
+                                                              with_delta ? 1 : 0);
+        return;
+    }
     kb_grad_h<<<grid > 0 ? grid : halo_wave(0, g.hc), HALO_BLOCK, halo_smem_bytes(0, g.hc), st>>>(
         g, c, s, q, spd, dq, qm, delta, with_delta ? 1 : 0);
 }
@@ -1019,6 +1170,10 @@ void launch_inner(const Geom &g, const Consts &c, const Sched &s, const double *
                   const double *dq_in, double *dq_out, int block, int grid, cudaStream_t st) {
     (void)block;
     (void)c;
+    if (slot_passes(g.n)) {
+        kb_inner_s<<<nblk(g.n, SLOT_PTS), SLOT_BLOCK, 0, st>>>(g, s, dq0, dq_in, dq_out);
+        return;
+    }
     kb_inner_h<<<grid > 0 ? grid : halo_wave(1, g.hc), HALO_BLOCK, halo_smem_bytes(1, g.hc), st>>>(
         g, s, dq0, dq_in, dq_out);
 }
