@@ -307,7 +307,7 @@ void lskum_host::build_halo(int n, int kp, const int *conn, const int *nbhs,
         }
         std::sort(rows.begin(), rows.end());
         rows.erase(std::unique(rows.begin(), rows.end()), rows.end());
-        if ((int)rows.size() > HALO_CAP) continue;  // gathered directly
+        if ((int)rows.size() > HALO_CAP_WIDE) continue;  // gathered directly
         auto pos = [&](int k) {
             return (unsigned char)(std::lower_bound(rows.begin(), rows.end(), k) - rows.begin());
         };

@@ -38,21 +38,24 @@ __device__ __forceinline__ void halo_wait() {
 // The row indices of a warp's two tiles: lane l holds those of pair rows l,
 // l + 32, l + 64 and l + 96 (row u of the pair being row u of the first
 // tile's halo, hrow[h0 + u], or row u - hn0 of the second's).
+template <int CAP>
 struct HaloIdx {
     int h0 = 0, hn0 = 0, h1 = 0, hn1 = 0;
-    int kr[2 * HALO_CAP / 32] = {0, 0, 0, 0};
+    int kr[2 * CAP / 32] = {};
 };
 
 // One chunk: both tiles' halo ranges and row indices, and this lane's point
 // (i < 0: none), its stencil size and the size of its tile's halo.
+template <int CAP>
 struct HaloChunk {
-    HaloIdx x;
+    HaloIdx<CAP> x;
     int i = -1, nb = 0, hn = 0;
 };
 
+template <int CAP>
 __device__ __forceinline__ void halo_chunk(const Geom &g, const Sched &s, const SchedSmem &ss,
-                                           int ntiles, int ch, int lane, HaloChunk &c) {
-    c = HaloChunk();
+                                           int ntiles, int ch, int lane, HaloChunk<CAP> &c) {
+    c = HaloChunk<CAP>();
     if (2 * ch >= ntiles) return;
     const int half = lane / TILE, jl = lane % TILE;
 #pragma unroll
@@ -78,7 +81,7 @@ __device__ __forceinline__ void halo_chunk(const Geom &g, const Sched &s, const 
     }
     const int hnt = c.x.hn0 + c.x.hn1;
 #pragma unroll
-    for (int w = 0; w < 2 * HALO_CAP / 32; ++w) {
+    for (int w = 0; w < 2 * CAP / 32; ++w) {
         const int u = 32 * w + lane;
         c.x.kr[w] = u < hnt ? __ldg(g.hrow + (u < c.x.hn0 ? c.x.h0 + u : c.x.h1 + u - c.x.hn0))
                             : 0;
@@ -90,14 +93,14 @@ __device__ __forceinline__ void halo_chunk(const Geom &g, const Sched &s, const 
 // (u < hn0 ? sm0 + u : sm1 + u - hn0) + (a0 + p) * hc.  A copy takes its row
 // index from the lane holding it (a shuffle whose source register is the
 // same for the whole warp).
-template <int NP>
-__device__ __forceinline__ void stage_array(const void *base, int row_bytes, const HaloIdx &x,
-                                            int lane, double2 *sm0, double2 *sm1, int hc,
-                                            int a0) {
+template <int NP, int CAP>
+__device__ __forceinline__ void stage_array(const void *base, int row_bytes,
+                                            const HaloIdx<CAP> &x, int lane, double2 *sm0,
+                                            double2 *sm1, int hc, int a0) {
     const int hn0 = x.hn0, hn = x.hn0 + x.hn1;
     const char *b = static_cast<const char *>(base);
 #pragma unroll
-    for (int t = 0; t < 2 * HALO_CAP * NP / 32; ++t) {
+    for (int t = 0; t < 2 * CAP * NP / 32; ++t) {
         if (32 * t >= NP * hn) break;
         const int pc = 32 * t + lane, u = pc / NP, part = pc % NP;
         const int k = NP == 1 ? x.kr[t] : __shfl_sync(0xffffffffu, x.kr[t / NP], u & 31);
@@ -108,12 +111,13 @@ __device__ __forceinline__ void stage_array(const void *base, int row_bytes, con
 
 // An 8-byte value per halo row (row k at base + 8 k) into the first half of
 // shared array a.
-__device__ __forceinline__ void stage_array8(const void *base, const HaloIdx &x, int lane,
+template <int CAP>
+__device__ __forceinline__ void stage_array8(const void *base, const HaloIdx<CAP> &x, int lane,
                                              double2 *sm0, double2 *sm1, int hc, int a) {
     const int hn0 = x.hn0, hn = x.hn0 + x.hn1;
     const char *b = static_cast<const char *>(base);
 #pragma unroll
-    for (int t = 0; t < 2 * HALO_CAP / 32; ++t) {
+    for (int t = 0; t < 2 * CAP / 32; ++t) {
         if (32 * t >= hn) break;
         const int u = 32 * t + lane;
         double2 *d = (u < hn0 ? sm0 + u : sm1 + (u - hn0)) + a * hc;

@@ -49,7 +49,7 @@ struct Geom {
     // gathered directly).  The halo of a TILE-point tile is the sorted set of
     // rows its points read (the points themselves and their neighbours);
     // hoff[tile] .. hoff[tile + 1] index its rows in hrow (an empty range: the
-    // tile's halo exceeds HALO_CAP and its rows are gathered directly).
+    // tile's halo exceeds HALO_CAP_WIDE and its rows are gathered directly).
     // hloc[p * hkp + r] is slot r's row within the tile's halo, hloc[p * hkp
     // + hkp - 1] the point's own; hc = the largest halo, the staging stride.
     const int *hoff = nullptr;
@@ -67,8 +67,13 @@ struct Geom {
     // (xx, xy, yy, unused)
     const double *minv = nullptr;
 };
-// rows a tile halo stages at most (its local row indices are bytes)
-constexpr int HALO_CAP = 64;
+// Rows a tile halo stages at most (its local row indices are bytes): an O-grid's
+// tiles have some 54, those of a renumbered cloud of points about 58 and a few
+// over 64.  A grid whose largest is over HALO_CAP takes the passes' wide forms:
+// gathered directly, those few tiles (4% of a cloud of 40,000 points) set the
+// passes' time (an iteration with one inner iteration FP64 195.7 us, 169.6 with
+// the wide forms; FP32 113.3 and 98.1).
+constexpr int HALO_CAP = 64, HALO_CAP_WIDE = 96;
 
 struct Consts {
     double cfl, power, euler, pi, gm1;  // gm1 = gamma - 1

@@ -208,6 +208,7 @@ __device__ __forceinline__ void grad32_sums(const Consts &c, const Geom32 &f, in
     }
 }
 
+template <int CAP>
 __global__ void __launch_bounds__(HALO32_BLOCK, HALO32_MIN_BLOCKS)
 kb_grad32_h(Geom g, Consts c, Geom32 f, Sched s, const float4 *__restrict__ q,
             const double *__restrict__ spd, float *__restrict__ dq, float *__restrict__ qm,
@@ -220,7 +221,7 @@ kb_grad32_h(Geom g, Consts c, Geom32 f, Sched s, const float4 *__restrict__ q,
     const int half = lane / TILE, stride = gridDim.x * wpb;
     using H = HaloRows32;
     double2 *sm0 = hsm + (2 * warp) * HA32 * g.hc, *sm1 = sm0 + HA32 * g.hc;
-    HaloChunk cur;
+    HaloChunk<CAP> cur;
     for (int ch = blockIdx.x * wpb + warp; 2 * ch < ntiles; ch += stride) {
         halo_chunk(g, s, ss, ntiles, ch, lane, cur);
         if (!live) return;
@@ -779,15 +780,18 @@ int flux32_per_sm() { return FLUX32_MIN_BLOCKS; }
 namespace {
 // dynamic shared memory of the halo kernels at staging stride hc
 size_t halo32_smem(int hc) { return halo_bytes(HALO32_BLOCK / 32, HA32, hc); }
-// one wave of resident blocks of a halo kernel (kind 0: D pass, 1: I pass)
-int halo32_wave(int kind, int hc) {
+// blocks of the D pass's halo kernel, as halo_grid of the FP64 passes
+int halo32_grid(int hc, int grid) {
+    const bool wide = hc > HALO_CAP + 1;
+    if (grid > 0 && !wide) return grid;
     int dev = 0, sms = 1, nb = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    (void)kind;  // the D pass only
-    cudaError_t e =
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_grad32_h, HALO32_BLOCK, halo32_smem(hc));
-    return std::max(sms, 1) * std::max(1, e == cudaSuccess ? nb : 1);
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &nb, wide ? kb_grad32_h<HALO_CAP_WIDE> : kb_grad32_h<HALO_CAP>, HALO32_BLOCK,
+        halo32_smem(hc));
+    const int wave = std::max(sms, 1) * std::max(1, e == cudaSuccess ? nb : 1);
+    return grid > 0 ? std::min(grid, wave) : wave;
 }
 }  // namespace
 
@@ -800,7 +804,7 @@ int batch_occupancy32(int kind, int block, size_t smem) {
     // the D pass: its tile-halo kernel at the largest staging stride, which
     // every grid with halos runs
     if (kind == 0)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_grad32_h, HALO32_BLOCK,
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_grad32_h<HALO_CAP>, HALO32_BLOCK,
                                                           halo32_smem(HALO_CAP + 1));
     else if (kind == 1)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_inner32, block, smem);
@@ -826,7 +830,8 @@ void launch_grad32(const Geom &g, const Consts &c, const Geom32 &f, const Sched 
                                                                 with_delta ? 1 : 0);
         return;
     }
-    kb_grad32_h<<<grid > 0 ? grid : halo32_wave(0, g.hc), HALO32_BLOCK, halo32_smem(g.hc), st>>>(
+    auto *kernel = g.hc > HALO_CAP + 1 ? kb_grad32_h<HALO_CAP_WIDE> : kb_grad32_h<HALO_CAP>;
+    kernel<<<halo32_grid(g.hc, grid), HALO32_BLOCK, halo32_smem(g.hc), st>>>(
         g, c, f, s, q, spd, dq, qm, delta, with_delta ? 1 : 0);
 }
 

@@ -96,28 +96,26 @@ constexpr int HA_I = 5, HA_D = 4;
 // 0.076 ms at 1.024M points at 5 blocks an SM); the I pass, whose rows are
 // larger, takes the grid's own: what shared memory it leaves is L1, where the
 // tiles' common rows are found (0.082 ms, 0.090 with the fixed stride).
-template <int nA>
-struct HaloStride;
-template <>
-struct HaloStride<HA_D> {
-    static constexpr int hc = HALO_CAP + 1;
-    __host__ __device__ constexpr HaloStride(int) {}
-};
-template <>
-struct HaloStride<HA_I> {
+template <int nA, int CAP>
+struct HaloStride {
     int hc;
     __host__ __device__ constexpr HaloStride(int h) : hc(h) {}
+};
+template <>
+struct HaloStride<HA_D, HALO_CAP> {
+    static constexpr int hc = HALO_CAP + 1;
+    __host__ __device__ constexpr HaloStride(int) {}
 };
 constexpr int HALO_BLOCK = 128;  // four warps, a half-warp per tile
 // resident blocks per SM (96 registers), measured at 1.024M points: the D pass
 // 0.082 ms at 4, 0.076 at 5, 0.089 at 6; the I pass 0.089, 0.082, 0.097
 constexpr int HALO_MIN_BLOCKS_D = 5, HALO_MIN_BLOCKS_I = 5;
 
-template <int nA>
+template <int nA, int CAP>
 struct HaloRows {
     static constexpr int OXY = nA == HA_I ? 0 : 2, ODQ = 1, OSPD = 3;
     const double2 *sm;
-    HaloStride<nA> st;
+    HaloStride<nA, CAP> st;
     HaloLoc loc;
     // i < 0: no point (nothing is loaded)
     __device__ __forceinline__ HaloRows(const Geom &g, const double2 *sm_, int i)
@@ -263,12 +261,12 @@ __device__ __forceinline__ void st8w(double *p, const double a[4], const double 
 // q, (x, y) and dq; nA = HA_D copies q, (x, y) and, with spd != nullptr, spd.
 // Stages a chunk's halo rows: the D pass q (two pieces a row), (x, y) and,
 // with spd != nullptr, spd; the I pass (x, y) and dq (four pieces a row).
-template <int nA>
+template <int nA, int CAP>
 __device__ __forceinline__ void stage_halo(const Geom &g, const R4 *q, const double *dq,
-                                           const double *spd, const HaloIdx &x, int lane,
+                                           const double *spd, const HaloIdx<CAP> &x, int lane,
                                            double2 *sm0, double2 *sm1) {
-    using H = HaloRows<nA>;
-    const HaloStride<nA> st(g.hc);
+    using H = HaloRows<nA, CAP>;
+    const HaloStride<nA, CAP> st(g.hc);
     if (nA == HA_D) stage_array<2>(q, 32, x, lane, sm0, sm1, st.hc, 0);
     stage_array<1>(g.xy, 16, x, lane, sm0, sm1, st.hc, H::OXY);
     if (nA == HA_I) stage_array<4>(dq, 64, x, lane, sm0, sm1, st.hc, H::ODQ);
@@ -280,6 +278,7 @@ __device__ __forceinline__ void stage_halo(const Geom &g, const R4 *q, const dou
 // tile whose halo was too large to stage reads its rows directly.  No block
 // barrier but the schedule load; the lanes of a warp meet at __syncwarp
 // before the rows are read and before they are overwritten.
+template <int CAP>
 __global__ void __launch_bounds__(HALO_BLOCK, HALO_MIN_BLOCKS_I)
 kb_inner_h(Geom g, Sched s, const double *__restrict__ dq0,
            const double *__restrict__ dq_in, double *__restrict__ dq_out) {
@@ -290,12 +289,12 @@ kb_inner_h(Geom g, Sched s, const double *__restrict__ dq0,
     const int wpb = blockDim.x / 32, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int half = lane / TILE, stride = gridDim.x * wpb;
     double2 *sm0 = hsm + (2 * warp) * HA_I * g.hc, *sm1 = sm0 + HA_I * g.hc;
-    HaloChunk cur;
+    HaloChunk<CAP> cur;
     for (int ch = blockIdx.x * wpb + warp; 2 * ch < ntiles; ch += stride) {
         halo_chunk(g, s, ss, ntiles, ch, lane, cur);
         if (!live) return;
         stage_halo<HA_I>(g, nullptr, dq_in, nullptr, cur.x, lane, sm0, sm1);
-        const HaloRows<HA_I> hr(g, half ? sm1 : sm0, cur.hn > 0 ? cur.i : -1);
+        const HaloRows<HA_I, CAP> hr(g, half ? sm1 : sm0, cur.hn > 0 ? cur.i : -1);
         double ax[4], ay[4];
         if (cur.i >= 0) ld8w(dq0 + 8 * (size_t)cur.i, ax, ay);
         halo_wait();
@@ -312,6 +311,7 @@ kb_inner_h(Geom g, Sched s, const double *__restrict__ dq0,
     }
 }
 
+template <int CAP>
 __global__ void __launch_bounds__(HALO_BLOCK, HALO_MIN_BLOCKS_D)
 kb_grad_h(Geom g, Consts c, Sched s, const R4 *__restrict__ q, const double *__restrict__ spd,
           double *__restrict__ dq, double *__restrict__ qm, double *__restrict__ delta,
@@ -322,14 +322,14 @@ kb_grad_h(Geom g, Consts c, Sched s, const R4 *__restrict__ q, const double *__r
     const int ntiles = sched_begin(s, ss, live);
     const int wpb = blockDim.x / 32, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int half = lane / TILE, stride = gridDim.x * wpb;
-    double2 *sm0 = hsm + (2 * warp) * HA_D * HaloStride<HA_D>::hc,
-            *sm1 = sm0 + HA_D * HaloStride<HA_D>::hc;
-    HaloChunk cur;
+    const HaloStride<HA_D, CAP> st(g.hc);
+    double2 *sm0 = hsm + (2 * warp) * HA_D * st.hc, *sm1 = sm0 + HA_D * st.hc;
+    HaloChunk<CAP> cur;
     for (int ch = blockIdx.x * wpb + warp; 2 * ch < ntiles; ch += stride) {
         halo_chunk(g, s, ss, ntiles, ch, lane, cur);
         if (!live) return;
         stage_halo<HA_D>(g, q, nullptr, with_delta ? spd : nullptr, cur.x, lane, sm0, sm1);
-        const HaloRows<HA_D> hr(g, half ? sm1 : sm0, cur.hn > 0 ? cur.i : -1);
+        const HaloRows<HA_D, CAP> hr(g, half ? sm1 : sm0, cur.hn > 0 ? cur.i : -1);
         halo_wait();
         __syncwarp();
         if (cur.i >= 0) {
@@ -1083,16 +1083,21 @@ void launch_flux_coef(const Geom &g, int base, int n, int nw, int no, double pow
 
 // staging memory of a block of the halo kernels: two tiles a warp
 size_t halo_smem_bytes(int kind, int hc) {
-    return kind == 0 ? halo_bytes(HALO_BLOCK / 32, HA_D, HaloStride<HA_D>::hc)
+    return kind == 0 ? halo_bytes(HALO_BLOCK / 32, HA_D, std::max(hc, HALO_CAP + 1))
                      : halo_bytes(HALO_BLOCK / 32, HA_I, hc);
 }
 
 cudaError_t init_kernels() {
-    cudaError_t e = cudaFuncSetAttribute(kb_grad_h, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)halo_smem_bytes(0, HALO_CAP + 1));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(kb_inner_h, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)halo_smem_bytes(1, HALO_CAP + 1));
+    cudaError_t e = cudaSuccess;
+    auto room = [&](auto *kernel, int kind, int cap) {
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)halo_smem_bytes(kind, cap + 1));
+    };
+    room(kb_grad_h<HALO_CAP>, 0, HALO_CAP);
+    room(kb_grad_h<HALO_CAP_WIDE>, 0, HALO_CAP_WIDE);
+    room(kb_inner_h<HALO_CAP>, 1, HALO_CAP);
+    room(kb_inner_h<HALO_CAP_WIDE>, 1, HALO_CAP_WIDE);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(kb_flux<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  FLUX_SMEM);
@@ -1131,26 +1136,31 @@ int batch_occupancy(int kind, bool fp32, int block, size_t smem) {
     // the D and I passes: their tile-halo kernels (blocks of HALO_BLOCK
     // threads, the largest staging stride), which every grid with halos runs
     if (kind == 0)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_grad_h, HALO_BLOCK,
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_grad_h<HALO_CAP>, HALO_BLOCK,
                                                           halo_smem_bytes(0, HALO_CAP + 1));
     else if (kind == 1)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_inner_h, HALO_BLOCK,
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_inner_h<HALO_CAP>, HALO_BLOCK,
                                                           halo_smem_bytes(1, HALO_CAP + 1));
     else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_flux<false>, block,
                                                           FLUX_SMEM);
     return e == cudaSuccess ? nb : 1;
 }
 
-// one wave of resident blocks of a halo kernel (kind 0: D pass, 1: I pass)
-int halo_wave(int kind, int hc) {
-    int dev = 0, sms = 1, nb = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+// blocks of a halo kernel (kind 0: D pass, 1: I pass): `grid`, but no more than
+// one wave of the wide forms, or one wave (grid == 0)
+int halo_grid(int kind, int hc, int grid) {
+    const bool wide = hc > HALO_CAP + 1;
+    if (grid > 0 && !wide) return grid;
     const size_t smem = halo_smem_bytes(kind, hc);
-    cudaError_t e = kind == 0
-        ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_grad_h, HALO_BLOCK, smem)
-        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_inner_h, HALO_BLOCK, smem);
-    return std::max(sms, 1) * std::max(1, e == cudaSuccess ? nb : 1);
+    int nb = 0;
+    auto ask = [&](auto *kernel) {
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, HALO_BLOCK, smem);
+    };
+    const cudaError_t e =
+        kind == 0 ? (wide ? ask(kb_grad_h<HALO_CAP_WIDE>) : ask(kb_grad_h<HALO_CAP>))
+                  : (wide ? ask(kb_inner_h<HALO_CAP_WIDE>) : ask(kb_inner_h<HALO_CAP>));
+    const int wave = sm_count() * std::max(1, e == cudaSuccess ? nb : 1);
+    return grid > 0 ? std::min(grid, wave) : wave;
 }
 
 void launch_grad(const Geom &g, const Consts &c, const Sched &s, const R4 *q, const double *spd,
@@ -1162,7 +1172,8 @@ void launch_grad(const Geom &g, const Consts &c, const Sched &s, const R4 *q, co
                                                               with_delta ? 1 : 0);
         return;
     }
-    kb_grad_h<<<grid > 0 ? grid : halo_wave(0, g.hc), HALO_BLOCK, halo_smem_bytes(0, g.hc), st>>>(
+    auto *kernel = g.hc > HALO_CAP + 1 ? kb_grad_h<HALO_CAP_WIDE> : kb_grad_h<HALO_CAP>;
+    kernel<<<halo_grid(0, g.hc, grid), HALO_BLOCK, halo_smem_bytes(0, g.hc), st>>>(
         g, c, s, q, spd, dq, qm, delta, with_delta ? 1 : 0);
 }
 
@@ -1174,7 +1185,8 @@ void launch_inner(const Geom &g, const Consts &c, const Sched &s, const double *
         kb_inner_s<<<nblk(g.n, SLOT_PTS), SLOT_BLOCK, 0, st>>>(g, s, dq0, dq_in, dq_out);
         return;
     }
-    kb_inner_h<<<grid > 0 ? grid : halo_wave(1, g.hc), HALO_BLOCK, halo_smem_bytes(1, g.hc), st>>>(
+    auto *kernel = g.hc > HALO_CAP + 1 ? kb_inner_h<HALO_CAP_WIDE> : kb_inner_h<HALO_CAP>;
+    kernel<<<halo_grid(1, g.hc, grid), HALO_BLOCK, halo_smem_bytes(1, g.hc), st>>>(
         g, s, dq0, dq_in, dq_out);
 }
 
