@@ -47,7 +47,8 @@ struct TanState {
     const Dual *obc;              // outer points: 8 Duals per point
     R4 *pv[2], *pt[2];            // prim
     R4 *qv[2], *qt[2];            // q
-    double *dqv[2], *dqt[2];      // dq [n][8]
+    double *dqv[3], *dqt[3];      // dq [n][8]: the D pass's, then the inner iterations' in turn
+    double *mt;                   // derivative of the stencil's normal matrix [n][4]
     double *qmv, *qmt;            // qm [n][8]
     double *dlv, *dlt;            // delta
     double *spv, *spt;            // spd
@@ -71,14 +72,12 @@ __device__ __forceinline__ void ld_dual8(const double *v, const double *t, int i
         b[m] = Dual(v[8 * (size_t)i + 4 + m], t[8 * (size_t)i + 4 + m]);
     }
 }
-__device__ __forceinline__ void st_dual8(double *v, double *t, int i, const Dual a[4],
-                                         const Dual b[4]) {
-    for (int m = 0; m < 4; ++m) {
-        v[8 * (size_t)i + m] = a[m].v;
-        t[8 * (size_t)i + m] = a[m].d;
-        v[8 * (size_t)i + 4 + m] = b[m].v;
-        t[8 * (size_t)i + 4 + m] = b[m].d;
-    }
+// four doubles in one 256-bit read-only load; p is 32-byte aligned and not written
+// by the kernel that reads it
+__device__ __forceinline__ void ld4nc(const double *p, double v[4]) {
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+        : "l"(p));
 }
 __device__ __forceinline__ void xy_dual(const Geom &g, const TanState &s, int i, Dual &x,
                                         Dual &y) {
@@ -100,99 +99,180 @@ __global__ void k_t_init(int n, TanState s, int cur, int qc) {
     s.spt[i] = spd.d;
 }
 
+// The tangents of the D and I passes by slots, as kb_grad_s and kb_inner_s of the
+// primal: eight lanes a point, a slot's lane leaves its fields in shared memory
+// (T_F doubles a field, T_P a point: distinct banks) and lane l sums component l
+// and its derivative.  The solve's derivative comes from the stored inverse L of
+// the normal matrix M: o = L s, do = L (ds - dM o).
+// At 64,000 points 21 and 24 us; a thread a point, summing and solving on Duals,
+// 28 and 35.
+constexpr int T_PTS = TB / LPP, T_F = 9, T_P = 116;
+
+// L s of both components, value and derivative, on each lane: the lane holds the
+// sum of component l & 3 along x (l < 4) or y.
+struct TSolve {
+    double ox, oy, tx, ty;
+    __device__ __forceinline__ TSolve(const Geom &g, const TanState &s, int i, int l, Dual sum) {
+        const unsigned full = 0xffffffffu;
+        const Dual o(__shfl_xor_sync(full, sum.v, 4), __shfl_xor_sync(full, sum.d, 4));
+        ox = oy = tx = ty = 0.0;
+        if (i < 0) return;
+        const Dual sx = l < 4 ? sum : o, sy = l < 4 ? o : sum;
+        double L[4], M[4];
+        ld4nc(g.minv + 4 * (size_t)i, L);
+        ld4nc(s.mt + 4 * (size_t)i, M);
+        ox = L[0] * sx.v + L[1] * sy.v;
+        oy = L[1] * sx.v + L[2] * sy.v;
+        const double dx = sx.d - (M[0] * ox + M[2] * oy), dy = sy.d - (M[2] * ox + M[1] * oy);
+        tx = L[0] * dx + L[1] * dy;
+        ty = L[1] * dx + L[2] * dy;
+    }
+};
+
 // eval_q_derivatives_d + func_delta_d (q_variables_d.F90, state_update_d.F90)
 __global__ void __launch_bounds__(TB)
 k_t_grad(Geom g, Consts c, TanState s, int qc, int with_delta) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= g.n) return;
-    Dual xi, yi, qi[4];
-    xy_dual(g, s, i, xi, yi);
-    ld_dual4(s.qv[qc], s.qt[qc], i, qi);
-    Dual qmax[4], qmin[4], sdxq[4], sdyq[4];
-    for (int m = 0; m < 4; ++m) {
-        qmax[m] = qi[m];
-        qmin[m] = qi[m];
+    __shared__ double sm[T_PTS * T_P];
+    const unsigned full = 0xffffffffu;
+    const int l = threadIdx.x % LPP, m = l & 3;
+    int i = blockIdx.x * T_PTS + threadIdx.x / LPP;
+    double *row = sm + threadIdx.x / LPP * T_P;
+    if (i >= g.n) i = -1;
+    int nb = 0;
+    Dual xi, yi, qi;
+    if (i >= 0) {
+        nb = g.nbhs[i];
+        xy_dual(g, s, i, xi, yi);
+        qi = Dual(reinterpret_cast<const double *>(s.qv[qc] + i)[m],
+                  reinterpret_cast<const double *>(s.qt[qc] + i)[m]);
     }
-    Dual sdx2, sdy2, sdxy, min_delt(1.0);
-    const int nb = g.nbhs[i];
-    for (int r = 0; r < nb; ++r) {
-        const int k = g.conn[r * g.n + i];
-        Dual xk, yk, qk[4];
-        xy_dual(g, s, k, xk, yk);
-        ld_dual4(s.qv[qc], s.qt[qc], k, qk);
-        for (int m = 0; m < 4; ++m) {
-            if (qk[m] > qmax[m]) qmax[m] = qk[m];
-            if (qk[m] < qmin[m]) qmin[m] = qk[m];
+    Dual sum, ext = qi, dmin(1.0);
+    int dslot = -1;  // of the smallest time step: the first, as in slot order
+    const int nbw = __reduce_max_sync(full, nb);
+    for (int r0 = 0; r0 < nbw; r0 += LPP) {
+        const int r = r0 + l;
+        if (r < nb) {
+            const int k = g.conn[(size_t)r * g.n + i];
+            double qv[4], qt[4];
+            ld4nc(reinterpret_cast<const double *>(s.qv[qc] + k), qv);
+            ld4nc(reinterpret_cast<const double *>(s.qt[qc] + k), qt);
+            Dual xk, yk;
+            xy_dual(g, s, k, xk, yk);
+            const Dual delx = xk - xi, dely = yk - yi;
+#pragma unroll
+            for (int f = 0; f < 4; ++f) {
+                row[f * T_F + l] = qv[f];
+                row[(4 + f) * T_F + l] = qt[f];
+            }
+            row[8 * T_F + l] = delx.v;
+            row[9 * T_F + l] = dely.v;
+            row[10 * T_F + l] = delx.d;
+            row[11 * T_F + l] = dely.d;
+            if (with_delta) {
+                Dual delta_t = sqrt(delx * delx + dely * dely) / Dual(s.spv[k], s.spt[k]);
+                delta_t = Dual(c.cfl) * delta_t;
+                if (dmin > delta_t) {
+                    dmin = delta_t;
+                    dslot = r;
+                }
+            }
         }
-        const Dual delx = xk - xi, dely = yk - yi;
-        const Dual dist = sqrt(delx * delx + dely * dely);
-        sdx2 = sdx2 + delx * delx;
-        sdy2 = sdy2 + dely * dely;
-        sdxy = sdxy + delx * dely;
-        for (int m = 0; m < 4; ++m) {
-            sdxq[m] = sdxq[m] + delx * (qk[m] - qi[m]);
-            sdyq[m] = sdyq[m] + dely * (qk[m] - qi[m]);
+        __syncwarp();
+        const double *qf = row + m * T_F, *wf = row + (8 + l / 4) * T_F;
+#pragma unroll
+        for (int j = 0; j < LPP; ++j) {
+            if (r0 + j >= nb) break;
+            const Dual qk(qf[j], qf[4 * T_F + j]), d(wf[j], wf[2 * T_F + j]);
+            if (l < 4 ? qk > ext : qk < ext) ext = qk;
+            sum += d * (qk - qi);
         }
-        if (with_delta) {
-            Dual delta_t = dist / Dual(s.spv[k], s.spt[k]);
-            delta_t = Dual(c.cfl) * delta_t;
-            if (min_delt > delta_t) min_delt = delta_t;
-        }
+        __syncwarp();
     }
-    const Dual one_by_det = Dual(1.0) / (sdx2 * sdy2 - sdxy * sdxy);
-    Dual dx[4], dy[4];
-    for (int m = 0; m < 4; ++m) {
-        dx[m] = (sdxq[m] * sdy2 - sdyq[m] * sdxy) * one_by_det;
-        dy[m] = (sdyq[m] * sdx2 - sdxq[m] * sdxy) * one_by_det;
-    }
-    st_dual8(s.dqv[0], s.dqt[0], i, dx, dy);
-    st_dual8(s.qmv, s.qmt, i, qmax, qmin);
     if (with_delta) {
-        s.dlv[i] = min_delt.v;
-        s.dlt[i] = min_delt.d;
+#pragma unroll
+        for (int o = 4; o; o >>= 1) {
+            const Dual d(__shfl_xor_sync(full, dmin.v, o), __shfl_xor_sync(full, dmin.d, o));
+            const int ds = __shfl_xor_sync(full, dslot, o);
+            if (dmin > d || (dmin.v == d.v && ds < dslot)) {
+                dmin = d;
+                dslot = ds;
+            }
+        }
+    }
+    const TSolve o(g, s, i, l, sum);
+    if (i < 0) return;
+    const size_t at = 8 * (size_t)i + l;
+    s.dqv[0][at] = l < 4 ? o.ox : o.oy;
+    s.dqt[0][at] = l < 4 ? o.tx : o.ty;
+    s.qmv[at] = ext.v;
+    s.qmt[at] = ext.d;
+    if (with_delta && l == 0) {
+        s.dlv[i] = dmin.v;
+        s.dlt[i] = dmin.d;
     }
 }
 
-// eval_q_inner_loop_d + eval_update_innerloop_d: dq buffer a -> a ^ 1
+// eval_q_inner_loop_d + eval_update_innerloop_d, dq buffer a -> b, in the
+// primal's form dq0 + dq_i / 2 - L s / 2, s = sum of d (d . dq_k)
 __global__ void __launch_bounds__(TB)
-k_t_inner(Geom g, TanState s, int qc, int a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= g.n) return;
-    Dual xi, yi, qi[4], dxi[4], dyi[4];
-    xy_dual(g, s, i, xi, yi);
-    ld_dual4(s.qv[qc], s.qt[qc], i, qi);
-    ld_dual8(s.dqv[a], s.dqt[a], i, dxi, dyi);
-    Dual sdx2, sdy2, sdxy, sdxq[4], sdyq[4];
-    const int nb = g.nbhs[i];
-    for (int r = 0; r < nb; ++r) {
-        const int k = g.conn[r * g.n + i];
-        Dual xk, yk, qk[4], dxk[4], dyk[4];
-        xy_dual(g, s, k, xk, yk);
-        ld_dual4(s.qv[qc], s.qt[qc], k, qk);
-        ld_dual8(s.dqv[a], s.dqt[a], k, dxk, dyk);
-        const Dual delx = xk - xi, dely = yk - yi;
-        sdx2 = sdx2 + delx * delx;
-        sdy2 = sdy2 + dely * dely;
-        sdxy = sdxy + delx * dely;
-        for (int m = 0; m < 4; ++m) {
-            const Dual temp1 = qi[m] - Dual(0.5) * (delx * dxi[m] + dely * dyi[m]);
-            const Dual temp2 = qk[m] - Dual(0.5) * (delx * dxk[m] + dely * dyk[m]);
-            sdxq[m] = sdxq[m] + (delx * (temp2 - temp1));
-            sdyq[m] = sdyq[m] + (dely * (temp2 - temp1));
+k_t_inner(Geom g, TanState s, int a, int b) {
+    __shared__ double sm[T_PTS * T_P];
+    const unsigned full = 0xffffffffu;
+    const int l = threadIdx.x % LPP, m = l & 3;
+    int i = blockIdx.x * T_PTS + threadIdx.x / LPP;
+    double *row = sm + threadIdx.x / LPP * T_P;
+    if (i >= g.n) i = -1;
+    int nb = 0;
+    Dual xi, yi;
+    if (i >= 0) {
+        nb = g.nbhs[i];
+        xy_dual(g, s, i, xi, yi);
+    }
+    Dual sum;
+    const int nbw = __reduce_max_sync(full, nb);
+    for (int r0 = 0; r0 < nbw; r0 += LPP) {
+        const int r = r0 + l;
+        if (r < nb) {
+            const int k = g.conn[(size_t)r * g.n + i];
+            double xv[4], yv[4], xt[4], yt[4];
+            ld4nc(s.dqv[a] + 8 * (size_t)k, xv);
+            ld4nc(s.dqv[a] + 8 * (size_t)k + 4, yv);
+            ld4nc(s.dqt[a] + 8 * (size_t)k, xt);
+            ld4nc(s.dqt[a] + 8 * (size_t)k + 4, yt);
+            Dual xk, yk;
+            xy_dual(g, s, k, xk, yk);
+            const Dual delx = xk - xi, dely = yk - yi;
+#pragma unroll
+            for (int f = 0; f < 4; ++f) {
+                const Dual t = delx * Dual(xv[f], xt[f]) + dely * Dual(yv[f], yt[f]);
+                row[f * T_F + l] = t.v;
+                row[(4 + f) * T_F + l] = t.d;
+            }
+            row[8 * T_F + l] = delx.v;
+            row[9 * T_F + l] = dely.v;
+            row[10 * T_F + l] = delx.d;
+            row[11 * T_F + l] = dely.d;
         }
+        __syncwarp();
+        const double *tf = row + m * T_F, *wf = row + (8 + l / 4) * T_F;
+#pragma unroll
+        for (int j = 0; j < LPP; ++j) {
+            if (r0 + j >= nb) break;
+            sum += Dual(wf[j], wf[2 * T_F + j]) * Dual(tf[j], tf[4 * T_F + j]);
+        }
+        __syncwarp();
     }
-    const Dual one_by_det = Dual(1.0) / (sdx2 * sdy2 - sdxy * sdxy);
-    Dual dx[4], dy[4];
-    for (int m = 0; m < 4; ++m) {
-        dx[m] = one_by_det * (sdxq[m] * sdy2 - sdyq[m] * sdxy);
-        dy[m] = one_by_det * (sdyq[m] * sdx2 - sdxq[m] * sdxy);
-    }
-    st_dual8(s.dqv[a ^ 1], s.dqt[a ^ 1], i, dx, dy);
+    const TSolve o(g, s, i, l, sum);
+    if (i < 0) return;
+    const size_t at = 8 * (size_t)i + l;
+    s.dqv[b][at] = s.dqv[0][at] + 0.5 * s.dqv[a][at] - 0.5 * (l < 4 ? o.ox : o.oy);
+    s.dqt[b][at] = s.dqt[0][at] + 0.5 * s.dqt[a][at] - 0.5 * (l < 4 ? o.tx : o.ty);
 }
 
 // The split lists' solve coefficients (k_flux_coef of the primal) as Duals:
 // per point and list a, b of the slot weight c = a dels + b deln (y lists: the
-// roles swapped).  Geometry: once per call.
+// roles swapped); and the derivative of the whole stencil's normal matrix.
+// Geometry: once per call.
 __global__ void __launch_bounds__(TB)
 k_t_coef(Geom g, TanState s, Dual *__restrict__ co) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -203,10 +283,14 @@ k_t_coef(Geom g, TanState s, Dual *__restrict__ co) {
     const Dual nx(g.nrm[i].x, s.nrm_t[i].x), ny(g.nrm[i].y, s.nrm_t[i].y);
     const unsigned long long bits[2] = {g.mx[i], g.my[i]};
     Dual sxx[4], syy[4], sxy[4];
+    double mxx = 0.0, myy = 0.0, mxy = 0.0;
     for (int r = 0; r < g.nbhs[i]; ++r) {
         Dual xk, yk;
         xy_dual(g, s, g.conn[(size_t)r * g.n + i], xk, yk);
         const Dual delx = xk - xi, dely = yk - yi;
+        mxx += 2.0 * delx.v * delx.d;
+        myy += 2.0 * dely.v * dely.d;
+        mxy += delx.v * dely.d + delx.d * dely.v;
         const Dual dels = delx * ny - dely * nx, deln = delx * nx + dely * ny;
         const Dual a = dels * dels, b = deln * deln, c = dels * deln;
 #pragma unroll
@@ -224,6 +308,10 @@ k_t_coef(Geom g, TanState s, Dual *__restrict__ co) {
         co[8 * (size_t)i + 2 * L] = none ? Dual() : (L < 2 ? syy[L] : sxx[L]) * ob;
         co[8 * (size_t)i + 2 * L + 1] = none ? Dual() : -(sxy[L] * ob);
     }
+    s.mt[4 * (size_t)i] = mxx;
+    s.mt[4 * (size_t)i + 1] = myy;
+    s.mt[4 * (size_t)i + 2] = mxy;
+    s.mt[4 * (size_t)i + 3] = 0.0;
 }
 
 // limited_qtilde (flux_math.cuh) on Duals.
@@ -634,9 +722,13 @@ int tan_setup(mfcfd_t *h) {
             take(s.pt[b], n);
             take(s.qv[b], n);
             take(s.qt[b], n);
+        }
+        for (int b = 0; b < 3; ++b) {
+            if (b > h->p.inner_iterations) break;
             take(s.dqv[b], (size_t)8 * n);
             take(s.dqt[b], (size_t)8 * n);
         }
+        take(s.mt, (size_t)4 * n);
         take(s.qmv, (size_t)8 * n);
         take(s.qmt, (size_t)8 * n);
         take(s.dlv, n);
@@ -714,10 +806,11 @@ extern "C" int mfcfd_tangent(mfcfd_t *h, int objective, int n_iters, const doubl
     for (int it = 0; it < n_iters; ++it) {
         const int A = cur, B = cur ^ 1;
         for (int rk = 1; rk <= rks; ++rk) {
-            k_t_grad<<<nblk(n, TB), TB, 0, str>>>(h->geom, h->consts, s, qc, rk == 1 ? 1 : 0);
+            auto dq = [](int t) { return t == 0 ? 0 : 2 - (t & 1); };  // buffer of iteration t
+            k_t_grad<<<nblk(n, T_PTS), TB, 0, str>>>(h->geom, h->consts, s, qc, rk == 1 ? 1 : 0);
             for (int t = 1; t <= m; ++t)
-                k_t_inner<<<nblk(n, TB), TB, 0, str>>>(h->geom, s, qc, (t - 1) & 1);
-            k_t_flux<<<nblk(n, TB / LPP), TB, 0, str>>>(h->geom, s, qc, m & 1, w.coef, w.fs);
+                k_t_inner<<<nblk(n, T_PTS), TB, 0, str>>>(h->geom, s, dq(t - 1), dq(t));
+            k_t_flux<<<nblk(n, TB / LPP), TB, 0, str>>>(h->geom, s, qc, dq(m), w.coef, w.fs);
             k_t_update<<<nblk(n, TB), TB, 0, str>>>(h->geom, h->consts, s, w.fs, A, B, qc, rk,
                                                    rk == rks ? 1 : 0);
             qc ^= 1;
