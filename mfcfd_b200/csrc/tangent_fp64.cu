@@ -65,13 +65,6 @@ __device__ __forceinline__ void st_dual4(R4 *v, R4 *t, int i, const Dual x[4]) {
     v[i] = R4{x[0].v, x[1].v, x[2].v, x[3].v};
     t[i] = R4{x[0].d, x[1].d, x[2].d, x[3].d};
 }
-__device__ __forceinline__ void ld_dual8(const double *v, const double *t, int i, Dual a[4],
-                                         Dual b[4]) {
-    for (int m = 0; m < 4; ++m) {
-        a[m] = Dual(v[8 * (size_t)i + m], t[8 * (size_t)i + m]);
-        b[m] = Dual(v[8 * (size_t)i + 4 + m], t[8 * (size_t)i + 4 + m]);
-    }
-}
 // four doubles in one 256-bit read-only load; p is 32-byte aligned and not written
 // by the kernel that reads it
 __device__ __forceinline__ void ld4nc(const double *p, double v[4]) {
@@ -367,11 +360,12 @@ __device__ __forceinline__ void flux_split_dual(const KStateT<Dual> &s, Dual u, 
 
 // cal_flux_residual_d: eight lanes a point, one slot a lane, and the pooled
 // slot weights of the primal flux pass; the sum of the list derivatives as
-// four values, then four derivatives, into fs [n][8].  94 us at 64,000 points;
-// a thread a point, with both states recomputed for each list and four list
-// sums of Duals, spilled at 255 registers and took 354.  Bound by latency at 8
-// warps an SM.
-__global__ void __launch_bounds__(TB)
+// four values, then four derivatives, into fs [n][8].  67 us at 64,000 points
+// with one state at a time and the neighbour's own list of each direction (3
+// blocks of 168 registers; 77 at 2 blocks, 73 at 4, which spill); 95 with both
+// states live and a loop over the lists, which a warp ran for both; 354 as a
+// thread a point with list sums of Duals.  Bound by latency at 12 warps an SM.
+__global__ void __launch_bounds__(TB, 3)
 k_t_flux(Geom g, TanState s, int qc, int dqa, const Dual *__restrict__ coef,
          double *__restrict__ fs) {
     const int lane = threadIdx.x % LPP;
@@ -387,62 +381,86 @@ k_t_flux(Geom g, TanState s, int qc, int dqa, const Dual *__restrict__ coef,
         xy_dual(g, s, k, xk, yk);
         const Dual nx(g.nrm[i].x, s.nrm_t[i].x), ny(g.nrm[i].y, s.nrm_t[i].y);
         const Dual delx = xk - xi, dely = yk - yi;
-        Dual qt[2][4];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int p = h ? k : i;
-            Dual q[4], dx[4], dy[4], hi[4], lo[4];
-            ld_dual4(s.qv[qc], s.qt[qc], p, q);
-            ld_dual8(s.dqv[dqa], s.dqt[dqa], p, dx, dy);
-            ld_dual8(s.qmv, s.qmt, p, hi, lo);
-            const double eps2 = g.eps2[p];
-#pragma unroll
-            for (int m = 0; m < 4; ++m)
-                qt[h][m] = limited_dual(delx * dx[m] + dely * dy[m], q[m], hi[m], lo[m], eps2);
-        }
-        KStateT<Dual> si, sk;
-        {
-            const double qi[4] = {qt[0][0].v, qt[0][1].v, qt[0][2].v, qt[0][3].v};
-            const double qk[4] = {qt[1][0].v, qt[1][1].v, qt[1][2].v, qt[1][3].v};
-            KState vi, vk;
-            double ui[2], uk[2];
-            kstate_pair(qi, qk, nx.v, ny.v, 0.56418958354775628695, vi, vk, ui, uk);
-            si = kstate_dual(vi, ui, qt[0], nx, ny);
-            sk = kstate_dual(vk, uk, qt[1], nx, ny);
-        }
         const Dual dels = delx * ny - dely * nx, deln = delx * nx + dely * ny;
         const Dual *co = coef + 8 * (size_t)i;
-        // the lists holding the neighbour, two of a direction only when its
-        // projection is exactly 0
-        const unsigned long long mx = g.mx[i], my = g.my[i];
+        // the lists holding the neighbour: one of each direction (lx, ly), in
+        // both only when its projection is exactly 0 (tx, ty)
+        const unsigned long long mx = g.mx[i] >> r, my = g.my[i] >> r;
+        const int lx = mx & 1ull ? 0 : 1, ly = my & 1ull ? 0 : 1;
+        const bool tx = (mx & (mx >> 32)) & 1ull, ty = (my & (my >> 32)) & 1ull;
+        Dual Dt[4], Dn[4];  // differences of the fluxes along t and n
+        // the point's state (h = 0), then the neighbour's, one at a time: both at
+        // once take 255 registers
 #pragma unroll 1
-        for (int l = 0; l < 2; ++l) {
-            const double sg = l ? -1.0 : 1.0;
-            if ((mx >> (r + 32 * l)) & 1ull) {
-                const Dual w = co[2 * l] * dels + co[2 * l + 1] * deln;
-                Dual Gi[4], Gk[4];
-                if (kind == KIND_INTERIOR) {
-                    flux_split_dual(si, si.ut, si.un, si.B1, si.e1, sg, Gi);
-                    flux_split_dual(sk, sk.ut, sk.un, sk.B1, sk.e1, sg, Gk);
-                } else {
-                    const Dual s2(kind == KIND_WALL ? -1.0 : 1.0);
-                    flux_quad<Dual>(si, Dual(sg), s2, Gi);
-                    flux_quad<Dual>(sk, Dual(sg), s2, Gk);
-                }
+        for (int h = 0; h < 2; ++h) {
+            const int p = h ? k : i;
+            const double sgn = h ? 1.0 : -1.0;
+            Dual qt[4];
+            {
+                double qv[4], qd[4], xv[4], yv[4], xd[4], yd[4], hv[4], lv[4], hd[4], ld[4];
+                ld4nc(reinterpret_cast<const double *>(s.qv[qc] + p), qv);
+                ld4nc(reinterpret_cast<const double *>(s.qt[qc] + p), qd);
+                ld4nc(s.dqv[dqa] + 8 * (size_t)p, xv);
+                ld4nc(s.dqv[dqa] + 8 * (size_t)p + 4, yv);
+                ld4nc(s.dqt[dqa] + 8 * (size_t)p, xd);
+                ld4nc(s.dqt[dqa] + 8 * (size_t)p + 4, yd);
+                ld4nc(s.qmv + 8 * (size_t)p, hv);
+                ld4nc(s.qmv + 8 * (size_t)p + 4, lv);
+                ld4nc(s.qmt + 8 * (size_t)p, hd);
+                ld4nc(s.qmt + 8 * (size_t)p + 4, ld);
+                const double eps2 = g.eps2[p];
 #pragma unroll
-                for (int m = 0; m < 4; ++m) v[m] += w * (Gk[m] - Gi[m]);
+                for (int m = 0; m < 4; ++m)
+                    qt[m] = limited_dual(delx * Dual(xv[m], xd[m]) + dely * Dual(yv[m], yd[m]),
+                                         Dual(qv[m], qd[m]), Dual(hv[m], hd[m]),
+                                         Dual(lv[m], ld[m]), eps2);
             }
-            if ((my >> (r + 32 * l)) & 1ull) {
-                const Dual w = co[4 + 2 * l] * deln + co[5 + 2 * l] * dels;
-                Dual Gi[4], Gk[4];
-                flux_split_dual(si, si.un, si.ut, si.B2, si.e2, sg, Gi);
-                flux_split_dual(sk, sk.un, sk.ut, sk.B2, sk.e2, sg, Gk);
-                v[0] += w * (Gk[0] - Gi[0]);
-                v[1] += w * (Gk[2] - Gi[2]);
-                v[2] += w * (Gk[1] - Gi[1]);
-                v[3] += w * (Gk[3] - Gi[3]);
+            KStateT<Dual> st;
+            {
+                const double q[4] = {qt[0].v, qt[1].v, qt[2].v, qt[3].v};
+                KState vs, same;
+                double u[2], w[2];
+                kstate_pair(q, q, nx.v, ny.v, 0.56418958354775628695, vs, same, u, w);
+                st = kstate_dual(vs, u, qt, nx, ny);
+            }
+            auto along_t = [&](int l, Dual G[4]) {
+                const double sg = l ? -1.0 : 1.0;
+                if (kind == KIND_INTERIOR)
+                    flux_split_dual(st, st.ut, st.un, st.B1, st.e1, sg, G);
+                else
+                    flux_quad<Dual>(st, Dual(sg), Dual(kind == KIND_WALL ? -1.0 : 1.0), G);
+            };
+            auto along_n = [&](int l, Dual G[4]) {
+                flux_split_dual(st, st.un, st.ut, st.B2, st.e2, l ? -1.0 : 1.0, G);
+            };
+            Dual G[4];
+            along_t(lx, G);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) Dt[m] = h ? G[m] - Dt[m] : G[m];
+            along_n(ly, G);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) Dn[m] = h ? G[m] - Dn[m] : G[m];
+            if (tx) {
+                const Dual w = Dual(sgn) * (co[2] * dels + co[3] * deln);
+                along_t(1, G);
+#pragma unroll
+                for (int m = 0; m < 4; ++m) v[m] += w * G[m];
+            }
+            if (ty) {
+                const Dual w = Dual(sgn) * (co[6] * deln + co[7] * dels);
+                along_n(1, G);
+                v[0] += w * G[0];
+                v[1] += w * G[2];
+                v[2] += w * G[1];
+                v[3] += w * G[3];
             }
         }
+        const Dual wx = co[2 * lx] * dels + co[2 * lx + 1] * deln;
+        const Dual wy = co[4 + 2 * ly] * deln + co[5 + 2 * ly] * dels;
+        v[0] += wx * Dt[0] + wy * Dn[0];
+        v[1] += wx * Dt[1] + wy * Dn[2];
+        v[2] += wx * Dt[2] + wy * Dn[1];
+        v[3] += wx * Dt[3] + wy * Dn[3];
     }
     __syncwarp();
     // lane t of a point gets entry t of (four values, four derivatives)
