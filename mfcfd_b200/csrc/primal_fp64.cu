@@ -1048,15 +1048,17 @@ int sm_count() {
 }  // namespace
 
 // Split of a flux pass for `tiles` scheduled tiles (`per_sm` resident blocks).
-// Up to one tile a resident block, the block's warps share the tile (a round
-// each): FP64 11.4 us against 16.4 at 4,000 points, 17.9 both at 16,000.
+// Up to two tiles a resident block, the block's warps share the tile (a round
+// each): FP64 11.4 us against 16.4 at 4,000 points; an iteration at 10,000 points
+// 60.2 against 65.8, 16,000 70.4 / 71.6, 18,500 73.4 / 73.5, 24,000 93.9 / 88.8;
+// FP32 at 12,000 47.9 / 50.1, 20,000 55.0 / 57.2, 24,000 67.3 / 62.2.
 // Beyond that a warp takes chunks of one tile or, for less idle lanes in the
 // updates (1.15 times the rate), of two, whichever its whole number of turns
 // makes cheaper: FP64, one against two tiles, 45.8 / 52.2 us at 91,000
 // points, 38.6 / 37.6 at 64,000, 112 / 105 at 256,000, 417 / 389 at 1,024,000.
 FluxShape flux_shape(int tiles, int per_sm) {
     const int blocks = sm_count() * per_sm, warps = blocks * FLUX_WARPS;
-    if (tiles <= blocks) return FluxShape{1, 1};
+    if (tiles <= 2 * blocks) return FluxShape{1, 1};
     const double one = 1.15 * nblk(tiles, warps), two = 2.0 * nblk(tiles, 2 * warps);
     return FluxShape{one < two ? 1 : 2, 0};
 }

@@ -19,7 +19,9 @@ pytestmark = pytest.mark.gpu
     (16, 9, dict(mach=0.8)),                     # 9 tiles
     (33, 17, dict(mach=0.8)),                    # 561 points: a last tile of one
     (96, 98, dict(mach=0.8)),                    # 588 tiles: a block a tile on 148 SMs
-    (96, 99, dict(mach=0.8)),                    # 594: a warp a tile
+    (96, 99, dict(mach=0.8)),                    # 594: two for some
+    (132, 143, dict(mach=0.8)),                  # 1,180: a block two tiles
+    (132, 144, dict(mach=0.8)),                  # 1,188: a warp a tile
     (192, 197, dict(mach=0.8)),                  # 2,364: one turn
     (192, 198, dict(mach=0.8)),                  # 2,376: two turns, or two tiles a warp
     (61, 23, dict(mach=0.8, power=-2.0)),
@@ -45,7 +47,9 @@ def test_flux_pass_paths(ni, nj, flow):
     (16, 9, 0.1),      # 9 tiles
     (33, 17, 0.1),     # a last tile of one point
     (120, 98, 0.1),    # 735 tiles: a block a tile on 148 SMs
-    (120, 99, 0.1),    # 743: a warp a tile
+    (120, 99, 0.1),    # 743: two for some
+    (152, 155, 0.1),   # 1,473: a block two tiles
+    (152, 156, 0.1),   # 1,482: a warp a tile
     (240, 197, 0.1),   # 2,955: one turn
     (240, 198, 0.1),   # 2,970: two turns, or two tiles a warp
     (62, 24, 0.0),     # ties
