@@ -28,6 +28,11 @@ namespace {
 
 constexpr int BLK = 128;
 constexpr int GROUPS = BLK / LPP;
+// Lanes a point of the neighbours' sides on a small grid (slot_passes; their
+// blocks are then about one wave), a transposed slot a lane in turn: adjoint of 8
+// iterations with one inner iteration, 4 lanes / 1: 2.38 / 2.63 ms at 1,536
+// points, 3.85 / 4.15 at 16,000, 4.81 / 4.87 at 24,000, 6.63 / 6.55 at 40,000.
+constexpr int FEW_LANES = 4;
 constexpr double OBT = 1.0 / 3.0;
 constexpr double TBT = 2.0 / 3.0;
 
@@ -44,6 +49,19 @@ __device__ __forceinline__ void ld4nc(const double *p, double v[4]) {
     asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
         : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
         : "l"(p));
+}
+
+// Sum of v over W neighbouring lanes (whole warps).
+template <int W>
+__device__ __forceinline__ double lane_sum(double v) {
+#pragma unroll
+    for (int o = W / 2; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+template <int W>
+__device__ __forceinline__ void lanes_sum(double v[4]) {
+#pragma unroll
+    for (int m = 0; m < 4; ++m) v[m] = lane_sum<W>(v[m]);
 }
 
 // A kinetic state from its tape entry (rho, p/rho, B1, B2, e1, e2, u1, u2)
@@ -565,6 +583,7 @@ constexpr int NBR_BLK = 128;
 // 128 registers (256,000 points: 77 us with the solve's records; before those 74,
 // 79 at 3 blocks, 91 with a record of the primitive state's adjoint)
 constexpr int NBR_MIN_BLOCKS = 4;
+template <int W>
 __global__ void __launch_bounds__(NBR_BLK, NBR_MIN_BLOCKS)
 k_flux_b_nbr(Geom g, const R4 *__restrict__ q_in, const double *__restrict__ dq,
              const double *__restrict__ qm, const int *__restrict__ tptr,
@@ -572,8 +591,9 @@ k_flux_b_nbr(Geom g, const R4 *__restrict__ q_in, const double *__restrict__ dq,
              double *__restrict__ qb, double *__restrict__ dqb, double *__restrict__ qmb,
              double *__restrict__ xb, double *__restrict__ yb, double2 *__restrict__ back,
              double *__restrict__ rec) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= g.n) return;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, w = t % W;
+    const bool in_range = t / W < g.n;
+    const int k = in_range ? t / W : g.n - 1;  // (the last block's other lanes: no slots)
     const R4 kv = ld4(q_in + k);
     const double qk[4] = {kv.a, kv.b, kv.c, kv.d};
     double dxk[4], dyk[4], qmaxk[4], qmink[4];
@@ -584,8 +604,8 @@ k_flux_b_nbr(Geom g, const R4 *__restrict__ q_in, const double *__restrict__ dq,
     double qkb[4] = {0, 0, 0, 0}, dxkb[4] = {0, 0, 0, 0}, dykb[4] = {0, 0, 0, 0},
            qmaxkb[4] = {0, 0, 0, 0}, qminkb[4] = {0, 0, 0, 0};
     double xkb = 0.0, ykb = 0.0;
-    const int e1 = tptr[k + 1];
-    for (int e = tptr[k]; e < e1; ++e) {
+    const int e1 = in_range ? tptr[k + 1] : 0;
+    for (int e = tptr[k] + w; e < e1; e += W) {
         const int slot = tlist[e];
         const int i = slot / g.kp, r = slot - i * g.kp;
         const double2 pi_ = g.xy[i];
@@ -601,6 +621,14 @@ k_flux_b_nbr(Geom g, const R4 *__restrict__ q_in, const double *__restrict__ dq,
         ykb += dd.y + dyr;
         back[(size_t)r * g.n + i] = make_double2(dxr, dyr);
     }
+    lanes_sum<W>(qkb);
+    lanes_sum<W>(dxkb);
+    lanes_sum<W>(dykb);
+    lanes_sum<W>(qmaxkb);
+    lanes_sum<W>(qminkb);
+    xkb = lane_sum<W>(xkb);
+    ykb = lane_sum<W>(ykb);
+    if (w > 0 || !in_range) return;
     add_pairs(qb + 4 * (size_t)k, qkb, 4);
     double v8[8];
 #pragma unroll
@@ -827,21 +855,23 @@ k_grad_b(Geom g, Consts c, const R4 *__restrict__ q, const double *__restrict__ 
 // q's adjoint is complete then, and goes on to the primitive state
 // (eval_q_variables_b).  40 us at 256,000 points (5 blocks an SM; 45 at 4, 49 at
 // 6); 62 and a pass of 10 for the primitive state with the longer record.
+template <int W>
 __global__ void __launch_bounds__(BLK, 5)
 k_grad_b_nbr(Geom g, Consts c, const R4 *__restrict__ q, const R4 *__restrict__ prim,
              const double *__restrict__ qmb, const double *__restrict__ deltab,
              const int *__restrict__ tptr, const int *__restrict__ tlist,
              const double *__restrict__ rec, const double *__restrict__ qb,
              double *__restrict__ pb, double *__restrict__ xb, double *__restrict__ yb) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= g.n) return;
-    double qk[4], qkb[4], pkb[4] = {0, 0, 0, 0}, xkb = 0.0, ykb = 0.0;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, w = t % W;
+    const bool in_range = t / W < g.n;
+    const int k = in_range ? t / W : g.n - 1;  // (the last block's other lanes: no slots)
+    double qk[4], qkb[4] = {0, 0, 0, 0}, pkb[4] = {0, 0, 0, 0}, xkb = 0.0, ykb = 0.0;
     ld4nc(reinterpret_cast<const double *>(q + k), qk);
-    ld4nc(qb + 4 * (size_t)k, qkb);
+    if (w == 0) ld4nc(qb + 4 * (size_t)k, qkb);
     const R4 P = ld4(prim + k);
     const double2 pk = g.xy[k];
-    const int e1 = tptr[k + 1];
-    for (int e = tptr[k]; e < e1; ++e) {
+    const int e1 = in_range ? tptr[k + 1] : 0;
+    for (int e = tptr[k] + w; e < e1; e += W) {
         const int slot = tlist[e];
         const int i = slot / g.kp, r = slot - i * g.kp;
         double zx[4], zy[4], M[4], qi[4];
@@ -883,6 +913,11 @@ k_grad_b_nbr(Geom g, Consts c, const R4 *__restrict__ q, const R4 *__restrict__ 
         xkb += delxb;
         ykb += delyb;
     }
+    lanes_sum<W>(qkb);
+    lanes_sum<W>(pkb);
+    xkb = lane_sum<W>(xkb);
+    ykb = lane_sum<W>(ykb);
+    if (w > 0 || !in_range) return;
     q_from_prim_b(P.a, P.b, P.c, P.d, qkb, pkb);
     add_pairs(pb + 4 * (size_t)k, pkb, 4);
     xb[k] += xkb;
@@ -1074,8 +1109,10 @@ void launch_flux_b(const Geom &g, const R4 *q_in, const double *dq, const double
                                                reinterpret_cast<const double *>(fr), frb, qb,
                                                dqb, qmb, xb, yb, nxb, nyb, deltab, nbrec, kst);
     double2 *bk = reinterpret_cast<double2 *>(back);
-    k_flux_b_nbr<<<nblk(g.n, NBR_BLK), NBR_BLK, 0, s>>>(g, q_in, dq, qm, tptr, tlist, nbrec, in,
-                                                       qb, dqb, qmb, xb, yb, bk, rec);
+    const bool few = slot_passes(g.n);
+    auto *nbr = few ? k_flux_b_nbr<FEW_LANES> : k_flux_b_nbr<1>;
+    nbr<<<nblk(g.n, NBR_BLK / (few ? FEW_LANES : 1)), NBR_BLK, 0, s>>>(
+        g, q_in, dq, qm, tptr, tlist, nbrec, in, qb, dqb, qmb, xb, yb, bk, rec);
 }
 
 void launch_inner_b(const Geom &g, const double *dq_in, LsqIn in, bool first, double *dqb,
@@ -1095,7 +1132,10 @@ void launch_grad_b(const Geom &g, const Consts &c, const R4 *q, const R4 *prim,
         k_grad_b<true><<<nb, BLK, 0, s>>>(g, c, q, spdA, qmb, deltab, bk, qb, xb, yb, rec);
     else
         k_grad_b<false><<<nb, BLK, 0, s>>>(g, c, q, spdA, qmb, deltab, bk, qb, xb, yb, rec);
-    k_grad_b_nbr<<<nb, BLK, 0, s>>>(g, c, q, prim, qmb, deltab, tptr, tlist, rec, qb, pb, xb, yb);
+    const bool few = slot_passes(g.n);
+    auto *nbr = few ? k_grad_b_nbr<FEW_LANES> : k_grad_b_nbr<1>;
+    nbr<<<nblk(g.n, BLK / (few ? FEW_LANES : 1)), BLK, 0, s>>>(g, c, q, prim, qmb, deltab, tptr,
+                                                               tlist, rec, qb, pb, xb, yb);
 }
 
 void launch_gather(int n, const int *tptr, const int *tlist, const double *contrib, double *pb,

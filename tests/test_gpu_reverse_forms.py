@@ -3,7 +3,7 @@ change: several inner iterations (the D pass's derivatives enter every one),
 neighbours exactly on an axis (a grid without jitter: in both lists of a
 direction), stencils of up to 20 slots (the flux reverse's later rounds) that
 are not symmetric, point counts around the blocks of 64 and 128, first-order
-time stepping.  Both derivatives are exact up to rounding, which some 1e2
+time stepping; the small grids' forms and, past 21,000 points, the others.  Both derivatives are exact up to rounding, which some 1e2
 operations a term and a few passes keep below 1e-9 of the sum of the terms'
 sizes."""
 import numpy as np
@@ -36,6 +36,8 @@ def _widen(g, seed):
     (32, 12, 0.0, 1, "ssprk43", False),   # ties
     (31, 13, 0.1, 0, "ssprk43", True),    # up to 20 slots
     (31, 13, 0.0, 3, "first", True),
+    (200, 108, 0.1, 1, "first", False),   # 21,600: past the small grids' forms on 148 SMs
+    (200, 108, 0.0, 2, "ssprk43", True),
 ])
 def test_adjoint_and_tangent_agree(gpu, ni, nj, jitter, inner, tscheme, wide):
     g = naca_ogrid(ni, nj, seed=15, first_spacing=5e-3, jitter=jitter)
