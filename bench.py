@@ -552,7 +552,7 @@ def main():
                 "dCl": abs(float(cl32[0] - cl64[0])), "dCd": abs(float(cd32[0] - cd64[0])),
                 "Cl_fp64": float(cl64[0]), "Cd_fp64": float(cd64[0]),
                 "kernel_ms": {k: float(v) for k, v in kt32.items()},
-                "note": "FP32 state, fluxes and Kahan sums; the state update's arithmetic, "
+                "note": "FP32 state and fluxes, summed in FP64; the state update's arithmetic, "
                         "the geometry (LSQ inverses, formed once), the residual and the "
                         "forces in FP64; dCl/dCd against the FP64 run after the same "
                         "iterations, 'accuracy' after --fp32-check-iters from freestream"}
@@ -595,7 +595,7 @@ def main():
     roofline.update({
         "kernel": "kb_flux (flux residual + state update, one SSPRK stage)",
         "fp64_pipe_active_frac": _profile_value("fp64_pipe_active_frac"),
-        "note": ("kb_flux is bound by FP64 latency (exp/erf/div chains), not by HBM: "
+        "note": ("kb_flux is bound by issue and FP64 latency, not by HBM: "
                  "achieved/peak is its FP64 work rate against the measured FMA peak; "
                  "the hbm object gives its algorithmic bytes against the copy peak")})
     iter_bytes = ab["iteration"] * grid.n
