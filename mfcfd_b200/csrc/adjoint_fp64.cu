@@ -101,10 +101,7 @@ __device__ __forceinline__ void add_pairs(double *dst, const double *v, int n) {
     }
 }
 
-#ifndef ADJ_MIN_BLOCKS
-#define ADJ_MIN_BLOCKS 3
-#endif
-__global__ void __launch_bounds__(BLK, ADJ_MIN_BLOCKS)
+__global__ void __launch_bounds__(BLK, 3)
 k_update_b(Geom g, Consts c, AdjConsts a, const R4 *__restrict__ prim_in,
            const R4 *__restrict__ prim_old, const R4 *__restrict__ fr,
            const double *__restrict__ pb_out, double *__restrict__ pb_in,

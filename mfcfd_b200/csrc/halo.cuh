@@ -36,8 +36,8 @@ __device__ __forceinline__ void halo_wait() {
 }
 
 // The row indices of a warp's two tiles: lane l holds those of pair rows l,
-// l + 32, l + 64 and l + 96 (row u of the pair being row u of the first
-// tile's halo, hrow[h0 + u], or row u - hn0 of the second's).
+// l + 32, l + 64, ... (row u of the pair being row u of the first tile's halo,
+// hrow[h0 + u], or row u - hn0 of the second's).
 template <int CAP>
 struct HaloIdx {
     int h0 = 0, hn0 = 0, h1 = 0, hn1 = 0;

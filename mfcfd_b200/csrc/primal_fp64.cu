@@ -249,18 +249,10 @@ __device__ __forceinline__ void st8w(double *p, const double a[4], const double 
                  "d"(b[2]), "d"(b[3]) : "memory");
 }
 
-// Copies the halo rows of a warp's two tiles (hrow ranges [h0, h0 + hn0) and
-// [h1, h1 + hn1), row u of the pair being row u of the first tile's halo or
-// row u - hn0 of the second's) into their shared-memory arrays sm0 / sm1.
-// Consecutive lanes copy consecutive 16-byte pieces of a row array -- the
-// pieces of one row, then those of the next row in the halo's ascending
-// order -- so that runs of neighbouring rows come in whole 128-byte lines.
-// Lane l first loads the row indices of pair rows l, l + 32, l + 64 and
-// l + 96; a copy takes its row index from the lane holding it (a shuffle
-// whose source register is the same for the whole warp).  nA = HA_I copies
-// q, (x, y) and dq; nA = HA_D copies q, (x, y) and, with spd != nullptr, spd.
-// Stages a chunk's halo rows: the D pass q (two pieces a row), (x, y) and,
-// with spd != nullptr, spd; the I pass (x, y) and dq (four pieces a row).
+// Stages a chunk's halo rows (stage_array): the D pass q (two pieces a row),
+// (x, y) and, with spd != nullptr, spd; the I pass (x, y) and dq (four pieces a
+// row).  Consecutive lanes copy consecutive 16-byte pieces of a row array, so
+// that runs of neighbouring rows come in whole 128-byte lines.
 template <int nA, int CAP>
 __device__ __forceinline__ void stage_halo(const Geom &g, const R4 *q, const double *dq,
                                            const double *spd, const HaloIdx<CAP> &x, int lane,
