@@ -282,7 +282,7 @@ void lskum_host::build_halo(int n, int kp, const int *conn, const int *nbhs,
                             const std::vector<std::pair<int, int>> &ranges, HostHalo &out) {
     const int ntile = (n + TILE - 1) / TILE;
     out.hkp = ((kp + 1 + 7) / 8) * 8;
-    out.hc = 0;
+    out.hc = out.hmost = 0;
     out.off.assign((size_t)ntile + 1, 0);
     out.rows.clear();
     out.loc.assign((size_t)n * out.hkp, 0);
@@ -316,7 +316,7 @@ void lskum_host::build_halo(int n, int kp, const int *conn, const int *nbhs,
             for (int r = 0; r < nbhs[p]; ++r) l[r] = pos(conn[(size_t)r * n + p]);
             l[out.hkp - 1] = pos(p);
         }
-        out.hc = std::max(out.hc, (int)rows.size());
+        out.hmost = std::max(out.hmost, (int)rows.size());
         out.rows.insert(out.rows.end(), rows.begin(), rows.end());
     }
     out.off[ntile] = (int)out.rows.size();
@@ -324,7 +324,7 @@ void lskum_host::build_halo(int n, int kp, const int *conn, const int *nbhs,
     // row's 16-byte pieces in consecutive arrays fall on different banks
     // (C2 I pass: 0.091 ms; 0.109 with no padding, 0.097 - 0.101 at two to
     // seven more than a multiple of eight)
-    if (out.hc > 0) out.hc += (9 - out.hc % 8) % 8;
+    if (out.hmost > 0) out.hc = out.hmost + (9 - out.hmost % 8) % 8;
 }
 
 int lskum_host::reset_run(mfcfd_t *h, int it_first) {
@@ -884,6 +884,7 @@ static int create_handle(const mfcfd_grid *grid, const mfcfd_params *params, int
         h->geom.hloc = h->d_hloc;
         h->geom.hkp = halo.hkp;
         h->geom.hc = halo.hc;
+        h->geom.hmost = halo.hmost;
     }
     if (!h->fp32) {
         // on the stream of the uploads above, and before the copies below

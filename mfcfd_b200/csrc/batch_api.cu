@@ -649,6 +649,7 @@ int mfcfd_batch_create(int n_inst, const mfcfd_grid *const *grids, const mfcfd_p
         b->geom.hloc = b->d_hloc;
         b->geom.hkp = halo.hkp;
         b->geom.hc = halo.hc;
+        b->geom.hmost = halo.hmost;
     }
     if (!b->fp32) {
         // on the stream of the uploads above, and before the copies below

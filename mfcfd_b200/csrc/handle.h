@@ -124,7 +124,7 @@ struct HostGrid {
 struct HostHalo {
     std::vector<int> off, rows;
     std::vector<unsigned char> loc;
-    int hkp = 0, hc = 0;
+    int hkp = 0, hc = 0, hmost = 0;
 };
 
 namespace lskum_host {

@@ -51,11 +51,12 @@ struct Geom {
     // hoff[tile] .. hoff[tile + 1] index its rows in hrow (an empty range: the
     // tile's halo exceeds HALO_CAP_WIDE and its rows are gathered directly).
     // hloc[p * hkp + r] is slot r's row within the tile's halo, hloc[p * hkp
-    // + hkp - 1] the point's own; hc = the largest halo, the staging stride.
+    // + hkp - 1] the point's own; hmost = the largest halo, hc = the staging
+    // stride (hmost padded: it does not tell how many rows a tile has).
     const int *hoff = nullptr;
     const int *hrow = nullptr;
     const unsigned char *hloc = nullptr;
-    int hkp = 0, hc = 0;
+    int hkp = 0, hc = 0, hmost = 0;
     // FP64 flux pass, fixed per grid: per point and split list the two
     // coefficients of the list's least-squares solve ([n][8], launch_flux_coef),
     // and with power != 0 the weight of every slot ([kp][n]; else nullptr: 1).
@@ -74,6 +75,8 @@ struct Geom {
 // passes' time (an iteration with one inner iteration FP64 195.7 us, 169.6 with
 // the wide forms; FP32 113.3 and 98.1).
 constexpr int HALO_CAP = 64, HALO_CAP_WIDE = 96;
+// whether a grid's staged tiles need the wide forms
+inline bool wide_halos(const Geom &g) { return g.hmost > HALO_CAP; }
 
 struct Consts {
     double cfl, power, euler, pi, gm1;  // gm1 = gamma - 1

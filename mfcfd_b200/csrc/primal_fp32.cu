@@ -801,15 +801,15 @@ namespace {
 // dynamic shared memory of the halo kernels at staging stride hc
 size_t halo32_smem(int hc) { return halo_bytes(HALO32_BLOCK / 32, HA32, hc); }
 // blocks of the D pass's halo kernel, as halo_grid of the FP64 passes
-int halo32_grid(int hc, int grid) {
-    const bool wide = hc > HALO_CAP + 1;
+int halo32_grid(const Geom &g, int grid) {
+    const bool wide = wide_halos(g);
     if (grid > 0 && !wide) return grid;
     int dev = 0, sms = 1, nb = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &nb, wide ? kb_grad32_h<HALO_CAP_WIDE> : kb_grad32_h<HALO_CAP>, HALO32_BLOCK,
-        halo32_smem(hc));
+        halo32_smem(g.hc));
     const int wave = std::max(sms, 1) * std::max(1, e == cudaSuccess ? nb : 1);
     return grid > 0 ? std::min(grid, wave) : wave;
 }
@@ -850,8 +850,8 @@ void launch_grad32(const Geom &g, const Consts &c, const Geom32 &f, const Sched 
                                                                 with_delta ? 1 : 0);
         return;
     }
-    auto *kernel = g.hc > HALO_CAP + 1 ? kb_grad32_h<HALO_CAP_WIDE> : kb_grad32_h<HALO_CAP>;
-    kernel<<<halo32_grid(g.hc, grid), HALO32_BLOCK, halo32_smem(g.hc), st>>>(
+    auto *kernel = wide_halos(g) ? kb_grad32_h<HALO_CAP_WIDE> : kb_grad32_h<HALO_CAP>;
+    kernel<<<halo32_grid(g, grid), HALO32_BLOCK, halo32_smem(g.hc), st>>>(
         g, c, f, s, q, spd, dq, qm, delta, with_delta ? 1 : 0);
 }
 

@@ -1142,10 +1142,10 @@ int batch_occupancy(int kind, bool fp32, int block, size_t smem) {
 
 // blocks of a halo kernel (kind 0: D pass, 1: I pass): `grid`, but no more than
 // one wave of the wide forms, or one wave (grid == 0)
-int halo_grid(int kind, int hc, int grid) {
-    const bool wide = hc > HALO_CAP + 1;
+int halo_grid(int kind, const Geom &g, int grid) {
+    const bool wide = wide_halos(g);
     if (grid > 0 && !wide) return grid;
-    const size_t smem = halo_smem_bytes(kind, hc);
+    const size_t smem = halo_smem_bytes(kind, g.hc);
     int nb = 0;
     auto ask = [&](auto *kernel) {
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, HALO_BLOCK, smem);
@@ -1166,8 +1166,8 @@ void launch_grad(const Geom &g, const Consts &c, const Sched &s, const R4 *q, co
                                                               with_delta ? 1 : 0);
         return;
     }
-    auto *kernel = g.hc > HALO_CAP + 1 ? kb_grad_h<HALO_CAP_WIDE> : kb_grad_h<HALO_CAP>;
-    kernel<<<halo_grid(0, g.hc, grid), HALO_BLOCK, halo_smem_bytes(0, g.hc), st>>>(
+    auto *kernel = wide_halos(g) ? kb_grad_h<HALO_CAP_WIDE> : kb_grad_h<HALO_CAP>;
+    kernel<<<halo_grid(0, g, grid), HALO_BLOCK, halo_smem_bytes(0, g.hc), st>>>(
         g, c, s, q, spd, dq, qm, delta, with_delta ? 1 : 0);
 }
 
@@ -1179,8 +1179,8 @@ void launch_inner(const Geom &g, const Consts &c, const Sched &s, const double *
         kb_inner_s<<<nblk(g.n, SLOT_PTS), SLOT_BLOCK, 0, st>>>(g, s, dq0, dq_in, dq_out);
         return;
     }
-    auto *kernel = g.hc > HALO_CAP + 1 ? kb_inner_h<HALO_CAP_WIDE> : kb_inner_h<HALO_CAP>;
-    kernel<<<halo_grid(1, g.hc, grid), HALO_BLOCK, halo_smem_bytes(1, g.hc), st>>>(
+    auto *kernel = wide_halos(g) ? kb_inner_h<HALO_CAP_WIDE> : kb_inner_h<HALO_CAP>;
+    kernel<<<halo_grid(1, g, grid), HALO_BLOCK, halo_smem_bytes(1, g.hc), st>>>(
         g, s, dq0, dq_in, dq_out);
 }
 
