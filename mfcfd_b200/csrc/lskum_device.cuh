@@ -49,7 +49,7 @@ struct Geom {
     // gathered directly).  The halo of a TILE-point tile is the sorted set of
     // rows its points read (the points themselves and their neighbours);
     // hoff[tile] .. hoff[tile + 1] index its rows in hrow (an empty range: the
-    // tile's halo exceeds HALO_CAP_WIDE and its rows are gathered directly).
+    // tile's halo exceeds the grid's cap and its rows are gathered directly).
     // hloc[p * hkp + r] is slot r's row within the tile's halo, hloc[p * hkp
     // + hkp - 1] the point's own; hmost = the largest halo, hc = the staging
     // stride (hmost padded: it does not tell how many rows a tile has).
@@ -70,10 +70,10 @@ struct Geom {
 };
 // Rows a tile halo stages at most (its local row indices are bytes): an O-grid's
 // tiles have some 54, those of a renumbered cloud of points about 58 and a few
-// over 64.  A grid whose largest is over HALO_CAP takes the passes' wide forms:
-// gathered directly, those few tiles (4% of a cloud of 40,000 points) set the
-// passes' time (an iteration with one inner iteration FP64 195.7 us, 169.6 with
-// the wide forms; FP32 113.3 and 98.1).
+// over 64.  HALO_CAP, or HALO_CAP_WIDE and the passes' wide forms where that pays
+// (wide_halos_pay): gathered directly, the few large tiles (4% of a cloud of
+// 40,000 points) can set the passes' time (an iteration with one inner iteration
+// FP64 195.7 us, 169.6 with the wide forms; FP32 113.3 and 98.1).
 constexpr int HALO_CAP = 64, HALO_CAP_WIDE = 96;
 // whether a grid's staged tiles need the wide forms
 inline bool wide_halos(const Geom &g) { return g.hmost > HALO_CAP; }

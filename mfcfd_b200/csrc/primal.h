@@ -105,6 +105,9 @@ struct StageBufs {
 // then the neighbour's reconstruction rho p/rho B1 B2 erf1 erf2 u1 u2
 constexpr int KS_TAPE = 16;
 
+// whether the wide halo forms pay for a grid with `over` of its tiles' halos over
+// HALO_CAP rows
+bool wide_halos_pay(int tiles, int over);
 // whether the D and I passes of a grid of n points go by slots
 bool slot_passes(int n);
 

@@ -1062,6 +1062,27 @@ FluxShape flux_shape(int tiles, int per_sm) {
 // 70.4 / 79.5, 24,000 76.4 / 77.6, 32,000 86.7 / 86.7).
 bool slot_passes(int n) { return nblk(n, SLOT_PTS) <= 9 * sm_count(); }
 
+// The wide halo forms for a grid with `over` tiles of more than HALO_CAP rows.
+// They cost every tile a block an SM (and the D pass its fixed stride); a tile
+// gathered directly costs its warp a longer chain, which sets the pass's time while
+// a warp has few chunks.  An iteration with one inner iteration on 148 SMs, wide /
+// narrow with the large tiles gathered, by the share of large tiles:
+//   points   precision  one tile    0.1%         0.5%         1%           2%
+//    90,000  FP64   us  263 / 276   260 / 275    277 / 284    278 / 285    302 / 309
+//   256,000  FP64       583 / 587   608 / 603    623 / 631    642 / 663    656 / 685
+//   256,000  FP32       349 / 340   349 / 351    365 / 377    366 / 383    360 / 379
+//   520,000  FP64      1201 / 1165 1260 / 1280  1269 / 1283  1289 / 1315  1313 / 1386
+//   520,000  FP32       651 / 640   670 / 666    667 / 663    671 / 689    679 / 700
+//   700,000  FP64      1575 / 1519 1638 / 1578  1680 / 1669  1691 / 1679  1721 / 1759
+//   700,000  FP32       865 / 836   871 / 859    883 / 900    889 / 901    902 / 942
+//  1,024,000 FP64      2253 / 2174 2327 / 2221       -       2407 / 2385  2439 / 2423
+//  1,024,000 FP32      1253 / 1216 1250 / 1252       -       1274 / 1294  1279 / 1332
+//  4,096,000 FP64      8804 / 8504 9140 / 8617       -       9308 / 9014  9463 / 9289
+//  4,096,000 FP32      4723 / 4556 4738 / 4599       -       4788 / 4743  4834 / 4869
+// Hence: from 200 tiles an SM on (five chunks a resident warp), narrow up to a
+// share of 0.5%.
+bool wide_halos_pay(int tiles, int over) { return tiles < 200 * sm_count() || 200LL * over > tiles; }
+
 // flux-pass blocks that give every chunk its warp (or its block)
 int flux_grid_blocks(int n, bool fp32) {
     const int tiles = nblk(n, TILE);

@@ -9,6 +9,7 @@ import numpy as np
 import pytest
 
 import oracle
+from mfcfd_b200.batch import Batch
 from mfcfd_b200.grid import INTERIOR, OUTER, WALL, naca_ogrid
 from mfcfd_b200.solver import Solver
 from tests.helpers import max_rel
@@ -44,12 +45,12 @@ def halo_sizes(g):
     return np.array([len(halo(g, order, inv, t)) for t in range(-(-g.n // TILE))])
 
 
-def grown(kind, sms=148):
+def grown(kind, sms=148, ni=200, nj=None):
     """A ring-ordered grid past the slots' line, the halos of some tiles grown to
     the wanted rows: their points take the nearest points outside the halo, one
     each in turn."""
     tiles, even, odd = GROWN[kind]
-    g = naca_ogrid(200, max(120, SLOTS * sms // 200 + 2), seed=5, spacing="arc",
+    g = naca_ogrid(ni, nj or max(120, SLOTS * sms // ni + 2), seed=5, spacing="arc",
                    first_spacing="match")
     order = order_of(g)
     inv = np.empty(g.n, np.int64)
@@ -59,7 +60,7 @@ def grown(kind, sms=148):
         want = (odd if t % 2 else even) - len(rows)
         assert want >= 0
         pts = order[t * TILE:(t + 1) * TILE]
-        near = range(max(0, pts[0] - 1200), min(g.n, pts[-1] + 1200))
+        near = range(max(0, pts[0] - 6 * ni), min(g.n, pts[-1] + 6 * ni))
         near = np.array([k for k in near if inv[k] not in rows and g.flag_1[k] == INTERIOR])
         d2 = (g.x[near] - g.x[pts[8]]) ** 2 + (g.y[near] - g.y[pts[8]]) ** 2
         for a, k in enumerate(near[np.argsort(d2, kind="stable")[:want]]):
@@ -129,3 +130,27 @@ def test_shuffled_grids_past_the_slots_match_the_oracle(gpu, frac):
     share = [float(np.mean(s)) for s in (sizes <= 64, (sizes > 64) & (sizes <= 96), sizes > 96)]
     assert share[2] > 0.9 if frac == 1.0 else min(share) > 0.02, share
     check(g, inner=2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "fp32_mixed"])
+def test_few_large_tiles_of_a_large_grid(gpu, precision):
+    """Two tiles of 65 rows in a grid past the line from which the wide forms need a
+    share of the tiles: gathered directly, with the same bits as in a batch whose
+    other grid takes both to the wide forms."""
+    sms = sm_count()
+    large = grown("65", sms, ni=800, nj=200 * TILE * sms // 800 + 8)
+    small = grown("many 66", sms)
+    assert large.n // TILE > 200 * sms and (large.n + small.n) // TILE < 200 * (len(MANY) + 2)
+    flow = dict(cfl=0.1, vl_const=5.0, mach=0.8, aoa=1.5, inner_iterations=1)
+    with Batch([large, small], [dict(flow, precision=precision) for _ in range(2)]) as b:
+        b.run(2)
+        many = b.get_state(0)
+    with Solver(large, precision=precision, **flow) as s:
+        s.run(2)
+        assert np.array_equal(s.get_state(), many)
+    if precision == "fp64":
+        o = oracle.Oracle(large, **flow)
+        o.run(2)
+        assert max_rel(many, o.prim()) < 1e-10
+        o.close()
