@@ -51,42 +51,27 @@ __device__ __forceinline__ void stf8w(float *p, const float a[4], const float b[
 // where dq0 = L sum_k w d (q_k - q_i) is the D pass's result of this stage
 // and L M = I turns the point's own term into dq_i/2.  Equal in exact
 // arithmetic; only the neighbours' derivatives are gathered (no q).
-// The loads of U slots are issued together: four while the pass's arrays stay in
-// L2 (up to INNER32_AHEAD points: 10.2 -> 9.9 us at 91,000 points, 15.9 -> 14.0
-// at 256,000; an iteration with three inner iterations 431 -> 411 us).  Beyond,
-// more rows in flight cost L2 hits: 19.7 -> 20.7 us at 400,000 points, 51.5 ->
-// 56.9 at 1.024M.
-constexpr int INNER32_AHEAD = 320000;
-template <int U>
+// One slot at a time, as the compiler unrolls it: asking for four slots' loads
+// together is 1 - 3% slower (8 slots / 20 slots a point, an iteration with three
+// inner iterations: 90,000 points 168 / 306 us, 170 / 313 with four together;
+// 256,000 402 / 861, 408 / 874; a pass at 1.024M points 49.7 / 89.1, 51.5 / 94.0).
 __device__ __forceinline__ void
 inner32_point(const Geom &g, const Geom32 &f, const float *__restrict__ dq0,
               const float *__restrict__ dq_in, float *__restrict__ dq_out, int i) {
     float tx[4] = {0.f, 0.f, 0.f, 0.f}, ty[4] = {0.f, 0.f, 0.f, 0.f};
     const int nb = g.nbhs[i];
-    for (int r0 = 0; r0 < nb; r0 += U) {
-        int kk[U];
-        float2 dd[U];
+    for (int r = 0; r < nb; ++r) {
+        const int k = g.conn[(size_t)r * g.n + i];
+        const float2 d = __ldg(f.dxy + (size_t)r * g.n + i);
+        const float w = f.w ? __ldg(f.w + (size_t)r * g.n + i) : 1.0f;
+        float dxk[4], dyk[4];
+        ldf8w(dq_in + 8 * (size_t)k, dxk, dyk);
+        const float wdx = w * d.x, wdy = w * d.y;
 #pragma unroll
-        for (int j = 0; j < U; ++j) {
-            const int r = min(r0 + j, nb - 1);
-            kk[j] = __ldg(g.conn + (size_t)r * g.n + i);
-            dd[j] = __ldg(f.dxy + (size_t)r * g.n + i);
-        }
-        float dxk[U][4], dyk[U][4];
-#pragma unroll
-        for (int j = 0; j < U; ++j) ldf8w(dq_in + 8 * (size_t)kk[j], dxk[j], dyk[j]);
-#pragma unroll
-        for (int j = 0; j < U; ++j) {
-            if (r0 + j >= nb) break;
-            const float2 d = dd[j];
-            const float w = f.w ? __ldg(f.w + (size_t)(r0 + j) * g.n + i) : 1.0f;
-            const float wdx = w * d.x, wdy = w * d.y;
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const float pk = fmaf(d.x, dxk[j][m], d.y * dyk[j][m]);
-                tx[m] = fmaf(wdx, pk, tx[m]);
-                ty[m] = fmaf(wdy, pk, ty[m]);
-            }
+        for (int m = 0; m < 4; ++m) {
+            const float pk = fmaf(d.x, dxk[m], d.y * dyk[m]);
+            tx[m] = fmaf(wdx, pk, tx[m]);
+            ty[m] = fmaf(wdy, pk, ty[m]);
         }
     }
     float dxi[4], dyi[4], dx0[4], dy0[4];
@@ -102,7 +87,6 @@ inner32_point(const Geom &g, const Geom32 &f, const float *__restrict__ dq0,
     stf8w(dq_out + 8 * (size_t)i, dx, dy);
 }
 
-template <int U>
 __global__ void __launch_bounds__(GRAD_BLOCK)
 kb_inner32(Geom g, Geom32 f, Sched s, const float *__restrict__ dq0,
            const float *__restrict__ dq_in, float *__restrict__ dq_out) {
@@ -112,7 +96,7 @@ kb_inner32(Geom g, Geom32 f, Sched s, const float *__restrict__ dq0,
     for (int vp = blockIdx.x * blockDim.x + threadIdx.x; vp < total;
          vp += gridDim.x * blockDim.x) {
         const int i = sched_point(s, ss, vp);
-        if (i >= 0 && live) inner32_point<U>(g, f, dq0, dq_in, dq_out, i);
+        if (i >= 0 && live) inner32_point(g, f, dq0, dq_in, dq_out, i);
     }
 }
 
@@ -827,7 +811,7 @@ int batch_occupancy32(int kind, int block, size_t smem) {
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_grad32_h<HALO_CAP>, HALO32_BLOCK,
                                                           halo32_smem(HALO_CAP + 1));
     else if (kind == 1)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_inner32<1>, block, smem);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_inner32, block, smem);
     else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_flux32, block, smem);
     return e == cudaSuccess ? nb : 1;
 }
@@ -863,8 +847,7 @@ void launch_inner32(const Geom &g, const Consts &c, const Geom32 &f, const Sched
         kb_inner32_s<<<nblk(g.n, SLOT_PTS), SLOT_BLOCK, 0, st>>>(g, f, s, dq0, dq_in, dq_out);
         return;
     }
-    auto *kernel = g.n <= INNER32_AHEAD ? kb_inner32<4> : kb_inner32<1>;
-    kernel<<<wave32(1, block, 0, grid), block, 0, st>>>(g, f, s, dq0, dq_in, dq_out);
+    kb_inner32<<<wave32(1, block, 0, grid), block, 0, st>>>(g, f, s, dq0, dq_in, dq_out);
 }
 
 void launch_flux32(const Geom &g, const Consts &c, const Sched &s, const StageBufs32 &b,
