@@ -149,7 +149,10 @@ int mfcfd_adjoint_many(int n_handles, mfcfd_t *const *handles, int objective, in
  * the final state and dJ/de along the direction.  For the gradient of
  * mfcfd_adjoint over the same iterations, dJ/de = sum_i dJdx_i dx_i +
  * dJdy_i dy_i.  The handle's state is left unchanged.  FP64 handles with
- * power == 0 only (else MFCFD_ERR_ARG). */
+ * power == 0 only (else MFCFD_ERR_ARG).
+ * Device memory: the call needs about 1.1 KB a point.  Up to 128 MB of it stays
+ * with the handle for the next call, until mfcfd_destroy or the handle's first
+ * mfcfd_adjoint; a larger workspace is released before the call returns. */
 int mfcfd_tangent(mfcfd_t *h, int objective, int n_iters, const double *dx, const double *dy,
                   double *J, double *dJ);
 

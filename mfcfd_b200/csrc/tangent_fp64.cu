@@ -681,12 +681,19 @@ inline int nblk(int n, int b) { return (n + b - 1) / b; }
 
 }  // namespace
 
-// Device workspace of mfcfd_tangent, kept with the handle: one allocation,
-// made by the first call (27 allocations and frees a call took longer than ten
-// iterations of 64,000 points) and given back by mfcfd_destroy or when the
-// adjoint needs the memory (drop_tangent).
+// Device workspace of mfcfd_tangent: one allocation of about 1.1 KB a point (27
+// allocations and frees a call took longer than ten iterations of 64,000 points).
+// Up to TAN_KEEP bytes it stays with the handle until mfcfd_destroy or until the
+// handle's adjoint is set up (drop_tangent): an allocation and its release take 0.65 ms at
+// best and 1.8 on average at 77 MB, of 4.4 ms for ten iterations of 64,000 points.
+// A larger one (from some 120,000 points on) is released by the call itself, so
+// that other handles and the caller's own allocator find the memory a call found
+// (ten iterations, kept / released: 256,000 points 17.6 / 18.7 ms, 1,024,000 points
+// 67.5 / 69.8).
+constexpr size_t TAN_KEEP = 128u << 20;
 struct TanWork {
     char *block = nullptr;
+    size_t bytes = 0;
     TanState s{};
     double2 *xy_t = nullptr, *nrm_t = nullptr;
     Dual *obc = nullptr, *coef = nullptr;
@@ -769,6 +776,7 @@ int tan_setup(mfcfd_t *h) {
             delete w;
             return cuda_fail(h, e, "mfcfd_tangent cudaMalloc");
         }
+        w->bytes = bytes;
     }
     w->s.xy_t = w->xy_t;
     w->s.nrm_t = w->nrm_t;
@@ -802,6 +810,13 @@ extern "C" int mfcfd_tangent(mfcfd_t *h, int objective, int n_iters, const doubl
     CK(dg.err);
     CK(cudaStreamSynchronize(h->stream));
     if (int st = tan_setup(h)) return st;
+    // on every way out (cudaFree waits for the device)
+    struct Release {
+        mfcfd_t *h;
+        ~Release() {
+            if (h->tan && h->tan->bytes > TAN_KEEP) lskum_host::drop_tangent(h);
+        }
+    } release{h};
     const TanWork &w = *h->tan;
     const TanState &s = w.s;
     cudaStream_t str = h->stream;
