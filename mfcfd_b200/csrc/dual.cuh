@@ -1,9 +1,9 @@
 // Forward-mode (tangent) scalar: a value and its directional derivative.
 //
-// The primal device templates (reconstruct, kstate, split and quadrant
-// fluxes, q_from_prim, prim_to_conserved, conserved_ubar) instantiated on
-// Dual give the tangent of the reference's routines, like the Tapenade
-// `_d` routines of src_mpi_forward/sensitivity_files (q_lskum_d.F90:28-89).
+// The primal device templates (quadrant fluxes, q_from_prim,
+// prim_to_conserved, conserved_ubar) instantiated on Dual give the tangent of
+// the reference's routines, like the Tapenade `_d` routines of
+// src_mpi_forward/sensitivity_files (q_lskum_d.F90:28-89).
 // Comparisons act on values, so a branch (limiter threshold, max/min, the
 // time-step minimum) passes the derivative of the branch taken.
 #pragma once

@@ -100,55 +100,6 @@ __device__ __forceinline__ void q_from_prim(double rho, double u1, double u2, do
     q_from_prim_t<double>(rho, u1, u2, pr, q);
 }
 
-// q_variables.F90:230-256 qtilde_to_primitive.  T is double on the FP64
-// path and float on the FP32-mixed path; the literals keep their values.
-template <class T>
-__device__ __forceinline__ void qtilde_to_primitive(const T qt[4], T gm1, T &u1, T &u2, T &rho,
-                                                    T &pr) {
-    T beta = -qt[3] * T(0.5);
-    T temp = T(0.5) / beta;
-    u1 = qt[1] * temp;
-    u2 = qt[2] * temp;
-    T temp1 = qt[0] + beta * (u1 * u1 + u2 * u2);
-    T temp2 = temp1 - (log(beta) / gm1);
-    rho = exp(temp2);
-    pr = rho * temp;
-}
-
-// limiters.F90:64-110 venkat_limiter, one component.
-template <class T>
-__device__ __forceinline__ T venkat_phi(T qtilde, T q, T qmax, T qmin, T eps2) {
-    T del_neg = qtilde - q;
-    if (fabs(del_neg) <= T(MFCFD_VENKAT_THR)) return T(1.0);
-    T del_pos = del_neg > T(0.0) ? qmax - q : qmin - q;
-    T num = (del_pos * del_pos) + eps2;
-    num = num * del_neg + T(2.0) * del_neg * del_neg * del_pos;
-    T den = del_pos * del_pos + T(2.0) * del_neg * del_neg;
-    den = den + del_neg * del_pos + eps2;
-    den = den * del_neg;
-    T temp = num / den;
-    return temp < T(1.0) ? temp : T(1.0);
-}
-
-// Limited reconstruction of one point towards one neighbour direction,
-// straight to primitive variables (the qtilde lines of *_fluxes.F90, e.g.
-// interior_fluxes.F90:158-172).  t = delx*dq(1,:) + dely*dq(2,:) is formed
-// once and used for both the unlimited and the limited qtilde, exactly as the
-// reference recomputes it.
-template <class T>
-__device__ __forceinline__ void reconstruct(const T q[4], const T dqx[4], const T dqy[4],
-                                            const T qmax[4], const T qmin[4], T eps2, T delx,
-                                            T dely, T gm1, T &u1, T &u2, T &rho, T &pr) {
-    T qt[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        T t = delx * dqx[r] + dely * dqy[r];
-        T phi = venkat_phi<T>(q[r] - T(0.5) * t, q[r], qmax[r], qmin[r], eps2);
-        qt[r] = q[r] - T(0.5) * phi * t;
-    }
-    qtilde_to_primitive<T>(qt, gm1, u1, u2, rho, pr);
-}
-
 // The per-state part shared by split_fluxes.F90 and quadrant_fluxes.F90: the
 // state in the point's (t, n) frame and the two Maxwellian half-moments.
 template <class T>
@@ -157,39 +108,17 @@ struct KStateT {
 };
 using KState = KStateT<double>;
 
+// erf(x) given exp(-x*x), the scalar statement of what the FP32 flux pass
+// evaluates on pairs (kstate2 of primal_fp32.cu): Abramowitz & Stegun 7.1.26
+// (after Hastings), erf(|x|) = 1 - t (a1 + t (a2 + t (a3 + t (a4 + t a5))))
+// exp(-x^2), t = 1 / (1 + p |x|), absolute error below 1.5e-7 (5.3e-7 evaluated in
+// FP32; tests/test_erf32.py reads the coefficients here, tests/test_erf32_pairs.py
+// holds kstate2's to them) -- the split fluxes use erf only in 1 +- erf, so the
+// absolute error is what counts -- reusing the exponential the Maxwellian moments
+// take anyway (1.024M points: FP32 flux pass 0.316 -> 0.304 ms; |dCl| against the
+// FP64 loop after 50 iterations 1.0e-7 with the library erff, 6e-9 with this).
 template <class T>
-__device__ __forceinline__ KStateT<T> kstate(T u1, T u2, T rho, T pr, T nx, T ny, T pi) {
-    KStateT<T> s;
-    T tx = ny, ty = -nx;
-    s.ut = u1 * tx + u2 * ty;
-    s.un = u1 * nx + u2 * ny;
-    T beta = T(0.5) * rho / pr;
-    T sb = sqrt(beta);
-    T S1 = s.ut * sb;
-    T S2 = s.un * sb;
-    T spb = sqrt(pi * beta);
-    s.B1 = T(0.5) * exp(-S1 * S1) / spb;
-    s.B2 = T(0.5) * exp(-S2 * S2) / spb;
-    s.e1 = erf(S1);
-    s.e2 = erf(S2);
-    s.pbr = pr / rho;
-    s.usq = s.ut * s.ut + s.un * s.un;
-    s.rho = rho;
-    return s;
-}
-
-// erf(x) given exp(-x*x).  FP64: the library erf.  FP32 (the flux pass
-// evaluates it on pairs, kstate2 of primal_fp32.cu): Abramowitz &
-// Stegun 7.1.26 (after Hastings), erf(|x|) = 1 - t (a1 + t (a2 + t (a3 + t
-// (a4 + t a5)))) exp(-x^2), t = 1 / (1 + p |x|), absolute error below
-// 1.5e-7 (5.3e-7 evaluated in FP32; tests/test_erf32.py) -- the split
-// fluxes use erf only in 1 +- erf, so the absolute error is what counts --
-// reusing the exponential the Maxwellian moments take anyway (C2: FP32 flux pass 0.316 -> 0.304 ms; |dCl| against the FP64
-// loop after 50 iterations 1.0e-7 with the library erff, 6e-9 with this).
-template <class T>
-__device__ __forceinline__ T erf_with_exp(T x, T) {
-    return erf(x);
-}
+__device__ T erf_with_exp(T x, T e);
 template <>
 __device__ __forceinline__ float erf_with_exp<float>(float x, float e) {
     const float ax = fabsf(x);
@@ -200,38 +129,6 @@ __device__ __forceinline__ float erf_with_exp<float>(float x, float e) {
     p = p * t - 0.284496736f;
     p = p * t + 0.254829592f;
     return copysignf(1.0f - (p * t) * e, x);
-}
-
-// split_fluxes.F90:8-96 flux_Gxp (s1 = +1) / flux_Gxn (s1 = -1)
-template <class T>
-__device__ __forceinline__ void flux_gx(const KStateT<T> &s, T s1, T G[4]) {
-    T A1 = T(0.5) * (T(1.0) + s1 * s.e1);
-    G[0] = s.rho * (s.ut * A1 + s1 * s.B1);
-    T temp1 = s.pbr + s.ut * s.ut;
-    T temp2 = temp1 * A1 + s1 * (s.ut * s.B1);
-    G[1] = s.rho * temp2;
-    temp1 = s.ut * s.un * A1 + s1 * (s.un * s.B1);
-    G[2] = s.rho * temp1;
-    temp1 = (T(7.0) * s.pbr) + s.usq;
-    temp2 = T(0.5) * s.ut * temp1 * A1;
-    temp1 = (T(6.0) * s.pbr) + s.usq;
-    G[3] = s.rho * (temp2 + s1 * (T(0.5) * temp1 * s.B1));
-}
-
-// split_fluxes.F90:99-190 flux_Gyp (s2 = +1) / flux_Gyn (s2 = -1)
-template <class T>
-__device__ __forceinline__ void flux_gy(const KStateT<T> &s, T s2, T G[4]) {
-    T A2 = T(0.5) * (T(1.0) + s2 * s.e2);
-    G[0] = s.rho * (s.un * A2 + s2 * s.B2);
-    T temp1 = s.pbr + s.un * s.un;
-    T temp2 = temp1 * A2 + s2 * (s.un * s.B2);
-    G[2] = s.rho * temp2;
-    temp1 = s.ut * s.un * A2 + s2 * (s.ut * s.B2);
-    G[1] = s.rho * temp1;
-    temp1 = (T(7.0) * s.pbr) + s.usq;
-    temp2 = T(0.5) * s.un * temp1 * A2;
-    temp1 = (T(6.0) * s.pbr) + s.usq;
-    G[3] = s.rho * (temp2 + s2 * (T(0.5) * temp1 * s.B2));
 }
 
 // quadrant_fluxes.F90:12-248: GxI (s1=-1,s2=-1), GxII (+1,-1), GxIII (+1,+1),
