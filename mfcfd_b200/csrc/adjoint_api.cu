@@ -205,7 +205,8 @@ int adj_setup(mfcfd_t *h) {
     CK(dmalloc(&a->nxb, n));
     CK(dmalloc(&a->nyb, n));
     CK(dmalloc(&a->contrib, (size_t)n * kp * ADJ_CW));
-    if (dmalloc(&a->tks, (size_t)rks * n * kp * KS_TAPE) != cudaSuccess) {
+    if (h->state_tape &&
+        dmalloc(&a->tks, (size_t)rks * n * kp * KS_TAPE) != cudaSuccess) {
         a->tks = nullptr;
         cudaGetLastError();  // an allocation failure is not sticky; clear it
     }

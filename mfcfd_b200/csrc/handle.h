@@ -14,8 +14,8 @@
 
 using namespace lskum;
 
-struct AdjointState;
-struct TanWork;  // adjoint buffers (adjoint_api.cu), created on first use
+struct AdjointState;  // adjoint buffers (adjoint_api.cu), created on first use
+struct TanWork;       // mfcfd_tangent's workspace (tangent_fp64.cu)
 
 struct mfcfd {
     int dev = 0;
@@ -82,6 +82,7 @@ struct mfcfd {
     std::string err;
     std::vector<double> shape_cp;
     AdjointState *adj = nullptr;
+    bool state_tape = true;     // false (tests only): the adjoint does without its state tape
     TanWork *tan = nullptr;     // mfcfd_tangent's device workspace
     int *d_perm = nullptr;      // perm on the device
     // device address of the fixed residue-history array of mfcfd_run_noalloc
