@@ -130,14 +130,19 @@ def test_adjoint_without_state_tape(gpu, probe, ni, nj, inner, tscheme, jitter, 
     g = naca_ogrid(ni, nj, seed=15, first_spacing=5e-3, jitter=jitter)
     if wide:
         g = _widen(g, 3)
-    grads = []
+    import torch
+    grads, used = [], []
     for tape in (True, False):
         with Solver(g, cfl=0.2, vl_const=5.0, mach=0.7, aoa=2.0, inner_iterations=inner,
                     tscheme=tscheme) as s:
             if not tape:
                 probe.probe_no_state_tape(s.h)
             s.run(2)
+            free = torch.cuda.mem_get_info(0)[0]
             grads.append(s.adjoint(2, "cd"))
+            used.append(free - torch.cuda.mem_get_info(0)[0])
+    if g.n > 20000:  # (128 bytes a slot and stage; the driver allocates in 2 MB pages)
+        assert used[0] - used[1] > 128 * int(g.nbhs.max()) * g.n - (4 << 20)
     (J0, x0, y0, n0), (J1, x1, y1, n1) = grads
     assert J0 == J1 and n0 == n1
     for a, b in ((x0, x1), (y0, y1)):
