@@ -1141,8 +1141,8 @@ int wave(int kind, int block, size_t smem, int grid) {
 }
 }  // namespace
 
-// the flux pass's shared memory is static (independent of the stencil size)
-size_t flux_smem_bytes(int) { return 0; }
+// the flux pass's shared memory does not depend on the stencil size
+size_t flux_smem_bytes(int) { return FLUX_SMEM; }
 
 int batch_occupancy(int kind, bool fp32, int block, size_t smem) {
     if (fp32) return batch_occupancy32(kind, block, smem);
@@ -1156,8 +1156,7 @@ int batch_occupancy(int kind, bool fp32, int block, size_t smem) {
     else if (kind == 1)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_inner_h<HALO_CAP>, HALO_BLOCK,
                                                           halo_smem_bytes(1, HALO_CAP + 1));
-    else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_flux<false>, block,
-                                                          FLUX_SMEM);
+    else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_flux<false>, block, smem);
     return e == cudaSuccess ? nb : 1;
 }
 
@@ -1208,7 +1207,7 @@ void launch_inner(const Geom &g, const Consts &c, const Sched &s, const double *
 void launch_flux(const Geom &g, const Consts &c, const Sched &s, const StageBufs &b, int rk,
                  bool last, int grid, int tiles, cudaStream_t st) {
     const FluxShape f = flux_shape(tiles, FLUX_MIN_BLOCKS);
-    const int gr = wave(2, FLUX_BLOCK, 0, grid);
+    const int gr = wave(2, FLUX_BLOCK, FLUX_SMEM, grid);
     constexpr int sm = FLUX_SMEM;
     if (b.kstape)
         kb_flux<true><<<gr, FLUX_BLOCK, sm, st>>>(g, c, s, b, rk, last ? 1 : 0, f.ct, f.coop);
