@@ -398,12 +398,14 @@ __device__ __forceinline__ F2 f2(float x, float y) {
 }
 __device__ __forceinline__ F2 f2(float x) { return f2(x, x); }
 __device__ __forceinline__ float lo(F2 a) {
-    float x, y;
+    float x;
+    [[maybe_unused]] float y;
     asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
     return x;
 }
 __device__ __forceinline__ float hi(F2 a) {
-    float x, y;
+    float y;
+    [[maybe_unused]] float x;
     asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
     return y;
 }

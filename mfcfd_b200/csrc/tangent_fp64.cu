@@ -545,7 +545,7 @@ constexpr int TF = 512;
 __global__ void __launch_bounds__(TF)
 k_t_forces(Geom g, TanState s, TanShape t, int cur, double mach, double cos_t, double sin_t,
            int objective, double *out) {
-    __shared__ Dual th[TF], tv[TF];
+    __shared__ double2 th[TF], tv[TF];  // value, derivative
     __shared__ int ts[TF];
     const double pr_inf = 1.0 / 1.4;
     const Dual temp(0.5 * 1.0 * mach * mach);
@@ -566,16 +566,17 @@ k_t_forces(Geom g, TanState s, TanShape t, int cur, double mach, double cos_t, d
                 const Dual nx(g.nrm[m].x, s.nrm_t[m].x), ny(g.nrm[m].y, s.nrm_t[m].y);
                 Dual cp = Dual(s.pv[cur][m].d, s.pt[cur][m].d) - Dual(pr_inf);
                 cp = -cp / temp;
-                th[threadIdx.x] = cp * nx * ds;
-                tv[threadIdx.x] = cp * ny * ds;
+                const Dual h = cp * nx * ds, v = cp * ny * ds;
+                th[threadIdx.x] = make_double2(h.v, h.d);
+                tv[threadIdx.x] = make_double2(v.v, v.d);
                 ts[threadIdx.x] = t.shape[j];
             }
             __syncthreads();
             if (threadIdx.x == 0)
                 for (int q = 0; q < min(TF, t.npts - j0); ++q)
                     if (ts[q] == sh) {
-                        H += th[q];
-                        V += tv[q];
+                        H += Dual(th[q].x, th[q].y);
+                        V += Dual(tv[q].x, tv[q].y);
                     }
             __syncthreads();
         }
