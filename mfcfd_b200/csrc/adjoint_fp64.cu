@@ -43,14 +43,6 @@ __device__ __forceinline__ void ld8a(const double *p, double a[4], double b[4]) 
     b[0] = t2.x; b[1] = t2.y; b[2] = t3.x; b[3] = t3.y;
 }
 
-// Four doubles in one 256-bit read-only load (ld.global.nc.v4.f64, sm_100);
-// p is 32-byte aligned and not written by the kernel that reads it.
-__device__ __forceinline__ void ld4nc(const double *p, double v[4]) {
-    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-        : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
-        : "l"(p));
-}
-
 // Sum of v over W neighbouring lanes (whole warps).
 template <int W>
 __device__ __forceinline__ double lane_sum(double v) {

@@ -27,6 +27,18 @@ __device__ __forceinline__ R4 ld4(const R4 *p) {
     double2 u = __ldg(q), v = __ldg(q + 1);
     return R4{u.x, u.y, v.x, v.y};
 }
+// Four doubles in one 256-bit read-only load (ld.global.nc.v4.f64, sm_100);
+// p is 32-byte aligned and not written by the kernel that reads it.
+__device__ __forceinline__ void ld4nc(const double *p, double v[4]) {
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+        : "l"(p));
+}
+__device__ __forceinline__ R4 ld4w(const R4 *p) {
+    double v[4];
+    ld4nc(reinterpret_cast<const double *>(p), v);
+    return R4{v[0], v[1], v[2], v[3]};
+}
 __device__ __forceinline__ void st4(R4 *p, double a, double b, double c, double d) {
     double2 *q = reinterpret_cast<double2 *>(p);
     q[0] = make_double2(a, b);

@@ -38,19 +38,7 @@ constexpr int FLUX_MIN_BLOCKS = 4;
 constexpr double OBT = 1.0 / 3.0;        // state_update.F90:19-20
 constexpr double TBT = 2.0 / 3.0;
 
-// Rows in 256-bit read-only loads (ld.global.nc.v4.f64, sm_100): a 32-byte
-// q row in one load, a 64-byte dq row in two (the D and I passes' rows of
-// tiles without a staged halo, the I pass's dq0 row).  R4 rows and dq rows
-// are 32-byte aligned.  The flux pass uses them for its 64-byte dq and qm
-// rows only: its 32-byte q rows in the wide form made it spill.
-__device__ __forceinline__ R4 ld4w(const R4 *p) {
-    R4 r;
-    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-        : "=d"(r.a), "=d"(r.b), "=d"(r.c), "=d"(r.d)
-        : "l"(p));
-    return r;
-}
-
+// A 64-byte row (dq, qm; 32-byte aligned) in two 256-bit loads.
 __device__ __forceinline__ void ld8w(const double *p, double a[4], double b[4]) {
     const R4 u = ld4w(reinterpret_cast<const R4 *>(p));
     const R4 v = ld4w(reinterpret_cast<const R4 *>(p + 4));

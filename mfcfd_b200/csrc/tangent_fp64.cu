@@ -65,13 +65,6 @@ __device__ __forceinline__ void st_dual4(R4 *v, R4 *t, int i, const Dual x[4]) {
     v[i] = R4{x[0].v, x[1].v, x[2].v, x[3].v};
     t[i] = R4{x[0].d, x[1].d, x[2].d, x[3].d};
 }
-// four doubles in one 256-bit read-only load; p is 32-byte aligned and not written
-// by the kernel that reads it
-__device__ __forceinline__ void ld4nc(const double *p, double v[4]) {
-    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-        : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
-        : "l"(p));
-}
 __device__ __forceinline__ void xy_dual(const Geom &g, const TanState &s, int i, Dual &x,
                                         Dual &y) {
     const double2 p = g.xy[i], d = s.xy_t[i];
