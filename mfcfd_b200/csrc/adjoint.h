@@ -58,7 +58,7 @@ void launch_update_b(const Geom &g, const Consts &c, const AdjConsts &a, const R
 // kinetic states and own reconstruction; writes nbrec [n][kp][NBREC]) and
 // k_flux_b_nbr per neighbour over the transposed stencil (the neighbour's
 // reconstruction; writes back [n][kp] (delx, dely) adjoint parts that
-// belong to the point as well), then k_back_sum adds those to the point.
+// belong to the point as well; k_grad_b adds those to the point).
 // nbrec and back share one buffer of n*kp*(NBREC+2) doubles.  dqb and rec
 // receive dq's adjoint (with inner iterations; otherwise the record holds all
 // that is needed of it) and the records of the solve that made dq.

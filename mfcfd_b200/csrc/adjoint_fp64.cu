@@ -72,7 +72,7 @@ __device__ __forceinline__ KState kst_taped(const double *v, double nx, double n
     s.usq = fma(v[6], v[6], v[7] * v[7]);
     return s;
 }
-// state_update_b (state_update.F90:10-141, reverse)
+
 // Stores n (even) doubles as 16-byte pairs; dst is 16-byte aligned (records
 // are an even number of doubles from an aligned base).
 __device__ __forceinline__ void st_pairs(double *dst, const double *v, int n) {
@@ -93,6 +93,7 @@ __device__ __forceinline__ void add_pairs(double *dst, const double *v, int n) {
     }
 }
 
+// state_update_b (state_update.F90:10-141, reverse)
 __global__ void __launch_bounds__(BLK, 3)
 k_update_b(Geom g, Consts c, AdjConsts a, const R4 *__restrict__ prim_in,
            const R4 *__restrict__ prim_old, const R4 *__restrict__ fr,
@@ -756,9 +757,10 @@ k_inner_b(Geom g, const double *__restrict__ dq_in, LsqIn in, int first,
 // neighbours (the solve's adjoint z comes in the record), the neighbours that
 // gave qmax, qmin and the time step -- left packed in the record's last field,
 // 5 bits each and 0 for none, for k_grad_b_nbr -- and the parts of delx/dely's
-// adjoint that k_flux_b_nbr left in back.  33 us at 256,000 points, 45 with the
-// time step (7 blocks an SM; 83 and 55 at 6, 38 and 56 at 8); 66 and a pass of
-// 12 for back when it summed the solve again and wrote a record of 24 doubles.
+// adjoint that k_flux_b_nbr left in back.  256,000 points, without / with the time
+// step: 33 / 45 us at 7 blocks an SM, 81 / 54 at 6 (measured twice: without the step
+// the compiler's code at that bound is the slower), 38 / 55 at 8; 66 and a pass of 12
+// for back when it summed the solve again and wrote a record of 24 doubles.
 template <bool with_delta>
 __global__ void __launch_bounds__(BLK, 7)
 k_grad_b(Geom g, Consts c, const R4 *__restrict__ q, const double *__restrict__ spdA,

@@ -164,7 +164,7 @@ int batch_wave(const mfcfd_batch_t *b, int kind, int block) {
 // Launch shape from (block, waves) or (block, points per thread): waves > 0
 // sizes every pass to that many waves of resident blocks; otherwise ppt
 // (1, 2, 4) gives each thread of the point passes ppt points and each warp
-// of the flux pass ppt chunks of two tiles (ppt 1: every point its thread).
+// of the flux pass ppt chunks (flux_shape; ppt 1: every point its thread).
 void set_shape(mfcfd_batch_t *b, int block, int waves, int ppt = 1) {
     b->point_block = block;
     const int fmax = flux_grid_blocks(b->ntiles * TILE, b->fp32);

@@ -227,7 +227,8 @@ void launch_init_state32(const Geom &g, const float4 *prim, float4 *q, double *s
 // float4 prim -> FP64 rows (for the force sums and diagnostics)
 void launch_widen(const float4 *in, R4 *out, int n, cudaStream_t s);
 
-// Shape-point force sums (compute_cl_cd_cm), serial in grid order.
+// Shape-point force sums (compute_cl_cd_cm) of one block, in a fixed order that does
+// not depend on the launch.
 struct ShapeTab {
     int npts, shapes;
     const int *idx;        // renumbered point

@@ -160,7 +160,9 @@ struct HaloRows32 {
     __device__ __forceinline__ double spdv(int l) const { return sm[OSPD * hc + l].x; }
 };
 
-// grad32_point's sums over the rows of R (the same arithmetic)
+// q_variables.F90:41-112 eval_q_derivatives and state_update.F90:190-236
+// func_delta over the rows of R, in slot order, with FP32 sums (the FP64 pass's
+// grad_sums)
 template <class Rows>
 __device__ __forceinline__ void grad32_sums(const Consts &c, const Geom32 &f, int n, Rows R,
                                             int nb, int with_delta, int i, float dx[4],

@@ -15,8 +15,8 @@
 //
 // Layout in HBM (renumbered points: wall | outer | interior): one 32-byte
 // row per point for prim and q, 64-byte rows for dq and qm, 16-byte rows for
-// (x, y) and (nx, ny); stencils as ELL columns conn[slot][point] so the
-// thread-per-point passes read them coalesced.
+// (x, y) and (nx, ny); stencils as ELL columns conn[slot][point] so that lanes of
+// neighbouring points read them coalesced.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -722,7 +722,7 @@ update_point(const Geom &g, const Consts &c, const StageBufs &b, int rk, int las
     const double nx = nn.x, ny = nn.y;
     double res_sqr = 0.0;
     {
-                const double delta = b.delta[i];
+        const double delta = b.delta[i];
         const R4 P = ld4(b.prim_in + i), O = rk == 3 ? ld4(b.prim_old + i) : R4{0, 0, 0, 0};
         double fr[4];
 #pragma unroll

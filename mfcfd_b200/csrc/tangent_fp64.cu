@@ -10,10 +10,10 @@
 // that direction.  For the reverse-mode gradient g of mfcfd_adjoint,
 // dJ/de = <g, (dx, dy)> (the dot-product test).
 //
-// The D and I passes and the state update are thread-per-point passes over the
-// primal's device templates (q_from_prim, prim_to_conserved, conserved_ubar)
-// instantiated on Dual; the flux pass has the primal's split of the work and
-// forms (flux_math.cuh), differentiated.  min_dist is data, as in the
+// The D, I and flux passes have the primal's split of the work (eight lanes a
+// point, a slot a lane) and its forms (flux_math.cuh), differentiated; the state
+// update is a thread-per-point pass over the primal's device templates
+// (q_from_prim, prim_to_conserved, conserved_ubar) instantiated on Dual.  min_dist is data, as in the
 // reference.
 #include <cuda_runtime.h>
 
